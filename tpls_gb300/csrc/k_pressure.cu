@@ -32,6 +32,8 @@
 
 #include <vector>
 
+#include "tpls_mg.cuh"
+#include "tpls_pair.cuh"
 #include "tpls_pressure.h"
 
 namespace tpls {
@@ -47,6 +49,7 @@ struct PLevel {
   double cx, cy, cz;
   void *b = nullptr, *e = nullptr, *e2 = nullptr, *r = nullptr, *t = nullptr;
   void *thomas = nullptr;  // [3 classes][nz][2] = (cprime, inv_den)
+  int halved = 0;  // red-black level whose three axes are coarsened below it: the k_mg_* kernels
   int point = 0;  // near-isotropic level: red-black Gauss-Seidel instead of z-lines
   double invd[3][3];  // point smoother: 1/diagonal by x class (first, interior, last) and z class
 };
@@ -54,9 +57,11 @@ struct PLevel {
 struct PoissonSolver {
   int nx, ny, nz, N;
   std::vector<PLevel> lv;
-  double *cinv = nullptr;  // coarsest pseudo-inverse (nc x nc), or null
+  double *cinv = nullptr;  // coarsest pseudo-inverse (nc x nc; FP32 levels: transposed), or null
   int coarse_sweeps = 0;
-  double *x = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr, *bvec = nullptr;
+  double *x = nullptr, *r = nullptr, *p = nullptr, *q = nullptr, *bvec = nullptr;
+  void *z = nullptr;           // preconditioned residual, in the level type
+  float *r32 = nullptr;        // FP32 levels: r rounded once, for the V-cycle
   double *bin = nullptr;     // inlet ghost-row data (ny*nz)
   double *part = nullptr;    // reduction partials (3 * rblk)
   unsigned *counter = nullptr;  // last-block ticket of the reductions
@@ -215,8 +220,8 @@ __global__ void __launch_bounds__(PB)
 // b -= mean(b); r = b - A x; ||b||^2, ||r||^2
 __global__ void __launch_bounds__(PB)
     k_init_r(int nx, int ny, int nz, double cx, double cy, double cz, double invN, double rtol, CgCtl ctl,
-             double *s, double *__restrict__ b, const double *__restrict__ x, double *__restrict__ r, double *part,
-             unsigned *counter) {
+             double *s, double *__restrict__ b, const double *__restrict__ x, double *__restrict__ r,
+             float *__restrict__ r32, double *part, unsigned *counter) {
   const double mb = s[S_SUMB] * invN;
   double v[2] = {0.0, 0.0};
   ROW_LOOP(nx, ny, nz) {
@@ -225,6 +230,7 @@ __global__ void __launch_bounds__(PB)
     b[c] = bb;
     const double rr = bb - applyA<double, double>(x, i, j, k, nx, ny, nz, cx, cy, cz);
     r[c] = rr;
+    if (r32) r32[c] = float_bits(rr);
     v[0] += bb * bb;
     v[1] += rr * rr;
   }
@@ -237,13 +243,36 @@ __global__ void __launch_bounds__(PB)
   }
 }
 
-// sum z, sum r, r.z -> mean(z), rz_new = r.(z - mean z), beta = rz_new/rz
+// FP64 levels: the mean of z is not removed.  A maps a constant to zero and r
+// has zero sum, so neither r.z nor the iterates' differences see it, and the
+// write-back sets the solution's mean; it cost three FP64 operations per
+// point and iteration of the 16 outside the V-cycle.  (An FP32 level's z
+// answers a last-bit change of r by FP32 roundings, which later steps of the
+// FP32-mixed form amplify to its own accuracy of 1e-7: its CG keeps the
+// order of every sum.)
+__device__ __forceinline__ void cg_beta(double *s, double rz) {
+  s[S_BETA] = (s[S_IT] == 0.0) ? 0.0 : rz / s[S_RZ];
+  s[S_RZ] = rz;
+}
+
+// r.z -> beta (levels whose last smoothing sweep does not form it)
 __global__ void __launch_bounds__(PB)
-    k_zdot(int N, double invN, const double *__restrict__ r, const double *__restrict__ z, double *part,
+    k_rdot(int N, const double *__restrict__ r, const double *__restrict__ z, double *part, unsigned *counter,
+           double *s) {
+  double v[1] = {0.0};
+  GRID_STRIDE(c, N) v[0] = fma(r[c], z[c], v[0]);
+  double tot[1];
+  if (reduce_last<1>(v, part, counter, tot) && threadIdx.x == 0) cg_beta(s, tot[0]);
+}
+
+// FP32 levels: sum z, sum r, r.z -> mean(z), rz_new = r.(z - mean z),
+// beta = rz_new/rz
+__global__ void __launch_bounds__(PB)
+    k_zdot(int N, double invN, const double *__restrict__ r, const float *__restrict__ z, double *part,
            unsigned *counter, double *s) {
   double v[3] = {0.0, 0.0, 0.0};
   GRID_STRIDE(c, N) {
-    const double zz = z[c], rr = r[c];
+    const double zz = widen_bits(z[c]), rr = r[c];
     v[0] += zz;
     v[1] += rr;
     v[2] += rr * zz;
@@ -251,19 +280,77 @@ __global__ void __launch_bounds__(PB)
   double tot[3];
   if (reduce_last<3>(v, part, counter, tot) && threadIdx.x == 0) {
     const double zm = tot[0] * invN;
-    const double rzn = tot[2] - zm * tot[1];
-    s[S_BETA] = (s[S_IT] == 0.0) ? 0.0 : rzn / s[S_RZ];
     s[S_ZMEAN] = zm;
-    s[S_RZ] = rzn;
+    cg_beta(s, tot[2] - zm * tot[1]);
   }
 }
 
-// p = (z - mean z) + beta p
+// The last red half-sweep of the finest level and r.z of its result (b is r).
 __global__ void __launch_bounds__(PB)
-    k_pupdate(int N, const double *__restrict__ s, const double *__restrict__ z, double *__restrict__ p) {
-  const double zm = s[S_ZMEAN], beta = s[S_BETA];
+    k_mg_half_dot(const __grid_constant__ MgLev<double> L, const double *__restrict__ b, double *e, int kz,
+                  double *part, unsigned *counter, double *s) {
+  const MgBlk B = mg_block(L, kz);
+  double v[1] = {0.0};
+  if (B.in) {
+    const int nx = L.nx, plane = nx * L.ny;
+    const int jm = (B.j > 0) ? -nx : plane - nx, jp = (B.j < L.ny - 1) ? nx : nx - plane;
+    int c = 2 * B.i2 + nx * B.j + plane * B.k0;
+    const double2 zero = {0.0, 0.0};
+    double2 pm = (B.k0 > 0) ? *reinterpret_cast<const double2 *>(e + c - plane) : zero;
+    double2 p0 = *reinterpret_cast<const double2 *>(e + c);
+    for (int k = B.k0; k < B.k1; k++, c += plane) {
+      const double2 pp = (k < L.nz - 1) ? *reinterpret_cast<const double2 *>(e + c + plane) : zero;
+      const double2 bb = *reinterpret_cast<const double2 *>(b + c);
+      const int odd = (B.j + k) & 1;
+      const double z = mg_relax(L, B, e, odd ? bb.y : bb.x, odd, c, jm, jp, k, pm, p0, pp);
+      e[c + odd] = z;
+      v[0] = fma(odd ? bb.y : bb.x, z, fma(odd ? bb.x : bb.y, odd ? p0.x : p0.y, v[0]));
+      pm = p0;
+      p0 = pp;
+    }
+  }
+  double tot[1];
+  if (reduce_last<1>(v, part, counter, tot) && threadIdx.x == 0) cg_beta(s, tot[0]);
+}
+
+// k_mg_up of the finest level (FP64, b is r), with r.z of its result.
+template <int CX, int CY, int CZ>
+__global__ void __launch_bounds__(PB)
+    k_mg_up_dot(const __grid_constant__ MgLev<double> L, const double *__restrict__ b, const double *__restrict__ ec,
+                double *__restrict__ e, double *part, unsigned *counter, double *s) {
+  using T = MgTile<CX, CY, CZ>;
+  __shared__ double se[T::EN];
+  __shared__ double ss[T::SN];
+  const int gx = (L.nx / 2 + CX - 1) / CX, gy = (L.ny / 2 + CY - 1) / CY;
+  const int x0 = (blockIdx.x % gx) * T::FX, y0 = (blockIdx.x / gx % gy) * T::FY, z0 = blockIdx.x / (gx * gy) * T::FZ;
+  mg_up_tile<double, CX, CY, CZ>(L, b, ec, se, ss, x0, y0, z0);
+  double v[1] = {0.0};
+  for (int q = threadIdx.x; q < T::FX * T::FY * T::FZ; q += PB) {
+    const int lx = q % T::FX, ly = q / T::FX % T::FY, lz = q / (T::FX * T::FY);
+    if (x0 + lx < L.nx && y0 + ly < L.ny && z0 + lz < L.nz) {
+      const size_t c = x0 + lx + L.nx * (y0 + ly + (size_t)L.ny * (z0 + lz));
+      const double z = se[lx + 2 + T::EX * (ly + 2 + T::EY * (lz + 2))];
+      e[c] = z;
+      v[0] = fma(b[c], z, v[0]);
+    }
+  }
+  double tot[1];
+  if (reduce_last<1>(v, part, counter, tot) && threadIdx.x == 0) cg_beta(s, tot[0]);
+}
+
+// p = z + beta p, z without its mean on FP32 levels (the first iteration's
+// beta is 0 and p not read)
+template <typename R>
+__global__ void __launch_bounds__(PB)
+    k_pupdate(int N, const double *__restrict__ s, const R *__restrict__ z, double *__restrict__ p) {
+  const double beta = s[S_BETA];
+  const bool first = (__double_as_longlong(beta) == 0);
   const int c = blockIdx.x * PB + threadIdx.x;
-  if (c < N) p[c] = (z[c] - zm) + beta * p[c];
+  if (c >= N) return;
+  double zz;
+  if constexpr (sizeof(R) == sizeof(float)) zz = widen_bits(z[c]) - s[S_ZMEAN];
+  else zz = z[c];
+  p[c] = first ? zz : fma(beta, p[c], zz);
 }
 
 // q = A p; p.q -> alpha = rz / p.q
@@ -284,13 +371,15 @@ __global__ void __launch_bounds__(PB)
 // x += alpha p; r -= alpha q; ||r||^2
 __global__ void __launch_bounds__(PB)
     k_axpy(int N, CgCtl ctl, double *s, const double *__restrict__ p, const double *__restrict__ q,
-           double *__restrict__ x, double *__restrict__ r, double *part, unsigned *counter) {
+           double *__restrict__ x, double *__restrict__ r, float *__restrict__ r32, double *part,
+           unsigned *counter) {
   const double alpha = s[S_ALPHA];
   double v[1] = {0.0};
   GRID_STRIDE(c, N) {
     x[c] += alpha * p[c];
     const double rr = r[c] - alpha * q[c];
     r[c] = rr;
+    if (r32) r32[c] = float_bits(rr);
     v[0] += rr * rr;
   }
   double tot[1];
@@ -330,11 +419,10 @@ __global__ void k_writeback(Geo g, double dy, double invN, const double *__restr
 }
 
 // ---------------------------------------------------------------------------
-// multigrid kernels.  R is the arithmetic type of the level (double, or
-// float for the FP32 preconditioner); TB, TE, TO the storage types of the
-// right-hand side, the input iterate and the output (the finest level of
-// the FP32 preconditioner reads the FP64 CG residual and writes the FP64
-// preconditioned vector directly).
+// multigrid kernels of the levels k_mg_* (tpls_mg.cuh) do not cover: axes
+// that do not halve, anisotropic couplings, odd y extents.  R is the type of
+// the level (double, or float for the FP32 preconditioner, whose finest
+// right-hand side is the CG residual rounded once per iteration).
 template <typename R>
 struct LevArgs {
   int nx, ny, nz;
@@ -345,10 +433,10 @@ struct LevArgs {
 // zero_init: ei == 0.
 constexpr int LJB = 64;  // threads per block of the line smoother (one column each)
 
-template <typename R, typename TB, typename TE, typename TO>
+template <typename R>
 __global__ void __launch_bounds__(LJB)
     k_line_jacobi(LevArgs<R> L, R omega, R one_m_omega, int zero_init, const R *__restrict__ thomas,
-                  const TB *__restrict__ b, const TE *__restrict__ ei, R *__restrict__ t, TO *__restrict__ eo) {
+                  const R *__restrict__ b, const R *__restrict__ ei, R *__restrict__ t, R *__restrict__ eo) {
   const int col = blockIdx.x * LJB + threadIdx.x;
   const int nx = L.nx, ny = L.ny, nz = L.nz;
   if (col >= nx * ny) return;
@@ -360,11 +448,11 @@ __global__ void __launch_bounds__(LJB)
   R y = (R)0;
   for (int k = 0; k < nz; k++) {
     const int c = col + plane * k;
-    R rhs = (R)b[c];
+    R rhs = b[c];
     if (!zero_init) {
-      R nb = L.cy * ((R)ei[c + jm] + (R)ei[c + jp]);
-      if (i > 0) nb += L.cx * (R)ei[c - 1];
-      if (i < nx - 1) nb += L.cx * (R)ei[c + 1];
+      R nb = L.cy * (ei[c + jm] + ei[c + jp]);
+      if (i > 0) nb += L.cx * ei[c - 1];
+      if (i < nx - 1) nb += L.cx * ei[c + 1];
       rhs += nb;
     }
     y = (rhs + L.cz * y) * th[2 * k + 1];
@@ -374,7 +462,7 @@ __global__ void __launch_bounds__(LJB)
   for (int k = nz - 1; k >= 0; k--) {
     const int c = col + plane * k;
     xn = t[c] - ((k < nz - 1) ? th[2 * k] * xn : (R)0);
-    eo[c] = (TO)(zero_init ? omega * xn : one_m_omega * (R)ei[c] + omega * xn);
+    eo[c] = zero_init ? omega * xn : one_m_omega * ei[c] + omega * xn;
   }
 }
 
@@ -384,10 +472,10 @@ __global__ void __launch_bounds__(LJB)
 // the damped result.  Dynamic shared memory: nz * 32 values of R.
 constexpr int LJ2_T = 256;
 
-template <typename R, typename TB, typename TE, typename TO>
+template <typename R>
 __global__ void __launch_bounds__(LJ2_T)
     k_line_jacobi2(LevArgs<R> L, R omega, R one_m_omega, int zero_init, const R *__restrict__ thomas,
-                   const TB *__restrict__ b, const TE *__restrict__ ei, TO *__restrict__ eo) {
+                   const R *__restrict__ b, const R *__restrict__ ei, R *__restrict__ eo) {
   extern __shared__ __align__(16) unsigned char lj2_raw[];
   R *buf = reinterpret_cast<R *>(lj2_raw);  // [nz][32]
   const int nx = L.nx, ny = L.ny, nz = L.nz, ncol = nx * ny, plane = nx * ny;
@@ -401,11 +489,11 @@ __global__ void __launch_bounds__(LJ2_T)
     R rhs = (R)0;
     if (mycol < ncol) {
       const int c = mycol + plane * k;
-      rhs = (R)b[c];
+      rhs = b[c];
       if (!zero_init) {
-        R nb = L.cy * ((R)ei[c + jm] + (R)ei[c + jp]);
-        if (ci > 0) nb += L.cx * (R)ei[c - 1];
-        if (ci < nx - 1) nb += L.cx * (R)ei[c + 1];
+        R nb = L.cy * (ei[c + jm] + ei[c + jp]);
+        if (ci > 0) nb += L.cx * ei[c - 1];
+        if (ci < nx - 1) nb += L.cx * ei[c + 1];
         rhs += nb;
       }
     }
@@ -435,7 +523,7 @@ __global__ void __launch_bounds__(LJ2_T)
     const int k = t >> 5, col = col0 + (t & 31);
     if (col < ncol) {
       const int c = col + plane * k;
-      eo[c] = (TO)(zero_init ? omega * buf[t] : one_m_omega * (R)ei[c] + omega * buf[t]);
+      eo[c] = zero_init ? omega * buf[t] : one_m_omega * ei[c] + omega * buf[t];
     }
   }
 }
@@ -458,9 +546,9 @@ struct InvD {
   R v[3][3];
 };
 
-template <typename R, typename TB, typename TE, typename TO>
-__global__ void k_rbgs(LevArgs<R> L, InvD<R> inv, int colour, int zero_init, int copy, const TB *__restrict__ b,
-                       const TE *ein, TO *eout) {
+template <typename R>
+__global__ void k_rbgs(LevArgs<R> L, InvD<R> inv, int colour, int zero_init, int copy, const R *__restrict__ b,
+                       const R *ein, R *eout) {
   const int nx = L.nx, ny = L.ny, nz = L.nz;
   const int i2 = blockIdx.x * MG_BX + threadIdx.x, j = blockIdx.y * MG_BY + threadIdx.y, k = blockIdx.z;
   if (2 * i2 >= nx || j >= ny) return;
@@ -472,32 +560,32 @@ __global__ void k_rbgs(LevArgs<R> L, InvD<R> inv, int colour, int zero_init, int
     if (i >= nx) break;
     const int c = i + nx * j + plane * k;
     if (((i + j + k) & 1) == colour) {
-      R acc = (R)b[c];
+      R acc = b[c];
       if (!zero_init) {
         R sx = (R)0, sz = (R)0;
-        if (i > 0) sx += (R)ein[c - 1];
-        if (i < nx - 1) sx += (R)ein[c + 1];
-        if (k > 0) sz += (R)ein[c - plane];
-        if (k < nz - 1) sz += (R)ein[c + plane];
+        if (i > 0) sx += ein[c - 1];
+        if (i < nx - 1) sx += ein[c + 1];
+        if (k > 0) sz += ein[c - plane];
+        if (k < nz - 1) sz += ein[c + plane];
         acc = fma(L.cx, sx, acc);
-        acc = fma(L.cy, (R)ein[c + jm] + (R)ein[c + jp], acc);
+        acc = fma(L.cy, ein[c + jm] + ein[c + jp], acc);
         acc = fma(L.cz, sz, acc);
       }
       const int xc = (nx == 1) ? 1 : ((i == 0) ? 0 : ((i == nx - 1) ? 2 : 1));
-      eout[c] = (TO)(acc * inv.v[xc][zc]);
+      eout[c] = acc * inv.v[xc][zc];
     } else if (copy) {
-      eout[c] = (TO)ein[c];
+      eout[c] = ein[c];
     }
   }
 }
 
-template <typename R, typename TB, typename TE>
-__global__ void k_residual(LevArgs<R> L, const TB *__restrict__ b, const TE *__restrict__ e, R *__restrict__ r) {
+template <typename R>
+__global__ void k_residual(LevArgs<R> L, const R *__restrict__ b, const R *__restrict__ e, R *__restrict__ r) {
   const int nx = L.nx, ny = L.ny, nz = L.nz;
   const int i = blockIdx.x * MG_BX + threadIdx.x, j = blockIdx.y * MG_BY + threadIdx.y, k = blockIdx.z;
   if (i >= nx || j >= ny) return;
   const int c = i + nx * (j + ny * k);
-  r[c] = (R)b[c] - applyA<R, TE>(e, i, j, k, nx, ny, nz, L.cx, L.cy, L.cz);
+  r[c] = b[c] - applyA<R, R>(e, i, j, k, nx, ny, nz, L.cx, L.cy, L.cz);
 }
 
 // 1-D restriction stencil: fine indices and weights contributing to coarse c
@@ -589,19 +677,49 @@ __global__ void k_restrict_axis(int ax, int periodic, int nx, int ny, int nz, in
   out[i + nx * (j + ny * k)] = acc * scale;
 }
 
-// coarsest grid: e = Cinv b (one block; the pseudo-inverse and the
-// products stay FP64 in both forms)
-template <typename T>
-__global__ void k_coarse_solve(int n, const double *__restrict__ cinv, const T *__restrict__ b, T *__restrict__ e) {
-  __shared__ double sb[512];
-  for (int a = threadIdx.x; a < n; a += blockDim.x) sb[a] = (double)b[a];
+// coarsest grid: e = Cinv b (the pseudo-inverse and the products stay FP64
+// in both forms).  One block with a thread per row of a row-major matrix took
+// 27.8 us at 192 unknowns and 144 us at 504 (every lane on its own row of a
+// 2 MB matrix, one SM's FP64 pipe).
+// FP64 levels: one warp per row, eight rows per block, lanes along the row
+// (4.6 us at 192).
+constexpr int CSB = 8;
+__global__ void __launch_bounds__(CSB * 32)
+    k_coarse_solve(int n, const double *__restrict__ cinv, const double *__restrict__ b, double *__restrict__ e) {
+  const int a = blockIdx.x * CSB + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (a >= n) return;
+  const double *row = cinv + (size_t)a * n;
+  double acc = 0.0;
+  for (int q = lane; q < n; q += 32) acc = fma(row[q], b[q], acc);
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  if (lane == 0) e[a] = acc;
+}
+// FP32 levels: a thread per row, eight rows per block, the products summed in
+// the row's order (see cg_beta) by one warp, from shared memory where all the
+// block's rows are brought at once (of the transposed matrix: eight
+// neighbouring entries per load); bound by the chain of n dependent FMAs.
+constexpr int CS32 = 8;
+__global__ void __launch_bounds__(256)
+    k_coarse_solve32(int n, const double *__restrict__ cinvt, const float *__restrict__ b, float *__restrict__ e) {
+  __shared__ double sb[512], sm[512 * CS32];
+  const int a0 = blockIdx.x * CS32, m = min(CS32, n - a0);
+  for (int q = threadIdx.x; q < n; q += 256) sb[q] = widen_bits(b[q]);
+#pragma unroll 4
+  for (int q = threadIdx.x; q < n * CS32; q += 256)
+    sm[q] = (q % CS32 < m) ? cinvt[(size_t)(q / CS32) * n + a0 + q % CS32] : 0.0;
   __syncthreads();
-  for (int a = threadIdx.x; a < n; a += blockDim.x) {
-    const double *row = cinv + (size_t)a * n;
+  if (threadIdx.x < m) {
     double acc = 0.0;
-    for (int q = 0; q < n; q++) acc += row[q] * sb[q];
-    e[a] = (T)acc;
+#pragma unroll 8
+    for (int q = 0; q < n; q++) acc = fma(sm[q * CS32 + threadIdx.x], sb[q], acc);
+    e[a0 + threadIdx.x] = (float)acc;
   }
+}
+static void coarse_solve(int n, const double *cinv, const double *b, double *e, cudaStream_t st) {
+  k_coarse_solve<<<(n + CSB - 1) / CSB, CSB * 32, 0, st>>>(n, cinv, b, e);
+}
+static void coarse_solve(int n, const double *cinvt, const float *b, float *e, cudaStream_t st) {
+  k_coarse_solve32<<<(n + CS32 - 1) / CS32, 256, 0, st>>>(n, cinvt, b, e);
 }
 
 // ---------------------------------------------------------------------------
@@ -695,11 +813,12 @@ static std::vector<double> thomas_factors(const PLevel &L) {
     if (e_ != cudaSuccess) return e_; \
   } while (0)
 
-template <typename R, typename TB, typename TE, typename TO>
+template <typename R>
 static cudaError_t lj2_attr() {
-  return cudaFuncSetAttribute(k_line_jacobi2<R, TB, TE, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              200 * 1024);
+  return cudaFuncSetAttribute(k_line_jacobi2<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
 }
+
+static size_t mg_dot_blocks(const PLevel &L);
 
 cudaError_t poisson_create(const Geo &g, double cx, double cy, double cz, int fp32,
                            PoissonSolver **out) {
@@ -736,6 +855,7 @@ cudaError_t poisson_create(const Geo &g, double cx, double cy, double cz, int fp
     c.cz = c.czs ? f.cz / 4.0 : f.cz;
     S->lv.push_back(c);
   }
+  if (S->lv.size() == 1 && S->lv[0].n <= 512) S->fp32 = 0;  // one dense FP64 solve: nothing to run in FP32
   const size_t esz = S->fp32 ? sizeof(float) : sizeof(double);
   for (size_t l = 0; l < S->lv.size(); l++) {
     PLevel &L = S->lv[l];
@@ -750,13 +870,19 @@ cudaError_t poisson_create(const Geo &g, double cx, double cy, double cz, int fp
           const double nbz = (L.nz == 1) ? 0.0 : ((q == 1) ? 2.0 : 1.0);
           L.invd[a][q] = 1.0 / (L.cx * nbx + 2.0 * L.cy + L.cz * nbz);
         }
+      if (l + 1 < S->lv.size()) {
+        const PLevel &c = S->lv[l + 1];
+        L.halved = L.point && c.cxs && c.cys && c.czs;
+      }
     }
     const size_t bytes = esz * (size_t)L.n;
     if (l > 0) PCK(cudaMalloc(&L.b, bytes));
-    PCK(cudaMalloc(&L.e, bytes));
-    PCK(cudaMalloc(&L.e2, bytes));
-    PCK(cudaMalloc(&L.r, bytes));
-    PCK(cudaMalloc(&L.t, bytes));
+    if (l > 0) PCK(cudaMalloc(&L.e, bytes));
+    if (!L.halved) {
+      PCK(cudaMalloc(&L.e2, bytes));
+      PCK(cudaMalloc(&L.r, bytes));
+      PCK(cudaMalloc(&L.t, bytes));
+    }
     std::vector<double> th = thomas_factors(L);
     if (S->fp32) {
       std::vector<float> thf(th.begin(), th.end());
@@ -768,15 +894,19 @@ cudaError_t poisson_create(const Geo &g, double cx, double cy, double cz, int fp
     }
   }
   if (S->fp32) {
-    PCK((lj2_attr<float, double, float, float>()));
-    PCK((lj2_attr<float, double, float, double>()));
-    PCK((lj2_attr<float, float, float, float>()));
+    PCK(lj2_attr<float>());
   } else {
-    PCK((lj2_attr<double, double, double, double>()));
+    PCK(lj2_attr<double>());
   }
   const PLevel &C = S->lv.back();
   if (C.n <= 512) {
     std::vector<double> M = coarse_pinv(C);
+    if (S->fp32) {  // by columns (the rounded matrix is not exactly symmetric)
+      std::vector<double> Mt(M.size());
+      for (int a = 0; a < C.n; a++)
+        for (int q = 0; q < C.n; q++) Mt[(size_t)q * C.n + a] = M[(size_t)a * C.n + q];
+      M.swap(Mt);
+    }
     PCK(cudaMalloc(&S->cinv, M.size() * sizeof(double)));
     PCK(cudaMemcpy(S->cinv, M.data(), M.size() * sizeof(double), cudaMemcpyHostToDevice));
   } else {
@@ -785,13 +915,21 @@ cudaError_t poisson_create(const Geo &g, double cx, double cy, double cz, int fp
   const size_t nb = sizeof(double) * (size_t)S->N;
   PCK(cudaMalloc(&S->x, nb));
   PCK(cudaMalloc(&S->r, nb));
-  PCK(cudaMalloc(&S->z, nb));
+  PCK(cudaMalloc(&S->z, S->fp32 ? nb / 2 : nb));
+  if (S->fp32) PCK(cudaMalloc((void **)&S->r32, nb / 2));
   PCK(cudaMalloc(&S->p, nb));
   PCK(cudaMalloc(&S->q, nb));
   PCK(cudaMalloc(&S->bvec, nb));
   PCK(cudaMalloc(&S->bin, sizeof(double) * (size_t)g.ny * g.nz));
   S->rblk = nblocks(S->N) < 1216 ? nblocks(S->N) : 1216;  // 8 blocks per SM on 152 SMs
-  PCK(cudaMalloc(&S->part, sizeof(double) * (size_t)S->rblk * 3));
+  {
+    size_t np = (size_t)S->rblk * 3;  // reductions of up to three sums, or one partial per block of k_mg_half_dot
+    if (S->lv[0].halved) {
+      const size_t nb = S->fp32 ? 0 : mg_dot_blocks(S->lv[0]);
+      if (nb > np) np = nb;
+    }
+    PCK(cudaMalloc(&S->part, sizeof(double) * np));
+  }
   PCK(cudaMalloc(&S->counter, sizeof(unsigned)));
   PCK(cudaMemset(S->counter, 0, sizeof(unsigned)));
   PCK(cudaMalloc(&S->s, sizeof(double) * S_COUNT));
@@ -815,6 +953,7 @@ void poisson_destroy(PoissonSolver *S) {
   cudaFree(S->x);
   cudaFree(S->r);
   cudaFree(S->z);
+  cudaFree(S->r32);
   cudaFree(S->p);
   cudaFree(S->q);
   cudaFree(S->bvec);
@@ -850,7 +989,10 @@ size_t poisson_footprint(const Geo &g, int fp32, size_t (*rnd)(size_t)) {
   }
   const size_t N = (size_t)g.nx * g.ny * g.nz;
   tot += 6 * rnd(sizeof(double) * N) + rnd(sizeof(double) * (size_t)g.ny * g.nz);
-  tot += rnd(sizeof(double) * 3 * 1216) + rnd(sizeof(unsigned)) + rnd(sizeof(double) * S_COUNT);
+  // reduction partials: three sums of 1216 blocks, or one of every block that forms r.z, at most one per 16 x 4 x 4
+  // points while there are few and one per 32 x 8 x 4 beyond
+  const size_t blk = (size_t)(g.nx / 32 + 1) * (g.ny / 8 + 1) * (g.nz / 4 + 1);
+  tot += rnd(sizeof(double) * (blk > 8 * 1216 ? blk : 8 * 1216)) + rnd(sizeof(unsigned)) + rnd(sizeof(double) * S_COUNT);
   return tot;
 }
 
@@ -866,17 +1008,16 @@ static LevArgs<R> largs(const PLevel &L) {
   return a;
 }
 
-template <typename R, typename TB, typename TE, typename TO>
-static void line_sweep(const PLevel &L, R w, R w1, int zero_init, const TB *b, const TE *ei, TO *eo,
-                       cudaStream_t st) {
+template <typename R>
+static void line_sweep(const PLevel &L, R w, R w1, int zero_init, const R *b, const R *ei, R *eo, cudaStream_t st) {
   const LevArgs<R> A = largs<R>(L);
   const R *th = static_cast<const R *>(L.thomas);
   const size_t smem = sizeof(R) * 32 * (size_t)L.nz;
   if (smem <= 200 * 1024) {
-    k_line_jacobi2<R, TB, TE, TO><<<(L.nx * L.ny + 31) / 32, LJ2_T, smem, st>>>(A, w, w1, zero_init, th, b, ei, eo);
+    k_line_jacobi2<R><<<(L.nx * L.ny + 31) / 32, LJ2_T, smem, st>>>(A, w, w1, zero_init, th, b, ei, eo);
   } else {
-    k_line_jacobi<R, TB, TE, TO><<<(L.nx * L.ny + LJB - 1) / LJB, LJB, 0, st>>>(A, w, w1, zero_init, th, b, ei,
-                                                                                static_cast<R *>(L.t), eo);
+    k_line_jacobi<R><<<(L.nx * L.ny + LJB - 1) / LJB, LJB, 0, st>>>(A, w, w1, zero_init, th, b, ei,
+                                                                   static_cast<R *>(L.t), eo);
   }
 }
 
@@ -944,83 +1085,185 @@ static InvD<R> invd_of(const PLevel &L) {
   return v;
 }
 
+template <typename R>
+static MgLev<R> mglev(const PLevel &L) {
+  MgLev<R> m;
+  m.nx = L.nx;
+  m.ny = L.ny;
+  m.nz = L.nz;
+  m.cx = (R)L.cx;
+  m.cy = (R)L.cy;
+  m.cz = (R)L.cz;
+  for (int a = 0; a < 3; a++)
+    for (int q = 0; q < 3; q++) {
+      m.inv[a][q] = (R)L.invd[a][q];
+      m.tx[a][q] = (R)(L.cx * L.invd[a][q]);
+      m.ty[a][q] = (R)(L.cy * L.invd[a][q]);
+      m.tz[a][q] = (R)(L.cz * L.invd[a][q]);
+    }
+  return m;
+}
+
+// Levels a thread of the k_mg_* pair kernels marches: 8 where the level
+// still gives 8 blocks of 256 threads per SM (152), fewer below, so that the
+// coarse levels, which are short of blocks, spread over the SMs.  Even.
+static int mg_columns(const PLevel &L) {
+  return ((L.nx / 2 + MGP_X - 1) / MGP_X) * ((L.ny + MGP_Y - 1) / MGP_Y);
+}
+static int mg_kz(const PLevel &L) {
+  int kz = 8;
+  while (kz > 2 && mg_columns(L) * ((L.nz + kz - 1) / kz) < 8 * 152) kz /= 2;
+  return kz;
+}
+static int mg_blocks(const PLevel &L, int kz) { return mg_columns(L) * ((L.nz + kz - 1) / kz); }
+
+// Which form a halved level takes: levels of more points run the five passes
+// (fewest operations), smaller ones the two tile launches.
+constexpr int MG_SPLIT64 = 200000, MG_SPLIT32 = 300000;
+template <typename R>
+static bool mg_split(const PLevel &L) {
+  return L.n > (sizeof(R) == sizeof(double) ? MG_SPLIT64 : MG_SPLIT32);
+}
+static int mg_tiles(const PLevel &L, int cx, int cy, int cz) {
+  return ((L.nx / 2 + cx - 1) / cx) * ((L.ny / 2 + cy - 1) / cy) * ((L.nz / 2 + cz - 1) / cz);
+}
+// blocks of the launch that forms r.z on the finest level (FP64)
+static size_t mg_dot_blocks(const PLevel &L) {
+  return mg_split<double>(L) ? mg_blocks(L, mg_kz(L)) : mg_tiles(L, 8, 2, 2);
+}
+
 // pre-smoothing from a zero start into e2: z-line Jacobi, or red then black
-template <typename R, typename TB>
-static void pre_smooth(const PLevel &L, R w, R w1, const TB *b, R *e2, cudaStream_t st, long *nl) {
+template <typename R>
+static void pre_smooth(const PLevel &L, R w, R w1, const R *b, R *e2, cudaStream_t st, long *nl) {
   if (!L.point) {
-    line_sweep<R, TB, R, R>(L, w, w1, 1, b, nullptr, e2, st);
+    line_sweep<R>(L, w, w1, 1, b, nullptr, e2, st);
     (*nl)++;
     return;
   }
   const LevArgs<R> A = largs<R>(L);
   const dim3 grd = mg_grid((L.nx + 1) / 2, L.ny, L.nz);
-  k_rbgs<R, TB, R, R><<<grd, dim3(MG_BX, MG_BY), 0, st>>>(A, invd_of<R>(L), 0, 1, 0, b, e2, e2);
-  k_rbgs<R, TB, R, R><<<grd, dim3(MG_BX, MG_BY), 0, st>>>(A, invd_of<R>(L), 1, 0, 0, b, e2, e2);
+  k_rbgs<R><<<grd, dim3(MG_BX, MG_BY), 0, st>>>(A, invd_of<R>(L), 0, 1, 0, b, e2, e2);
+  k_rbgs<R><<<grd, dim3(MG_BX, MG_BY), 0, st>>>(A, invd_of<R>(L), 1, 0, 0, b, e2, e2);
   *nl += 2;
 }
 
 // post-smoothing of e2 into res: z-line Jacobi, or black (in place) then red
 // (with the black values copied), the adjoint order of the pre-smoothing
-template <typename R, typename TB, typename TO>
-static void post_smooth(const PLevel &L, R w, R w1, const TB *b, R *e2, TO *res, cudaStream_t st, long *nl) {
+template <typename R>
+static void post_smooth(const PLevel &L, R w, R w1, const R *b, R *e2, R *res, cudaStream_t st, long *nl) {
   if (!L.point) {
-    line_sweep<R, TB, R, TO>(L, w, w1, 0, b, e2, res, st);
+    line_sweep<R>(L, w, w1, 0, b, e2, res, st);
     (*nl)++;
     return;
   }
   const LevArgs<R> A = largs<R>(L);
   const dim3 grd = mg_grid((L.nx + 1) / 2, L.ny, L.nz);
-  k_rbgs<R, TB, R, R><<<grd, dim3(MG_BX, MG_BY), 0, st>>>(A, invd_of<R>(L), 1, 0, 0, b, e2, e2);
-  k_rbgs<R, TB, R, TO><<<grd, dim3(MG_BX, MG_BY), 0, st>>>(A, invd_of<R>(L), 0, 0, 1, b, e2, res);
+  k_rbgs<R><<<grd, dim3(MG_BX, MG_BY), 0, st>>>(A, invd_of<R>(L), 1, 0, 0, b, e2, e2);
+  k_rbgs<R><<<grd, dim3(MG_BX, MG_BY), 0, st>>>(A, invd_of<R>(L), 0, 0, 1, b, e2, res);
   *nl += 2;
 }
 
-// one symmetric V-cycle: out = M b0.  Every level pre-smooths into its
-// scratch e2 (one damped line-Jacobi sweep from zero), restricts the
-// residual, adds the prolonged coarse correction into e2 and post-smooths
-// from e2 into its result buffer (out on the finest level, e elsewhere).
-// R: level type; the finest level reads b0 and writes out in FP64.
+// Coarse levels per block of k_mg_restrict: up to 8 while every SM keeps four
+// blocks (each block also forms the residual of two fine levels of its
+// neighbours).
+static void mg_restrict_grid(const PLevel &L, int ncz, int *czb, int *blocks) {
+  const int gxy = ((L.nx + MGR_FX - 1) / MGR_FX) * ((L.ny + MGR_FY - 1) / MGR_FY);
+  *czb = 8;
+  while (*czb > 1 && gxy * ((ncz + *czb - 1) / *czb) < 4 * 152) *czb /= 2;
+  *blocks = gxy * ((ncz + *czb - 1) / *czb);
+}
+
+// b -> the coarse right-hand side bc (ncz levels); the five-pass form keeps
+// the pre-smoothed iterate in e.
 template <typename R>
-static cudaError_t vcycle(PoissonSolver *S, const double *b0, double *out, cudaStream_t st, long *nl) {
+static cudaError_t mg_down_level(const MgLev<R> &M, const PLevel &L, int ncz, const R *b, R *e, R *bc,
+                                 cudaStream_t st, long *nl) {
+  if (mg_split<R>(L)) {
+    const int kz = mg_kz(L);
+    int czb, nb;
+    mg_restrict_grid(L, ncz, &czb, &nb);
+    if constexpr (sizeof(R) == sizeof(double)) k_mg_black<<<mg_blocks(L, kz), 256, 0, st>>>(M, b, e, kz);
+    else k_mg_pre<<<mg_blocks(L, kz), 256, 0, st>>>(M, b, e, kz);
+    k_mg_restrict<R><<<nb, 256, 0, st>>>(M, b, e, bc, czb);
+    *nl += 2;
+  } else {
+    k_mg_down<R, 8, 2, 2><<<mg_tiles(L, 8, 2, 2), 256, 0, st>>>(M, b, bc);
+    *nl += 1;
+  }
+  return cudaGetLastError();
+}
+
+// b and the coarse correction ec -> e; FP64: on the finest level r.z too.
+static cudaError_t mg_up_level(PoissonSolver *S, const MgLev<double> &M, const PLevel &L, bool finest,
+                               const double *b, const double *ec, double *e, cudaStream_t st, long *nl) {
+  if (mg_split<double>(L)) {
+    const int kz = mg_kz(L), nb = mg_blocks(L, kz);
+    k_mg_prolong<<<nb, 256, 0, st>>>(M, b, ec, e, kz);
+    k_mg_half<<<nb, 256, 0, st>>>(M, 1, b, e, kz);
+    if (finest) k_mg_half_dot<<<nb, PB, 0, st>>>(M, b, e, kz, S->part, S->counter, S->s);
+    else k_mg_half<<<nb, 256, 0, st>>>(M, 0, b, e, kz);
+    *nl += 3;
+  } else {
+    const int nb = mg_tiles(L, 8, 2, 2);
+    if (finest) k_mg_up_dot<8, 2, 2><<<nb, PB, 0, st>>>(M, b, ec, e, S->part, S->counter, S->s);
+    else k_mg_up<double, 8, 2, 2><<<nb, 256, 0, st>>>(M, b, ec, e);
+    *nl += 1;
+  }
+  return cudaGetLastError();
+}
+static cudaError_t mg_up_level(PoissonSolver *, const MgLev<float> &M, const PLevel &L, bool, const float *b,
+                               const float *ec, float *e, cudaStream_t st, long *nl) {
+  if (mg_split<float>(L)) {
+    const int kz = mg_kz(L), nb = mg_blocks(L, kz);
+    k_mg_prolong32<<<nb, 256, 0, st>>>(M, b, ec, e, kz);
+    k_mg_half<<<nb, 256, 0, st>>>(M, 1, b, e, kz);
+    k_mg_half<<<nb, 256, 0, st>>>(M, 0, b, e, kz);
+    *nl += 3;
+  } else {
+    k_mg_up<float, 8, 2, 2><<<mg_tiles(L, 8, 2, 2), 256, 0, st>>>(M, b, ec, e);
+    *nl += 1;
+  }
+  return cudaGetLastError();
+}
+
+// r.z and beta of the preconditioned residual out.
+static cudaError_t mg_dot(PoissonSolver *S, const double *out, cudaStream_t st, long *nl) {
+  if (S->lv.size() > 1 && S->lv[0].halved) return cudaSuccess;  // formed by mg_up_level
+  k_rdot<<<S->rblk, PB, 0, st>>>(S->N, S->r, out, S->part, S->counter, S->s);
+  (*nl)++;
+  return cudaGetLastError();
+}
+static cudaError_t mg_dot(PoissonSolver *S, const float *out, cudaStream_t st, long *nl) {
+  k_zdot<<<S->rblk, PB, 0, st>>>(S->N, 1.0 / (double)S->N, S->r, out, S->part, S->counter, S->s);
+  (*nl)++;
+  return cudaGetLastError();
+}
+
+// one symmetric V-cycle: out = M b0, and r.z into the CG scalars.  A level
+// whose axes are all coarsened runs the k_mg_* kernels in place in its
+// result array (L.halved); the others pre-smooth into their scratch e2 (one
+// damped line-Jacobi sweep from zero, or red-black), restrict the residual,
+// add the prolonged coarse correction into e2 and post-smooth into the
+// result (out on the finest level, e elsewhere).  R: level type.
+template <typename R>
+static cudaError_t vcycle(PoissonSolver *S, const R *b0, R *out, cudaStream_t st, long *nl) {
   const int nlev = (int)S->lv.size();
   const R w = (R)S->omega, w1 = (R)(1.0 - S->omega);
   auto lvp = [](void *p) { return static_cast<R *>(p); };
-  if (nlev == 1) {
-    PLevel &L = S->lv[0];
-    if (S->cinv) {
-      k_coarse_solve<double><<<1, 256, 0, st>>>(L.n, S->cinv, b0, out);
-      (*nl)++;
-      return cudaGetLastError();
-    }
-    // single level without a dense inverse: damped line-Jacobi sweeps
-    R *cur = lvp(L.e2), *oth = lvp(L.e);
-    line_sweep<R, double, R, R>(L, w, w1, 1, b0, nullptr, cur, st);
-    (*nl)++;
-    for (int sw = 1; sw < S->coarse_sweeps - 1; sw++) {
-      line_sweep<R, double, R, R>(L, w, w1, 0, b0, cur, oth, st);
-      (*nl)++;
-      R *tmp = cur;
-      cur = oth;
-      oth = tmp;
-    }
-    line_sweep<R, double, R, double>(L, w, w1, 0, b0, cur, out, st);
-    (*nl)++;
-    return cudaGetLastError();
-  }
   for (int l = 0; l < nlev; l++) {
     PLevel &L = S->lv[l];
-    const R *b = lvp(L.b);
-    R *res = lvp(L.e);
+    const R *b = (l == 0) ? b0 : lvp(L.b);
+    R *res = (l == 0) ? out : lvp(L.e);
     if (l == nlev - 1) {
       if (S->cinv) {
-        k_coarse_solve<R><<<1, 256, 0, st>>>(L.n, S->cinv, b, res);
+        coarse_solve(L.n, S->cinv, b, res, st);
         (*nl)++;
-      } else {
+      } else {  // no dense inverse: damped line-Jacobi sweeps
         R *cur = lvp(L.e2), *oth = res;
-        line_sweep<R, R, R, R>(L, w, w1, 1, b, nullptr, cur, st);
+        line_sweep<R>(L, w, w1, 1, b, nullptr, cur, st);
         (*nl)++;
         for (int sw = 1; sw < S->coarse_sweeps; sw++) {
-          line_sweep<R, R, R, R>(L, w, w1, 0, b, cur, oth, st);
+          line_sweep<R>(L, w, w1, 0, b, cur, oth, st);
           (*nl)++;
           R *tmp = cur;
           cur = oth;
@@ -1031,32 +1274,34 @@ static cudaError_t vcycle(PoissonSolver *S, const double *b0, double *out, cudaS
       PCK(cudaGetLastError());
       break;
     }
-    const LevArgs<R> A = largs<R>(L);
-    if (l == 0) {
-      pre_smooth<R, double>(L, w, w1, b0, lvp(L.e2), st, nl);
-      k_residual<R, double, R><<<mg_grid(L.nx, L.ny, L.nz), dim3(MG_BX, MG_BY), 0, st>>>(A, b0, lvp(L.e2),
-                                                                                    lvp(L.r));
-    } else {
-      pre_smooth<R, R>(L, w, w1, b, lvp(L.e2), st, nl);
-      k_residual<R, R, R><<<mg_grid(L.nx, L.ny, L.nz), dim3(MG_BX, MG_BY), 0, st>>>(A, b, lvp(L.e2), lvp(L.r));
-    }
     const PLevel &C = S->lv[l + 1];
-    PCK(restrict_chain<R>(L, C, lvp(L.r), lvp(L.t), lvp(C.b), st, nl));
+    if (L.halved) {
+      const MgLev<R> M = mglev<R>(L);
+      PCK(mg_down_level(M, L, C.nz, b, res, lvp(C.b), st, nl));
+      continue;
+    }
+    const LevArgs<R> A = largs<R>(L);
+    pre_smooth<R>(L, w, w1, b, lvp(L.e2), st, nl);
+    k_residual<R><<<mg_grid(L.nx, L.ny, L.nz), dim3(MG_BX, MG_BY), 0, st>>>(A, b, lvp(L.e2), lvp(L.r));
     *nl += 1;
+    PCK(restrict_chain<R>(L, C, lvp(L.r), lvp(L.t), lvp(C.b), st, nl));
     PCK(cudaGetLastError());
   }
   for (int l = nlev - 2; l >= 0; l--) {
     PLevel &L = S->lv[l];
     const PLevel &C = S->lv[l + 1];
-    const LevArgs<R> A = largs<R>(L);
-    PCK(prolong_chain<R>(L, C, lvp(C.e), lvp(L.t), lvp(L.e2), st, nl));
-    if (l == 0)
-      post_smooth<R, double, double>(L, w, w1, b0, lvp(L.e2), out, st, nl);
-    else
-      post_smooth<R, R, R>(L, w, w1, lvp(L.b), lvp(L.e2), lvp(L.e), st, nl);
+    const R *b = (l == 0) ? b0 : lvp(L.b);
+    R *res = (l == 0) ? out : lvp(L.e);
+    if (L.halved) {
+      const MgLev<R> M = mglev<R>(L);
+      PCK(mg_up_level(S, M, L, l == 0, b, lvp(C.e), res, st, nl));
+    } else {
+      PCK(prolong_chain<R>(L, C, lvp(C.e), lvp(L.t), lvp(L.e2), st, nl));
+      post_smooth<R>(L, w, w1, b, lvp(L.e2), res, st, nl);
+    }
     PCK(cudaGetLastError());
   }
-  return cudaSuccess;
+  return mg_dot(S, out, st, nl);
 }
 
 // The solve in three parts: set-up (b, x0 = p_old, r0 and the first
@@ -1076,7 +1321,7 @@ static cudaError_t solve_begin(PoissonSolver *S, const Geo &g, const Phys &ph, c
                                          static_cast<const double *>(u3), u_inlet, pres_old, S->bvec, S->x, S->bin,
                                          S->part, S->counter, S->s);
   k_init_r<<<rb, PB, 0, st>>>(F.nx, F.ny, F.nz, F.cx, F.cy, F.cz, 1.0 / (double)N, rtol, ctl, S->s, S->bvec,
-                              S->x, S->r, S->part, S->counter);
+                              S->x, S->r, S->r32, S->part, S->counter);
   *nl += 2;
   return cudaGetLastError();
 }
@@ -1084,12 +1329,18 @@ static cudaError_t solve_begin(PoissonSolver *S, const Geo &g, const Phys &ph, c
 static cudaError_t solve_iteration(PoissonSolver *S, const CgCtl &ctl, cudaStream_t st, long *nl) {
   const int N = S->N, rb = S->rblk;
   const PLevel &F = S->lv[0];
-  PCK(S->fp32 ? vcycle<float>(S, S->r, S->z, st, nl) : vcycle<double>(S, S->r, S->z, st, nl));
-  k_zdot<<<rb, PB, 0, st>>>(N, 1.0 / (double)N, S->r, S->z, S->part, S->counter, S->s);
-  k_pupdate<<<nblocks(N), PB, 0, st>>>(N, S->s, S->z, S->p);
+  if (S->fp32) {
+    float *z = static_cast<float *>(S->z);
+    PCK(vcycle<float>(S, S->r32, z, st, nl));
+    k_pupdate<float><<<nblocks(N), PB, 0, st>>>(N, S->s, z, S->p);
+  } else {
+    double *z = static_cast<double *>(S->z);
+    PCK(vcycle<double>(S, S->r, z, st, nl));
+    k_pupdate<double><<<nblocks(N), PB, 0, st>>>(N, S->s, z, S->p);
+  }
   k_apply_dot<<<rb, PB, 0, st>>>(F.nx, F.ny, F.nz, F.cx, F.cy, F.cz, S->p, S->q, S->part, S->counter, S->s);
-  k_axpy<<<rb, PB, 0, st>>>(N, ctl, S->s, S->p, S->q, S->x, S->r, S->part, S->counter);
-  *nl += 4;
+  k_axpy<<<rb, PB, 0, st>>>(N, ctl, S->s, S->p, S->q, S->x, S->r, S->r32, S->part, S->counter);
+  *nl += 3;
   return cudaGetLastError();
 }
 

@@ -58,6 +58,18 @@ __device__ __forceinline__ float dif(F2 a, F2 b) { return (a.h - b.h) + (a.l - b
 __device__ __forceinline__ float val(F2 a) { return a.h + a.l; }
 __device__ __forceinline__ float round_bits(double x) { return val(split_bits(x)); }
 
+// (float)x, round to nearest even, by operations on the two 32-bit words (a
+// conversion instruction would hold the FP64 pipe); values outside FP32's
+// normal range convert by the instruction
+__device__ __forceinline__ float float_bits(double x) {
+  const unsigned int hi = (unsigned int)__double2hiint(x), lo = (unsigned int)__double2loint(x);
+  const unsigned int a = hi & 0x7fffffffu;
+  if (a - 0x38100000u >= 0x47e00000u - 0x38100000u) return (a | lo) == 0 ? __uint_as_float(hi) : (float)x;
+  const unsigned int m = __funnelshift_l(lo, a - 0x38000000u, 3), rem = lo & 0x1fffffffu;
+  const unsigned int up = (rem > 0x10000000u || (rem == 0x10000000u && (m & 1u))) ? 1u : 0u;
+  return __uint_as_float((m + up) | (hi & 0x80000000u));
+}
+
 // order of two pairs of the same normalisation (both from split_bits, or
 // both from an error-free sum): by hi, then by lo
 __device__ __forceinline__ F2 pmin(F2 a, F2 b) { return (b.h < a.h || (b.h == a.h && b.l < a.l)) ? b : a; }
