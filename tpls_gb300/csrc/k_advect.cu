@@ -384,8 +384,7 @@ cudaError_t launch_to_float(const double *a, float *b, size_t n, cudaStream_t st
 }
 
 // exchange2d on one GPU: rows 0 <- ny, ny+1 <- 1 over x = 0..nx+1.
-template <typename T>
-__global__ void k_exchange(Geo g, T *a, int nzp) {
+__global__ void k_exchange(Geo g, double *a, int nzp) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int k = blockIdx.y;
   if (i > g.nx + 1 || k >= nzp) return;
@@ -395,14 +394,36 @@ __global__ void k_exchange(Geo g, T *a, int nzp) {
 
 cudaError_t launch_exchange(const Geo &g, double *a, int nzp, cudaStream_t st) {
   dim3 blk(128), grd((g.nx + 2 + 127) / 128, nzp);
-  k_exchange<double><<<grd, blk, 0, st>>>(g, a, nzp);
+  k_exchange<<<grd, blk, 0, st>>>(g, a, nzp);
   return cudaGetLastError();
 }
-cudaError_t launch_exchange(const Geo &g, float *a, int nzp, cudaStream_t st) {
-  dim3 blk(128), grd((g.nx + 2 + 127) / 128, nzp);
-  k_exchange<float><<<grd, blk, 0, st>>>(g, a, nzp);
+template <typename T>
+struct ExSet {
+  T *a[3];
+  int nzp[3];
+};
+template <typename T>
+__global__ void k_exchange_set(Geo g, ExSet<T> s) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y, q = blockIdx.z;
+  if (i > g.nx + 1 || k >= s.nzp[q]) return;
+  T *a = s.a[q];
+  a[TPLS_IDX(g, i, 0, k)] = a[TPLS_IDX(g, i, g.ny, k)];
+  a[TPLS_IDX(g, i, g.ny + 1, k)] = a[TPLS_IDX(g, i, 1, k)];
+}
+template <typename T>
+cudaError_t launch_exchange_set(const Geo &g, int n, T *const *a, const int *nzp, cudaStream_t st) {
+  ExSet<T> s = {};
+  int m = 0;
+  for (int q = 0; q < n; q++) {
+    s.a[q] = a[q];
+    s.nzp[q] = nzp[q];
+    if (nzp[q] > m) m = nzp[q];
+  }
+  k_exchange_set<T><<<dim3((g.nx + 2 + 127) / 128, m, n), 128, 0, st>>>(g, s);
   return cudaGetLastError();
 }
+template cudaError_t launch_exchange_set<double>(const Geo &, int, double *const *, const int *, cudaStream_t);
+template cudaError_t launch_exchange_set<float>(const Geo &, int, float *const *, const int *, cudaStream_t);
 
 // Deterministic final reduction of per-block partials (one block).
 __global__ void k_finish_sum(const double *part, int nparts, double *out, int nout) {

@@ -100,51 +100,64 @@ __device__ __forceinline__ Rec<double> get_rec(int comp, const Geo &g, const Ref
   return q;
 }
 
-// Jacobi: x = J(xo) on the component's interior with its boundary rows.
-template <typename T, typename CS, int CC, int SW_X, int SW_Y>
+// The FP64 sweeps run every component of the set in one launch (gx blocks
+// along x each): the components are independent, and one after the other they
+// left a small channel's SMs idle (32 blocks per launch at 64x32x48) and
+// every launch with a tail of its own.
+// Jacobi: x = J(xo) on a component's interior with its boundary rows, ghost
+// rows included (out of place, so no row read is written); ZERO: xo = 0, so
+// x = b, the records' other entries neither read nor multiplied.
+template <int SW_X, int SW_Y, bool ZERO>
 __global__ void __launch_bounds__(SW_X *SW_Y)
-    k_jacobi_c(int comp_, Geo g, Helm h, const T *__restrict__ xo, const CS coef,
-               const double *__restrict__ P, const double *__restrict__ X, T *__restrict__ x, int fuse) {
-  const int comp = (CC >= 0) ? CC : comp_;
-  const int i = blockIdx.x * SW_X + threadIdx.x + 1, j = blockIdx.y * SW_Y + threadIdx.y + 1;
+    k_jacobi_c(Geo g, Helm h, const __grid_constant__ SweepSet64 S, int gx, const double *__restrict__ P) {
+  const int q3 = blockIdx.x / gx, comp = S.id[q3];
+  const int i = (blockIdx.x - q3 * gx) * SW_X + threadIdx.x + 1, j = blockIdx.y * SW_Y + threadIdx.y + 1;
   const int k = blockIdx.z + (comp == 2 ? 1 : 0);
   const int iend = (comp == 0) ? g.nx - 1 : g.nx;
-  if (i > iend || j > g.ny) return;
+  if (i > iend || j > g.ny || k > g.nz - 1) return;
   const int c = TPLS_IDX(g, i, j, k), sy = g.sy, sz = g.sz;
-  const Rec<T> q = get_rec(comp, g, coef, c, i, j, k, false);
-  const T xc = xo[c];
-  T zp, zm;
-  if (comp == 2) {
-    zp = xo[c + sz];
-    zm = xo[c - sz];
-  } else {  // walls folded into the record: the z slot multiplies the point itself
-    zp = (k == g.nz - 1) ? xc : xo[c + sz];
-    zm = (k == 0) ? xc : xo[c - sz];
+  double *x = S.x[q3];
+  double v;
+  if constexpr (ZERO) {
+    v = __ldg(S.coef[q3] + 8 * (size_t)rec_slot(g, c, i) + 6);
+  } else {
+    const double *__restrict__ xo = S.xo[q3];
+    const Rec<double> q = get_rec(comp, g, S.coef[q3], c, i, j, k, false);
+    const double xc = xo[c];
+    double zp, zm;
+    if (comp == 2) {
+      zp = xo[c + sz];
+      zm = xo[c - sz];
+    } else {  // walls folded into the record: the z slot multiplies the point itself
+      zp = (k == g.nz - 1) ? xc : xo[c + sz];
+      zm = (k == 0) ? xc : xo[c - sz];
+    }
+    v = rec_apply(q, xo[c + 1], xo[c - 1], xo[c + sy], xo[c - sy], zp, zm);
   }
-  const T v = rec_apply(q, xo[c + 1], xo[c - 1], xo[c + sy], xo[c - sy], zp, zm);
-  put(g, x, i, j, k, v, fuse);
+  put(g, x, i, j, k, v, 1);
   const bool edge = (i == 1) || (i >= g.nx - 1) || (comp == 2 && (k == 1 || k == g.nz - 1));
-  if (edge) jacobi_bc(comp, g, h, x, X, P, i, j, k, v, fuse);
+  if (edge) jacobi_bc(comp, g, h, x, (const double *)nullptr, P, i, j, k, v, 1);
 }
 
 // 3-D checkerboard half-sweep (even iteration_time), one thread per point
 // of the colour.
-template <typename T, typename CS, int CC, int SW_X, int SW_Y>
+template <int SW_X, int SW_Y>
 __global__ void __launch_bounds__(SW_X *SW_Y)
-    k_sor_even_c(int comp_, Geo g, Helm h, T *__restrict__ x, const CS coef,
-                 const double *__restrict__ P, const double *__restrict__ X, int flg, int bc, int fuse) {
-  const int comp = (CC >= 0) ? CC : comp_;
-  const int i2 = blockIdx.x * SW_X + threadIdx.x, j = blockIdx.y * SW_Y + threadIdx.y + 1;
+    k_sor_even_c(Geo g, Helm h, const __grid_constant__ SweepSet64 S, int gx, const double *__restrict__ P, int flg,
+                 int bc, int fuse) {
+  const int q3 = blockIdx.x / gx, comp = S.id[q3];
+  const int i2 = (blockIdx.x - q3 * gx) * SW_X + threadIdx.x, j = blockIdx.y * SW_Y + threadIdx.y + 1;
   const int k = blockIdx.z + (comp == 2 ? 1 : 0);
   const int iend = (comp == 0) ? g.nx - 1 : g.nx;
-  if (i2 > (iend - 1) / 2 || j > g.ny) return;
+  if (i2 > (iend - 1) / 2 || j > g.ny || k > g.nz - 1) return;
   const int i = 2 * i2 + 1 + ((k + j + flg) & 1);
-  T v = 0;
+  double *__restrict__ x = S.x[q3];
+  double v = 0;
   if (i <= iend) {
     const int c = TPLS_IDX(g, i, j, k), sy = g.sy, sz = g.sz;
-    const Rec<T> q = get_rec(comp, g, coef, c, i, j, k, false);
-    const T xc = x[c];
-    T zp, zm;
+    const Rec<double> q = get_rec(comp, g, S.coef[q3], c, i, j, k, false);
+    const double xc = x[c];
+    double zp, zm;
     if (comp == 2) {
       zp = x[c + sz];
       zm = x[c - sz];
@@ -152,11 +165,11 @@ __global__ void __launch_bounds__(SW_X *SW_Y)
       zp = (k == g.nz - 1) ? xc : x[c + sz];
       zm = (k == 0) ? xc : x[c - sz];
     }
-    const T res = rec_apply(q, x[c + 1], x[c - 1], x[c + sy], x[c - sy], zp, zm);
-    v = xc + (T)1.2 * (res - xc);
+    const double res = rec_apply(q, x[c + 1], x[c - 1], x[c + sy], x[c - sy], zp, zm);
+    v = xc + 1.2 * (res - xc);
     put(g, x, i, j, k, v, fuse);
   }
-  if (bc) sor_bc(comp, g, h, x, X, P, i2, i, iend, v, j, k, fuse);
+  if (bc) sor_bc(comp, g, h, x, (const double *)nullptr, P, i2, i, iend, v, j, k, fuse);
 }
 
 // Odd-iteration half-sweep (2-D colouring, sequential in k).  Within such a
@@ -373,6 +386,14 @@ __device__ __forceinline__ T odd_write(int comp, const Geo &g, const Helm &h, T 
   return last;
 }
 
+// Shared memory of a block of the odd half-sweep: A and B (then y and P) of
+// a super-chunk, the chunk ends, and the values carried between super-chunks
+// or entering each warp's chunk (FP64) or the segment (FP32).
+template <typename T>
+struct OddShared {
+  T A[SOC_SC][32], B[SOC_SC][32], ey[SOC_W][32], ep[SOC_W][32], xin[sizeof(T) == 8 ? SOC_W : 1][32];
+};
+
 // One tile: 32 columns (x pairs from bx*32) of row j = by+1, the whole
 // column.  Every thread of the block runs it (it synchronises the block).
 // The segment kernel below runs the same phases by the helpers above, one
@@ -381,10 +402,10 @@ template <typename T, typename CS, int CC>
 __device__ __forceinline__ void sor_odd_c4_tile(int comp_, const Geo &g, const Helm &h, T *__restrict__ x,
                                                 const CS &coef, const double *__restrict__ P,
                                                 const double *__restrict__ X, int flg, int bc, int fuse, int bx,
-                                                int by) {
+                                                int by, OddShared<T> &sh) {
   const int comp = (CC >= 0) ? CC : comp_;
-  __shared__ T sA[SOC_SC][32], sB[SOC_SC][32];
-  __shared__ T ey[SOC_W][32], ep[SOC_W][32], scarry[32];
+  T(&sA)[SOC_SC][32] = sh.A, (&sB)[SOC_SC][32] = sh.B, (&ey)[SOC_W][32] = sh.ey, (&ep)[SOC_W][32] = sh.ep;
+  T(&scarry)[32] = sh.xin[0];
   const int j = by + 1;
   const int iend = (comp == 0) ? g.nx - 1 : g.nx;
   const int npair = (iend + 1) / 2;
@@ -490,24 +511,16 @@ __device__ __forceinline__ void sor_odd_c4_tile(int comp_, const Geo &g, const H
 // the block counts it in *kto, takes NaN as its entering value (the step's
 // pressure solve then reports DIVERGED_NAN) and still publishes, so no
 // later segment waits on it.
+// The columns of every component of the set form one list of tiles.
 template <typename T, typename CS, int CC>
-__global__ void __launch_bounds__(SOC_W * 32, sizeof(T) == 4 ? 6 : 5)  // 40 / 48 registers: 6 / 5 blocks per SM
-    k_sor_odd_seg(int comp_, Geo g, Helm h, T *__restrict__ x, const CS coef, const double *__restrict__ P,
-                  const double *__restrict__ X, int flg, int bc, int fuse, OddChain oc, int gx, int limit) {
+__device__ __forceinline__ void sor_odd_segment(int comp_, const Geo &g, const Helm &h, T *__restrict__ x,
+                                                const CS &coef, const double *__restrict__ P,
+                                                const double *__restrict__ X, int flg, int bc, int fuse,
+                                                const OddChain &oc, int limit, unsigned t, unsigned epoch, int nct,
+                                                int seg, int bx, int j, OddShared<T> &sh) {
   const int comp = (CC >= 0) ? CC : comp_;
-  __shared__ T sA[SOC_SC][32], sB[SOC_SC][32];
-  // the value entering each warp's chunk (FP64), or the segment's (FP32)
-  __shared__ T ey[SOC_W][32], ep[SOC_W][32], sxin[sizeof(T) == 8 ? SOC_W : 1][32];
-  __shared__ unsigned s_t, s_ep;
-  if (threadIdx.x == 0) {
-    s_t = atomicAdd(&oc.ctr[0], 1u);
-    s_ep = ld_acquire_u32(&oc.ctr[2]);
-  }
-  __syncthreads();
-  const unsigned t = s_t, epoch = s_ep;
-  const int nct = gx * g.ny;
-  const int seg = (int)(t / (unsigned)nct), ct = (int)(t - (unsigned)seg * nct);
-  const int bx = ct % gx, j = ct / gx + 1;
+  T(&sA)[SOC_SC][32] = sh.A, (&sB)[SOC_SC][32] = sh.B, (&ey)[SOC_W][32] = sh.ey, (&ep)[SOC_W][32] = sh.ep;
+  auto &sxin = sh.xin;
   const int iend = (comp == 0) ? g.nx - 1 : g.nx;
   const int npair = (iend + 1) / 2;
   const int par = (j + flg) & 1;
@@ -516,6 +529,7 @@ __global__ void __launch_bounds__(SOC_W * 32, sizeof(T) == 4 ? 6 : 5)  // 40 / 4
   const int i2 = bx * 32 + lane, i = 2 * i2 + 1 + par;
   const bool act = (i2 < npair) && (i <= iend);
   const int kc = k0 + seg * SOC_SC, n = min(SOC_SC, k1 - kc + 1);
+  if (n <= 0) return;  // w's columns are a level shorter: its last segment can be empty (none waits for it)
   constexpr int PER = SOC_SC / SOC_W;
   odd_produce_scan<T, CS>(comp, g, coef, x, i, j, act, k0, kc, n, sA, sB, ey, ep);
   if (w == 0) {
@@ -563,6 +577,42 @@ __global__ void __launch_bounds__(SOC_W * 32, sizeof(T) == 4 ? 6 : 5)  // 40 / 4
   __syncthreads();
   odd_write<T>(comp, g, h, x, X, P, bc, fuse, i2, i, j, iend, npair, kc, n, sxin[sizeof(T) == 8 ? w : 0][lane], sA,
                sB, ey, ep);
+}
+
+// One component's work on a tile, the component a compile-time constant for
+// the FP32 sweeps (their face averages differ by component).
+#define TPLS_BY_COMP(CALL)                        \
+  do {                                            \
+    if constexpr (sizeof(T) == sizeof(float)) {   \
+      if (comp == 0) CALL(0);                     \
+      else if (comp == 1) CALL(1);                \
+      else CALL(2);                               \
+    } else {                                      \
+      CALL(-1);                                   \
+    }                                             \
+  } while (0)
+
+template <typename T, typename CS>
+__global__ void __launch_bounds__(SOC_W * 32, sizeof(T) == 4 ? 6 : 5)  // 40 / 48 registers: 6 / 5 blocks per SM
+    k_sor_odd_seg(Geo g, Helm h, const __grid_constant__ SweepSet<T, CS> S, const double *__restrict__ P, int flg,
+                  int bc, int fuse, OddChain oc, int gx, int limit) {
+  __shared__ OddShared<T> sh;
+  __shared__ unsigned s_t, s_ep;
+  if (threadIdx.x == 0) {
+    s_t = atomicAdd(&oc.ctr[0], 1u);
+    s_ep = ld_acquire_u32(&oc.ctr[2]);
+  }
+  __syncthreads();
+  const unsigned t = s_t, epoch = s_ep;
+  const int nct = S.n * gx * g.ny;
+  const int seg = (int)(t / (unsigned)nct), ct = (int)(t - (unsigned)seg * nct);
+  const int q3 = ct / (gx * g.ny), tile = ct - q3 * gx * g.ny;
+  const int comp = S.id[q3];
+#define TPLS_SEG(CC)                                                                                              \
+  sor_odd_segment<T, CS, CC>(comp, g, h, S.x[q3], S.coef[q3], P, S.X[q3], flg, bc, fuse, oc, limit, t, epoch, nct, \
+                             seg, tile % gx, tile / gx + 1, sh)
+  TPLS_BY_COMP(TPLS_SEG);
+#undef TPLS_SEG
   if (threadIdx.x == 0) {  // the last block to leave resets the tickets and starts a new epoch
     __threadfence();
     if (atomicAdd(&oc.ctr[1], 1u) == gridDim.x - 1) {
@@ -574,11 +624,16 @@ __global__ void __launch_bounds__(SOC_W * 32, sizeof(T) == 4 ? 6 : 5)  // 40 / 4
   }
 }
 
-template <typename T, typename CS, int CC>
+template <typename T, typename CS>
 __global__ void __launch_bounds__(SOC_W * 32)
-    k_sor_odd_c4(int comp_, Geo g, Helm h, T *__restrict__ x, const CS coef,
-                 const double *__restrict__ P, const double *__restrict__ X, int flg, int bc, int fuse) {
-  sor_odd_c4_tile<T, CS, CC>(comp_, g, h, x, coef, P, X, flg, bc, fuse, blockIdx.x, blockIdx.y);
+    k_sor_odd_c4(Geo g, Helm h, const __grid_constant__ SweepSet<T, CS> S, const double *__restrict__ P, int gx,
+                 int flg, int bc, int fuse) {
+  __shared__ OddShared<T> sh;
+  const int q3 = blockIdx.x / gx, bx = blockIdx.x - q3 * gx, comp = S.id[q3];
+#define TPLS_COL(CC) \
+  sor_odd_c4_tile<T, CS, CC>(comp, g, h, S.x[q3], S.coef[q3], P, S.X[q3], flg, bc, fuse, bx, blockIdx.y, sh)
+  TPLS_BY_COMP(TPLS_COL);
+#undef TPLS_COL
 }
 
 // Multi-instance odd half-sweep of the FP32 sweeps of a batch: the tiles of
@@ -588,6 +643,7 @@ template <int CC>
 __global__ void __launch_bounds__(SOC_W * 32)
     k_odd_multi(const SweepMember *__restrict__ mem, const int *__restrict__ prefix, int n, int src, int flg,
                 int bc, unsigned *ctr) {
+  __shared__ OddShared<float> sh;
   __shared__ int s_t;
   const int total = prefix[n];
   for (;;) {
@@ -603,7 +659,7 @@ __global__ void __launch_bounds__(SOC_W * 32)
     const int gx = ((iend + 1) / 2 + 31) / 32;
     const int lt = t - prefix[m];
     sor_odd_c4_tile<float, MuCoef, CC>(CC, M.g, M.h, M.x[CC][src], M.s[CC], M.P, M.X[CC], flg, bc, M.fuse,
-                                       lt % gx, lt / gx);
+                                       lt % gx, lt / gx, sh);
   }
   if (threadIdx.x == 0) {
     __threadfence();
@@ -631,89 +687,106 @@ cudaError_t launch_odd_multi(int comp, const SweepMember *mem, const int *prefix
 
 cudaError_t sweep_init() { return cudaSuccess; }
 
-template <typename T, typename CS, int CC, int BX, int BY>
-static void jacobi_v(int comp, const Geo &g, const Helm &h, const T *xo, CS coef, const double *pres,
-                     const double *X, T *x, int fuse, cudaStream_t st) {
-  const int nk = (comp == 2) ? g.nz - 1 : g.nz;
-  const int iend = (comp == 0) ? g.nx - 1 : g.nx;
-  dim3 grd((iend + BX - 1) / BX, (g.ny + BY - 1) / BY, nk);
-  k_jacobi_c<T, CS, CC, BX, BY><<<grd, dim3(BX, BY), 0, st>>>(comp, g, h, xo, coef, pres, X, x, fuse);
-}
-
 // tile: the block shape (threads over i, or i pairs, by threads over j) the
 // autotuner chooses among for the Jacobi and even-SOR kernels: 0 = 32x4 (the
 // default), 1 = 32x8, 2 = 64x4, 3 = 16x8.
-template <typename T, typename CS, int CC>
-static cudaError_t jacobi_c(int comp, const Geo &g, const Phys &ph, const T *xo, CS coef, const double *pres,
-                            const double *X, T *x, int fuse, int tile, cudaStream_t st) {
+template <int BX, int BY>
+static void jacobi_v(const Geo &g, const Helm &h, const SweepSet64 &s, const double *pres, bool zero,
+                     cudaStream_t st) {
+  const int gx = (g.nx + BX - 1) / BX;
+  const dim3 grd(gx * s.n, (g.ny + BY - 1) / BY, g.nz), blk(BX, BY);
+  if (zero) k_jacobi_c<BX, BY, true><<<grd, blk, 0, st>>>(g, h, s, gx, pres);
+  else k_jacobi_c<BX, BY, false><<<grd, blk, 0, st>>>(g, h, s, gx, pres);
+}
+cudaError_t launch_jacobi_set(const Geo &g, const Phys &ph, const SweepSet64 &s, const double *pres, bool from_zero,
+                              cudaStream_t st, const SweepTiles &t) {
   const Helm h = helm_of(ph);
-  switch (tile) {
-    case 1: jacobi_v<T, CS, CC, 32, 8>(comp, g, h, xo, coef, pres, X, x, fuse, st); break;
-    case 2: jacobi_v<T, CS, CC, 64, 4>(comp, g, h, xo, coef, pres, X, x, fuse, st); break;
-    case 3: jacobi_v<T, CS, CC, 16, 8>(comp, g, h, xo, coef, pres, X, x, fuse, st); break;
-    default: jacobi_v<T, CS, CC, 32, 4>(comp, g, h, xo, coef, pres, X, x, fuse, st); break;
+  switch (t.jac) {
+    case 1: jacobi_v<32, 8>(g, h, s, pres, from_zero, st); break;
+    case 2: jacobi_v<64, 4>(g, h, s, pres, from_zero, st); break;
+    case 3: jacobi_v<16, 8>(g, h, s, pres, from_zero, st); break;
+    default: jacobi_v<32, 4>(g, h, s, pres, from_zero, st); break;
   }
   return cudaGetLastError();
 }
+cudaError_t launch_jacobi_set(const Geo &g, const Phys &ph, const SweepSet32 &s, const double *, bool, cudaStream_t st,
+                              const SweepTiles &t) {
+  return launch_sweep4(0, g, helm_of(ph), s, 0, 1, 1, t.jac, st);
+}
 
-template <typename T, typename CS, int CC, int BX, int BY>
-static void even_v(int comp, const Geo &g, const Helm &h, T *x, CS coef, const double *pres, const double *X,
-                   int flg, int bc, int fuse, cudaStream_t st) {
-  const int iend = (comp == 0) ? g.nx - 1 : g.nx;
-  const int npairs = (iend + 1) / 2;
-  const int nk = (comp == 2) ? g.nz - 1 : g.nz;
-  dim3 grd((npairs + BX - 1) / BX, (g.ny + BY - 1) / BY, nk);
-  k_sor_even_c<T, CS, CC, BX, BY><<<grd, dim3(BX, BY), 0, st>>>(comp, g, h, x, coef, pres, X, flg, bc, fuse);
+template <int BX, int BY>
+static void even_v(const Geo &g, const Helm &h, const SweepSet64 &s, const double *pres, int flg, int bc, int fuse,
+                   cudaStream_t st) {
+  const int gx = ((g.nx + 1) / 2 + BX - 1) / BX;
+  k_sor_even_c<BX, BY><<<dim3(gx * s.n, (g.ny + BY - 1) / BY, g.nz), dim3(BX, BY), 0, st>>>(g, h, s, gx, pres, flg,
+                                                                                          bc, fuse);
+}
+static cudaError_t even_set(const Geo &g, const Helm &h, const SweepSet64 &s, const double *pres, int flg, int bc,
+                            int fuse, int tile, cudaStream_t st) {
+  switch (tile) {
+    case 1: even_v<32, 8>(g, h, s, pres, flg, bc, fuse, st); break;
+    case 2: even_v<64, 4>(g, h, s, pres, flg, bc, fuse, st); break;
+    case 3: even_v<16, 8>(g, h, s, pres, flg, bc, fuse, st); break;
+    default: even_v<32, 4>(g, h, s, pres, flg, bc, fuse, st); break;
+  }
+  return cudaGetLastError();
+}
+// checkerboard half-sweep: four x points per thread (k_sweep32.cu)
+static cudaError_t even_set(const Geo &g, const Helm &h, const SweepSet32 &s, const double *, int flg, int bc,
+                            int fuse, int tile, cudaStream_t st) {
+  return launch_sweep4(1, g, h, s, flg, bc, fuse, tile, st);
 }
 
 int odd_chain_segments(const Geo &g) {
   const int gx = (((g.nx + 1) / 2) + 31) / 32;  // v and w have the most pairs
-  return ((g.nz - 1) / SOC_SC + 1) * gx * g.ny;
+  return 3 * ((g.nz - 1) / SOC_SC + 1) * gx * g.ny;
 }
 
-template <typename T, typename CS, int CC>
-static cudaError_t sor_c(int comp, const Geo &g, const Phys &ph, T *x, CS coef, const double *pres,
-                         const double *X, int flg, int iteration_time, int bc, int fuse, int tile_even,
-                         int tile_odd, cudaStream_t st, const OddChain *oc = nullptr) {
-  const int iend = (comp == 0) ? g.nx - 1 : g.nx;
-  const int npairs = (iend + 1) / 2;
-  const Helm h = helm_of(ph);
-  if (iteration_time % 2 == 0) {
-    switch (tile_even) {
-      case 1: even_v<T, CS, CC, 32, 8>(comp, g, h, x, coef, pres, X, flg, bc, fuse, st); break;
-      case 2: even_v<T, CS, CC, 64, 4>(comp, g, h, x, coef, pres, X, flg, bc, fuse, st); break;
-      case 3: even_v<T, CS, CC, 16, 8>(comp, g, h, x, coef, pres, X, flg, bc, fuse, st); break;
-      default: even_v<T, CS, CC, 32, 4>(comp, g, h, x, coef, pres, X, flg, bc, fuse, st); break;
-    }
-  } else {
-    (void)tile_odd;
-    const int gx = (npairs + 31) / 32;
-    const int k0 = (comp == 2) ? 1 : 0, nseg = (g.nz - 1 - k0) / SOC_SC + 1;
-    // one block per segment, chained, for columns of 3 or more segments:
-    // with 2, half the blocks wait on the other half for a larger share of
-    // their time than the extra blocks save (measured slower on the batched
-    // workload's grids, nz <= 128; faster at nz = 192 and 256)
-    if (oc && nseg >= 3 && oc->cap >= nseg * gx * g.ny) {
-      k_sor_odd_seg<T, CS, CC><<<nseg * gx * g.ny, SOC_W * 32, 0, st>>>(comp, g, h, x, coef, pres, X, flg, bc,
-                                                                       fuse, *oc, gx, 1 << 20);
-    } else {  // one block per 32 columns of a row, the column in super-chunks
-      dim3 grd(gx, g.ny, 1);
-      k_sor_odd_c4<T, CS, CC><<<grd, SOC_W * 32, 0, st>>>(comp, g, h, x, coef, pres, X, flg, bc, fuse);
-    }
+template <typename T, typename CS>
+static cudaError_t odd_set(const Geo &g, const Helm &h, const SweepSet<T, CS> &s, const double *pres, int flg, int bc,
+                           int fuse, cudaStream_t st, const OddChain *oc) {
+  const int gx = ((g.nx + 1) / 2 + 31) / 32, nseg = (g.nz - 1) / SOC_SC + 1;
+  const int blocks = nseg * s.n * gx * g.ny;
+  // one block per segment, chained, for columns of 3 or more segments: with
+  // 2, half the blocks wait on the other half for a larger share of their
+  // time than the extra blocks save (measured slower on the batched
+  // workload's grids, nz <= 128; faster at nz = 192 and 256)
+  if (oc && nseg >= 3 && oc->cap >= blocks) {
+    k_sor_odd_seg<T, CS><<<blocks, SOC_W * 32, 0, st>>>(g, h, s, pres, flg, bc, fuse, *oc, gx, 1 << 20);
+  } else {  // one block per 32 columns of a row, the column in super-chunks
+    k_sor_odd_c4<T, CS><<<dim3(gx * s.n, g.ny), SOC_W * 32, 0, st>>>(g, h, s, pres, gx, flg, bc, fuse);
   }
   return cudaGetLastError();
+}
+
+cudaError_t launch_sor_set(const Geo &g, const Phys &ph, const SweepSet64 &s, const double *pres, int flg,
+                           int iteration_time, int bc, int fuse_ghosts, cudaStream_t st, const SweepTiles &t,
+                           const OddChain *oc) {
+  if (iteration_time % 2 == 0) return even_set(g, helm_of(ph), s, pres, flg, bc, fuse_ghosts, t.even, st);
+  return odd_set(g, helm_of(ph), s, pres, flg, bc, fuse_ghosts, st, oc);
+}
+cudaError_t launch_sor_set(const Geo &g, const Phys &ph, const SweepSet32 &s, const double *pres, int flg,
+                           int iteration_time, int bc, int fuse_ghosts, cudaStream_t st, const SweepTiles &t,
+                           const OddChain *oc) {
+  if (iteration_time % 2 == 0) return even_set(g, helm_of(ph), s, pres, flg, bc, fuse_ghosts, t.even, st);
+  return odd_set(g, helm_of(ph), s, pres, flg, bc, fuse_ghosts, st, oc);
 }
 
 cudaError_t launch_sor_ref_odd(int comp, const Geo &g, const Phys &ph, double *x, const double *rhs,
                                const double *mu, int flg, cudaStream_t st, const OddChain *oc) {
   const Helm h = helm_of(ph);
+  SweepSet<double, RefCoef> s;
+  s.n = 1;
+  s.id[0] = comp;
+  s.x[0] = x;
   RefCoef r;
   r.mu = mu;
   r.rhs = rhs;
   r.ax2 = h.ax2;
   r.ay2 = h.ay2;
   r.az2 = h.az2;
-  return sor_c<double, RefCoef, -1>(comp, g, ph, x, r, nullptr, nullptr, flg, 1, 0, 0, 0, 0, st, oc);
+  s.coef[0] = r;
+  return odd_set(g, h, s, nullptr, flg, 0, 0, st, oc);
 }
 
 MuCoef mu_coef(const Phys &ph, const float *mu, const float *b, const float4 *bco) {
@@ -726,33 +799,6 @@ MuCoef mu_coef(const Phys &ph, const float *mu, const float *b, const float4 *bc
   m.ay2 = (float)h.ay2;
   m.az2 = (float)h.az2;
   return m;
-}
-
-cudaError_t launch_jacobi_c(int comp, const Geo &g, const Phys &ph, const double *xo, const double *coef,
-                            const double *pres, double *x, int fuse, cudaStream_t st, const SweepTiles &t) {
-  return jacobi_c<double, const double *, -1>(comp, g, ph, xo, coef, pres, nullptr, x, fuse, t.jac, st);
-}
-cudaError_t launch_jacobi_c(int comp, const Geo &g, const Phys &ph, const float *xo, const MuCoef &coef,
-                            const double *pres, const double *X, float *x, int fuse, cudaStream_t st,
-                            const SweepTiles &t) {
-  return launch_sweep4(0, comp, g, helm_of(ph), xo, x, coef, pres, X, 0, 1, fuse, t.jac, st);
-}
-cudaError_t launch_sor_c(int comp, const Geo &g, const Phys &ph, double *x, const double *coef,
-                         const double *pres, int flg, int iteration_time, int bc, int fuse, cudaStream_t st,
-                         const SweepTiles &t, const OddChain *oc) {
-  return sor_c<double, const double *, -1>(comp, g, ph, x, coef, pres, nullptr, flg, iteration_time, bc, fuse, t.even,
-                                          t.odd, st, oc);
-}
-cudaError_t launch_sor_c(int comp, const Geo &g, const Phys &ph, float *x, const MuCoef &coef,
-                         const double *pres, const double *X, int flg, int iteration_time, int bc, int fuse,
-                         cudaStream_t st, const SweepTiles &t, const OddChain *oc) {
-  if (iteration_time % 2 == 0)  // checkerboard half-sweep: four x points per thread (k_sweep32.cu)
-    return launch_sweep4(1, comp, g, helm_of(ph), x, x, coef, pres, X, flg, bc, fuse, t.even, st);
-  if (comp == 0)
-    return sor_c<float, MuCoef, 0>(comp, g, ph, x, coef, pres, X, flg, iteration_time, bc, fuse, t.even, t.odd, st, oc);
-  if (comp == 1)
-    return sor_c<float, MuCoef, 1>(comp, g, ph, x, coef, pres, X, flg, iteration_time, bc, fuse, t.even, t.odd, st, oc);
-  return sor_c<float, MuCoef, 2>(comp, g, ph, x, coef, pres, X, flg, iteration_time, bc, fuse, t.even, t.odd, st, oc);
 }
 
 // defect form: d = -X before the first sweep (the sweeps start from x = 0),

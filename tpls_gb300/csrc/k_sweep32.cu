@@ -24,6 +24,8 @@
 // outlet and fictitious point) add a per-row offset that is constant for the
 // whole momentum solve, computed once per component and step
 // (launch_bc32_prep).
+#include <type_traits>
+
 #include "tpls_sweep.cuh"
 
 namespace tpls {
@@ -221,17 +223,22 @@ __device__ __forceinline__ void sweep4_tile(const Geo &g, const Helm &h, const f
   load_b(g, s.b, q, i0, iend, j, k, par, act, bv);
   halo<true, true>(cc, ol, orr);
   halo_mu<CC>(m, ol, orr);
-  Faces f;
-  faces4<CC>(m, f);
   // per-axis scale: dt/(2 d^2), and a quarter of it for the averaged faces
   const float cx = (CC == 0) ? s.ax2 : 0.25f * s.ax2;
   const float cy = (CC == 1) ? s.ay2 : 0.25f * s.ay2;
   const float cz = (CC == 2) ? s.az2 : 0.25f * s.az2;
   float out[4] = {cc.v.x, cc.v.y, cc.v.z, cc.v.w};
+  // the points of x parity PAR (-1: all four); a half-sweep's parity is the
+  // same for the whole warp, so each parity has its own code and the faces of
+  // the other colour's points are not formed
+  auto relax = [&](auto parity) {
+    constexpr int PAR = decltype(parity)::value;
+    Faces f;
+    faces4<CC>(m, f);
 #pragma unroll
-  for (int e = 0; e < 4; e++) {
-    const bool upd = act && (i0 + e <= iend) && (MODE == M_JAC || (e & 1) == par);
-    if (upd) {
+    for (int e = 0; e < 4; e++) {
+      if (PAR >= 0 && (e & 1) != PAR) continue;
+      if (!act || i0 + e > iend) continue;
       const float xc = el(cc, e);
       float zpv = el(zp, e), zmv = el(zm, e);
       if (CC != 2) {  // no-slip ghost value -2 x(0) + x(1)/3 below k = 0 and above k = nz-1
@@ -249,7 +256,10 @@ __device__ __forceinline__ void sweep4_tile(const Geo &g, const Helm &h, const f
       const float v = fmaf(r, t, bv[e]);
       out[e] = (MODE == M_JAC) ? v : xc + 1.2f * (v - xc);
     }
-  }
+  };
+  if (MODE == M_JAC) relax(std::integral_constant<int, -1>{});
+  else if (par) relax(std::integral_constant<int, 1>{});
+  else relax(std::integral_constant<int, 0>{});
   // store: whole groups as one 16-byte store (in the half-sweep the other
   // colour's values are rewritten unchanged: nothing else writes them in
   // this launch), ragged ends point by point
@@ -296,11 +306,22 @@ __device__ __forceinline__ void sweep4_tile(const Geo &g, const Helm &h, const f
   }
 }
 
-template <int CC, int MODE, int BY>
-__global__ void __launch_bounds__(32 * BY)
-    k_sweep4(Geo g, Helm h, const float *__restrict__ xo, float *x, MuCoef s, const double *__restrict__ X,
-             int flg, int bc, int fuse) {
-  sweep4_tile<CC, MODE, BY>(g, h, xo, x, s, X, flg, bc, fuse, blockIdx.x, blockIdx.y, blockIdx.z);
+// gx: blocks along x per component; block column q * gx + bx runs tile bx of
+// the set's q-th component.
+// Registers: 56 for Jacobi (36 warps per SM), 64 for the half-sweep (32);
+// unbounded the compiler takes 80 and 24 warps do not cover the loads'
+// latency.
+template <int MODE, int BY>
+__global__ void __launch_bounds__(32 * BY, (MODE == M_JAC ? 36 : 32) / BY)
+    k_sweep4(Geo g, Helm h, const __grid_constant__ SweepSet32 s, int gx, int flg, int bc, int fuse) {
+  const int q = blockIdx.x / gx, bx = blockIdx.x - q * gx, comp = s.id[q];
+  if (comp == 0) {
+    sweep4_tile<0, MODE, BY>(g, h, s.xo[q], s.x[q], s.coef[q], s.X[q], flg, bc, fuse, bx, blockIdx.y, blockIdx.z);
+  } else if (comp == 1) {
+    sweep4_tile<1, MODE, BY>(g, h, s.xo[q], s.x[q], s.coef[q], s.X[q], flg, bc, fuse, bx, blockIdx.y, blockIdx.z);
+  } else if ((int)blockIdx.z < g.nz - 1) {
+    sweep4_tile<2, MODE, BY>(g, h, s.xo[q], s.x[q], s.coef[q], s.X[q], flg, bc, fuse, bx, blockIdx.y, blockIdx.z);
+  }
 }
 
 // tiles of the single-instance grid of component CC (4 rows per block)
@@ -349,35 +370,24 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-template <int CC, int MODE, int BY>
-cudaError_t launch4(const Geo &g, const Helm &h, const float *xo, float *x, const MuCoef &s, const double *X,
-                    int flg, int bc, int fuse, cudaStream_t st) {
-  const int iend = (CC == 0) ? g.nx - 1 : g.nx;
-  const int G = (iend + 3) / 4;
-  const int nk = (CC == 2) ? g.nz - 1 : g.nz;
-  dim3 grd((G + 31) / 32, (g.ny + BY - 1) / BY, nk);
-  k_sweep4<CC, MODE, BY><<<grd, dim3(32, BY), 0, st>>>(g, h, xo, x, s, X, flg, bc, fuse);
+template <int MODE, int BY>
+cudaError_t launch4(const Geo &g, const Helm &h, const SweepSet32 &s, int flg, int bc, int fuse, cudaStream_t st) {
+  const int gx = ((g.nx + 3) / 4 + 31) / 32;
+  dim3 grd(gx * s.n, (g.ny + BY - 1) / BY, g.nz);
+  k_sweep4<MODE, BY><<<grd, dim3(32, BY), 0, st>>>(g, h, s, gx, flg, bc, fuse);
   return cudaGetLastError();
 }
 
 // tile: rows per block (0: 4, 1: 8, 2: 2, 3: 1)
-template <int CC, int MODE>
-cudaError_t launch4_t(int tile, const Geo &g, const Helm &h, const float *xo, float *x, const MuCoef &s,
-                      const double *X, int flg, int bc, int fuse, cudaStream_t st) {
-  switch (tile) {
-    case 1: return launch4<CC, MODE, 8>(g, h, xo, x, s, X, flg, bc, fuse, st);
-    case 2: return launch4<CC, MODE, 2>(g, h, xo, x, s, X, flg, bc, fuse, st);
-    case 3: return launch4<CC, MODE, 1>(g, h, xo, x, s, X, flg, bc, fuse, st);
-    default: return launch4<CC, MODE, 4>(g, h, xo, x, s, X, flg, bc, fuse, st);
-  }
-}
-
 template <int MODE>
-cudaError_t by_comp(int comp, int tile, const Geo &g, const Helm &h, const float *xo, float *x, const MuCoef &s,
-                    const double *X, int flg, int bc, int fuse, cudaStream_t st) {
-  if (comp == 0) return launch4_t<0, MODE>(tile, g, h, xo, x, s, X, flg, bc, fuse, st);
-  if (comp == 1) return launch4_t<1, MODE>(tile, g, h, xo, x, s, X, flg, bc, fuse, st);
-  return launch4_t<2, MODE>(tile, g, h, xo, x, s, X, flg, bc, fuse, st);
+cudaError_t launch4_t(int tile, const Geo &g, const Helm &h, const SweepSet32 &s, int flg, int bc, int fuse,
+                      cudaStream_t st) {
+  switch (tile) {
+    case 1: return launch4<MODE, 8>(g, h, s, flg, bc, fuse, st);
+    case 2: return launch4<MODE, 2>(g, h, s, flg, bc, fuse, st);
+    case 3: return launch4<MODE, 1>(g, h, s, flg, bc, fuse, st);
+    default: return launch4<MODE, 4>(g, h, s, flg, bc, fuse, st);
+  }
 }
 
 // one thread per (j, k) row of the component
@@ -401,11 +411,10 @@ __global__ void k_bc32_prep(int comp, Geo g, Helm h, const double *__restrict__ 
 
 }  // namespace
 
-cudaError_t launch_sweep4(int mode, int comp, const Geo &g, const Helm &h, const float *xo, float *x,
-                          const MuCoef &s, const double *, const double *X, int flg, int bc, int fuse, int tile,
-                          cudaStream_t st) {
-  if (mode == M_JAC) return by_comp<M_JAC>(comp, tile, g, h, xo, x, s, X, flg, bc, fuse, st);
-  return by_comp<M_EVEN>(comp, tile, g, h, xo, x, s, X, flg, bc, fuse, st);
+cudaError_t launch_sweep4(int mode, const Geo &g, const Helm &h, const SweepSet32 &s, int flg, int bc, int fuse,
+                          int tile, cudaStream_t st) {
+  if (mode == M_JAC) return launch4_t<M_JAC>(tile, g, h, s, flg, bc, fuse, st);
+  return launch4_t<M_EVEN>(tile, g, h, s, flg, bc, fuse, st);
 }
 
 int sweep4_tiles(int comp, const Geo &g) {

@@ -1011,9 +1011,6 @@ static const double *mom32_base(tpls_ctx *c, int comp) { return comp == 0 ? c->u
 static size_t mom32_len(tpls_ctx *c, int comp) {
   return (size_t)c->px * (c->ny + 2) * nz_planes(comp == 2 ? 2 : 1, c->nz) + 8;
 }
-static int mom32_iters(tpls_ctx *c, int comp) {
-  return (comp == 0 ? c->prm.mom_u : (comp == 1 ? c->prm.mom_v : c->prm.mom_w)) / 2;
-}
 static int mom32_begin(tpls_ctx *c, int comp) {
   const double *base = mom32_base(c, comp);
   LCK(c, launch_defect_init(base - XOFF, c->x3f[comp][0] - XOFF, mom32_len(c, comp), c->st));
@@ -1035,63 +1032,65 @@ static int mom32_end(tpls_ctx *c, int comp, int N) {
   return TPLS_OK;
 }
 
-// One velocity component's Crank-Nicolson solve (main_ns_hybrid.F90:756-887)
-// on the iterate pair X: FP64, or in the FP32-mixed form the FP32 defect
-// d = x - base (base = the component's FP64 state), iterated from d = -base
-// (x = 0, the reference's start) and added back into out64 at the end.
+static int mom_iters(const tpls_ctx *c, int comp) {
+  return (comp == 0 ? c->prm.mom_u : (comp == 1 ? c->prm.mom_v : c->prm.mom_w)) / 2;
+}
+// The sweeps of the three components' Crank-Nicolson solves (main_ns_hybrid.
+// F90:756-887), which are independent of one another, in common launches:
+// iteration it of every component that has one.  X: the iterate pairs; FP64,
+// or in the FP32-mixed form the FP32 defects.
 template <typename T, typename CS>
-static int momentum(tpls_ctx *c, int comp, CS coef, T **X, int max_iteration, const double *base = nullptr,
-                    double *out64 = nullptr) {
+static int momentum_sweeps(tpls_ctx *c, const CS (&coef)[3], T *(&X)[3][2]) {
   const Geo &g = c->g;
-  const int nzp = nz_planes(comp == 2 ? 2 : 1, c->nz);
   const int fuse = (g.ny % 2 == 0);
-  const size_t n = (size_t)c->px * (c->ny + 2) * nzp + 8;
-  if constexpr (sizeof(T) == sizeof(float)) {
-    int s = mom32_begin(c, comp);
-    if (s) return s;
-  } else {
-    TCK(cudaMemsetAsync(X[0] - XOFF, 0, sizeof(T) * n, c->st));
-  }
-  const SweepTiles tl = c->tiles;
-  auto jac = [&](const T *src, T *dst) {
-    if constexpr (sizeof(T) == sizeof(float)) return launch_jacobi_c(comp, g, c->ph, src, coef, c->pres, base, dst,
-                                                                      fuse, c->st, tl);
-    else return launch_jacobi_c(comp, g, c->ph, src, coef, c->pres, dst, fuse, c->st, tl);
-  };
-  auto sor = [&](T *x, int flg, int it, int bc) {
-    if constexpr (sizeof(T) == sizeof(float)) return launch_sor_c(comp, g, c->ph, x, coef, c->pres, base, flg, it,
-                                                                   bc, fuse, c->st, tl, odd_chain(c));
-    else return launch_sor_c(comp, g, c->ph, x, coef, c->pres, flg, it, bc, fuse, c->st, tl, odd_chain(c));
-  };
-  const int N = max_iteration / 2;
-  for (int it = 1; it <= N; it++) {
-    T *src = X[(it - 1) % 2], *dst = X[it % 2];
+  int last = 0;
+  for (int q = 0; q < 3; q++) last = mom_iters(c, q) > last ? mom_iters(c, q) : last;
+  for (int it = 1; it <= last; it++) {
+    SweepSet<T, CS> s;
+    int nzp[3];
+    for (int q = 0; q < 3; q++) {
+      if (it > mom_iters(c, q)) continue;
+      nzp[s.n] = nz_planes(q == 2 ? 2 : 1, c->nz);
+      s.id[s.n] = q;
+      s.xo[s.n] = X[q][(it - 1) % 2];
+      s.x[s.n] = X[q][it % 2];
+      s.coef[s.n] = coef[q];
+      s.X[s.n] = mom32_base(c, q);
+      s.n++;
+    }
     {
       PhaseScope ps(c, TPLS_T_JACOBI);
-      LCK(c, jac(src, dst));
+      LCK(c, launch_jacobi_set(g, c->ph, s, c->pres, it == 1 && sizeof(T) == sizeof(double), c->st, c->tiles));
     }
-    if (!fuse) LCK(c, launch_exchange(g, dst, nzp, c->st));
-    {
-      PhaseScope ps(c, (it % 2) ? TPLS_T_SOR_ODD : TPLS_T_SOR);
-      LCK(c, sor(dst, 0, it, 0));
+    for (int flg = 0; flg < 2; flg++) {
+      {
+        PhaseScope ps(c, (it % 2) ? TPLS_T_SOR_ODD : TPLS_T_SOR);
+        LCK(c, launch_sor_set(g, c->ph, s, c->pres, flg, it, flg, fuse, c->st, c->tiles, odd_chain(c)));
+      }
+      if (!fuse) LCK(c, launch_exchange_set(g, s.n, s.x, nzp, c->st));
     }
-    if (!fuse) LCK(c, launch_exchange(g, dst, nzp, c->st));
-    {
-      PhaseScope ps(c, (it % 2) ? TPLS_T_SOR_ODD : TPLS_T_SOR);
-      LCK(c, sor(dst, 1, it, 1));
-    }
-    if (!fuse) LCK(c, launch_exchange(g, dst, nzp, c->st));
   }
-  if constexpr (sizeof(T) == sizeof(float)) {
-    return mom32_end(c, comp, N);
-  }
-  c->x3_final[comp] = N % 2;
-  const int nb = diff2_blocks(g, nzp);
-  if (N >= 1) {
-    LCK(c, launch_diff2(g, X[N % 2], X[(N - 1) % 2], nzp, c->part, c->st));
-    FSUM(c, c->part, nb, c->scal + SC_ERR_U + comp, c->st);
-  } else {
-    TCK(cudaMemsetAsync(c->scal + SC_ERR_U + comp, 0, sizeof(double), c->st));
+  return TPLS_OK;
+}
+
+// The FP64 solves, from the reference's start x = 0.
+static int momentum64(tpls_ctx *c) {
+  const double *const coef[3] = {c->coef[0], c->coef[1], c->coef[2]};
+  int s = momentum_sweeps<double, const double *>(c, coef, c->x3);
+  if (s) return s;
+  for (int q = 0; q < 3; q++) {
+    const int N = mom_iters(c, q), nzp = nz_planes(q == 2 ? 2 : 1, c->nz);
+    double **X = c->x3[q];
+    c->x3_final[q] = N % 2;
+    if (N >= 1) {
+      // one sweep: the iterate before it is the start, which no launch wrote
+      if (N == 1) TCK(cudaMemsetAsync(X[0] - XOFF, 0, sizeof(double) * ((size_t)c->px * (c->ny + 2) * nzp + 8), c->st));
+      LCK(c, launch_diff2(c->g, X[N % 2], X[(N - 1) % 2], nzp, c->part, c->st));
+      FSUM(c, c->part, diff2_blocks(c->g, nzp), c->scal + SC_ERR_U + q, c->st);
+    } else {
+      TCK(cudaMemsetAsync(X[0] - XOFF, 0, sizeof(double) * ((size_t)c->px * (c->ny + 2) * nzp + 8), c->st));
+      TCK(cudaMemsetAsync(c->scal + SC_ERR_U + q, 0, sizeof(double), c->st));
+    }
   }
   return TPLS_OK;
 }
@@ -1240,9 +1239,7 @@ static int step_back(tpls_ctx *c) {
   cudaStream_t st = c->st;
   // momentum sweeps (:756-887)
   int s;
-  if ((s = momentum<double, const double *>(c, 0, c->coef[0], c->x3[0], c->prm.mom_u))) return s;
-  if ((s = momentum<double, const double *>(c, 1, c->coef[1], c->x3[1], c->prm.mom_v))) return s;
-  if ((s = momentum<double, const double *>(c, 2, c->coef[2], c->x3[2], c->prm.mom_w))) return s;
+  if ((s = momentum64(c))) return s;
   double *u3 = c->x3[0][c->x3_final[0]], *v3 = c->x3[1][c->x3_final[1]], *w3 = c->x3[2][c->x3_final[2]];
   // pressure source (:892) and solve (:897-913)
   int its = 0, reason = 0;
@@ -1279,14 +1276,14 @@ static int step_once(tpls_ctx *c) {
 // FP64 results in x3[q][0]
 static int sweeps32(tpls_ctx *c) {
   int s;
-  const Phys &ph = c->ph;
-  if ((s = momentum<float>(c, 0, mu_coef(ph, c->mu32, c->bdef[0], c->bco32[0]), c->x3f[0], c->prm.mom_u, c->u2, c->x3[0][0])))
-    return s;
-  if ((s = momentum<float>(c, 1, mu_coef(ph, c->mu32, c->bdef[1], c->bco32[1]), c->x3f[1], c->prm.mom_v, c->v2, c->x3[1][0])))
-    return s;
-  if ((s = momentum<float>(c, 2, mu_coef(ph, c->mu32, c->bdef[2], c->bco32[2]), c->x3f[2], c->prm.mom_w, c->w2, c->x3[2][0])))
-    return s;
-  for (int q = 0; q < 3; q++) c->x3_final[q] = 0;
+  MuCoef coef[3];
+  for (int q = 0; q < 3; q++) {
+    coef[q] = mu_coef(c->ph, c->mu32, c->bdef[q], c->bco32[q]);
+    if ((s = mom32_begin(c, q))) return s;
+  }
+  if ((s = momentum_sweeps<float, MuCoef>(c, coef, c->x3f))) return s;
+  for (int q = 0; q < 3; q++)
+    if ((s = mom32_end(c, q, mom_iters(c, q)))) return s;
   return TPLS_OK;
 }
 
@@ -1371,9 +1368,7 @@ static int mixed_front(tpls_ctx *c) {
                             c->csf_w[s1], c->csf_w[s0], c->conv_w[s2], c->csf_w[s2], nullptr, nullptr, c->coef[2],
                             st));
     }
-    if ((s = momentum<double, const double *>(c, 0, c->coef[0], c->x3[0], c->prm.mom_u))) return s;
-    if ((s = momentum<double, const double *>(c, 1, c->coef[1], c->x3[1], c->prm.mom_v))) return s;
-    if ((s = momentum<double, const double *>(c, 2, c->coef[2], c->x3[2], c->prm.mom_w))) return s;
+    if ((s = momentum64(c))) return s;
   } else if (sten64) {
     {
       PhaseScope ps(c, TPLS_T_CSF);
@@ -1562,8 +1557,7 @@ int tpls_step_async(tpls_ctx *c, int nsteps) {
 // ---------------------------------------------------------------------------
 // Tile-shape autotuner of the momentum sweeps: each candidate block shape of
 // the Jacobi and even half-sweep kernels is timed with CUDA events on the
-// context's own records and iterate arrays (reps launches of the u
-// component), the fastest kept.  Results are cached per (grid, sweep
+// context's own records and iterate arrays (reps launches), the fastest kept.  Results are cached per (grid, sweep
 // precision) for the process, so batch members of one shape tune once.
 }  // extern "C"
 
@@ -1609,16 +1603,28 @@ int tpls_autotune(tpls_ctx *c, int reps) {
   TCK(cudaEventCreate(&e0));
   TCK(cudaEventCreate(&e1));
   auto launch = [&](int kind, const SweepTiles &t) -> cudaError_t {
-    // kind 0: Jacobi, 1: even half-sweep, 2: odd half-sweep (component u)
+    // kind 0: Jacobi, 1: even half-sweep, of the three components
     if (f32) {
-      float *a = c->x3f[0][0], *b = c->x3f[0][1];
-      const MuCoef mc = mu_coef(c->ph, c->mu32, c->bdef[0], c->bco32[0]);
-      if (kind == 0) return launch_jacobi_c(0, g, c->ph, a, mc, c->pres, c->u2, b, fuse, c->st, t);
-      return launch_sor_c(0, g, c->ph, b, mc, c->pres, c->u2, 0, kind == 1 ? 2 : 1, 1, fuse, c->st, t);
+      SweepSet32 w;
+      for (w.n = 0; w.n < 3; w.n++) {
+        w.id[w.n] = w.n;
+        w.xo[w.n] = c->x3f[w.n][0];
+        w.x[w.n] = c->x3f[w.n][1];
+        w.coef[w.n] = mu_coef(c->ph, c->mu32, c->bdef[w.n], c->bco32[w.n]);
+        w.X[w.n] = mom32_base(c, w.n);
+      }
+      if (kind == 0) return launch_jacobi_set(g, c->ph, w, c->pres, false, c->st, t);
+      return launch_sor_set(g, c->ph, w, c->pres, 0, 2, 1, fuse, c->st, t);
     }
-    double *a = c->x3[0][0], *b = c->x3[0][1];
-    if (kind == 0) return launch_jacobi_c(0, g, c->ph, a, c->coef[0], c->pres, b, fuse, c->st, t);
-    return launch_sor_c(0, g, c->ph, b, c->coef[0], c->pres, 0, kind == 1 ? 2 : 1, 1, fuse, c->st, t, odd_chain(c));
+    SweepSet64 w;
+    for (w.n = 0; w.n < 3; w.n++) {
+      w.id[w.n] = w.n;
+      w.xo[w.n] = c->x3[w.n][0];
+      w.x[w.n] = c->x3[w.n][1];
+      w.coef[w.n] = c->coef[w.n];
+    }
+    if (kind == 0) return launch_jacobi_set(g, c->ph, w, c->pres, false, c->st, t);
+    return launch_sor_set(g, c->ph, w, c->pres, 0, 2, 1, fuse, c->st, t);
   };
   SweepTiles best = c->tiles;
   // The odd half-sweep's chunking changes its rounding, so it is not tuned:
@@ -1756,7 +1762,7 @@ int tpls_batch_create(tpls_ctx *const *ctxs, int n, tpls_batch **out) {
 static int batch_multi_sweeps(tpls_batch *b) {
   const int n = (int)b->m.size();
   for (int comp = 0; comp < 3; comp++) {
-    const int N = mom32_iters(b->m[0], comp);
+    const int N = mom_iters(b->m[0], comp);
     const int *pf0 = b->dprefix + (0 * 3 + comp) * (n + 1), *pf1 = b->dprefix + (1 * 3 + comp) * (n + 1);
     for (int it = 1; it <= N; it++) {
       const int src = (it - 1) % 2, dst = it % 2;
@@ -1806,7 +1812,7 @@ static int batch_capture(tpls_batch *b, int ph) {
       e = cudaStreamWaitEvent(c->st, b->fork2, 0);
       if (e != cudaSuccess) break;
       c->capturing = true;
-      for (int comp = 0; comp < 3 && s == TPLS_OK; comp++) s = mom32_end(c, comp, mom32_iters(c, comp));
+      for (int comp = 0; comp < 3 && s == TPLS_OK; comp++) s = mom32_end(c, comp, mom_iters(c, comp));
       if (s == TPLS_OK) s = mixed_back(c);
       c->capturing = false;
       if (s == TPLS_OK) e = cudaEventRecord(b->join[q], c->st);
@@ -1839,7 +1845,7 @@ int tpls_batch_multi_sweeps(tpls_batch *b, int on) {
     for (tpls_ctx *c : b->m) {
       if (!c->mixed || !mixed_fp32_sweeps(c) || c->ny % 2 != 0) return TPLS_ERR_ARG;
       for (int comp = 0; comp < 3; comp++)
-        if (mom32_iters(c, comp) != mom32_iters(b->m[0], comp)) return TPLS_ERR_ARG;
+        if (mom_iters(c, comp) != mom_iters(b->m[0], comp)) return TPLS_ERR_ARG;
     }
     TCK(cudaGetDevice(&dev0));
     if (!b->dmem) {

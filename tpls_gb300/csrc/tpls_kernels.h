@@ -30,7 +30,9 @@ cudaError_t launch_advect(const Geo &g, const Phys &ph, const double *phi2,
 // exchange2d (mpi.f90:110) on one GPU: periodic copy of rows 0 and ny+1,
 // x = 0..nx+1, nzp planes.
 cudaError_t launch_exchange(const Geo &g, double *a, int nzp, cudaStream_t st);
-cudaError_t launch_exchange(const Geo &g, float *a, int nzp, cudaStream_t st);
+// The same for n arrays a[q] of nzp[q] planes in one launch.
+template <typename T>
+cudaError_t launch_exchange_set(const Geo &g, int n, T *const *a, const int *nzp, cudaStream_t st);
 // FP32-mixed form: WENO5 faces and flux divergence in FP32 on FP32 copies
 // of phi, u, v, w; conv2_phi written in FP64.
 cudaError_t launch_advect(const Geo &g, const Phys &ph, const float *phi2,
@@ -166,7 +168,7 @@ struct OddChain {
   double *kto = nullptr;     // waits that ran out (a context scalar)
   int cap = 0;               // segments the arrays hold
 };
-// Segments of the largest component's odd half-sweep on grid g.
+// Segments of the three components' odd half-sweeps on grid g.
 int odd_chain_segments(const Geo &g);
 
 // Coefficient source of the per-routine sweep entries: the FP64
@@ -182,20 +184,6 @@ struct RefCoef {
 cudaError_t launch_sor_ref_odd(int comp, const Geo &g, const Phys &ph, double *x, const double *rhs,
                                const double *mu, int flg, cudaStream_t st, const OddChain *oc);
 
-// Sweeps on the per-point coefficient records written by launch_mom_rhs
-// (coef != null there): same updates and boundary rows as launch_jacobi /
-// launch_sor with bc = 1.
-cudaError_t launch_jacobi_c(int comp, const Geo &g, const Phys &ph,
-                            const double *xo, const double *coef,
-                            const double *pres, double *x, int fuse_ghosts,
-                            cudaStream_t st, const SweepTiles &t = SweepTiles());
-// oc: the context's segment-chained odd half-sweep state (null: one block
-// walks each column, the same results).
-cudaError_t launch_sor_c(int comp, const Geo &g, const Phys &ph, double *x,
-                         const double *coef, const double *pres, int flg,
-                         int iteration_time, int bc, int fuse_ghosts,
-                         cudaStream_t st, const SweepTiles &t = SweepTiles(),
-                         const OddChain *oc = nullptr);
 // FP32 sweeps in defect form: x holds d = x - X for the FP64 base X (the
 // component's state).  Their coefficients are recomputed per point from the
 // FP32 viscosity field (face averages and Helmholtz diagonal: a few dozen
@@ -219,17 +207,40 @@ MuCoef mu_coef(const Phys &ph, const float *mu, const float *b, const float4 *bc
 // d(nx) + (X(nx) - X(nx+1)).  Differences taken from FP32 pairs.
 cudaError_t launch_bc32_prep(int comp, const Geo &g, const Phys &ph, const double *X, const double *P,
                              float4 *bco, cudaStream_t st);
-cudaError_t launch_jacobi_c(int comp, const Geo &g, const Phys &ph,
-                            const float *xo, const MuCoef &coef,
-                            const double *pres, const double *X, float *x,
-                            int fuse_ghosts, cudaStream_t st,
-                            const SweepTiles &t = SweepTiles());
-cudaError_t launch_sor_c(int comp, const Geo &g, const Phys &ph, float *x,
-                         const MuCoef &coef, const double *pres,
-                         const double *X, int flg, int iteration_time, int bc,
-                         int fuse_ghosts, cudaStream_t st,
-                         const SweepTiles &t = SweepTiles(),
-                         const OddChain *oc = nullptr);
+// The components one sweep launch runs: u, v and w solve independent systems
+// (each reads its own iterate, the pressure and coefficients fixed before the
+// sweeps), so a sweep of all three is one launch.  n entries; id: the
+// component (0 u, 1 v, 2 w); xo -> x (Jacobi) or x in place (half-sweeps);
+// CS: the coefficient records of launch_mom_rhs (double) or MuCoef (float);
+// X: the FP64 base of the float defect iterates.
+template <typename T, typename CS>
+struct SweepSet {
+  int n = 0;
+  int id[3] = {0, 0, 0};
+  const T *xo[3] = {nullptr, nullptr, nullptr};
+  T *x[3] = {nullptr, nullptr, nullptr};
+  CS coef[3];
+  const double *X[3] = {nullptr, nullptr, nullptr};
+};
+using SweepSet64 = SweepSet<double, const double *>;
+using SweepSet32 = SweepSet<float, MuCoef>;
+// Jacobi sweep with its boundary rows; from_zero: xo is zero and not read
+// (the reference's start), FP64 sets only.  Ghost rows are always written:
+// the sweep is out of place.
+cudaError_t launch_jacobi_set(const Geo &g, const Phys &ph, const SweepSet64 &s, const double *pres, bool from_zero,
+                              cudaStream_t st, const SweepTiles &t = SweepTiles());
+cudaError_t launch_jacobi_set(const Geo &g, const Phys &ph, const SweepSet32 &s, const double *pres, bool from_zero,
+                              cudaStream_t st, const SweepTiles &t = SweepTiles());
+// Half-sweep flg of iteration_time; bc: with the boundary rows; fuse_ghosts:
+// ghost rows written by the sweep (even ny).  oc: the context's state of the
+// segment-chained odd half-sweep (null: one block walks each column, the same
+// results).
+cudaError_t launch_sor_set(const Geo &g, const Phys &ph, const SweepSet64 &s, const double *pres, int flg,
+                           int iteration_time, int bc, int fuse_ghosts, cudaStream_t st,
+                           const SweepTiles &t = SweepTiles(), const OddChain *oc = nullptr);
+cudaError_t launch_sor_set(const Geo &g, const Phys &ph, const SweepSet32 &s, const double *pres, int flg,
+                           int iteration_time, int bc, int fuse_ghosts, cudaStream_t st,
+                           const SweepTiles &t = SweepTiles(), const OddChain *oc = nullptr);
 // d = -X (n elements) / x = X + d
 cudaError_t launch_defect_init(const double *X, float *d, size_t n, cudaStream_t st);
 cudaError_t launch_defect_apply(const double *X, const float *d, double *x, size_t n,

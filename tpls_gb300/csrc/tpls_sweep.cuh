@@ -212,9 +212,8 @@ cudaError_t launch_odd_multi(int comp, const SweepMember *mem, const int *prefix
 
 // FP32 Jacobi (mode 0) and checkerboard half-sweep (mode 1) with four x
 // points per thread (k_sweep32.cu); tile = rows per block choice.
-cudaError_t launch_sweep4(int mode, int comp, const Geo &g, const Helm &h, const float *xo, float *x,
-                          const MuCoef &s, const double *P, const double *X, int flg, int bc, int fuse, int tile,
-                          cudaStream_t st);
+cudaError_t launch_sweep4(int mode, const Geo &g, const Helm &h, const SweepSet32 &s, int flg, int bc, int fuse,
+                          int tile, cudaStream_t st);
 
 static inline Helm helm_of(const Phys &ph) {
   Helm h;
