@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "tpls_mg.cuh"
+#include "tpls_modes.cuh"
 #include "tpls_pair.cuh"
 #include "tpls_pressure.h"
 
@@ -59,6 +60,7 @@ struct PoissonSolver {
   std::vector<PLevel> lv;
   double *cinv = nullptr;  // coarsest pseudo-inverse (nc x nc; FP32 levels: transposed), or null
   int coarse_sweeps = 0;
+  double *modes = nullptr;  // coarsest level by modes: Qz, Qy, lambda_z, lambda_y
   double *x = nullptr, *r = nullptr, *p = nullptr, *q = nullptr, *bvec = nullptr;
   void *z = nullptr;           // preconditioned residual, in the level type
   float *r32 = nullptr;        // FP32 levels: r rounded once, for the V-cycle
@@ -433,7 +435,8 @@ struct LevArgs {
 // zero_init: ei == 0.
 constexpr int LJB = 64;  // threads per block of the line smoother (one column each)
 
-template <typename R>
+// TS: values per level of the factor table (k_line_jacobi3's carries four).
+template <typename R, int TS>
 __global__ void __launch_bounds__(LJB)
     k_line_jacobi(LevArgs<R> L, R omega, R one_m_omega, int zero_init, const R *__restrict__ thomas,
                   const R *__restrict__ b, const R *__restrict__ ei, R *__restrict__ t, R *__restrict__ eo) {
@@ -442,7 +445,7 @@ __global__ void __launch_bounds__(LJB)
   if (col >= nx * ny) return;
   const int i = col % nx, j = col / nx;
   const int cls = (nx == 1) ? 1 : ((i == 0) ? 0 : ((i == nx - 1) ? 2 : 1));
-  const R *th = thomas + (size_t)cls * nz * 2;
+  const R *th = thomas + (size_t)cls * nz * TS;
   const int plane = nx * ny;
   const int jm = (j > 0) ? -nx : nx * (ny - 1), jp = (j < ny - 1) ? nx : -nx * (ny - 1);
   R y = (R)0;
@@ -455,13 +458,13 @@ __global__ void __launch_bounds__(LJB)
       if (i < nx - 1) nb += L.cx * ei[c + 1];
       rhs += nb;
     }
-    y = (rhs + L.cz * y) * th[2 * k + 1];
+    y = (rhs + L.cz * y) * th[TS * k + 1];
     t[c] = y;
   }
   R xn = (R)0;
   for (int k = nz - 1; k >= 0; k--) {
     const int c = col + plane * k;
-    xn = t[c] - ((k < nz - 1) ? th[2 * k] * xn : (R)0);
+    xn = t[c] - ((k < nz - 1) ? th[TS * k] * xn : (R)0);
     eo[c] = zero_init ? omega * xn : one_m_omega * ei[c] + omega * xn;
   }
 }
@@ -469,15 +472,14 @@ __global__ void __launch_bounds__(LJB)
 // The same sweep for 32 columns per block in three phases: all threads
 // assemble the line right-hand sides into shared memory, one warp runs the
 // Thomas forward/backward substitution in shared memory, all threads write
-// the damped result.  Dynamic shared memory: nz * 32 values of R.
+// the damped result.  Dynamic shared memory: nz * 32 values of float.
 constexpr int LJ2_T = 256;
 
-template <typename R>
 __global__ void __launch_bounds__(LJ2_T)
-    k_line_jacobi2(LevArgs<R> L, R omega, R one_m_omega, int zero_init, const R *__restrict__ thomas,
-                   const R *__restrict__ b, const R *__restrict__ ei, R *__restrict__ eo) {
+    k_line_jacobi2(LevArgs<float> L, float omega, float one_m_omega, int zero_init, const float *__restrict__ thomas,
+                   const float *__restrict__ b, const float *__restrict__ ei, float *__restrict__ eo) {
   extern __shared__ __align__(16) unsigned char lj2_raw[];
-  R *buf = reinterpret_cast<R *>(lj2_raw);  // [nz][32]
+  float *buf = reinterpret_cast<float *>(lj2_raw);  // [nz][32]
   const int nx = L.nx, ny = L.ny, nz = L.nz, ncol = nx * ny, plane = nx * ny;
   const int col0 = blockIdx.x * 32;
   // every thread keeps one column (LJ2_T is a multiple of 32)
@@ -486,12 +488,12 @@ __global__ void __launch_bounds__(LJ2_T)
   const int jm = (cj > 0) ? -nx : nx * (ny - 1), jp = (cj < ny - 1) ? nx : -nx * (ny - 1);
   for (int t = threadIdx.x; t < nz * 32; t += LJ2_T) {
     const int k = t >> 5;
-    R rhs = (R)0;
+    float rhs = 0.0f;
     if (mycol < ncol) {
       const int c = mycol + plane * k;
       rhs = b[c];
       if (!zero_init) {
-        R nb = L.cy * (ei[c + jm] + ei[c + jp]);
+        float nb = L.cy * (ei[c + jm] + ei[c + jp]);
         if (ci > 0) nb += L.cx * ei[c - 1];
         if (ci < nx - 1) nb += L.cx * ei[c + 1];
         rhs += nb;
@@ -505,13 +507,13 @@ __global__ void __launch_bounds__(LJ2_T)
     if (col < ncol) {
       const int i = col % nx;
       const int cls = (nx == 1) ? 1 : ((i == 0) ? 0 : ((i == nx - 1) ? 2 : 1));
-      const R *th = thomas + (size_t)cls * nz * 2;
-      R y = (R)0;
+      const float *th = thomas + (size_t)cls * nz * 2;
+      float y = 0.0f;
       for (int k = 0; k < nz; k++) {
         y = (buf[k * 32 + threadIdx.x] + L.cz * y) * th[2 * k + 1];
         buf[k * 32 + threadIdx.x] = y;
       }
-      R xn = y;
+      float xn = y;
       for (int k = nz - 2; k >= 0; k--) {
         xn = buf[k * 32 + threadIdx.x] - th[2 * k] * xn;
         buf[k * 32 + threadIdx.x] = xn;
@@ -525,6 +527,71 @@ __global__ void __launch_bounds__(LJ2_T)
       const int c = col + plane * k;
       eo[c] = zero_init ? omega * buf[t] : one_m_omega * ei[c] + omega * buf[t];
     }
+  }
+}
+
+// FP64: the same sweep with the two substitutions in parallel.  Both are
+// recurrences v_k = a_k + m_k v_{k-1} whose multipliers m do not depend on the
+// data, so a warp takes 32 columns of one of LJ_W runs of levels, solves it
+// from zero, and the value entering the run times the (precomputed) product
+// of its multipliers is added once the runs below have been folded: chains of
+// nz/8 + 8 dependent FP64 operations instead of nz of two each (23 us at
+// 50x25x75 with one warp per block in the substitutions; 75 levels).
+// th: per class and level c', 1/den, the forward and the backward product
+// from the start of the level's run.
+constexpr int LJ_W = 8;
+static inline __host__ __device__ int lj_run(int nz) { return (nz + LJ_W - 1) / LJ_W; }
+
+__global__ void __launch_bounds__(32 * LJ_W)
+    k_line_jacobi3(LevArgs<double> L, double omega, double one_m_omega, int zero_init,
+                   const double *__restrict__ thomas, const double *__restrict__ b, const double *__restrict__ ei,
+                   double *__restrict__ eo) {
+  extern __shared__ __align__(16) unsigned char lj3_raw[];
+  double *buf = reinterpret_cast<double *>(lj3_raw);  // [nz][32]
+  __shared__ double se[LJ_W][32], sp[LJ_W][32];       // a run's end from zero, and its product
+  const int nx = L.nx, ny = L.ny, nz = L.nz, ncol = nx * ny, plane = nx * ny;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int col = min(blockIdx.x * 32 + lane, ncol - 1);  // past the end: the last column again, not stored
+  const bool own = blockIdx.x * 32 + lane < ncol;
+  const int i = col % nx, j = col / nx;
+  const int jm = (j > 0) ? -nx : nx * (ny - 1), jp = (j < ny - 1) ? nx : -nx * (ny - 1);
+  const int cls = (nx == 1) ? 1 : ((i == 0) ? 0 : ((i == nx - 1) ? 2 : 1));
+  const double *th = thomas + (size_t)cls * nz * 4;
+  const int run = lj_run(nz), k0 = min(w * run, nz), k1 = min(k0 + run, nz);
+  double y = 0.0;
+  for (int k = k0; k < k1; k++) {
+    const int c = col + plane * k;
+    double rhs = b[c];
+    if (!zero_init) {
+      double nb = L.cy * (ei[c + jm] + ei[c + jp]);
+      if (i > 0) nb = fma(L.cx, ei[c - 1], nb);
+      if (i < nx - 1) nb = fma(L.cx, ei[c + 1], nb);
+      rhs += nb;
+    }
+    y = fma(L.cz, y, rhs) * th[4 * k + 1];
+    buf[k * 32 + lane] = y;
+  }
+  se[w][lane] = y;
+  sp[w][lane] = k1 > k0 ? th[4 * (k1 - 1) + 2] : 1.0;
+  __syncthreads();
+  double in = 0.0;  // y entering this run
+  for (int v = 0; v < w; v++) in = fma(sp[v][lane], in, se[v][lane]);
+  __syncthreads();
+  double x = 0.0;  // from the top of the run down, zero above it
+  for (int k = k1 - 1; k >= k0; k--) {
+    const double yk = fma(th[4 * k + 2], in, buf[k * 32 + lane]);
+    x = (k < nz - 1) ? fma(-th[4 * k], x, yk) : yk;
+    buf[k * 32 + lane] = x;
+  }
+  se[w][lane] = x;
+  sp[w][lane] = k1 > k0 ? th[4 * k0 + 3] : 1.0;
+  __syncthreads();
+  in = 0.0;
+  for (int v = LJ_W - 1; v > w; v--) in = fma(sp[v][lane], in, se[v][lane]);
+  for (int k = k0; k < k1; k++) {
+    const int c = col + plane * k;
+    const double v = omega * fma(th[4 * k + 3], in, buf[k * 32 + lane]);
+    if (own) eo[c] = zero_init ? v : fma(one_m_omega, ei[c], v);
   }
 }
 
@@ -806,6 +873,43 @@ static std::vector<double> thomas_factors(const PLevel &L) {
   }
   return th;
 }
+// with the run products of k_line_jacobi3: forward multipliers cz/den (the
+// substitution is y_k = (rhs + cz y_{k-1})/den), backward -c'
+static std::vector<double> thomas_runs(const PLevel &L) {
+  const std::vector<double> th = thomas_factors(L);
+  std::vector<double> r((size_t)3 * L.nz * 4);
+  const int run = lj_run(L.nz);
+  for (int cls = 0; cls < 3; cls++) {
+    const double *t = &th[(size_t)cls * L.nz * 2];
+    double *o = &r[(size_t)cls * L.nz * 4];
+    for (int k0 = 0; k0 < L.nz; k0 += run) {
+      const int k1 = k0 + run < L.nz ? k0 + run : L.nz;
+      double p = 1.0;
+      for (int k = k0; k < k1; k++) {
+        p *= L.cz * t[2 * k + 1];
+        o[4 * k] = t[2 * k];
+        o[4 * k + 1] = t[2 * k + 1];
+        o[4 * k + 2] = p;
+      }
+      p = 1.0;
+      for (int k = k1 - 1; k >= k0; k--) {
+        p *= k < L.nz - 1 ? -t[2 * k] : 0.0;  // nothing above the last level
+        o[4 * k + 3] = p;
+      }
+    }
+  }
+  return r;
+}
+
+// Sweeps on a coarsest level without a dense inverse, and whether they run by
+// modes (FP64): the transforms take about nz + 2 ny operations per point and
+// the x recurrences 3 per sweep, against about 9.5 per sweep for the line
+// solves, whose serial part (nz dependent pairs of FP64 operations) is what
+// they wait for until a level has millions of points.
+constexpr int COARSE_SWEEPS = 40;
+static bool modes_pay(int nx, int ny, int nz) {
+  return nx <= 32 * MODE_PPL && nz + 2 * ny + 3 * COARSE_SWEEPS <= 400;
+}
 
 #define PCK(x)                        \
   do {                                \
@@ -813,9 +917,8 @@ static std::vector<double> thomas_factors(const PLevel &L) {
     if (e_ != cudaSuccess) return e_; \
   } while (0)
 
-template <typename R>
 static cudaError_t lj2_attr() {
-  return cudaFuncSetAttribute(k_line_jacobi2<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  return cudaFuncSetAttribute(k_line_jacobi2, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
 }
 
 static size_t mg_dot_blocks(const PLevel &L);
@@ -883,20 +986,21 @@ cudaError_t poisson_create(const Geo &g, double cx, double cy, double cz, int fp
       PCK(cudaMalloc(&L.r, bytes));
       PCK(cudaMalloc(&L.t, bytes));
     }
-    std::vector<double> th = thomas_factors(L);
     if (S->fp32) {
+      std::vector<double> th = thomas_factors(L);
       std::vector<float> thf(th.begin(), th.end());
       PCK(cudaMalloc(&L.thomas, thf.size() * sizeof(float)));
       PCK(cudaMemcpy(L.thomas, thf.data(), thf.size() * sizeof(float), cudaMemcpyHostToDevice));
     } else {
+      std::vector<double> th = thomas_runs(L);
       PCK(cudaMalloc(&L.thomas, th.size() * sizeof(double)));
       PCK(cudaMemcpy(L.thomas, th.data(), th.size() * sizeof(double), cudaMemcpyHostToDevice));
     }
   }
   if (S->fp32) {
-    PCK(lj2_attr<float>());
+    PCK(lj2_attr());
   } else {
-    PCK(lj2_attr<double>());
+    PCK(cudaFuncSetAttribute(k_line_jacobi3, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
   }
   const PLevel &C = S->lv.back();
   if (C.n <= 512) {
@@ -910,7 +1014,17 @@ cudaError_t poisson_create(const Geo &g, double cx, double cy, double cz, int fp
     PCK(cudaMalloc(&S->cinv, M.size() * sizeof(double)));
     PCK(cudaMemcpy(S->cinv, M.data(), M.size() * sizeof(double), cudaMemcpyHostToDevice));
   } else {
-    S->coarse_sweeps = 40;
+    S->coarse_sweeps = COARSE_SWEEPS;
+    if (!S->fp32 && modes_pay(C.nx, C.ny, C.nz)) {
+      std::vector<double> Qz, Qy, lz, ly;
+      neumann_basis(C.nz, Qz, lz);
+      periodic_basis(C.ny, Qy, ly);
+      Qz.insert(Qz.end(), Qy.begin(), Qy.end());
+      Qz.insert(Qz.end(), lz.begin(), lz.end());
+      Qz.insert(Qz.end(), ly.begin(), ly.end());
+      PCK(cudaMalloc(&S->modes, Qz.size() * sizeof(double)));
+      PCK(cudaMemcpy(S->modes, Qz.data(), Qz.size() * sizeof(double), cudaMemcpyHostToDevice));
+    }
   }
   const size_t nb = sizeof(double) * (size_t)S->N;
   PCK(cudaMalloc(&S->x, nb));
@@ -950,6 +1064,7 @@ void poisson_destroy(PoissonSolver *S) {
     cudaFree(L.thomas);
   }
   cudaFree(S->cinv);
+  cudaFree(S->modes);
   cudaFree(S->x);
   cudaFree(S->r);
   cudaFree(S->z);
@@ -975,13 +1090,16 @@ size_t poisson_footprint(const Geo &g, int fp32, size_t (*rnd)(size_t)) {
   int nx = g.nx, ny = g.ny, nz = g.nz, l = 0;
   while (true) {
     const size_t n = (size_t)nx * ny * nz;
-    tot += (l > 0 ? 5 : 4) * rnd(esz * n) + rnd(esz * 3 * nz * 2);
+    tot += (l > 0 ? 5 : 4) * rnd(esz * n) + rnd(esz * 3 * nz * (fp32 ? 2 : 4));
     if (n <= 512) {
       tot += rnd(sizeof(double) * n * n);
       break;
     }
     const int cx = (nx % 2 == 0 && nx >= 4), cy = (ny % 2 == 0 && ny >= 4), cz = (nz % 2 == 0 && nz >= 4);
-    if (!cx && !cy && !cz) break;
+    if (!cx && !cy && !cz) {
+      if (!fp32 && modes_pay(nx, ny, nz)) tot += rnd(sizeof(double) * ((size_t)nz * nz + (size_t)ny * ny + nz + ny));
+      break;
+    }
     nx = cx ? nx / 2 : nx;
     ny = cy ? ny / 2 : ny;
     nz = cz ? nz / 2 : nz;
@@ -1008,17 +1126,63 @@ static LevArgs<R> largs(const PLevel &L) {
   return a;
 }
 
-template <typename R>
-static void line_sweep(const PLevel &L, R w, R w1, int zero_init, const R *b, const R *ei, R *eo, cudaStream_t st) {
-  const LevArgs<R> A = largs<R>(L);
-  const R *th = static_cast<const R *>(L.thomas);
-  const size_t smem = sizeof(R) * 32 * (size_t)L.nz;
-  if (smem <= 200 * 1024) {
-    k_line_jacobi2<R><<<(L.nx * L.ny + 31) / 32, LJ2_T, smem, st>>>(A, w, w1, zero_init, th, b, ei, eo);
-  } else {
-    k_line_jacobi<R><<<(L.nx * L.ny + LJB - 1) / LJB, LJB, 0, st>>>(A, w, w1, zero_init, th, b, ei,
-                                                                   static_cast<R *>(L.t), eo);
-  }
+static void line_sweep(const PLevel &L, double w, double w1, int zero_init, const double *b, const double *ei,
+                       double *eo, cudaStream_t st) {
+  const LevArgs<double> A = largs<double>(L);
+  const double *th = static_cast<const double *>(L.thomas);
+  const size_t smem = sizeof(double) * 32 * (size_t)L.nz;
+  if (smem <= 200 * 1024)
+    k_line_jacobi3<<<(L.nx * L.ny + 31) / 32, 32 * LJ_W, smem, st>>>(A, w, w1, zero_init, th, b, ei, eo);
+  else
+    k_line_jacobi<double, 4><<<(L.nx * L.ny + LJB - 1) / LJB, LJB, 0, st>>>(A, w, w1, zero_init, th, b, ei,
+                                                                           static_cast<double *>(L.t), eo);
+}
+static void line_sweep(const PLevel &L, float w, float w1, int zero_init, const float *b, const float *ei, float *eo,
+                       cudaStream_t st) {
+  const LevArgs<float> A = largs<float>(L);
+  const float *th = static_cast<const float *>(L.thomas);
+  const size_t smem = sizeof(float) * 32 * (size_t)L.nz;
+  if (smem <= 200 * 1024)
+    k_line_jacobi2<<<(L.nx * L.ny + 31) / 32, LJ2_T, smem, st>>>(A, w, w1, zero_init, th, b, ei, eo);
+  else
+    k_line_jacobi<float, 2><<<(L.nx * L.ny + LJB - 1) / LJB, LJB, 0, st>>>(A, w, w1, zero_init, th, b, ei,
+                                                                          static_cast<float *>(L.t), eo);
+}
+
+// The coarsest level's sweeps by modes: b -> e; t and u are scratch of the
+// level's size.
+template <int PPL>
+static void mode_lines(const ModeSweeps &M, const double *Qy, const double *ly, const double *lz, const double *t,
+                       double *u, cudaStream_t st) {
+  k_mode_lines<PPL><<<dim3((M.ny + MODE_W - 1) / MODE_W, M.nz), 32 * MODE_W, 0, st>>>(M, Qy, ly, lz, t, u);
+}
+static cudaError_t coarse_modes(const PoissonSolver *S, const PLevel &L, const double *b, double *t, double *u,
+                                double *e, cudaStream_t st, long *nl) {
+  const ModeSweeps M = {L.nx, L.ny, L.nz, S->coarse_sweeps, L.cx, L.cy, L.cz, S->omega};
+  const double *Qz = S->modes, *Qy = Qz + (size_t)L.nz * L.nz, *lz = Qy + (size_t)L.ny * L.ny, *ly = lz + L.nz;
+  const int ncol = L.nx * L.ny, gc = (ncol + 31) / 32;
+  constexpr int T = 32 * MODE_W;
+  auto blocks = [](int warps) { return (warps + MODE_W - 1) / MODE_W; };
+  const int m4 = 2 * ((L.nz + 7) / 8), m1 = 2 * ((L.nz + 1) / 2);  // groups of four modes of one parity, of one
+  if (gc * m4 >= MODE_WARPS) k_modes_z<4><<<dim3(gc, blocks(m4)), T, 0, st>>>(L.nz, ncol, Qz, b, t);
+  else k_modes_z<1><<<dim3(gc, blocks(m1)), T, 0, st>>>(L.nz, ncol, Qz, b, t);
+  const int ppl = (L.nx + 31) / 32;
+  if (ppl == 1) mode_lines<1>(M, Qy, ly, lz, t, u, st);
+  else if (ppl == 2) mode_lines<2>(M, Qy, ly, lz, t, u, st);
+  else if (ppl <= 4) mode_lines<4>(M, Qy, ly, lz, t, u, st);
+  else mode_lines<MODE_PPL>(M, Qy, ly, lz, t, u, st);
+  const int gi = (L.nx + 31) / 32, r4 = (L.ny + 3) / 4;
+  if (gi * r4 * L.nz >= MODE_WARPS) k_points_y<4><<<dim3(gi, blocks(r4), L.nz), T, 0, st>>>(L.nx, L.ny, Qy, u, t);
+  else k_points_y<1><<<dim3(gi, blocks(L.ny), L.nz), T, 0, st>>>(L.nx, L.ny, Qy, u, t);
+  const int p1 = (L.nz + 1) / 2, p2 = (p1 + 1) / 2;  // pairs of points
+  if (gc * p2 >= MODE_WARPS) k_points_z<2><<<dim3(gc, blocks(p2)), T, 0, st>>>(L.nz, ncol, Qz, t, e);
+  else k_points_z<1><<<dim3(gc, blocks(p1)), T, 0, st>>>(L.nz, ncol, Qz, t, e);
+  *nl += 4;
+  return cudaGetLastError();
+}
+static cudaError_t coarse_modes(const PoissonSolver *, const PLevel &, const float *, float *, float *, float *,
+                                cudaStream_t, long *) {
+  return cudaErrorInvalidValue;  // FP32 levels keep the sweeps
 }
 
 // R = P^T / 2^d over the coarsened axes in the order x, y, z; the
@@ -1136,7 +1300,7 @@ static size_t mg_dot_blocks(const PLevel &L) {
 template <typename R>
 static void pre_smooth(const PLevel &L, R w, R w1, const R *b, R *e2, cudaStream_t st, long *nl) {
   if (!L.point) {
-    line_sweep<R>(L, w, w1, 1, b, nullptr, e2, st);
+    line_sweep(L, w, w1, 1, b, nullptr, e2, st);
     (*nl)++;
     return;
   }
@@ -1152,7 +1316,7 @@ static void pre_smooth(const PLevel &L, R w, R w1, const R *b, R *e2, cudaStream
 template <typename R>
 static void post_smooth(const PLevel &L, R w, R w1, const R *b, R *e2, R *res, cudaStream_t st, long *nl) {
   if (!L.point) {
-    line_sweep<R>(L, w, w1, 0, b, e2, res, st);
+    line_sweep(L, w, w1, 0, b, e2, res, st);
     (*nl)++;
     return;
   }
@@ -1258,12 +1422,14 @@ static cudaError_t vcycle(PoissonSolver *S, const R *b0, R *out, cudaStream_t st
       if (S->cinv) {
         coarse_solve(L.n, S->cinv, b, res, st);
         (*nl)++;
+      } else if (S->modes) {
+        PCK(coarse_modes(S, L, b, lvp(L.r), lvp(L.e2), res, st, nl));
       } else {  // no dense inverse: damped line-Jacobi sweeps
         R *cur = lvp(L.e2), *oth = res;
-        line_sweep<R>(L, w, w1, 1, b, nullptr, cur, st);
+        line_sweep(L, w, w1, 1, b, nullptr, cur, st);
         (*nl)++;
         for (int sw = 1; sw < S->coarse_sweeps; sw++) {
-          line_sweep<R>(L, w, w1, 0, b, cur, oth, st);
+          line_sweep(L, w, w1, 0, b, cur, oth, st);
           (*nl)++;
           R *tmp = cur;
           cur = oth;

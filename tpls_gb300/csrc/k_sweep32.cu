@@ -312,7 +312,7 @@ __device__ __forceinline__ void sweep4_tile(const Geo &g, const Helm &h, const f
 // unbounded the compiler takes 80 and 24 warps do not cover the loads'
 // latency.
 template <int MODE, int BY>
-__global__ void __launch_bounds__(32 * BY, (MODE == M_JAC ? 36 : 32) / BY)
+__global__ void __launch_bounds__(32 * BY, BY == 1 ? 32 : (MODE == M_JAC ? 36 : 32) / BY)
     k_sweep4(Geo g, Helm h, const __grid_constant__ SweepSet32 s, int gx, int flg, int bc, int fuse) {
   const int q = blockIdx.x / gx, bx = blockIdx.x - q * gx, comp = s.id[q];
   if (comp == 0) {
