@@ -63,6 +63,51 @@ __device__ __forceinline__ T weno_up(bool pos, T m2, T m1, T c0, T p1, T p2, T p
   return weno5(pos ? m2 : p3, pos ? m1 : p2, pos ? c0 : p1, pos ? p1 : c0, pos ? p2 : m1);
 }
 
+// FP64: the same weights and faces with fewer operations on GB300's FP64 pipe,
+// which bounds the kernel.  In the differences d_m = v_{m+1} - v_m and s_m =
+// d_{m+1} - d_m of the stencil the smoothness indicators are, up to the factor
+// 13/12 (which cancels in the weights; eps scales with it),
+//   q_m = s_m^2 + 3/13 t_m^2 + 12/13 eps,
+//   t_1 = s_1 + 2 d_2, t_2 = d_2 + d_3, t_3 = s_3 - 2 d_3,
+// and the three candidate values are v3 + g/6 with g_1 = 2 t_1 - d_2, g_2 =
+// t_2 + d_3, g_3 = d_3 - t_3, so the face is v3 + (sum n_m g_m)/(6 sum n_m):
+// 40 operations with the quotient of div_fast against 57 with the form above,
+// and smaller roundings (the correction is a small part of v3).
+struct Weno {
+  double d1, d2, d3, d4, s1, s2, s3;
+};
+__device__ __forceinline__ double weno_ratio(const Weno &w, double e1, double e2, double e3) {
+  // e_m = s_m^2 + 12/13 eps
+  const double c = 3.0 / 13.0;
+  const double t1 = fma(2.0, w.d2, w.s1), t2 = w.d2 + w.d3, t3 = fma(-2.0, w.d3, w.s3);
+  const double q1 = fma(c * t1, t1, e1), q2 = fma(c * t2, t2, e2), q3 = fma(c * t3, t3, e3);
+  const double m1 = q2 * q3, m2 = q1 * q3, m3 = q1 * q2;
+  const double n1 = m1 * m1, n2 = (6.0 * m2) * m2, n3 = (3.0 * m3) * m3;
+  const double num = fma(n1, fma(2.0, t1, -w.d2), fma(n2, t2 + w.d3, n3 * (w.d3 - t3)));
+  return div_fast(num, n1 + n2 + n3);
+}
+constexpr double WENO_E = TPLS_WENO_EPS * (12.0 / 13.0);
+
+__device__ __forceinline__ double weno_up64(bool pos, double m2, double m1, double c0, double p1, double p2,
+                                            double p3) {
+  const double v1 = pos ? m2 : p3, v2 = pos ? m1 : p2, v3 = pos ? c0 : p1, v4 = pos ? p1 : c0, v5 = pos ? p2 : m1;
+  Weno w;
+  w.d1 = v2 - v1;
+  w.d2 = v3 - v2;
+  w.d3 = v4 - v3;
+  w.d4 = v5 - v4;
+  w.s1 = w.d2 - w.d1;
+  w.s2 = w.d3 - w.d2;
+  w.s3 = w.d4 - w.d3;
+  return fma(weno_ratio(w, fma(w.s1, w.s1, WENO_E), fma(w.s2, w.s2, WENO_E), fma(w.s3, w.s3, WENO_E)), 1.0 / 6.0,
+             v3);
+}
+template <typename T>
+__device__ __forceinline__ T weno_face(bool pos, T m2, T m1, T c0, T p1, T p2, T p3) {
+  if constexpr (sizeof(T) == sizeof(double)) return weno_up64(pos, m2, m1, c0, p1, p2, p3);
+  else return weno_up(pos, m2, m1, c0, p1, p2, p3);
+}
+
 // dfx at u-index (iu, jp-1, kp-1): phi along x at p-row jp, level kp.
 // WENO for 3 <= iu <= nx-2, first-order upwind otherwise (weno.f90:45-100).
 template <typename T>
@@ -73,7 +118,7 @@ __device__ __forceinline__ T xface(const Geo &g, const T *__restrict__ phi,
   const T vel = u[TPLS_IDX(g, iu, ju, kp - 1)];
   const T *row = phi + TPLS_IDX(g, 0, jp, kp);
   if (iu >= 3 && iu <= g.nx - 2)
-    return weno_up(upwind_pos(vel), row[iu - 2], row[iu - 1], row[iu], row[iu + 1], row[iu + 2], row[iu + 3]);
+    return weno_face(upwind_pos(vel), row[iu - 2], row[iu - 1], row[iu], row[iu + 1], row[iu + 2], row[iu + 3]);
   return (upwind_pos(vel)) ? row[iu] : row[iu + 1];
 }
 
@@ -89,12 +134,16 @@ __device__ __forceinline__ T yface(const Geo &g, const T *__restrict__ phi,
   const T *col = phi + TPLS_IDX(g, ip, 0, kp);
   const int sy = g.sy;
 #define PY(jj) col[sy * wrapy((jj), ny)]
-  return weno_up(upwind_pos(vel), PY(jv - 2), PY(jv - 1), PY(jv), PY(jv + 1), PY(jv + 2), PY(jv + 3));
+  return weno_face(upwind_pos(vel), PY(jv - 2), PY(jv - 1), PY(jv), PY(jv + 1), PY(jv + 2), PY(jv + 3));
 #undef PY
 }
 
 constexpr int ADV_BX = 32, ADV_BY = 8;
-constexpr int ADV_KC = 16;  // z levels per thread (column chunk)
+// z levels per thread (column chunk): 16, halved to no less than 2 while the
+// grid has fewer than three blocks per SM.  A chunk forms one z-face more than
+// its levels; at 64x32x48, 24 blocks of 16 levels left 128 of 152 SMs idle
+// (285 us, against about 30 for its FP64 operations spread over all).
+constexpr int ADV_KC = 16;
 
 // One block covers 32 x 8 columns and a chunk of ADV_KC levels.  At each
 // level every thread computes the x-face right of its cell and the y-face
@@ -107,13 +156,13 @@ constexpr int ADV_KC = 16;  // z levels per thread (column chunk)
 template <typename T>
 __global__ void __launch_bounds__(ADV_BX *ADV_BY, 4)
     k_advect(Geo g, T rdx, T rdy, T rdz, const T *__restrict__ phi, const T *__restrict__ u,
-             const T *__restrict__ v, const T *__restrict__ w, double *__restrict__ conv) {
+             const T *__restrict__ v, const T *__restrict__ w, double *__restrict__ conv, int kc) {
   __shared__ T xs[2][ADV_BY][ADV_BX + 1];  // x-faces iu = i0-1 .. i0+31 per row
   __shared__ T ys[2][ADV_BY + 1][ADV_BX];  // y-faces jv = j0-1 .. j0+7 per column
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int i0 = blockIdx.x * ADV_BX + 1, j0 = blockIdx.y * ADV_BY + 1;
   const int i = i0 + tx, j = j0 + ty;
-  const int k0 = blockIdx.z * ADV_KC + 1, k1 = min(k0 + ADV_KC - 1, g.nz);
+  const int k0 = blockIdx.z * kc + 1, k1 = min(k0 + kc - 1, g.nz);
   const bool act = (i <= g.nx) && (j <= g.ny);
   const int ic = act ? i : 1, jc = act ? j : 1;  // clamped for inactive lanes
   const int jm = (jc == 1) ? g.ny : jc - 1;      // u/v/w row index j-1 (wrapped)
@@ -129,7 +178,7 @@ __global__ void __launch_bounds__(ADV_BX *ADV_BY, 4)
   // dfz at w-index (ic, jc-1, kw): WENO for 3 <= kw <= nz-2, arithmetic mean
   // otherwise (weno.f90:136-166)
   auto zface = [&](int kw, T c0, T c1, T c2, T c3, T c4, T c5) -> T {
-    if (kw >= 3 && kw <= g.nz - 2) return weno_up(upwind_pos(w[TPLS_IDX(g, ic, jm, kw)]), c0, c1, c2, c3, c4, c5);
+    if (kw >= 3 && kw <= g.nz - 2) return weno_face(upwind_pos(w[TPLS_IDX(g, ic, jm, kw)]), c0, c1, c2, c3, c4, c5);
     return (c2 + c3) / (T)2;
   };
   T c0 = zld(k0 - 3), c1 = zld(k0 - 2), c2 = zld(k0 - 1), c3 = zld(k0), c4 = zld(k0 + 1), c5 = zld(k0 + 2);
@@ -352,23 +401,29 @@ cudaError_t launch_advect_tma(const Geo &g, const Phys &ph, const void *map128, 
   return cudaGetLastError();
 }
 
+static int adv_levels(const Geo &g) {
+  const int gxy = ((g.nx + ADV_BX - 1) / ADV_BX) * ((g.ny + ADV_BY - 1) / ADV_BY);
+  int kc = ADV_KC;
+  while (kc > 2 && gxy * ((g.nz + kc - 1) / kc) < 3 * 152) kc /= 2;
+  return kc;
+}
+
 cudaError_t launch_advect(const Geo &g, const Phys &ph, const double *phi2,
                           const double *u2, const double *v2,
                           const double *w2, double *conv2_phi,
                           cudaStream_t st) {
-  dim3 blk(ADV_BX, ADV_BY),
-      grd((g.nx + ADV_BX - 1) / ADV_BX, (g.ny + ADV_BY - 1) / ADV_BY, (g.nz + ADV_KC - 1) / ADV_KC);
-  k_advect<double><<<grd, blk, 0, st>>>(g, 1.0 / ph.dx, 1.0 / ph.dy, 1.0 / ph.dz, phi2, u2, v2, w2,
-                                        conv2_phi);
+  const int kc = adv_levels(g);
+  dim3 blk(ADV_BX, ADV_BY), grd((g.nx + ADV_BX - 1) / ADV_BX, (g.ny + ADV_BY - 1) / ADV_BY, (g.nz + kc - 1) / kc);
+  k_advect<double><<<grd, blk, 0, st>>>(g, 1.0 / ph.dx, 1.0 / ph.dy, 1.0 / ph.dz, phi2, u2, v2, w2, conv2_phi, kc);
   return cudaGetLastError();
 }
 
 cudaError_t launch_advect(const Geo &g, const Phys &ph, const float *phi2, const float *u2, const float *v2,
                           const float *w2, double *conv2_phi, cudaStream_t st) {
-  dim3 blk(ADV_BX, ADV_BY),
-      grd((g.nx + ADV_BX - 1) / ADV_BX, (g.ny + ADV_BY - 1) / ADV_BY, (g.nz + ADV_KC - 1) / ADV_KC);
+  const int kc = adv_levels(g);
+  dim3 blk(ADV_BX, ADV_BY), grd((g.nx + ADV_BX - 1) / ADV_BX, (g.ny + ADV_BY - 1) / ADV_BY, (g.nz + kc - 1) / kc);
   k_advect<float><<<grd, blk, 0, st>>>(g, (float)(1.0 / ph.dx), (float)(1.0 / ph.dy), (float)(1.0 / ph.dz), phi2,
-                                       u2, v2, w2, conv2_phi);
+                                       u2, v2, w2, conv2_phi, kc);
   return cudaGetLastError();
 }
 

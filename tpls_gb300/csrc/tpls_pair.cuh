@@ -70,6 +70,31 @@ __device__ __forceinline__ float float_bits(double x) {
   return __uint_as_float((m + up) | (hi & 0x80000000u));
 }
 
+// 1/d to about 2^-44 for 2^-100 < |d| < 2^100: FP32 reciprocal of the leading
+// part and one Newton step in FP32 on the pair, joined by one FP64 addition.
+__device__ __forceinline__ double rcp_seed(double d) {
+  const F2 p = split_bits(d);
+  const float r = __fdividef(1.0f, p.h);
+  const float e = fmaf(-p.l, r, fmaf(-p.h, r, 1.0f));
+  return widen_bits(r) + widen_bits(r * e);
+}
+// |d| within 2^-100 .. 2^100 (also excludes 0, infinities and NaN)
+__device__ __forceinline__ bool rcp_range(double d) {
+  const unsigned int a = (unsigned int)__double2hiint(d) & 0x7fffffffu;
+  return a - (923u << 20) < (200u << 20);
+}
+// The quotient the hardware sequence would form, out of line: the callers'
+// common path is four FP64 operations instead of about nine.
+static __device__ __noinline__ double div_slow(double n, double d) { return n / d; }
+// n/d to within one ulp: quotient from the seed, its remainder by an FMA
+// (exact up to one rounding) and one correction.
+__device__ __forceinline__ double div_fast(double n, double d) {
+  if (!rcp_range(d)) return div_slow(n, d);
+  const double r = rcp_seed(d);
+  const double q = n * r;
+  return fma(fma(-d, q, n), r, q);
+}
+
 // order of two pairs of the same normalisation (both from split_bits, or
 // both from an error-free sum): by hi, then by lo
 __device__ __forceinline__ F2 pmin(F2 a, F2 b) { return (b.h < a.h || (b.h == a.h && b.l < a.l)) ? b : a; }
