@@ -126,161 +126,383 @@ __device__ __forceinline__ bool cd_valid(int comp, const Geo &g, int i, int k) {
   return true;
 }
 
-// The sweep coefficients of one point, divided by the Helmholtz diagonal
-// (jacobi_iteration_allflux.f90:84-90): x_new = cxp x[i+1] + cxm x[i-1] +
-// cyp x[j+1] + cym x[j-1] + czp x[k+1] + czm x[k-1] + rhs/diag.  For u and v
-// the wall ghost rule `-2 x(0) + x(1)/3` (and its top mirror) is folded in:
-// at k = 0 the czm slot multiplies the point itself and czp absorbs czm/3;
-// at k = nz-1 the czp slot multiplies the point itself and czm absorbs
-// czp/3.  One 64-byte record per point: (cxp, cxm, cyp, cym, czp, czm, b,
-// 1.2 czm), the last the factor of the odd half-sweep's column recurrence.
-__device__ __forceinline__ void store_rec(double *rec, double a0, double a1, double a2, double a3, double a4,
-                                          double a5, double a6) {
-  double2 *o = reinterpret_cast<double2 *>(rec);
-  o[0] = make_double2(a0, a1);
-  o[1] = make_double2(a2, a3);
-  o[2] = make_double2(a4, a5);
-  o[3] = make_double2(a6, 1.2 * a5);
-}
-
-// The record of one point of the FP64 sweeps.
+// FP64 stencils of the FP32-mixed form (TPLS_PART_MOM_STENCIL): conv and diff
+// in FP64, the defect right-hand side b = R / diag of the FP32 sweeps stored
+// FP32, R = dt (diff - AB3(conv) + AB3(csf)) (see k_mom_rhs_pair); the sweeps
+// rebuild the coefficients themselves.
 template <bool INTERIOR>
-__device__ __forceinline__ void write_coef(int comp, const Geo &g, const Helm &h, const FcT<double> &f,
-                                           double rhs, int k, double *__restrict__ rec) {
-  const double ax2 = h.ax2, ay2 = h.ay2, az2 = h.az2;
-  const double diag = 1.0 + ax2 * (f.px + f.mx) + ay2 * (f.py + f.my) + az2 * (f.pz + f.mz);
-  const double r = 1.0 / diag;
-  double czp = az2 * f.pz * r, czm = az2 * f.mz * r;
-  if (!INTERIOR && comp != 2) {
-    if (k == 0) {
-      czp += czm * (1.0 / 3.0);
-      czm = -2.0 * czm;
-    } else if (k == g.nz - 1) {
-      czm += czp * (1.0 / 3.0);
-      czp = -2.0 * czp;
-    }
-  }
-  store_rec(rec, ax2 * f.px * r, ax2 * f.mx * r, ay2 * f.py * r, ay2 * f.my * r, czp, czm, rhs * r);
-}
-
-// FP64 stencils.  TR = double: the FP64 form's right-hand side and 64-byte
-// sweep records (X64 = the component's FP64 state u2, v2 or w2); TR = float:
-// the FP32-mixed form with FP64 stencils, which stores the defect b alone.
-template <typename T, typename TR, bool INTERIOR>
-__device__ __forceinline__ void mom_rhs_point(int comp, const Geo &g, const Phys &ph, const Helm &hm,
-                                              const T *__restrict__ U, const T *__restrict__ V,
-                                              const T *__restrict__ W, const double *__restrict__ X64,
-                                              const T *__restrict__ mu, const T *__restrict__ fc,
-                                              const double *__restrict__ c1, const double *__restrict__ c0,
-                                              const double *__restrict__ s1, const double *__restrict__ s0,
-                                              double *__restrict__ conv2, double *__restrict__ csf2,
-                                              double *__restrict__ rhs, double *__restrict__ diff_out,
-                                              TR *__restrict__ coef, int i, int j, int k) {
+__device__ __forceinline__ void mom_b32_point(int comp, const Geo &g, const Phys &ph, const Helm &hm,
+                                              const double *__restrict__ U, const double *__restrict__ V,
+                                              const double *__restrict__ W, const double *__restrict__ mu,
+                                              const double *__restrict__ fc, const double *__restrict__ c1,
+                                              const double *__restrict__ c0, const double *__restrict__ s1,
+                                              const double *__restrict__ s0, double *__restrict__ conv2,
+                                              double *__restrict__ csf2, float *__restrict__ bdef, int i, int j,
+                                              int k) {
   const int c = TPLS_IDX(g, i, j, k);
-  CDT<T> cd = {(T)0, (T)0};
+  CDT<double> cd = {0.0, 0.0};
   const bool valid = cd_valid(comp, g, i, k);
-  FcT<T> f;
+  Fc f;
   if (valid) {
     f = faces(comp, g, mu, i, j, k);
     // 1/dx, 1/dy, 1/dz from the host (the same IEEE quotients, not three FP64
     // divisions per point on GB300's FP64 pipe)
-    cd = conv_diff<T, INTERIOR>(comp, g, (T)hm.rdx, (T)hm.rdy, (T)hm.rdz, U, V, W, f, i, j, k);
+    cd = conv_diff<double, INTERIOR>(comp, g, hm.rdx, hm.rdy, hm.rdz, U, V, W, f, i, j, k);
   }
   // main_ns_hybrid.F90:629-641 face averages of the CSF force
   double s2;
-  if (comp == 0) s2 = ((double)fc[TPLS_IDX(g, i + 1, j + 1, k + 1)] + (double)fc[TPLS_IDX(g, i, j + 1, k + 1)]) * 0.5;
-  else if (comp == 1) s2 = ((double)fc[TPLS_IDX(g, i, j + 1, k + 1)] + (double)fc[TPLS_IDX(g, i, j, k + 1)]) * 0.5;
-  else s2 = ((double)fc[TPLS_IDX(g, i, j + 1, k + 1)] + (double)fc[TPLS_IDX(g, i, j + 1, k)]) * 0.5;
-  const double dt = ph.dt, conv = (double)cd.conv, diff = (double)cd.diff;
-  if constexpr (sizeof(TR) == sizeof(float)) {
-    // FP32 defect-form sweeps: b = R / diag with R = dt (diff - AB3(conv) +
-    // AB3(csf)), the defect equation's right-hand side (see k_mom_rhs_pair),
-    // here in FP64; the sweeps rebuild the coefficients themselves
-    conv2[c] = conv;
-    csf2[c] = s2;
-    if (coef && valid) {
-      const double abc = (23.0 / 12.0) * conv - (4.0 / 3.0) * c1[c] + (5.0 / 12.0) * c0[c];
-      const double abs_ = (23.0 / 12.0) * s2 - (4.0 / 3.0) * s1[c] + (5.0 / 12.0) * s0[c];
-      const double diag =
-          1.0 + hm.ax2 * (f.px + f.mx) + hm.ay2 * (f.py + f.my) + hm.az2 * (f.pz + f.mz);
-      coef[rec_slot(g, c, i)] = (TR)(dt * (diff - abc + abs_) / diag);
-    }
-  } else {
-    const double X = X64[c];
-    // main_ns_hybrid.F90:743-751 (AB3 convection and CSF, CN diffusion)
-    const double r = X - dt * ((23.0 / 12.0) * conv - (4.0 / 3.0) * c1[c] + (5.0 / 12.0) * c0[c]) +
-                     (dt / 2.0) * diff +
-                     dt * ((23.0 / 12.0) * s2 - (4.0 / 3.0) * s1[c] + (5.0 / 12.0) * s0[c]);
-    conv2[c] = conv;
-    csf2[c] = s2;
-    if (rhs) rhs[c] = r;
-    if (diff_out) diff_out[c] = diff;
-    if (coef && valid) write_coef<INTERIOR>(comp, g, hm, f, r, k, coef + 8 * (size_t)rec_slot(g, c, i));
+  if (comp == 0) s2 = (fc[TPLS_IDX(g, i + 1, j + 1, k + 1)] + fc[TPLS_IDX(g, i, j + 1, k + 1)]) * 0.5;
+  else if (comp == 1) s2 = (fc[TPLS_IDX(g, i, j + 1, k + 1)] + fc[TPLS_IDX(g, i, j, k + 1)]) * 0.5;
+  else s2 = (fc[TPLS_IDX(g, i, j + 1, k + 1)] + fc[TPLS_IDX(g, i, j + 1, k)]) * 0.5;
+  conv2[c] = cd.conv;
+  csf2[c] = s2;
+  if (valid) {
+    const double abc = (23.0 / 12.0) * cd.conv - (4.0 / 3.0) * c1[c] + (5.0 / 12.0) * c0[c];
+    const double abs_ = (23.0 / 12.0) * s2 - (4.0 / 3.0) * s1[c] + (5.0 / 12.0) * s0[c];
+    const double diag = 1.0 + hm.ax2 * (f.px + f.mx) + hm.ay2 * (f.py + f.my) + hm.az2 * (f.pz + f.mz);
+    bdef[rec_slot(g, c, i)] = (float)(ph.dt * (cd.diff - abc + abs_) / diag);
   }
 }
 
 // CC: the velocity component at compile time.  The wall levels of u and v
 // (k = 0, nz-1) take their own copy of the point code by a block-uniform
 // branch, so the interior levels carry none of the wall forms.
-template <typename T, typename TR, int CC>
+template <int CC>
 __global__ void __launch_bounds__(MB_X *MB_Y)
-    k_mom_rhs(Geo g, Phys ph, Helm hm, const T *__restrict__ U, const T *__restrict__ V,
-              const T *__restrict__ W, const double *__restrict__ X64, const T *__restrict__ mu,
-              const T *__restrict__ fc, const double *__restrict__ c1, const double *__restrict__ c0,
-              const double *__restrict__ s1, const double *__restrict__ s0, double *__restrict__ conv2,
-              double *__restrict__ csf2, double *__restrict__ rhs, double *__restrict__ diff_out,
-              TR *__restrict__ coef) {
+    k_mom_b32(Geo g, Phys ph, Helm hm, const double *__restrict__ U, const double *__restrict__ V,
+              const double *__restrict__ W, const double *__restrict__ mu, const double *__restrict__ fc,
+              const double *__restrict__ c1, const double *__restrict__ c0, const double *__restrict__ s1,
+              const double *__restrict__ s0, double *__restrict__ conv2, double *__restrict__ csf2,
+              float *__restrict__ bdef) {
   const int i = blockIdx.x * MB_X + threadIdx.x + 1, j = blockIdx.y * MB_Y + threadIdx.y + 1;
   const int k = blockIdx.z;
   if (i > g.nx || j > g.ny) return;
   if (CC != 2 && (k == 0 || k == g.nz - 1))
-    mom_rhs_point<T, TR, false>(CC, g, ph, hm, U, V, W, X64, mu, fc, c1, c0, s1, s0, conv2, csf2, rhs, diff_out,
-                                coef, i, j, k);
+    mom_b32_point<false>(CC, g, ph, hm, U, V, W, mu, fc, c1, c0, s1, s0, conv2, csf2, bdef, i, j, k);
   else
-    mom_rhs_point<T, TR, true>(CC, g, ph, hm, U, V, W, X64, mu, fc, c1, c0, s1, s0, conv2, csf2, rhs, diff_out,
-                               coef, i, j, k);
-}
-
-template <typename T, typename TR = T>
-static cudaError_t mom_rhs(int comp, const Geo &g, const Phys &ph, const T *u2, const T *v2, const T *w2,
-                           const double *x64, const T *mu, const T *fcsf, const double *c1, const double *c0,
-                           const double *s1, const double *s0, double *conv2, double *csf2, double *rhs,
-                           double *diff_out, TR *coef, cudaStream_t st) {
-  const int nk = (comp == 2) ? g.nz + 1 : g.nz;
-  dim3 grd((g.nx + MB_X - 1) / MB_X, (g.ny + MB_Y - 1) / MB_Y, nk);
-  const Helm hm = helm_of(ph);
-  if (comp == 0)
-    k_mom_rhs<T, TR, 0><<<grd, dim3(MB_X, MB_Y), 0, st>>>(g, ph, hm, u2, v2, w2, x64, mu, fcsf, c1, c0, s1, s0,
-                                                          conv2, csf2, rhs, diff_out, coef);
-  else if (comp == 1)
-    k_mom_rhs<T, TR, 1><<<grd, dim3(MB_X, MB_Y), 0, st>>>(g, ph, hm, u2, v2, w2, x64, mu, fcsf, c1, c0, s1, s0,
-                                                          conv2, csf2, rhs, diff_out, coef);
-  else
-    k_mom_rhs<T, TR, 2><<<grd, dim3(MB_X, MB_Y), 0, st>>>(g, ph, hm, u2, v2, w2, x64, mu, fcsf, c1, c0, s1, s0,
-                                                          conv2, csf2, rhs, diff_out, coef);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_mom_rhs(int comp, const Geo &g, const Phys &ph,
-                           const double *u2, const double *v2,
-                           const double *w2, const double *mu,
-                           const double *fcsf, const double *c1,
-                           const double *c0, const double *s1,
-                           const double *s0, double *conv2, double *csf2,
-                           double *rhs, double *diff_out, double *coef, cudaStream_t st) {
-  const double *x64 = (comp == 0) ? u2 : (comp == 1) ? v2 : w2;
-  return mom_rhs<double>(comp, g, ph, u2, v2, w2, x64, mu, fcsf, c1, c0, s1, s0, conv2, csf2, rhs, diff_out,
-                         coef, st);
+    mom_b32_point<true>(CC, g, ph, hm, U, V, W, mu, fc, c1, c0, s1, s0, conv2, csf2, bdef, i, j, k);
 }
 
 cudaError_t launch_mom_rhs64r32(int comp, const Geo &g, const Phys &ph, const double *u2, const double *v2,
                                 const double *w2, const double *mu, const double *fcsf, const double *c1,
                                 const double *c0, const double *s1, const double *s0, double *conv2,
                                 double *csf2, float *bdef, cudaStream_t st) {
-  const double *x64 = (comp == 0) ? u2 : (comp == 1) ? v2 : w2;
-  return mom_rhs<double, float>(comp, g, ph, u2, v2, w2, x64, mu, fcsf, c1, c0, s1, s0, conv2, csf2, nullptr,
-                                nullptr, bdef, st);
+  const int nk = (comp == 2) ? g.nz + 1 : g.nz;
+  dim3 grd((g.nx + MB_X - 1) / MB_X, (g.ny + MB_Y - 1) / MB_Y, nk), blk(MB_X, MB_Y);
+  const Helm hm = helm_of(ph);
+  if (comp == 0) k_mom_b32<0><<<grd, blk, 0, st>>>(g, ph, hm, u2, v2, w2, mu, fcsf, c1, c0, s1, s0, conv2, csf2, bdef);
+  else if (comp == 1)
+    k_mom_b32<1><<<grd, blk, 0, st>>>(g, ph, hm, u2, v2, w2, mu, fcsf, c1, c0, s1, s0, conv2, csf2, bdef);
+  else k_mom_b32<2><<<grd, blk, 0, st>>>(g, ph, hm, u2, v2, w2, mu, fcsf, c1, c0, s1, s0, conv2, csf2, bdef);
+  return cudaGetLastError();
 }
+
+// ---------------------------------------------------------------------------
+// FP64 right-hand sides and sweep records (the FP64 form).  Bound by the FP64
+// pipe, so written for few operations (73 per point against 105 in the point
+// form above):
+//   * a thread marches kc levels of a column: the z faces' viscosity sums,
+//     shear and difference products of a level's upper face are the next
+//     level's lower face;
+//   * conv and diff share the normal stress p dE - m dW of the component's own
+//     axis; every axis' scales (1/2 of the centred difference, 1/4 of a
+//     four-cell average, the grid spacings) are one factor;
+//   * the AB3 and Crank-Nicolson combination is seven FMAs on factors that
+//     carry dt; 1/diag comes from rcp_seed and one Newton step.
+// All three components in one launch (gx blocks along x each).
+//
+// The record of one point (8 doubles): the neighbour coefficients divided by
+// the Helmholtz diagonal (jacobi_iteration_allflux.f90:84-90), x_new = cxp
+// x[i+1] + cxm x[i-1] + cyp x[j+1] + cym x[j-1] + czp x[k+1] + czm x[k-1] +
+// rhs/diag.  For u and v the wall ghost rule `-2 x(0) + x(1)/3` (and its top
+// mirror) is folded in: at k = 0 the czm slot multiplies the point itself and
+// czp absorbs czm/3; at k = nz-1 the czp slot multiplies the point itself and
+// czm absorbs czp/3.  Order (cxp, cxm, cyp, cym, czp, czm, b, 1.2 czm), the
+// last the factor of the odd half-sweep's column recurrence.
+struct MomK {
+  double vx, vy, vz;           // centred difference x velocity (sum of four where averaged)
+  double tx, ty, tz;           // shear of conv per axis: rd_own rd_axis (a quarter where averaged)
+  double lx, ly, lz;           // rd_axis^2 of diff (a quarter where averaged)
+  double ax, ay, az;           // dt/(2 d^2) (a quarter where averaged)
+  double k2, k1, k0, hd, l2, l1, l0;  // AB3 conv, CN diff and AB3 csf factors, dt included
+};
+struct MomArgs {
+  const double *U, *V, *W, *mu;
+  const double *f[3], *c1[3], *c0[3], *s1[3], *s0[3];
+  double *conv2[3], *csf2[3], *coef[3];
+  MomK q[3];
+};
+
+// The z face of a level as the level above needs it: the four-cell (w: single)
+// viscosity, its products with the shear difference and with the component's
+// own difference, and what the next face is formed from.
+struct MomFace {
+  double m, sh, own;
+};
+
+template <int CC>
+__device__ __forceinline__ void mom_column(const Geo &g, const MomArgs &A, int i, int j, int ka, int kb) {
+  const int sy = g.sy, sz = g.sz, my = g.sy, mz = g.szm, nz = g.nz;
+  const MomK &q = A.q[CC];
+  const double *__restrict__ U = A.U, *__restrict__ V = A.V, *__restrict__ W = A.W;
+  const double *__restrict__ S = (CC == 0) ? U : (CC == 1 ? V : W);
+  // the cell on the far side of the face: +x (u), -y (v), +z (w) of the near one
+  const int om = (CC == 0) ? 1 : (CC == 1 ? -my : mz);
+  const int oq = (CC == 0) ? 1 : (CC == 1 ? -sy : -sz);  // and in the velocity arrays, towards the other face point
+  const bool inside = CC != 0 || i <= g.nx - 1;
+  const double *f = A.f[CC], *c1 = A.c1[CC], *c0 = A.c0[CC], *s1 = A.s1[CC], *s0 = A.s0[CC];
+  double *conv2 = A.conv2[CC], *csf2 = A.csf2[CC], *coef = A.coef[CC];
+  double x = 0.0, mn = 0.0, mf = 0.0, ws = 0.0, fz = 0.0;
+  MomFace lo = {0.0, 0.0, 0.0};
+  // near-cell viscosity index of level k (u, v: level k+1 of the p-grid; w: k)
+  auto mi = [&](int k) { return TPLS_IDXM(g, i, j + 1, k + (CC == 2 ? 0 : 1)); };
+  bool started = false;
+  for (int k = ka; k <= kb; k++) {
+    const int c = TPLS_IDX(g, i, j, k);
+    const bool level = (CC != 2) || (k >= 1 && k <= nz - 1);
+    double conv = 0.0, diff = 0.0;
+    double px = 0.0, mx = 0.0, py = 0.0, myv = 0.0, pz = 0.0, mzv = 0.0, sx = 0.0, xc = 0.0;
+    const bool valid = inside && level;
+    if (valid) {
+      if (!started) {  // the lower face of the chunk's first level
+        started = true;
+        x = S[c];
+        mn = A.mu[mi(k)];
+        mf = A.mu[mi(k) + om];
+        if (CC == 2) {
+          lo.m = mn;
+          lo.own = mn * (x - S[c - sz]);
+        } else {
+          lo.m = (mn + mf) + (A.mu[mi(k) - mz] + A.mu[mi(k) - mz + om]);
+          const double w0 = W[c], w1 = W[c + oq];
+          ws = w0 + w1;
+          lo.sh = lo.m * (CC == 0 ? w1 - w0 : w0 - w1);
+          if (k > 0) lo.own = lo.m * (x - S[c - sz]);
+        }
+      }
+      const double xe = S[c + 1], xw = S[c - 1], xn = S[c + sy], xs = S[c - sy];
+      const double dE = xe - x, dW = x - xw, dN = xn - x, dS = x - xs;
+      // viscosity sums of the faces, and the level's upper face
+      const double *m = A.mu + mi(k);
+      const double near = mn + mf;  // the two cells of this point's own face
+      double mn1 = 0.0, mf1 = 0.0;
+      MomFace hi;
+      double xt = 0.0, dT, dB2, ws1 = 0.0;  // dB2: the centred difference's lower half
+      if (CC == 2) {
+        hi.m = mf;  // mu of level k+1
+        xt = S[c + sz];
+        dT = xt - x;
+        hi.sh = 0.0;
+        hi.own = hi.m * dT;
+        dB2 = x - S[c - sz];
+        mn1 = mf;
+        mf1 = m[2 * mz];
+        px = near + (m[1] + m[1 + mz]);
+        mx = near + (m[-1] + m[-1 + mz]);
+        py = near + (m[my] + m[my + mz]);
+        myv = near + (m[-my] + m[-my + mz]);
+        pz = hi.m;
+        mzv = lo.m;
+        sx = near;
+      } else {
+        mn1 = m[mz];
+        mf1 = m[mz + om];
+        hi.m = near + (mn1 + mf1);
+        const double w0 = W[c + sz], w1 = W[c + sz + oq];
+        ws1 = w0 + w1;
+        hi.sh = hi.m * (CC == 0 ? w1 - w0 : w0 - w1);
+        pz = hi.m;
+        mzv = lo.m;
+        if (CC == 0) {
+          px = mf;
+          mx = mn;
+          py = near + (m[my] + m[my + 1]);
+          myv = near + (m[-my] + m[-my + 1]);
+        } else {
+          px = near + (m[1] + m[1 - my]);
+          mx = near + (m[-1] + m[-1 - my]);
+          py = mn;
+          myv = mf;
+        }
+        sx = near;
+        dT = 0.0;
+        dB2 = 0.0;
+      }
+      // z differences; at the walls of u and v the ghost -2 x + x(k+-1)/3
+      double dz;
+      if (CC == 2) {
+        dz = dT + dB2;
+      } else if (k == 0) {
+        xt = S[c + sz];
+        dT = xt - x;
+        hi.own = hi.m * dT;
+        lo.own = lo.m * fma(-1.0 / 3.0, xt, 3.0 * x);
+        dz = x + xt;
+      } else if (k == nz - 1) {
+        const double xb = S[c - sz];
+        hi.own = hi.m * fma(1.0 / 3.0, xb, -3.0 * x);
+        dz = -(x + xb);
+      } else {
+        xt = S[c + sz];
+        dT = xt - x;
+        hi.own = hi.m * dT;
+        dz = xt - S[c - sz];
+      }
+      // velocities at the point (sums of four) and shear of the other two components
+      double vx, vy, vz, shx, shy;
+      if (CC == 0) {
+        const double a0 = V[c], a1 = V[c + 1], b0 = V[c + sy], b1 = V[c + 1 + sy];
+        vx = x;
+        vy = (a0 + a1) + (b0 + b1);
+        vz = ws + ws1;
+        shx = 0.0;
+        shy = fma(py, b1 - b0, -myv * (a1 - a0));
+      } else if (CC == 1) {
+        const double a0 = U[c - 1 - sy], a1 = U[c - 1], b0 = U[c - sy], b1 = U[c];
+        vx = (a0 + a1) + (b0 + b1);
+        vy = x;
+        vz = ws + ws1;
+        shx = fma(px, b1 - b0, -mx * (a1 - a0));
+        shy = 0.0;
+      } else {
+        const double a0 = U[c - 1 - sz], a1 = U[c - 1], b0 = U[c - sz], b1 = U[c];
+        const double d0 = V[c - sz], d1 = V[c], e0 = V[c + sy - sz], e1 = V[c + sy];
+        vx = (a0 + a1) + (b0 + b1);
+        vy = (d0 + d1) + (e0 + e1);
+        vz = x;
+        shx = fma(px, b1 - b0, -mx * (a1 - a0));
+        shy = fma(py, e1 - e0, -myv * (d1 - d0));
+      }
+      const double nx_ = fma(px, dE, -mx * dW), ny_ = fma(py, dN, -myv * dS), nz_ = hi.own - lo.own;
+      conv = q.vx * ((xe - xw) * vx);
+      conv = fma(q.vy, (xn - xs) * vy, conv);
+      conv = fma(q.vz, dz * vz, conv);
+      // shear of conv: the component's own axis shares diff's normal stress
+      if (CC == 0) {
+        conv = fma(-q.tx, nx_, conv);
+        conv = fma(-q.ty, shy, conv);
+        conv = fma(-q.tz, hi.sh - lo.sh, conv);
+      } else if (CC == 1) {
+        conv = fma(-q.tx, shx, conv);
+        conv = fma(-q.ty, ny_, conv);
+        conv = fma(-q.tz, hi.sh - lo.sh, conv);
+      } else {
+        conv = fma(-q.tx, shx, conv);
+        conv = fma(-q.ty, shy, conv);
+        conv = fma(-q.tz, nz_, conv);
+      }
+      diff = q.lx * nx_;
+      diff = fma(q.ly, ny_, diff);
+      diff = fma(q.lz, nz_, diff);
+      lo = hi;
+      xc = x;
+      x = xt;
+      mn = mn1;
+      mf = mf1;
+      ws = ws1;
+    }
+    // main_ns_hybrid.F90:629-641 face averages of the CSF force
+    double s2;
+    if (CC == 0) s2 = (f[TPLS_IDX(g, i + 1, j + 1, k + 1)] + f[TPLS_IDX(g, i, j + 1, k + 1)]) * 0.5;
+    else if (CC == 1) s2 = (f[TPLS_IDX(g, i, j + 1, k + 1)] + f[TPLS_IDX(g, i, j, k + 1)]) * 0.5;
+    else {
+      const double fn = f[TPLS_IDX(g, i, j + 1, k + 1)];
+      if (k == ka) fz = f[TPLS_IDX(g, i, j + 1, k)];
+      s2 = (fn + fz) * 0.5;
+      fz = fn;
+    }
+    conv2[c] = conv;
+    csf2[c] = s2;
+    if (valid) {
+      // main_ns_hybrid.F90:743-751 (AB3 convection and CSF, CN diffusion)
+      double r = fma(q.k2, conv, xc);
+      r = fma(q.k1, c1[c], r);
+      r = fma(q.k0, c0[c], r);
+      r = fma(q.hd, diff, r);
+      r = fma(q.l2, s2, r);
+      r = fma(q.l1, s1[c], r);
+      r = fma(q.l0, s0[c], r);
+      // the own axis' two faces are the two cells `near` sums (u: px + mx, v: py + my, w: pz + mz)
+      double d = fma(q.ax, CC == 0 ? sx : px + mx, 1.0);
+      d = fma(q.ay, CC == 1 ? sx : py + myv, d);
+      d = fma(q.az, CC == 2 ? sx : pz + mzv, d);
+      double h;
+      if (rcp_range(d)) {
+        h = rcp_seed(d);
+        h = fma(h, fma(-d, h, 1.0), h);
+      } else {
+        h = div_slow(1.0, d);
+      }
+      const double hx = q.ax * h, hy = q.ay * h, hz = q.az * h;
+      double czp = hz * pz, czm = hz * mzv;
+      if (CC != 2) {
+        if (k == 0) {
+          czp = fma(czm, 1.0 / 3.0, czp);
+          czm = -2.0 * czm;
+        } else if (k == nz - 1) {
+          czm = fma(czp, 1.0 / 3.0, czm);
+          czp = -2.0 * czp;
+        }
+      }
+      double2 *o = reinterpret_cast<double2 *>(coef + 8 * (size_t)rec_slot(g, c, i));
+      o[0] = make_double2(hx * px, hx * mx);
+      o[1] = make_double2(hy * py, hy * myv);
+      o[2] = make_double2(czp, czm);
+      o[3] = make_double2(r * h, 1.2 * czm);
+    }
+  }
+}
+
+// Levels per thread: 8, halved to no less than 2 while the three components
+// give fewer than eight blocks per SM.
+__global__ void __launch_bounds__(MB_X *MB_Y)
+    k_mom_rhs(Geo g, const __grid_constant__ MomArgs A, int gx, int kc) {
+  const int comp = blockIdx.x / gx, i = (blockIdx.x - comp * gx) * MB_X + threadIdx.x + 1;
+  const int j = blockIdx.y * MB_Y + threadIdx.y + 1;
+  const int last = (comp == 2) ? g.nz : g.nz - 1, ka = blockIdx.z * kc, kb = min(ka + kc - 1, last);
+  if (i > g.nx || j > g.ny || ka > last) return;
+  if (comp == 0) mom_column<0>(g, A, i, j, ka, kb);
+  else if (comp == 1) mom_column<1>(g, A, i, j, ka, kb);
+  else mom_column<2>(g, A, i, j, ka, kb);
+}
+
+cudaError_t launch_mom_rhs(const Geo &g, const Phys &ph, const double *u2, const double *v2, const double *w2,
+                           const double *mu, const MomFields &m, cudaStream_t st) {
+  const Helm hm = helm_of(ph);
+  MomArgs A;
+  A.U = u2;
+  A.V = v2;
+  A.W = w2;
+  A.mu = mu;
+  const double rd[3] = {hm.rdx, hm.rdy, hm.rdz}, a2[3] = {hm.ax2, hm.ay2, hm.az2};
+  for (int q = 0; q < 3; q++) {
+    A.f[q] = m.fcsf[q];
+    A.c1[q] = m.c1[q];
+    A.c0[q] = m.c0[q];
+    A.s1[q] = m.s1[q];
+    A.s0[q] = m.s0[q];
+    A.conv2[q] = m.conv2[q];
+    A.csf2[q] = m.csf2[q];
+    A.coef[q] = m.coef[q];
+    double v[3], t[3], l[3], a[3];
+    for (int d = 0; d < 3; d++) {
+      const double s = (d == q) ? 1.0 : 0.25;
+      v[d] = 0.5 * rd[d] * s;
+      t[d] = rd[q] * rd[d] * s;
+      l[d] = rd[d] * rd[d] * s;
+      a[d] = a2[d] * s;
+    }
+    A.q[q] = {v[0], v[1], v[2], t[0], t[1], t[2], l[0], l[1], l[2], a[0], a[1], a[2],
+              -ph.dt * (23.0 / 12.0), ph.dt * (4.0 / 3.0), -ph.dt * (5.0 / 12.0), ph.dt / 2.0,
+              ph.dt * (23.0 / 12.0), -ph.dt * (4.0 / 3.0), ph.dt * (5.0 / 12.0)};
+  }
+  const int gx = (g.nx + MB_X - 1) / MB_X, gy = (g.ny + MB_Y - 1) / MB_Y;
+  int kc = 8;
+  while (kc > 2 && 3 * gx * gy * ((g.nz + kc) / kc) < 8 * 152) kc /= 2;
+  k_mom_rhs<<<dim3(3 * gx, gy, (g.nz + kc) / kc), dim3(MB_X, MB_Y), 0, st>>>(g, A, gx, kc);
+  return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------------------
 // FP32 momentum stencils of the FP32-mixed form on the FP64 velocity state.
 //

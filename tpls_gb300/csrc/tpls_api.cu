@@ -1170,6 +1170,25 @@ static int dim_stage(tpls_ctx *c, const double *conv2_phi) {
   return TPLS_OK;
 }
 
+// The three components' right-hand side arrays of this history phase.
+static MomFields mom_fields(const tpls_ctx *c) {
+  const int s0 = c->phase % 3, s1 = (c->phase + 1) % 3, s2 = (c->phase + 2) % 3;
+  MomFields m;
+  double *const *conv[3] = {c->conv_u, c->conv_v, c->conv_w}, *const *csf[3] = {c->csf_u, c->csf_v, c->csf_w};
+  const double *f[3] = {c->fx, c->fy, c->fz};
+  for (int q = 0; q < 3; q++) {
+    m.fcsf[q] = f[q];
+    m.c1[q] = conv[q][s1];
+    m.c0[q] = conv[q][s0];
+    m.s1[q] = csf[q][s1];
+    m.s0[q] = csf[q][s0];
+    m.conv2[q] = conv[q][s2];
+    m.csf2[q] = csf[q][s2];
+    m.coef[q] = c->coef[q];
+  }
+  return m;
+}
+
 // The front of a step: viscosity, advection, level set, CSF and the
 // momentum right-hand sides.  Every state field but u2, v2, w2, pres and
 // pres_old is final after it (front_final).
@@ -1219,15 +1238,7 @@ static int step_front(tpls_ctx *c) {
   {
     PhaseScope rhs_scope(c, TPLS_T_MOM_RHS);
     // convective / diffusive terms and AB3 + CN right-hand sides (:728-751)
-    LCK(c, launch_mom_rhs(0, g, ph, c->u2, c->v2, c->w2, c->mu, c->fx, c->conv_u[s1], c->conv_u[s0],
-                          c->csf_u[s1], c->csf_u[s0], c->conv_u[s2], c->csf_u[s2], nullptr, nullptr, c->coef[0],
-                          st));
-    LCK(c, launch_mom_rhs(1, g, ph, c->u2, c->v2, c->w2, c->mu, c->fy, c->conv_v[s1], c->conv_v[s0],
-                          c->csf_v[s1], c->csf_v[s0], c->conv_v[s2], c->csf_v[s2], nullptr, nullptr, c->coef[1],
-                          st));
-    LCK(c, launch_mom_rhs(2, g, ph, c->u2, c->v2, c->w2, c->mu, c->fz, c->conv_w[s1], c->conv_w[s0],
-                          c->csf_w[s1], c->csf_w[s0], c->conv_w[s2], c->csf_w[s2], nullptr, nullptr, c->coef[2],
-                          st));
+    LCK(c, launch_mom_rhs(g, ph, c->u2, c->v2, c->w2, c->mu, mom_fields(c), st));
   }
   return TPLS_OK;
 }
@@ -1358,15 +1369,7 @@ static int mixed_front(tpls_ctx *c) {
     }
     {
       PhaseScope ps(c, TPLS_T_MOM_RHS);
-      LCK(c, launch_mom_rhs(0, g, ph, c->u2, c->v2, c->w2, c->mu, c->fx, c->conv_u[s1], c->conv_u[s0],
-                            c->csf_u[s1], c->csf_u[s0], c->conv_u[s2], c->csf_u[s2], nullptr, nullptr, c->coef[0],
-                            st));
-      LCK(c, launch_mom_rhs(1, g, ph, c->u2, c->v2, c->w2, c->mu, c->fy, c->conv_v[s1], c->conv_v[s0],
-                            c->csf_v[s1], c->csf_v[s0], c->conv_v[s2], c->csf_v[s2], nullptr, nullptr, c->coef[1],
-                            st));
-      LCK(c, launch_mom_rhs(2, g, ph, c->u2, c->v2, c->w2, c->mu, c->fz, c->conv_w[s1], c->conv_w[s0],
-                            c->csf_w[s1], c->csf_w[s0], c->conv_w[s2], c->csf_w[s2], nullptr, nullptr, c->coef[2],
-                            st));
+      LCK(c, launch_mom_rhs(g, ph, c->u2, c->v2, c->w2, c->mu, mom_fields(c), st));
     }
     if ((s = momentum64(c))) return s;
   } else if (sten64) {

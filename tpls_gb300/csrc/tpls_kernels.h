@@ -100,16 +100,15 @@ cudaError_t launch_csf(const Geo &g, const Phys &ph, const double *phi3,
 cudaError_t launch_visc(const Geo &g, const Phys &ph, const double *phi2,
                         float *mu, cudaStream_t st);
 
-// momentum_allflux.f90 + main_ns_hybrid.F90:629-641,743-751: per component
-// conv2, csf2 (history) and the AB3/CN right-hand side.
-cudaError_t launch_mom_rhs(int comp, const Geo &g, const Phys &ph,
-                           const double *u2, const double *v2,
-                           const double *w2, const double *mu,
-                           const double *fcsf, const double *c1,
-                           const double *c0, const double *s1,
-                           const double *s0, double *conv2, double *csf2,
-                           double *rhs, double *diff_out, double *coef,
-                           cudaStream_t st);
+// momentum_allflux.f90 + main_ns_hybrid.F90:629-641,743-751 of the three
+// components: conv2, csf2 (history) and the sweep records of the AB3/CN
+// right-hand side.
+struct MomFields {
+  const double *fcsf[3], *c1[3], *c0[3], *s1[3], *s0[3];
+  double *conv2[3], *csf2[3], *coef[3];
+};
+cudaError_t launch_mom_rhs(const Geo &g, const Phys &ph, const double *u2, const double *v2, const double *w2,
+                           const double *mu, const MomFields &m, cudaStream_t st);
 // FP32-mixed form: FP32 stencils on the FP64 velocity state split into
 // FP32 pairs by integer operations and FP32 viscosity, FP64 CSF force and
 // AB3 combination; writes the defect-form b of the FP32 sweeps (one float
