@@ -883,19 +883,21 @@ __global__ void k_diff2(Geo g, const T *__restrict__ a, const T *__restrict__ b,
     const T d = a[c] - b[c];
     e = d * d;
   }
-  __shared__ double s[MB_X * MB_Y / 32];
-  for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
-  const int t = threadIdx.y * MB_X + threadIdx.x;
+  const int t = threadIdx.y * MB_X + threadIdx.x, blk = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
   if constexpr (sizeof(T) == sizeof(float)) {
+    __shared__ double s[MB_X * MB_Y / 32];
+    for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
     if ((t & 31) == 0) s[t >> 5] = widen_bits(e);
+    __syncthreads();
+    if (t == 0) {
+      double acc = 0.0;
+      for (int q = 0; q < MB_X * MB_Y / 32; q++) acc += s[q];
+      part[blk] = acc;
+    }
   } else {
-    if ((t & 31) == 0) s[t >> 5] = e;
-  }
-  __syncthreads();
-  if (t == 0) {
-    double acc = 0.0;
-    for (int q = 0; q < MB_X * MB_Y / 32; q++) acc += s[q];
-    part[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = acc;
+    __shared__ double s[MB_X * MB_Y];
+    const double acc = block_sum<MB_X * MB_Y / 32>(e, t, s);
+    if (t == 0) part[blk] = acc;
   }
 }
 

@@ -2001,12 +2001,10 @@ __global__ void k_volume(Geo g, Phys ph, const double *__restrict__ phi, double 
     else hv = 0.5 + (p / (2.0 * ph.sw)) + (1.0 / (2.0 * TPLS_PI_SP)) * sin(TPLS_PI_SP * p / ph.sw);
     e = 1.0 - hv;
   }
-  for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
-  __shared__ double s[4];
+  __shared__ double s[128];
   const int t = threadIdx.y * 32 + threadIdx.x;
-  if ((t & 31) == 0) s[t >> 5] = e;
-  __syncthreads();
-  if (t == 0) part[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = s[0] + s[1] + s[2] + s[3];
+  const double a = block_sum<4>(e, t, s);
+  if (t == 0) part[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = a;
 }
 
 int tpls_timing_enable(tpls_ctx *c, int on) {

@@ -95,6 +95,41 @@ __device__ __forceinline__ double div_fast(double n, double d) {
   return fma(fma(-d, q, n), r, q);
 }
 
+// sqrt(a), correctly rounded, with one FP64 operation: an FP32 pair (sh, sl)
+// of the root to about 2^-43, joined to a double s0 by integer addition; the
+// exact residual a - s0^2 by one FMA; the correction c = residual / (2 s0) in
+// FP32, in units of s0's last place, rounded to an integer and added to the
+// bits.  c is known to 2^-21.4 of itself (rsqrtf's two ulps and four FP32
+// roundings), so where it lies that close to half-way between two integers,
+// or a sum leaves the binade, the library's sqrt decides (about 1 in 3000).
+// (a in 2^-60 .. 2^60; everything else goes there too.)
+static __device__ __noinline__ double sqrt_slow(double a) { return sqrt(a); }
+__device__ __forceinline__ double add_ulps(double x, int n) {
+  unsigned lo, hi;
+  asm("add.cc.u32 %0, %2, %4;\n\taddc.u32 %1, %3, %5;"
+      : "=r"(lo), "=r"(hi)
+      : "r"(__double2loint(x)), "r"(__double2hiint(x)), "r"(n), "r"(n >> 31));
+  return __hiloint2double((int)hi, (int)lo);
+}
+__device__ __forceinline__ double sqrt_rn(double a) {
+  if ((unsigned)__double2hiint(a) - (963u << 20) >= (120u << 20)) return sqrt_slow(a);
+  const F2 p = split_bits(a);
+  const float r = rsqrtf(p.h), hr = 0.5f * r;
+  const float sh = p.h * r;
+  const float sl = (fmaf(-sh, sh, p.h) + p.l) * hr;
+  const unsigned eb = __float_as_uint(sh) >> 23;
+  const float scale = __uint_as_float((306u - eb) << 23);  // 2^52 / 2^exponent(sh)
+  const double s = widen_bits(sh);
+  const double s0 = add_ulps(s, __float2int_rn(sl * scale));
+  const float cu = float_bits(fma(-s0, s0, a)) * hr * scale;
+  const float n = (cu + 12582912.0f) - 12582912.0f;  // nearest integer for |cu| < 2^22
+  const double r0 = add_ulps(s0, (int)n);
+  const int es = __double2hiint(s);
+  const bool sure = fabsf(cu - n) <= 0.5f - fmaf(fabsf(cu), 9.5367431640625e-7f, 1.52587890625e-5f) &&
+                    fabsf(cu) < 65536.0f && (((es ^ __double2hiint(s0)) | (es ^ __double2hiint(r0))) >> 20) == 0;
+  return sure ? r0 : sqrt_slow(a);
+}
+
 // order of two pairs of the same normalisation (both from split_bits, or
 // both from an error-free sum): by hi, then by lo
 __device__ __forceinline__ F2 pmin(F2 a, F2 b) { return (b.h < a.h || (b.h == a.h && b.l < a.l)) ? b : a; }
