@@ -225,6 +225,7 @@ class _Tiles:
 
     def load(self, a, i, j, k):
         nx, ny, nz = self.n
+        assert -ny <= j < 2 * ny  # one wrap
         return _Kernels.get(a, i + nx * (j % ny + ny * k))
 
     def relax(self, e, l, rhs, i, k):
@@ -293,6 +294,7 @@ class _Tiles:
             K = np.zeros((CZ + 4, CY + 4, CX + 4))
             for z, y, x in np.ndindex(K.shape):
                 ic, kc = min(max(x0 // 2 - 2 + x, 0), ncx - 1), min(max(z0 // 2 - 2 + z, 0), ncz - 1)
+                assert -ncy <= y0 // 2 - 2 + y < 2 * ncy
                 K[z, y, x] = _Kernels.get(ec, ic + ncx * ((y0 // 2 - 2 + y) % ncy + ncy * kc))
             Z = np.stack([lerp(K[pair(l)[0]], K[pair(l)[1]], not 0 <= z0 // 2 - 2 + pair(l)[1] < ncz)
                           for l in range(2 * CZ + 4)])
@@ -325,7 +327,7 @@ class _Tiles:
 
 
 @pytest.mark.parametrize("tile", [(8, 2, 2)])
-@pytest.mark.parametrize("size", [(4, 4, 4), (8, 6, 4), (34, 10, 10), (18, 4, 14)])
+@pytest.mark.parametrize("size", [(4, 4, 4), (8, 6, 4), (34, 10, 10), (18, 4, 14), (6, 8, 6)])
 def test_tile_kernels_equal_the_general_passes(size, tile):
     nx, ny, nz = size
     rng = np.random.default_rng(nx + ny)

@@ -58,7 +58,7 @@ struct PLevel {
 struct PoissonSolver {
   int nx, ny, nz, N;
   std::vector<PLevel> lv;
-  double *cinv = nullptr;  // coarsest pseudo-inverse (nc x nc; FP32 levels: transposed), or null
+  double *cinv = nullptr;  // coarsest pseudo-inverse (nc x nc), or null
   int coarse_sweeps = 0;
   double *modes = nullptr;  // coarsest level by modes: Qz, Qy, lambda_z, lambda_y
   double *x = nullptr, *r = nullptr, *p = nullptr, *q = nullptr, *bvec = nullptr;
@@ -117,24 +117,44 @@ static inline int nblocks(int n) { return (n + PB - 1) / PB; }
 // an atomic ticket) summing the partials in a fixed order.  The result does
 // not depend on scheduling.  Returns true in the last block, with the sums
 // in tot[] of thread 0.
+// A block's sums are the trees of its eight warps added in warp order.  The
+// trees run in shared memory, a level of all warps and sums at a time, so a
+// sum takes 17 FP64 warp instructions instead of the 48 of a shuffle tree in
+// every warp (most of them on idle lanes), in the same order: 1216 blocks of
+// three sums had spent 11 us on them, of a kernel of 33 us at 192x96x112.
+template <int NQ>
+__device__ __forceinline__ void block_sums(const double (&v)[NQ], double (&out)[NQ]) {  // in thread 0
+  __shared__ double sh[NQ][PB];
+  const int t = threadIdx.x;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NQ; q++) sh[q][t] = v[q];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    __syncthreads();
+    for (int m = t; m < NQ * (PB / 32) * o; m += PB) {
+      const int q = m / (PB / 32 * o), w = m / o % (PB / 32), l = m % o;
+      sh[q][32 * w + l] += sh[q][32 * w + l + o];
+    }
+  }
+  __syncthreads();
+  if (t == 0) {
+    for (int q = 0; q < NQ; q++) {
+      double a = 0.0;
+      for (int w = 0; w < PB / 32; w++) a += sh[q][32 * w];
+      out[q] = a;
+    }
+  }
+}
 template <int NQ>
 __device__ __forceinline__ bool reduce_last(double (&v)[NQ], double *part, unsigned *counter,
                                             double (&tot)[NQ]) {
-  __shared__ double sh[NQ][PB / 32];
   __shared__ bool last;
   const int nblk = gridDim.x;
-  for (int q = 0; q < NQ; q++) {
-    double a = v[q];
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-    if ((threadIdx.x & 31) == 0) sh[q][threadIdx.x >> 5] = a;
-  }
-  __syncthreads();
+  double a[NQ];
+  block_sums<NQ>(v, a);
   if (threadIdx.x == 0) {
-    for (int q = 0; q < NQ; q++) {
-      double a = 0.0;
-      for (int w = 0; w < PB / 32; w++) a += sh[q][w];
-      part[(size_t)q * nblk + blockIdx.x] = a;
-    }
+    for (int q = 0; q < NQ; q++) part[(size_t)q * nblk + blockIdx.x] = a[q];
     __threadfence();
     last = (atomicAdd(counter, 1u) == (unsigned)(nblk - 1));
   }
@@ -142,20 +162,11 @@ __device__ __forceinline__ bool reduce_last(double (&v)[NQ], double *part, unsig
   if (!last) return false;
   __threadfence();
   for (int q = 0; q < NQ; q++) {
-    double a = 0.0;
-    for (int b = threadIdx.x; b < nblk; b += PB) a += __ldcg(part + (size_t)q * nblk + b);
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-    if ((threadIdx.x & 31) == 0) sh[q][threadIdx.x >> 5] = a;
+    v[q] = 0.0;
+    for (int b = threadIdx.x; b < nblk; b += PB) v[q] += __ldcg(part + (size_t)q * nblk + b);
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int q = 0; q < NQ; q++) {
-      double a = 0.0;
-      for (int w = 0; w < PB / 32; w++) a += sh[q][w];
-      tot[q] = a;
-    }
-    *counter = 0u;
-  }
+  block_sums<NQ>(v, tot);
+  if (threadIdx.x == 0) *counter = 0u;
   return true;
 }
 
@@ -323,17 +334,19 @@ __global__ void __launch_bounds__(PB)
   using T = MgTile<CX, CY, CZ>;
   __shared__ double se[T::EN];
   __shared__ double ss[T::SN];
+  __shared__ double sb[T::EN];
   const int gx = (L.nx / 2 + CX - 1) / CX, gy = (L.ny / 2 + CY - 1) / CY;
   const int x0 = (blockIdx.x % gx) * T::FX, y0 = (blockIdx.x / gx % gy) * T::FY, z0 = blockIdx.x / (gx * gy) * T::FZ;
-  mg_up_tile<double, CX, CY, CZ>(L, b, ec, se, ss, x0, y0, z0);
+  mg_up_tile<double, CX, CY, CZ>(L, b, ec, se, ss, sb, x0, y0, z0);
   double v[1] = {0.0};
   for (int q = threadIdx.x; q < T::FX * T::FY * T::FZ; q += PB) {
     const int lx = q % T::FX, ly = q / T::FX % T::FY, lz = q / (T::FX * T::FY);
     if (x0 + lx < L.nx && y0 + ly < L.ny && z0 + lz < L.nz) {
       const size_t c = x0 + lx + L.nx * (y0 + ly + (size_t)L.ny * (z0 + lz));
-      const double z = se[lx + 2 + T::EX * (ly + 2 + T::EY * (lz + 2))];
+      const int o = lx + 2 + T::EX * (ly + 2 + T::EY * (lz + 2));
+      const double z = se[o];
       e[c] = z;
-      v[0] = fma(b[c], z, v[0]);
+      v[0] = fma(sb[o], z, v[0]);
     }
   }
   double tot[1];
@@ -745,48 +758,25 @@ __global__ void k_restrict_axis(int ax, int periodic, int nx, int ny, int nz, in
 }
 
 // coarsest grid: e = Cinv b (the pseudo-inverse and the products stay FP64
-// in both forms).  One block with a thread per row of a row-major matrix took
-// 27.8 us at 192 unknowns and 144 us at 504 (every lane on its own row of a
-// 2 MB matrix, one SM's FP64 pipe).
-// FP64 levels: one warp per row, eight rows per block, lanes along the row
-// (4.6 us at 192).
+// in both forms).  One warp per row, eight rows per block, lanes along the
+// row: 4.6 us at 192 unknowns, where one block with a thread per row took 27.8
+// us (144 us at 504: every lane on its own row of a 2 MB matrix, one SM's FP64
+// pipe, and a chain of 504 dependent FMAs).
 constexpr int CSB = 8;
+template <typename T>
 __global__ void __launch_bounds__(CSB * 32)
-    k_coarse_solve(int n, const double *__restrict__ cinv, const double *__restrict__ b, double *__restrict__ e) {
+    k_coarse_solve(int n, const double *__restrict__ cinv, const T *__restrict__ b, T *__restrict__ e) {
   const int a = blockIdx.x * CSB + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (a >= n) return;
   const double *row = cinv + (size_t)a * n;
   double acc = 0.0;
-  for (int q = lane; q < n; q += 32) acc = fma(row[q], b[q], acc);
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  if (lane == 0) e[a] = acc;
-}
-// FP32 levels: a thread per row, eight rows per block, the products summed in
-// the row's order (see cg_beta) by one warp, from shared memory where all the
-// block's rows are brought at once (of the transposed matrix: eight
-// neighbouring entries per load); bound by the chain of n dependent FMAs.
-constexpr int CS32 = 8;
-__global__ void __launch_bounds__(256)
-    k_coarse_solve32(int n, const double *__restrict__ cinvt, const float *__restrict__ b, float *__restrict__ e) {
-  __shared__ double sb[512], sm[512 * CS32];
-  const int a0 = blockIdx.x * CS32, m = min(CS32, n - a0);
-  for (int q = threadIdx.x; q < n; q += 256) sb[q] = widen_bits(b[q]);
 #pragma unroll 4
-  for (int q = threadIdx.x; q < n * CS32; q += 256)
-    sm[q] = (q % CS32 < m) ? cinvt[(size_t)(q / CS32) * n + a0 + q % CS32] : 0.0;
-  __syncthreads();
-  if (threadIdx.x < m) {
-    double acc = 0.0;
-#pragma unroll 8
-    for (int q = 0; q < n; q++) acc = fma(sm[q * CS32 + threadIdx.x], sb[q], acc);
-    e[a0 + threadIdx.x] = (float)acc;
+  for (int q = lane; q < n; q += 32) {
+    if constexpr (sizeof(T) == sizeof(float)) acc = fma(row[q], widen_bits(b[q]), acc);
+    else acc = fma(row[q], b[q], acc);
   }
-}
-static void coarse_solve(int n, const double *cinv, const double *b, double *e, cudaStream_t st) {
-  k_coarse_solve<<<(n + CSB - 1) / CSB, CSB * 32, 0, st>>>(n, cinv, b, e);
-}
-static void coarse_solve(int n, const double *cinvt, const float *b, float *e, cudaStream_t st) {
-  k_coarse_solve32<<<(n + CS32 - 1) / CS32, 256, 0, st>>>(n, cinvt, b, e);
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  if (lane == 0) e[a] = (T)acc;
 }
 
 // ---------------------------------------------------------------------------
@@ -1005,12 +995,6 @@ cudaError_t poisson_create(const Geo &g, double cx, double cy, double cz, int fp
   const PLevel &C = S->lv.back();
   if (C.n <= 512) {
     std::vector<double> M = coarse_pinv(C);
-    if (S->fp32) {  // by columns (the rounded matrix is not exactly symmetric)
-      std::vector<double> Mt(M.size());
-      for (int a = 0; a < C.n; a++)
-        for (int q = 0; q < C.n; q++) Mt[(size_t)q * C.n + a] = M[(size_t)a * C.n + q];
-      M.swap(Mt);
-    }
     PCK(cudaMalloc(&S->cinv, M.size() * sizeof(double)));
     PCK(cudaMemcpy(S->cinv, M.data(), M.size() * sizeof(double), cudaMemcpyHostToDevice));
   } else {
@@ -1420,7 +1404,7 @@ static cudaError_t vcycle(PoissonSolver *S, const R *b0, R *out, cudaStream_t st
     R *res = (l == 0) ? out : lvp(L.e);
     if (l == nlev - 1) {
       if (S->cinv) {
-        coarse_solve(L.n, S->cinv, b, res, st);
+        k_coarse_solve<R><<<(L.n + CSB - 1) / CSB, CSB * 32, 0, st>>>(L.n, S->cinv, b, res);
         (*nl)++;
       } else if (S->modes) {
         PCK(coarse_modes(S, L, b, lvp(L.r), lvp(L.e2), res, st, nl));

@@ -415,15 +415,16 @@ __global__ void __launch_bounds__(256) k_mg_restrict(const __grid_constant__ MgL
 }
 
 // ---------------------------------------------------------------------------
-// The same level in two launches, for FP32 levels of any size and for FP64
-// levels too small to fill the pipe: a block takes a coarse tile CX x CY x CZ
-// with the fine points around it in shared memory and runs all the passes of
-// the level on it, recomputing the halo (2.3 to 3 times the operations of
-// the passes above, which only FP32 or a short level can afford).  Every
-// value is formed by the operations of the general passes (k_rbgs,
-// k_residual, k_restrict_axis, k_prolong_axis) in their order, so the result
-// equals theirs bit for bit in either precision: products that a sum would
-// absorb into one rounding are kept apart (mul_rn).
+// The same level in two launches, for levels too small to fill the GPU: a
+// block takes a coarse tile CX x CY x CZ with the fine points around it in
+// shared memory and runs all the passes of the level on it, recomputing the
+// halo.  All loads of a block are issued before the first is used.
+// FP32: every value is formed by the operations of the general passes
+// (k_rbgs, k_residual, k_restrict_axis, k_prolong_axis) in their order, so the
+// result equals theirs bit for bit; products that a sum would absorb into one
+// rounding are kept apart (mul_rn).  FP64: the fewer operations of the five
+// passes above (a warp's FP64 instruction holds its scheduler's unit for about
+// 80 cycles, which is what a small level waits for beside its launches).
 template <int CX, int CY, int CZ>
 struct MgTile {
   static constexpr int FX = 2 * CX, FY = 2 * CY, FZ = 2 * CZ;
@@ -436,11 +437,34 @@ struct MgTile {
   static_assert(XN + YN <= DN && KN + ZN <= EN, "reused shared memory");
 };
 
-__device__ __forceinline__ int mg_mod(int j, int n) {  // n even: the colour of a row survives the wrap
-  j %= n;
-  return j < 0 ? j + n : j;
-}
+// y wrap; a tile reaches no further than one period beyond either end (the
+// smallest extents included: ny 4 and 2 coarse rows).  n even: the colour of a
+// row survives.
+__device__ __forceinline__ int mg_wrap(int j, int n) { return j < 0 ? j + n : (j >= n ? j - n : j); }
 __device__ __forceinline__ int mg_xc(int i, int nx) { return i == 0 ? 0 : (i == nx - 1 ? 2 : 1); }
+
+// The points of a level around a tile (its extents DX x DY x DZ from fine
+// point x0, y0, z0 on; y periodic, zero beyond the x and z walls), all loads
+// issued together.
+template <int DX, int DY, int DZ, typename R>
+struct MgLoad {
+  static constexpr int N = DX * DY * DZ, LI = (N + 255) / 256;
+  R v[LI];
+  __device__ __forceinline__ void load(const R *__restrict__ b, int nx, int ny, int nz, int x0, int y0, int z0,
+                                       int t) {
+#pragma unroll
+    for (int m = 0; m < LI; m++) {
+      const int q = t + 256 * m, lz = q / (DX * DY), ly = q / DX % DY, lx = q % DX;
+      const int i = x0 + lx, j = mg_wrap(y0 + ly, ny), k = z0 + lz;
+      v[m] = (q < N && i >= 0 && i < nx && k >= 0 && k < nz) ? b[i + nx * (j + (size_t)ny * k)] : (R)0;
+    }
+  }
+  __device__ __forceinline__ void store(R *s, int t) {
+#pragma unroll
+    for (int m = 0; m < LI; m++)
+      if (t + 256 * m < N) s[t + 256 * m] = v[m];
+  }
+};
 
 // The Gauss-Seidel value of local point q of a tile of row length DX and
 // plane DXY (zeros beyond the x and z walls).
@@ -456,63 +480,104 @@ template <typename R, int CX, int CY, int CZ>
 __global__ void __launch_bounds__(256) k_mg_down(const __grid_constant__ MgLev<R> L, const R *__restrict__ b,
                                                  R *__restrict__ bc) {
   using T = MgTile<CX, CY, CZ>;
+  constexpr bool F32 = sizeof(R) == sizeof(float);
   __shared__ R se[T::DN];
   __shared__ R sr[T::RN];
-  R *sx = se, *sy = se + T::XN;  // after the residual
+  __shared__ R sb[F32 ? T::DN : 1];  // FP32: b, for the residual
+  R *sx = se, *sy = se + T::XN;      // after the residual
   const int nx = L.nx, ny = L.ny, nz = L.nz;
   const int ncx = nx / 2, ncy = ny / 2, ncz = nz / 2;
   const int gx = (ncx + CX - 1) / CX, gy = (ncy + CY - 1) / CY;
   const int x0 = (blockIdx.x % gx) * T::FX, y0 = (blockIdx.x / gx % gy) * T::FY, z0 = blockIdx.x / (gx * gy) * T::FZ;
   const int t = threadIdx.x;
-  // red points: b / d; black: b
-  for (int q = t; q < T::DN; q += 256) {
-    const int lz = q / (T::DX * T::DY), ly = q / T::DX % T::DY, lx = q % T::DX;
-    const int i = x0 - 3 + lx, j = mg_mod(y0 - 3 + ly, ny), k = z0 - 3 + lz;
-    R v = (R)0;
-    if (i >= 0 && i < nx && k >= 0 && k < nz) {
-      v = b[i + nx * (j + (size_t)ny * k)];
-      if (((i + j + k) & 1) == 0) v = mul_rn(v, L.inv[mg_xc(i, nx)][mg_zc(k, nz)]);
+  {
+    MgLoad<T::DX, T::DY, T::DZ, R> ld;
+    ld.load(b, nx, ny, nz, x0 - 3, y0 - 3, z0 - 3, t);
+    if constexpr (F32) {  // red points: b / d
+      ld.store(sb, t);
+#pragma unroll
+      for (int m = 0; m < ld.LI; m++) {
+        const int q = t + 256 * m, lz = q / (T::DX * T::DY), ly = q / T::DX % T::DY, lx = q % T::DX;
+        const int i = x0 - 3 + lx, k = z0 - 3 + lz;
+        if ((lx + ly + lz) & 1)  // i + j + k = lx + ly + lz - 9 even (x0, y0, z0 are even)
+          ld.v[m] = mul_rn(ld.v[m], L.inv[mg_xc(i, nx)][mg_zc(k, nz)]);
+      }
     }
-    se[q] = v;
+    ld.store(se, t);
   }
   __syncthreads();
-  // black points of the tile and two points around it; x0, y0, z0 are even
+  // black points of the tile and two points around it
   for (int q = t; q < (T::DX - 2) / 2 * (T::DY - 2) * (T::DZ - 2); q += 256) {
     constexpr int HX = (T::DX - 2) / 2;
     const int lz = 1 + q / (HX * (T::DY - 2)), ly = 1 + q / HX % (T::DY - 2);
     const int lx = 2 + 2 * (q % HX) - ((ly + lz) & 1);  // lx + ly + lz even: i + j + k = lx + ly + lz - 9 odd
     const int i = x0 - 3 + lx, k = z0 - 3 + lz, o = lx + T::DX * (ly + T::DY * lz);
-    if (i >= 0 && i < nx && k >= 0 && k < nz) se[o] = mg_tile_relax<T::DX, T::DX * T::DY>(L, se, o, se[o], i, k);
+    if (i >= 0 && i < nx && k >= 0 && k < nz) {
+      if constexpr (F32) {
+        se[o] = mg_tile_relax<T::DX, T::DX * T::DY>(L, se, o, se[o], i, k);
+      } else {  // from b alone: the red neighbours' 1/d is in the couplings (zeros beyond the walls)
+        const int xc = mg_xc(i, nx), zc = mg_zc(k, nz);
+        R acc = fma(L.tx[mg_xc(max(i - 1, 0), nx)][zc], se[o - 1], se[o]);
+        acc = fma(L.tx[mg_xc(min(i + 1, nx - 1), nx)][zc], se[o + 1], acc);
+        acc = fma(L.ty[xc][zc], se[o - T::DX] + se[o + T::DX], acc);
+        acc = fma(L.tz[xc][mg_zc(max(k - 1, 0), nz)], se[o - T::DX * T::DY], acc);
+        acc = fma(L.tz[xc][mg_zc(min(k + 1, nz - 1), nz)], se[o + T::DX * T::DY], acc);
+        se[o] = acc * L.inv[xc][zc];
+      }
+    }
   }
   __syncthreads();
-  const R d = (R)2 * (L.cx + L.cy + L.cz);
-  for (int q = t; q < T::RN; q += 256) {
-    const int lz = q / (T::RX * T::RY), ly = q / T::RX % T::RY, lx = q % T::RX;
-    const int i = x0 - 1 + lx, j = mg_mod(y0 - 1 + ly, ny), k = z0 - 1 + lz;
-    R r = (R)0;
-    if (i >= 0 && i < nx && k >= 0 && k < nz) {
-      const int o = (lx + 2) + T::DX * ((ly + 2) + T::DY * (lz + 2));
-      const R v = se[o];
-      const R xm = (i > 0) ? se[o - 1] : v, xp = (i < nx - 1) ? se[o + 1] : v;
-      const R zm = (k > 0) ? se[o - T::DX * T::DY] : v, zp = (k < nz - 1) ? se[o + T::DX * T::DY] : v;
-      R a = mul_rn(d, v);
-      a = fma(-L.cx, xm + xp, a);
-      a = fma(-L.cy, se[o - T::DX] + se[o + T::DX], a);
-      r = b[i + nx * (j + (size_t)ny * k)] - fma(-L.cz, zm + zp, a);
+  if constexpr (F32) {  // the residual of every point
+    const R d = (R)2 * (L.cx + L.cy + L.cz);
+    for (int q = t; q < T::RN; q += 256) {
+      const int lz = q / (T::RX * T::RY), ly = q / T::RX % T::RY, lx = q % T::RX;
+      const int i = x0 - 1 + lx, k = z0 - 1 + lz;
+      R r = (R)0;
+      if (i >= 0 && i < nx && k >= 0 && k < nz) {
+        const int o = (lx + 2) + T::DX * ((ly + 2) + T::DY * (lz + 2));
+        const R v = se[o];
+        const R xm = (i > 0) ? se[o - 1] : v, xp = (i < nx - 1) ? se[o + 1] : v;
+        const R zm = (k > 0) ? se[o - T::DX * T::DY] : v, zp = (k < nz - 1) ? se[o + T::DX * T::DY] : v;
+        R a = mul_rn(d, v);
+        a = fma(-L.cx, xm + xp, a);
+        a = fma(-L.cy, se[o - T::DX] + se[o + T::DX], a);
+        r = sb[o] - fma(-L.cz, zm + zp, a);
+      }
+      sr[q] = r;
     }
-    sr[q] = r;
+  } else {  // of the red points: the sum of the black couplings
+    constexpr int HX = T::RX / 2;
+    for (int q = t; q < HX * T::RY * T::RZ; q += 256) {
+      const int lz = q / (HX * T::RY), ly = q / HX % T::RY, lx = 2 * (q % HX) + 1 - ((ly + lz) & 1);
+      const int i = x0 - 1 + lx, k = z0 - 1 + lz, o = (lx + 2) + T::DX * ((ly + 2) + T::DY * (lz + 2));
+      R r = (R)0;
+      if (i >= 0 && i < nx && k >= 0 && k < nz) {
+        // beyond a wall the tile holds zeros
+        r = L.cx * (se[o - 1] + se[o + 1]);
+        r = fma(L.cy, se[o - T::DX] + se[o + T::DX], r);
+        r = fma(L.cz, se[o - T::DX * T::DY] + se[o + T::DX * T::DY], r);
+      }
+      sr[lx + T::RX * (ly + T::RY * lz)] = r;  // lx + ly + lz odd: i + j + k even
+    }
   }
   __syncthreads();
   for (int q = t; q < T::XN; q += 256) {
     const int ix = q % CX, row = q / CX, ic = x0 / 2 + ix;  // row = ly + RY lz
     const R *p = sr + T::RX * row + 2 * ix;
-    sx[q] = mg_taps(ic == 0 ? (R)1 : (R)0.75, ic == ncx - 1 ? (R)1 : (R)0.75, p[0], p[1], p[2], p[3]);
+    if constexpr (F32) {
+      sx[q] = mg_taps(ic == 0 ? (R)1 : (R)0.75, ic == ncx - 1 ? (R)1 : (R)0.75, p[0], p[1], p[2], p[3]);
+    } else {  // taps 1 3 3 1, red where lx + ly + lz is odd; 4 where a wall reflects the missing one (zero here)
+      const bool odd = !((row % T::RY + row / T::RY) & 1);
+      const R w = (odd ? ic == 0 : ic == ncx - 1) ? (R)4 : (R)3;
+      sx[q] = fma(w, odd ? p[1] : p[2], odd ? p[3] : p[0]);
+    }
   }
   __syncthreads();
   for (int q = t; q < T::YN; q += 256) {
     const int ix = q % CX, iy = q / CX % CY, lz = q / (CX * CY);
     const R *p = sx + ix + CX * (2 * iy + T::RY * lz);
-    sy[q] = mg_taps((R)0.75, (R)0.75, p[0], p[CX], p[2 * CX], p[3 * CX]);
+    if constexpr (F32) sy[q] = mg_taps((R)0.75, (R)0.75, p[0], p[CX], p[2 * CX], p[3 * CX]);
+    else sy[q] = fma((R)3, p[CX] + p[2 * CX], p[0] + p[3 * CX]);
   }
   __syncthreads();
   for (int q = t; q < CX * CY * CZ; q += 256) {
@@ -520,76 +585,110 @@ __global__ void __launch_bounds__(256) k_mg_down(const __grid_constant__ MgLev<R
     const int ic = x0 / 2 + ix, jc = y0 / 2 + iy, kc = z0 / 2 + iz;
     if (ic < ncx && jc < ncy && kc < ncz) {
       const R *p = sy + ix + CX * (iy + CY * 2 * iz);
-      const R v = mg_taps(kc == 0 ? (R)1 : (R)0.75, kc == ncz - 1 ? (R)1 : (R)0.75, p[0], p[CX * CY], p[2 * CX * CY],
-                          p[3 * CX * CY]);
-      bc[ic + ncx * (jc + (size_t)ncy * kc)] = v * (R)0.125;
+      const R p0 = p[0], p1 = p[CX * CY], p2 = p[2 * CX * CY], p3 = p[3 * CX * CY];
+      R v;
+      if constexpr (F32) {
+        v = mg_taps(kc == 0 ? (R)1 : (R)0.75, kc == ncz - 1 ? (R)1 : (R)0.75, p0, p1, p2, p3) * (R)0.125;
+      } else {
+        v = fma(kc == 0 ? (R)4 : (R)3, p1, p0);
+        v = (fma(kc == ncz - 1 ? (R)4 : (R)3, p2, p3) + v) * (R)(1.0 / 512.0);
+      }
+      bc[ic + ncx * (jc + (size_t)ncy * kc)] = v;
     }
   }
 }
 
+// Coarse tile with two cells around it, clamped at the walls, y periodic.
+template <int KX, int KY, int KZ, typename R>
+struct MgLoadCoarse {
+  static constexpr int N = KX * KY * KZ, LI = (N + 255) / 256;
+  R v[LI];
+  __device__ __forceinline__ void load(const R *__restrict__ ec, int ncx, int ncy, int ncz, int x0, int y0, int z0,
+                                       int t) {
+#pragma unroll
+    for (int m = 0; m < LI; m++) {
+      const int q = t + 256 * m, lz = q / (KX * KY), ly = q / KX % KY, lx = q % KX;
+      const int ic = min(max(x0 + lx, 0), ncx - 1), jc = mg_wrap(y0 + ly, ncy), kc = min(max(z0 + lz, 0), ncz - 1);
+      v[m] = q < N ? ec[ic + ncx * (jc + (size_t)ncy * kc)] : (R)0;
+    }
+  }
+};
+
 // e of the tile after the coarse correction and the post-smoothing; every
 // thread of the block returns from it with the tile in se (local point 2 =
-// the tile's first).
+// the tile's first), its right-hand side in sb.
 template <typename R, int CX, int CY, int CZ>
 __device__ __forceinline__ void mg_up_tile(const MgLev<R> &L, const R *__restrict__ b, const R *__restrict__ ec, R *se,
-                                           R *ss, int x0, int y0, int z0) {
+                                           R *ss, R *sb, int x0, int y0, int z0) {
   using T = MgTile<CX, CY, CZ>;
+  constexpr bool F32 = sizeof(R) == sizeof(float);
   R *sk = se, *sz = se + T::KN;  // before the fine values
   const int nx = L.nx, ny = L.ny, nz = L.nz;
   const int ncx = nx / 2, ncy = ny / 2, ncz = nz / 2;
   const int t = threadIdx.x;
-  for (int q = t; q < T::KN; q += 256) {
-    const int lz = q / (T::KX * T::KY), ly = q / T::KX % T::KY, lx = q % T::KX;
-    const int ic = min(max(x0 / 2 - 2 + lx, 0), ncx - 1), jc = mg_mod(y0 / 2 - 2 + ly, ncy);
-    const int kc = min(max(z0 / 2 - 2 + lz, 0), ncz - 1);
-    sk[q] = ec[ic + ncx * (jc + (size_t)ncy * kc)];
+  {
+    MgLoad<T::EX, T::EY, T::EZ, R> lb;
+    MgLoadCoarse<T::KX, T::KY, T::KZ, R> lc;
+    lc.load(ec, ncx, ncy, ncz, x0 / 2 - 2, y0 / 2 - 2, z0 / 2 - 2, t);
+    lb.load(b, nx, ny, nz, x0 - 2, y0 - 2, z0 - 2, t);
+#pragma unroll
+    for (int m = 0; m < lc.LI; m++)
+      if (t + 256 * m < lc.N) sk[t + 256 * m] = lc.v[m];
+    lb.store(sb, t);
   }
   __syncthreads();
+  // one axis of the interpolation: FP32 as the general passes (3/4 and 1/4; a cell at a wall alone), FP64 3 and 1 (the
+  // wall's clamped cell counts twice), scaled by 1/64 at the end
+  auto lerp = [](R a, R c, bool wall) -> R {
+    if constexpr (F32) return mg_lerp(a, c, wall);
+    else return fma((R)3, a, c);
+  };
   // fine index f = f0 - 2 + l; its cell is local (l >> 1) + 1, the next one on
   // its side one below for even l, one above for odd
   for (int q = t; q < T::ZN; q += 256) {
     const int lz = q / (T::KX * T::KY), col = q % (T::KX * T::KY), c0 = (lz >> 1) + 1;
     const int c1 = (lz & 1) ? c0 + 1 : c0 - 1, kc1 = z0 / 2 - 2 + c1;
-    sz[q] = mg_lerp(sk[col + T::KX * T::KY * c0], sk[col + T::KX * T::KY * c1], kc1 < 0 || kc1 >= ncz);
+    sz[q] = lerp(sk[col + T::KX * T::KY * c0], sk[col + T::KX * T::KY * c1], kc1 < 0 || kc1 >= ncz);
   }
   __syncthreads();
   for (int q = t; q < T::SN; q += 256) {
     const int lx = q % T::KX, ly = q / T::KX % T::EY, lz = q / (T::KX * T::EY), c0 = (ly >> 1) + 1;
     const int c1 = (ly & 1) ? c0 + 1 : c0 - 1;
     const R *p = sz + lx + T::KX * T::KY * lz;
-    ss[q] = mg_lerp(p[T::KX * c0], p[T::KX * c1], false);
+    ss[q] = lerp(p[T::KX * c0], p[T::KX * c1], false);
   }
   __syncthreads();
-  // red points of the tile and two points around it: b / d + P e_c; black: 0 until relaxed
-  for (int q = t; q < T::EN; q += 256) {
-    const int lx = q % T::EX, ly = q / T::EX % T::EY, lz = q / (T::EX * T::EY);
-    const int i = x0 - 2 + lx, k = z0 - 2 + lz;
+  // red points of the tile and two points around it: b / d + P e_c; black: zero until relaxed
+  constexpr int HE = T::EX / 2;
+  for (int q = t; q < HE * T::EY * T::EZ; q += 256) {
+    const int lz = q / (HE * T::EY), ly = q / HE % T::EY, odd = (ly + lz) & 1, lx = 2 * (q % HE) + odd;
+    const int i = x0 - 2 + lx, k = z0 - 2 + lz, o = lx + T::EX * (ly + T::EY * lz);
     R v = (R)0;
-    if (((lx + ly + lz) & 1) == 0 && i >= 0 && i < nx && k >= 0 && k < nz) {
-      const int j = mg_mod(y0 - 2 + ly, ny), c0 = (lx >> 1) + 1, c1 = (lx & 1) ? c0 + 1 : c0 - 1;
-      const int ic1 = x0 / 2 - 2 + c1;
+    if (i >= 0 && i < nx && k >= 0 && k < nz) {
+      const int c0 = (lx >> 1) + 1, c1 = (lx & 1) ? c0 + 1 : c0 - 1, ic1 = x0 / 2 - 2 + c1;
       const R *p = ss + T::KX * (ly + T::EY * lz);
-      v = mul_rn(b[i + nx * (j + (size_t)ny * k)], L.inv[mg_xc(i, nx)][mg_zc(k, nz)]) +
-          mg_lerp(p[c0], p[c1], ic1 < 0 || ic1 >= ncx);
+      const R d = L.inv[mg_xc(i, nx)][mg_zc(k, nz)], w = lerp(p[c0], p[c1], ic1 < 0 || ic1 >= ncx);
+      if constexpr (F32) v = mul_rn(sb[o], d) + w;
+      else v = fma(sb[o], d, w * (R)(1.0 / 64.0));
     }
-    se[q] = v;
+    se[o] = v;
+    se[o + 1 - 2 * odd] = (R)0;
   }
   __syncthreads();
   for (int q = t; q < (T::EX - 2) / 2 * (T::EY - 2) * (T::EZ - 2); q += 256) {
     constexpr int HX = (T::EX - 2) / 2;
     const int lz = 1 + q / (HX * (T::EY - 2)), ly = 1 + q / HX % (T::EY - 2);
     const int lx = 1 + 2 * (q % HX) + ((ly + lz) & 1);  // lx + ly + lz odd
-    const int i = x0 - 2 + lx, j = mg_mod(y0 - 2 + ly, ny), k = z0 - 2 + lz, o = lx + T::EX * (ly + T::EY * lz);
+    const int i = x0 - 2 + lx, k = z0 - 2 + lz, o = lx + T::EX * (ly + T::EY * lz);
     if (i >= 0 && i < nx && k >= 0 && k < nz)
-      se[o] = mg_tile_relax<T::EX, T::EX * T::EY>(L, se, o, b[i + nx * (j + (size_t)ny * k)], i, k);
+      se[o] = mg_tile_relax<T::EX, T::EX * T::EY>(L, se, o, sb[o], i, k);
   }
   __syncthreads();
   for (int q = t; q < T::FX / 2 * T::FY * T::FZ; q += 256) {
     const int lz = 2 + q / (T::FX / 2 * T::FY), ly = 2 + q / (T::FX / 2) % T::FY;
     const int lx = 2 + 2 * (q % (T::FX / 2)) + ((ly + lz) & 1);  // even sum
-    const int i = x0 - 2 + lx, j = y0 - 2 + ly, k = z0 - 2 + lz, o = lx + T::EX * (ly + T::EY * lz);
-    if (i < nx && j < ny && k < nz)
-      se[o] = mg_tile_relax<T::EX, T::EX * T::EY>(L, se, o, b[i + nx * (j + (size_t)ny * k)], i, k);
+    const int i = x0 - 2 + lx, k = z0 - 2 + lz, o = lx + T::EX * (ly + T::EY * lz);
+    if (i < nx && y0 - 2 + ly < ny && k < nz) se[o] = mg_tile_relax<T::EX, T::EX * T::EY>(L, se, o, sb[o], i, k);
   }
   __syncthreads();
 }
@@ -600,9 +699,10 @@ __global__ void __launch_bounds__(256) k_mg_up(const __grid_constant__ MgLev<R> 
   using T = MgTile<CX, CY, CZ>;
   __shared__ R se[T::EN];
   __shared__ R ss[T::SN];
+  __shared__ R sb[T::EN];
   const int gx = (L.nx / 2 + CX - 1) / CX, gy = (L.ny / 2 + CY - 1) / CY;
   const int x0 = (blockIdx.x % gx) * T::FX, y0 = (blockIdx.x / gx % gy) * T::FY, z0 = blockIdx.x / (gx * gy) * T::FZ;
-  mg_up_tile<R, CX, CY, CZ>(L, b, ec, se, ss, x0, y0, z0);
+  mg_up_tile<R, CX, CY, CZ>(L, b, ec, se, ss, sb, x0, y0, z0);
   for (int q = threadIdx.x; q < T::FX * T::FY * T::FZ; q += 256) {
     const int lx = q % T::FX, ly = q / T::FX % T::FY, lz = q / (T::FX * T::FY);
     if (x0 + lx < L.nx && y0 + ly < L.ny && z0 + lz < L.nz)
