@@ -214,9 +214,15 @@ __device__ __forceinline__ void st_release_u32(unsigned *p, unsigned v) {
 
 // Phases 1 and 2 of one super-chunk (levels kc .. kc+n-1) of a tile: A and B
 // of every (level, column) pair into sA/sB, then each warp's chunk scanned
-// in place (y and P), its ends into ey/ep.  Synchronises the block.  The
-// form of the FP32 sweeps (latency-bound): a warp per level, all (level,
-// column) pairs independent so that their loads overlap.
+// in place (y and P), its ends into ey/ep.  Synchronises the block.  A warp
+// per level, all (level, column) pairs independent.
+// The FP32 sweeps are bound by the latency of the loads, and more warps hide
+// it better than more loads per warp: one level at a time in 32 registers (8
+// blocks, all 64 warps of an SM) measured 404 us per half-sweep of three
+// components at 512x256x256, four levels in flight at 40 registers (6
+// blocks) 470.  Lanes past the row's end take the row's first point of this
+// colour (and store nothing), which frees the loads of their predicates: 404
+// against 422.
 template <typename T, typename CS>
 __device__ __forceinline__ void odd_produce_scan_levels(int comp, const Geo &g, const CS &coef,
                                                         const T *__restrict__ x, int i, int j, bool act, int k0,
@@ -225,14 +231,15 @@ __device__ __forceinline__ void odd_produce_scan_levels(int comp, const Geo &g, 
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int sy_ = g.sy, sz = g.sz, nz = g.nz;
   constexpr int PER = SOC_SC / SOC_W;
-#pragma unroll 4
+  const int ic = (sizeof(T) == 4 && !act) ? 1 + ((i & 1) ^ 1) : i;
+#pragma unroll(sizeof(T) == 4 ? 1 : 4)
   for (int r = 0; r < PER; r++) {
     const int lk = w + r * SOC_W, k = kc + lk;
     if (lk < n) {
       T A = 0, B = 0;
-      if (act) {
-        const int c = TPLS_IDX(g, i, j, k);
-        const Rec<T> q = get_rec(comp, g, coef, c, i, j, k, true);
+      if (sizeof(T) == 4 || act) {
+        const int c = TPLS_IDX(g, ic, j, k);
+        const Rec<T> q = get_rec(comp, g, coef, c, ic, j, k, true);
         const T xc = x[c];
         T zp;
         if (comp == 2) zp = x[c + sz];
@@ -247,7 +254,7 @@ __device__ __forceinline__ void odd_produce_scan_levels(int comp, const Geo &g, 
           A = xc + (T)1.2 * (fma(q.zm, zm, part) - xc);
         } else {
           A = xc + (T)1.2 * (part - xc);
-          B = (T)1.2 * q.zm;
+          B = (sizeof(T) == 8) ? q.bz : (T)1.2 * q.zm;
         }
       }
       sA[lk][lane] = A;
@@ -414,55 +421,12 @@ __device__ __forceinline__ void sor_odd_c4_tile(int comp_, const Geo &g, const H
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int i2 = bx * 32 + lane, i = 2 * i2 + 1 + par;
   const bool act = (i2 < npair) && (i <= iend);
-  const int sy_ = g.sy, sz = g.sz, nz = g.nz;
   constexpr int PER = SOC_SC / SOC_W;
   T carry = 0;  // x of the level below the super-chunk (k0 has B = 0)
   for (int kc = k0; kc <= k1; kc += SOC_SC) {
     const int n = min(SOC_SC, k1 - kc + 1);
-    // 1. produce
-#pragma unroll 4
-    for (int r = 0; r < PER; r++) {
-      const int lk = w + r * SOC_W, k = kc + lk;
-      if (lk < n) {
-        T A = 0, B = 0;
-        if (act) {
-          const int c = TPLS_IDX(g, i, j, k);
-          const Rec<T> q = get_rec(comp, g, coef, c, i, j, k, true);
-          const T xc = x[c];
-          T zp;
-          if (comp == 2) zp = x[c + sz];
-          else zp = (k == nz - 1) ? xc : x[c + sz];
-          T part = fma(q.xp, x[c + 1], q.b);
-          part = fma(q.xm, x[c - 1], part);
-          part = fma(q.yp, x[c + sy_], part);
-          part = fma(q.ym, x[c - sy_], part);
-          part = fma(q.zp, zp, part);
-          if (k == k0) {  // the point below is a wall value (w) or the point itself (u, v)
-            const T zm = (comp == 2) ? x[c - sz] : xc;
-            A = xc + (T)1.2 * (fma(q.zm, zm, part) - xc);
-          } else {
-            A = xc + (T)1.2 * (part - xc);
-            B = (sizeof(T) == 8) ? q.bz : (T)1.2 * q.zm;
-          }
-        }
-        sA[lk][lane] = A;
-        sB[lk][lane] = B;
-      }
-    }
-    __syncthreads();
-    // 2. scan of this warp's levels
+    odd_produce_scan_levels<T, CS>(comp, g, coef, x, i, j, act, k0, kc, n, sA, sB, ey, ep);  // 1. produce, 2. scan
     const int lb = w * PER, le = min(n, lb + PER);
-    T yv = 0, pv = 1;
-    for (int lk = lb; lk < le; lk++) {
-      const T B = sB[lk][lane];
-      yv = fma(B, yv, sA[lk][lane]);
-      pv = B * pv;
-      sA[lk][lane] = yv;
-      sB[lk][lane] = pv;
-    }
-    ey[w][lane] = yv;  // an empty chunk passes x_in through (y 0, P 1)
-    ep[w][lane] = pv;
-    __syncthreads();
     // 3. fold and write
     T xin = carry;
     for (int v = 0; v < w; v++) xin = fma(ep[v][lane], xin, ey[v][lane]);
@@ -498,7 +462,7 @@ __device__ __forceinline__ void sor_odd_c4_tile(int comp_, const Geo &g, const H
 }
 
 // Odd half-sweep with one block per super-chunk of a tile (segment), for
-// columns of 3 or more segments (FP64 records, the FP32 sweeps and the
+// columns of several segments (odd_set; FP64 records, the FP32 sweeps and the
 // per-routine entries alike), so a launch has nz/64 times the blocks of
 // the whole-column form and the blocks' load, scan and write phases
 // overlap.
@@ -593,7 +557,7 @@ __device__ __forceinline__ void sor_odd_segment(int comp_, const Geo &g, const H
   } while (0)
 
 template <typename T, typename CS>
-__global__ void __launch_bounds__(SOC_W * 32, sizeof(T) == 4 ? 6 : 5)  // 40 / 48 registers: 6 / 5 blocks per SM
+__global__ void __launch_bounds__(SOC_W * 32, sizeof(T) == 4 ? 8 : 5)  // 32 / 48 registers: 8 / 5 blocks per SM
     k_sor_odd_seg(Geo g, Helm h, const __grid_constant__ SweepSet<T, CS> S, const double *__restrict__ P, int flg,
                   int bc, int fuse, OddChain oc, int gx, int limit) {
   __shared__ OddShared<T> sh;
@@ -625,7 +589,7 @@ __global__ void __launch_bounds__(SOC_W * 32, sizeof(T) == 4 ? 6 : 5)  // 40 / 4
 }
 
 template <typename T, typename CS>
-__global__ void __launch_bounds__(SOC_W * 32)
+__global__ void __launch_bounds__(SOC_W * 32, sizeof(T) == 4 ? 8 : 1)
     k_sor_odd_c4(Geo g, Helm h, const __grid_constant__ SweepSet<T, CS> S, const double *__restrict__ P, int gx,
                  int flg, int bc, int fuse) {
   __shared__ OddShared<T> sh;
@@ -747,11 +711,12 @@ static cudaError_t odd_set(const Geo &g, const Helm &h, const SweepSet<T, CS> &s
                            int fuse, cudaStream_t st, const OddChain *oc) {
   const int gx = ((g.nx + 1) / 2 + 31) / 32, nseg = (g.nz - 1) / SOC_SC + 1;
   const int blocks = nseg * s.n * gx * g.ny;
-  // one block per segment, chained, for columns of 3 or more segments: with
-  // 2, half the blocks wait on the other half for a larger share of their
-  // time than the extra blocks save (measured slower on the batched
-  // workload's grids, nz <= 128; faster at nz = 192 and 256)
-  if (oc && nseg >= 3 && oc->cap >= blocks) {
+  // One block per segment, chained, for columns of 2 (FP32) or 3 (FP64) and
+  // more segments.  With 2, half the blocks wait on the other half: the FP32
+  // sweeps gain more from twice the blocks (16 half-sweeps at 192x96x112: 722
+  // us, whole columns 764), the FP64 ones, bound by the FP64 pipe, do not
+  // (128x64x96: 720, whole columns 646).
+  if (oc && nseg >= (sizeof(T) == 4 ? 2 : 3) && oc->cap >= blocks) {
     k_sor_odd_seg<T, CS><<<blocks, SOC_W * 32, 0, st>>>(g, h, s, pres, flg, bc, fuse, *oc, gx, 1 << 20);
   } else {  // one block per 32 columns of a row, the column in super-chunks
     k_sor_odd_c4<T, CS><<<dim3(gx * s.n, g.ny), SOC_W * 32, 0, st>>>(g, h, s, pres, gx, flg, bc, fuse);

@@ -49,20 +49,16 @@ __device__ __forceinline__ float ex(const Row &w, int e) { return e < 0 ? w.l : 
 // Row segment at p (i = 4q+1 of the row), in two steps so that a thread
 // issues every load before it waits for any: issue() loads the 16 bytes and,
 // for the lanes that own them, the x-1 / x+4 neighbours (lane 0 its left one;
-// the last lane, or the last active group, its right one); halo() then
-// takes the other lanes' neighbours from the adjacent lanes.  halo() is
-// called by every lane of the warp (the shuffles need all of them);
-// inactive lanes load nothing.
+// the last lane, or the last group, its right one); halo() then takes the
+// other lanes' neighbours from the adjacent lanes.  Every lane of the warp
+// runs both: lanes past the row's last group take that group again (and store
+// nothing), so no load or operation is predicated on them.
 template <bool L, bool R, bool NC>
-__device__ __forceinline__ void issue(Row &w, const float *p, bool act, bool own_l, bool own_r) {
-  w.v = make_float4(0.f, 0.f, 0.f, 0.f);
-  w.l = w.r = 0.f;
-  if (act) {
-    const float4 *p4 = reinterpret_cast<const float4 *>(p);
-    w.v = NC ? __ldg(p4) : *p4;
-    if (L && own_l) w.l = NC ? __ldg(p - 1) : p[-1];
-    if (R && own_r) w.r = NC ? __ldg(p + 4) : p[4];
-  }
+__device__ __forceinline__ void issue(Row &w, const float *p, bool own_l, bool own_r) {
+  const float4 *p4 = reinterpret_cast<const float4 *>(p);
+  w.v = NC ? __ldg(p4) : *p4;
+  if (L && own_l) w.l = NC ? __ldg(p - 1) : p[-1];
+  if (R && own_r) w.r = NC ? __ldg(p + 4) : p[4];
 }
 template <bool L, bool R>
 __device__ __forceinline__ void halo(Row &w, bool own_l, bool own_r) {
@@ -84,31 +80,31 @@ struct MuRows {
 
 template <int CC>
 __device__ __forceinline__ void issue_mu(MuRows &m, const Geo &g, const float *__restrict__ mu, int i0, int j, int k,
-                                         bool act, bool ol, bool orr) {
+                                         bool ol, bool orr) {
   const int sy = g.sy, sz = g.szm;
   if (CC == 0) {
     const float *b = mu + TPLS_IDXM(g, i0, j + 1, k + 1);
-    issue<false, true, true>(m.r[0], b, act, ol, orr);       // (j+1, k+1)
-    issue<false, true, true>(m.r[1], b + sy, act, ol, orr);  // (j+2, k+1)
-    issue<false, true, true>(m.r[2], b - sy, act, ol, orr);  // (j, k+1)
-    issue<false, true, true>(m.r[3], b + sz, act, ol, orr);  // (j+1, k+2)
-    issue<false, true, true>(m.r[4], b - sz, act, ol, orr);  // (j+1, k)
+    issue<false, true, true>(m.r[0], b, ol, orr);       // (j+1, k+1)
+    issue<false, true, true>(m.r[1], b + sy, ol, orr);  // (j+2, k+1)
+    issue<false, true, true>(m.r[2], b - sy, ol, orr);  // (j, k+1)
+    issue<false, true, true>(m.r[3], b + sz, ol, orr);  // (j+1, k+2)
+    issue<false, true, true>(m.r[4], b - sz, ol, orr);  // (j+1, k)
   } else if (CC == 1) {
     const float *b = mu + TPLS_IDXM(g, i0, j + 1, k + 1);
-    issue<true, true, true>(m.r[0], b, act, ol, orr);              // (j+1, k+1)
-    issue<true, true, true>(m.r[1], b - sy, act, ol, orr);         // (j, k+1)
-    issue<false, false, true>(m.r[2], b + sz, act, ol, orr);       // (j+1, k+2)
-    issue<false, false, true>(m.r[3], b + sz - sy, act, ol, orr);  // (j, k+2)
-    issue<false, false, true>(m.r[4], b - sz, act, ol, orr);       // (j+1, k)
-    issue<false, false, true>(m.r[5], b - sz - sy, act, ol, orr);  // (j, k)
+    issue<true, true, true>(m.r[0], b, ol, orr);              // (j+1, k+1)
+    issue<true, true, true>(m.r[1], b - sy, ol, orr);         // (j, k+1)
+    issue<false, false, true>(m.r[2], b + sz, ol, orr);       // (j+1, k+2)
+    issue<false, false, true>(m.r[3], b + sz - sy, ol, orr);  // (j, k+2)
+    issue<false, false, true>(m.r[4], b - sz, ol, orr);       // (j+1, k)
+    issue<false, false, true>(m.r[5], b - sz - sy, ol, orr);  // (j, k)
   } else {
     const float *b = mu + TPLS_IDXM(g, i0, j + 1, k);
-    issue<true, true, true>(m.r[0], b, act, ol, orr);              // (j+1, k)
-    issue<true, true, true>(m.r[1], b + sz, act, ol, orr);         // (j+1, k+1)
-    issue<false, false, true>(m.r[2], b + sy, act, ol, orr);       // (j+2, k)
-    issue<false, false, true>(m.r[3], b + sy + sz, act, ol, orr);  // (j+2, k+1)
-    issue<false, false, true>(m.r[4], b - sy, act, ol, orr);       // (j, k)
-    issue<false, false, true>(m.r[5], b - sy + sz, act, ol, orr);  // (j, k+1)
+    issue<true, true, true>(m.r[0], b, ol, orr);              // (j+1, k)
+    issue<true, true, true>(m.r[1], b + sz, ol, orr);         // (j+1, k+1)
+    issue<false, false, true>(m.r[2], b + sy, ol, orr);       // (j+2, k)
+    issue<false, false, true>(m.r[3], b + sy + sz, ol, orr);  // (j+2, k+1)
+    issue<false, false, true>(m.r[4], b - sy, ol, orr);       // (j, k)
+    issue<false, false, true>(m.r[5], b - sy + sz, ol, orr);  // (j, k+1)
   }
 }
 template <int CC>
@@ -170,17 +166,18 @@ __device__ __forceinline__ void faces4(const MuRows &m, Faces &f) {
 // b of the four points (record-slot order: odd i in the first half of the
 // row, even i in the second, so each parity's two values are one aligned
 // 8-byte load: the b arrays carry no x offset); `par` < 0 loads all four,
-// else the two points of that x parity.
-__device__ __forceinline__ void load_b(const Geo &g, const float *__restrict__ b, int q, int i0, int iend, int j, int k,
-                                       int par, bool act, float *out) {
+// else the two points of that x parity.  (Points past the row's end read its
+// padding, for values that are not stored.)
+__device__ __forceinline__ void load_b(const Geo &g, const float *__restrict__ b, int q, int j, int k, int par,
+                                       float *out) {
   const float *rb = b + g.sy * j + g.sz * k + 2 * q;
   out[0] = out[1] = out[2] = out[3] = 0.f;
-  if (act && par != 1) {  // i = 4q+1, 4q+3
+  if (par != 1) {  // i = 4q+1, 4q+3
     const float2 v = __ldg(reinterpret_cast<const float2 *>(rb));
     out[0] = v.x;
     out[2] = v.y;
   }
-  if (act && par != 0 && i0 + 1 <= iend) {  // i = 4q+2, 4q+4
+  if (par != 0) {  // i = 4q+2, 4q+4
     const float2 v = __ldg(reinterpret_cast<const float2 *>(rb + (g.sy >> 1)));
     out[1] = v.x;
     out[3] = v.y;
@@ -194,35 +191,42 @@ template <int CC, int MODE, int BY>
 __device__ __forceinline__ void sweep4_tile(const Geo &g, const Helm &h, const float *__restrict__ xo, float *x,
                                             const MuCoef &s, const double *__restrict__ X, int flg, int bc,
                                             int fuse, int bx, int by, int bz) {
-  const int lane = threadIdx.x, q = bx * 32 + lane;
+  const int lane = threadIdx.x;
   const int j = by * BY + threadIdx.y + 1;
   if (j > g.ny) return;  // uniform per warp
   const int nx = g.nx, nz = g.nz, sy = g.sy, sz = g.sz;
   const int k = bz + ((CC == 2) ? 1 : 0);
   const int iend = (CC == 0) ? nx - 1 : nx;
   const int G = (iend + 3) >> 2;
-  const bool act = q < G;
+  const bool act = bx * 32 + lane < G;
+  const int q = act ? bx * 32 + lane : G - 1;
   const bool ol = (lane == 0), orr = (lane == 31) || (q + 1 >= G);
   const int i0 = 4 * q + 1;
-  const bool full = act && (i0 + 3 <= iend);
   constexpr bool NC = (MODE == M_JAC);  // only the Jacobi source is read-only
   const float *xr = (MODE == M_JAC) ? xo : x;
   const float *pc = xr + (i0 + sy * j + sz * k);
   // every load of the thread first, then the shuffles
-  const bool has_zp = (CC == 2) || (k + 1 <= nz - 1), has_zm = (CC == 2) || (k >= 1);
   Row cc, yp, ym, zp, zm;
   MuRows m;
-  issue<true, true, NC>(cc, pc, act, ol, orr);
-  issue<false, false, NC>(yp, pc + sy, act, ol, orr);
-  issue<false, false, NC>(ym, pc - sy, act, ol, orr);
-  issue<false, false, NC>(zp, pc + sz, act && has_zp, ol, orr);
-  issue<false, false, NC>(zm, pc - sz, act && has_zm, ol, orr);
-  issue_mu<CC>(m, g, s.mu, i0, j, k, act, ol, orr);
+  issue<true, true, NC>(cc, pc, ol, orr);
+  issue<false, false, NC>(yp, pc + sy, ol, orr);
+  issue<false, false, NC>(ym, pc - sy, ol, orr);
+  issue<false, false, NC>(zp, (CC == 2 || k < nz - 1) ? pc + sz : pc, ol, orr);
+  issue<false, false, NC>(zm, (CC == 2 || k > 0) ? pc - sz : pc, ol, orr);
+  issue_mu<CC>(m, g, s.mu, i0, j, k, ol, orr);
   const int par = (MODE == M_JAC) ? -1 : ((k + j + flg) & 1);
   float bv[4];
-  load_b(g, s.b, q, i0, iend, j, k, par, act, bv);
+  load_b(g, s.b, q, j, k, par, bv);
   halo<true, true>(cc, ol, orr);
   halo_mu<CC>(m, ol, orr);
+  if (CC != 2) {  // no-slip ghost value -2 x(0) + x(1)/3 below k = 0 and above k = nz-1 (uniform per block)
+    auto ghost = [](float4 in, float4 c) {
+      return make_float4(fmaf(in.x, 1.0f / 3.0f, -2.0f * c.x), fmaf(in.y, 1.0f / 3.0f, -2.0f * c.y),
+                         fmaf(in.z, 1.0f / 3.0f, -2.0f * c.z), fmaf(in.w, 1.0f / 3.0f, -2.0f * c.w));
+    };
+    if (k == 0) zm.v = ghost(zp.v, cc.v);
+    if (k == nz - 1) zp.v = ghost(zm.v, cc.v);
+  }
   // per-axis scale: dt/(2 d^2), and a quarter of it for the averaged faces
   const float cx = (CC == 0) ? s.ax2 : 0.25f * s.ax2;
   const float cy = (CC == 1) ? s.ay2 : 0.25f * s.ay2;
@@ -238,20 +242,14 @@ __device__ __forceinline__ void sweep4_tile(const Geo &g, const Helm &h, const f
 #pragma unroll
     for (int e = 0; e < 4; e++) {
       if (PAR >= 0 && (e & 1) != PAR) continue;
-      if (!act || i0 + e > iend) continue;
       const float xc = el(cc, e);
-      float zpv = el(zp, e), zmv = el(zm, e);
-      if (CC != 2) {  // no-slip ghost value -2 x(0) + x(1)/3 below k = 0 and above k = nz-1
-        if (k == 0) zmv = fmaf(zpv, 1.0f / 3.0f, -2.0f * xc);
-        if (k == nz - 1) zpv = fmaf(zmv, 1.0f / 3.0f, -2.0f * xc);
-      }
       float d = fmaf(cx, f.px[e] + f.mx[e], 1.0f);
       d = fmaf(cy, f.py[e] + f.my[e], d);
       d = fmaf(cz, f.pz[e] + f.mz[e], d);
       const float r = __fdividef(1.0f, d);  // d >= 1: the fast reciprocal is within 2 ulp
       const float tx = fmaf(f.px[e], ex(cc, e + 1), f.mx[e] * ex(cc, e - 1));
       const float ty = fmaf(f.py[e], el(yp, e), f.my[e] * el(ym, e));
-      const float tz = fmaf(f.pz[e], zpv, f.mz[e] * zmv);
+      const float tz = fmaf(f.pz[e], el(zp, e), f.mz[e] * el(zm, e));
       const float t = fmaf(cx, tx, fmaf(cy, ty, cz * tz));
       const float v = fmaf(r, t, bv[e]);
       out[e] = (MODE == M_JAC) ? v : xc + 1.2f * (v - xc);
@@ -263,18 +261,19 @@ __device__ __forceinline__ void sweep4_tile(const Geo &g, const Helm &h, const f
   // store: whole groups as one 16-byte store (in the half-sweep the other
   // colour's values are rewritten unchanged: nothing else writes them in
   // this launch), ragged ends point by point
+  if (!act) return;
   float *po = x + (i0 + sy * j + sz * k);
-  if (full) {
+  if (i0 + 3 <= iend) {
     const float4 o = make_float4(out[0], out[1], out[2], out[3]);
     *reinterpret_cast<float4 *>(po) = o;
     if (fuse && j == g.ny) *reinterpret_cast<float4 *>(po - sy * g.ny) = o;
     if (fuse && j == 1) *reinterpret_cast<float4 *>(po + sy * g.ny) = o;
-  } else if (act) {
+  } else {
 #pragma unroll
     for (int e = 0; e < 4; e++)
       if (i0 + e <= iend && (MODE == M_JAC || (e & 1) == par)) put(g, x, i0 + e, j, k, out[e], fuse);
   }
-  if (!act || (MODE != M_JAC && !bc)) return;
+  if (MODE != M_JAC && !bc) return;
   // boundary rows (the post-sweep ones of main_ns_hybrid.F90:784-799,
   // 826-836, 860-879): x(0) = x(1) + off.x; u: x(nx) = x(nx-1) + off.y and
   // x(nx+1) = off.z; v, w: x(nx+1) = x(nx) + off.y.  x(1) and x(iend) are
@@ -308,11 +307,15 @@ __device__ __forceinline__ void sweep4_tile(const Geo &g, const Helm &h, const f
 
 // gx: blocks along x per component; block column q * gx + bx runs tile bx of
 // the set's q-th component.
-// Registers: 56 for Jacobi (36 warps per SM), 64 for the half-sweep (32);
-// unbounded the compiler takes 80 and 24 warps do not cover the loads'
-// latency.
+// Bound by issue and the loads' latency (DRAM at 40%).  Registers: 64 for
+// Jacobi (32 warps per SM), 72 for the half-sweep (28): without the lanes'
+// predicates on the row's end (issue()) these hold every load in flight.
+// Warps per SM against time per sweep of three components at 512x256x256,
+// Jacobi: 40 -> 413 us, 36 -> 381, 32 -> 350, 28 -> 355, 24 -> 385; even half:
+// 36 -> 389, 32 -> 350, 28 -> 340, 24 -> 357.  (Predicated, at 36 and 32
+// warps: 400 and 356.)
 template <int MODE, int BY>
-__global__ void __launch_bounds__(32 * BY, BY == 1 ? 32 : (MODE == M_JAC ? 36 : 32) / BY)
+__global__ void __launch_bounds__(32 * BY, BY == 1 ? 32 : (MODE == M_JAC ? 32 : 28) / BY)
     k_sweep4(Geo g, Helm h, const __grid_constant__ SweepSet32 s, int gx, int flg, int bc, int fuse) {
   const int q = blockIdx.x / gx, bx = blockIdx.x - q * gx, comp = s.id[q];
   if (comp == 0) {
