@@ -16,6 +16,7 @@
 // only b (4 bytes), cutting a Jacobi point from ~40 to ~16 bytes of traffic.
 // Templated on the arithmetic type and the coefficient source (records, or
 // MuCoef).
+#include <type_traits>
 #include "tpls_sweep.cuh"
 
 namespace tpls {
@@ -77,27 +78,33 @@ __device__ __forceinline__ Rec<float> get_rec(int comp, const Geo &g, const MuCo
   return q;
 }
 
-// The per-routine entries' coefficients (sor_iteration_allflux.f90 on host
-// arrays): face viscosities of the FP64 viscosity_aug and the right-hand
-// side, divided by the Helmholtz diagonal, the wall rule folded into the z
-// slots as in the records.
-__device__ __forceinline__ Rec<double> get_rec(int comp, const Geo &g, const RefCoef &s, int c, int i, int j, int k,
-                                               bool) {
-  const FcT<double> f = faces<double>(comp, g, s.mu, i, j, k);
-  const double diag = 1.0 + s.ax2 * (f.px + f.mx) + s.ay2 * (f.py + f.my) + s.az2 * (f.pz + f.mz);
-  const double r = 1.0 / diag;
-  double czp = s.az2 * f.pz * r, czm = s.az2 * f.mz * r;
-  if (comp != 2) {
-    if (k == 0) {
-      czp += czm * (1.0 / 3.0);
-      czm = -2.0 * czm;
-    } else if (k == g.nz - 1) {
-      czm += czp * (1.0 / 3.0);
-      czp = -2.0 * czp;
-    }
+// The per-routine entries (sor_iteration_allflux.f90 on host arrays): A and B
+// of point (i, j, k) of the odd half-sweep from the FP64 viscosity (ref_point),
+// x the field, zp its value above (unused at the wall levels of u and v).
+// near and lo in, near1 and hi out, as ref_point.  (111 us per half-sweep of a
+// component at 192x96x144; with the coefficients normalised one by one by a
+// division 163.)
+template <int CC>
+__device__ __forceinline__ void ref_odd(const Geo &g, const RefCoef &s, const double *__restrict__ x,
+                                        const double *m, int c, int k, int k0, double xc, double zp, double near,
+                                        double lo, double &near1, double &hi, double &A, double &B) {
+  double h;
+  double t = ref_point<CC>(g, s, m, near, lo, s.rhs[c], x[c + 1], x[c - 1], x[c + g.sy], x[c - g.sy], hi, near1, h);
+  double below = lo;  // weight of the point below
+  double zt = zp;
+  if (CC != 2 && k == g.nz - 1) {  // ghost -2 x + x(k-1)/3 above
+    zt = -2.0 * xc;
+    below = fma(hi, 1.0 / 3.0, lo);
   }
-  Rec<double> q = {s.ax2 * f.px * r, s.ax2 * f.mx * r, s.ay2 * f.py * r, s.ay2 * f.my * r, czp, czm, s.rhs[c] * r, 1.2 * czm};
-  return q;
+  t = fma(s.cz, hi * zt, t);
+  B = 0.0;
+  if (k == k0) {  // the wall value (w) or the ghost -2 x + x(k+1)/3 (u, v) below
+    const double zm = (CC == 2) ? x[c - g.sz] : fma(zp, 1.0 / 3.0, -2.0 * xc);
+    t = fma(s.cz, lo * zm, t);
+  } else {
+    B = ((1.2 * s.cz) * h) * below;
+  }
+  A = fma(1.2, fma(t, h, -xc), xc);
 }
 
 // The FP64 sweeps run every component of the set in one launch (gx blocks
@@ -223,7 +230,7 @@ __device__ __forceinline__ void st_release_u32(unsigned *p, unsigned v) {
 // blocks) 470.  Lanes past the row's end take the row's first point of this
 // colour (and store nothing), which frees the loads of their predicates: 404
 // against 422.
-template <typename T, typename CS>
+template <typename T, typename CS, int CC>
 __device__ __forceinline__ void odd_produce_scan_levels(int comp, const Geo &g, const CS &coef,
                                                         const T *__restrict__ x, int i, int j, bool act, int k0,
                                                         int kc, int n, T (*sA)[32], T (*sB)[32], T (*ey)[32],
@@ -239,22 +246,30 @@ __device__ __forceinline__ void odd_produce_scan_levels(int comp, const Geo &g, 
       T A = 0, B = 0;
       if (sizeof(T) == 4 || act) {
         const int c = TPLS_IDX(g, ic, j, k);
-        const Rec<T> q = get_rec(comp, g, coef, c, ic, j, k, true);
         const T xc = x[c];
         T zp;
-        if (comp == 2) zp = x[c + sz];
-        else zp = (k == nz - 1) ? xc : x[c + sz];
-        T part = fma(q.xp, x[c + 1], q.b);
-        part = fma(q.xm, x[c - 1], part);
-        part = fma(q.yp, x[c + sy_], part);
-        part = fma(q.ym, x[c - sy_], part);
-        part = fma(q.zp, zp, part);
-        if (k == k0) {  // the point below is a wall value (w) or the point itself (u, v)
-          const T zm = (comp == 2) ? x[c - sz] : xc;
-          A = xc + (T)1.2 * (fma(q.zm, zm, part) - xc);
+        if constexpr (std::is_same<CS, RefCoef>::value) {
+          const double *m = ref_cell<CC>(g, coef, ic, j, k);
+          double near, lo, near1, hi;
+          ref_begin<CC>(g, m, near, lo);
+          zp = (CC == 2 || k < nz - 1) ? x[c + sz] : 0.0;
+          ref_odd<CC>(g, coef, x, m, c, k, k0, xc, zp, near, lo, near1, hi, A, B);
         } else {
-          A = xc + (T)1.2 * (part - xc);
-          B = (sizeof(T) == 8) ? q.bz : (T)1.2 * q.zm;
+          const Rec<T> q = get_rec(comp, g, coef, c, ic, j, k, true);
+          if (comp == 2) zp = x[c + sz];
+          else zp = (k == nz - 1) ? xc : x[c + sz];
+          T part = fma(q.xp, x[c + 1], q.b);
+          part = fma(q.xm, x[c - 1], part);
+          part = fma(q.yp, x[c + sy_], part);
+          part = fma(q.ym, x[c - sy_], part);
+          part = fma(q.zp, zp, part);
+          if (k == k0) {  // the point below is a wall value (w) or the point itself (u, v)
+            const T zm = (comp == 2) ? x[c - sz] : xc;
+            A = xc + (T)1.2 * (fma(q.zm, zm, part) - xc);
+          } else {
+            A = xc + (T)1.2 * (part - xc);
+            B = (sizeof(T) == 8) ? q.bz : (T)1.2 * q.zm;
+          }
         }
       }
       sA[lk][lane] = A;
@@ -285,12 +300,12 @@ __device__ __forceinline__ void odd_produce_scan_levels(int comp, const Geo &g, 
 // record and the segment kernel's once-per-block fold, this form measured
 // 10% faster than the level form for the FP64 sweeps at 256x128x192 and
 // 11% slower for the FP32 sweeps at 512x256x256.
-template <typename T, typename CS>
+template <typename T, typename CS, int CC>
 __device__ __forceinline__ void odd_produce_scan(int comp, const Geo &g, const CS &coef, const T *__restrict__ x,
                                                  int i, int j, bool act, int k0, int kc, int n,
                                                  T (*sA)[32], T (*sB)[32], T (*ey)[32], T (*ep)[32]) {
   if constexpr (sizeof(T) == 4) {
-    odd_produce_scan_levels<T, CS>(comp, g, coef, x, i, j, act, k0, kc, n, sA, sB, ey, ep);
+    odd_produce_scan_levels<T, CS, CC>(comp, g, coef, x, i, j, act, k0, kc, n, sA, sB, ey, ep);
   } else {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int sy_ = g.sy, sz = g.sz, nz = g.nz;
@@ -299,27 +314,45 @@ __device__ __forceinline__ void odd_produce_scan(int comp, const Geo &g, const C
     T yv = 0, pv = 1;
     int c = act ? TPLS_IDX(g, i, j, kc + lb) : 0;
     T xc = (act && lb < le) ? x[c] : (T)0;
+    constexpr bool REF = std::is_same<CS, RefCoef>::value;
+    double near = 0.0, lo = 0.0;  // REF: viscosities carried up the column
+    const double *m = nullptr;
+    if constexpr (REF) {
+      if (act && lb < le) {
+        m = ref_cell<CC>(g, coef, i, j, kc + lb);
+        ref_begin<CC>(g, m, near, lo);
+      }
+    }
 #pragma unroll
     for (int l = 0; l < PER; l++) {
       const int lk = lb + l, k = kc + lk;
       if (lk < le) {
         T A = 0, B = 0;
         if (act) {
-          const Rec<T> q = get_rec(comp, g, coef, c, i, j, k, true);
           T zp;
-          if (comp == 2) zp = x[c + sz];
-          else zp = (k == nz - 1) ? xc : x[c + sz];
-          T part = fma(q.xp, x[c + 1], q.b);
-          part = fma(q.xm, x[c - 1], part);
-          part = fma(q.yp, x[c + sy_], part);
-          part = fma(q.ym, x[c - sy_], part);
-          part = fma(q.zp, zp, part);
-          if (k == k0) {
-            const T zm = (comp == 2) ? x[c - sz] : xc;
-            A = xc + (T)1.2 * (fma(q.zm, zm, part) - xc);
+          if constexpr (REF) {
+            double near1, hi;
+            zp = (CC == 2 || k < nz - 1) ? x[c + sz] : 0.0;
+            ref_odd<CC>(g, coef, x, m, c, k, k0, xc, zp, near, lo, near1, hi, A, B);
+            near = near1;
+            lo = hi;
+            m += g.szm;
           } else {
-            A = xc + (T)1.2 * (part - xc);
-            B = q.bz;
+            const Rec<T> q = get_rec(comp, g, coef, c, i, j, k, true);
+            if (comp == 2) zp = x[c + sz];
+            else zp = (k == nz - 1) ? xc : x[c + sz];
+            T part = fma(q.xp, x[c + 1], q.b);
+            part = fma(q.xm, x[c - 1], part);
+            part = fma(q.yp, x[c + sy_], part);
+            part = fma(q.ym, x[c - sy_], part);
+            part = fma(q.zp, zp, part);
+            if (k == k0) {
+              const T zm = (comp == 2) ? x[c - sz] : xc;
+              A = xc + (T)1.2 * (fma(q.zm, zm, part) - xc);
+            } else {
+              A = xc + (T)1.2 * (part - xc);
+              B = q.bz;
+            }
           }
           xc = zp;  // x(k+1), the centre of the next level (unused after k = nz-1)
           c += sz;
@@ -425,7 +458,7 @@ __device__ __forceinline__ void sor_odd_c4_tile(int comp_, const Geo &g, const H
   T carry = 0;  // x of the level below the super-chunk (k0 has B = 0)
   for (int kc = k0; kc <= k1; kc += SOC_SC) {
     const int n = min(SOC_SC, k1 - kc + 1);
-    odd_produce_scan_levels<T, CS>(comp, g, coef, x, i, j, act, k0, kc, n, sA, sB, ey, ep);  // 1. produce, 2. scan
+    odd_produce_scan_levels<T, CS, CC>(comp, g, coef, x, i, j, act, k0, kc, n, sA, sB, ey, ep);  // 1. produce, 2. scan
     const int lb = w * PER, le = min(n, lb + PER);
     // 3. fold and write
     T xin = carry;
@@ -495,7 +528,7 @@ __device__ __forceinline__ void sor_odd_segment(int comp_, const Geo &g, const H
   const int kc = k0 + seg * SOC_SC, n = min(SOC_SC, k1 - kc + 1);
   if (n <= 0) return;  // w's columns are a level shorter: its last segment can be empty (none waits for it)
   constexpr int PER = SOC_SC / SOC_W;
-  odd_produce_scan<T, CS>(comp, g, coef, x, i, j, act, k0, kc, n, sA, sB, ey, ep);
+  odd_produce_scan<T, CS, CC>(comp, g, coef, x, i, j, act, k0, kc, n, sA, sB, ey, ep);
   if (w == 0) {
     T xin = 0;  // k0 has B = 0
     if (seg > 0) {
@@ -544,10 +577,11 @@ __device__ __forceinline__ void sor_odd_segment(int comp_, const Geo &g, const H
 }
 
 // One component's work on a tile, the component a compile-time constant for
-// the FP32 sweeps (their face averages differ by component).
+// the sweeps that form face viscosities (FP32, per-routine entries: these
+// differ by component).
 #define TPLS_BY_COMP(CALL)                        \
   do {                                            \
-    if constexpr (sizeof(T) == sizeof(float)) {   \
+    if constexpr (!std::is_same<CS, const double *>::value) { \
       if (comp == 0) CALL(0);                     \
       else if (comp == 1) CALL(1);                \
       else CALL(2);                               \
@@ -737,21 +771,14 @@ cudaError_t launch_sor_set(const Geo &g, const Phys &ph, const SweepSet32 &s, co
   return odd_set(g, helm_of(ph), s, pres, flg, bc, fuse_ghosts, st, oc);
 }
 
-cudaError_t launch_sor_ref_odd(int comp, const Geo &g, const Phys &ph, double *x, const double *rhs,
-                               const double *mu, int flg, cudaStream_t st, const OddChain *oc) {
-  const Helm h = helm_of(ph);
+cudaError_t launch_ref_odd(int comp, const Geo &g, const RefCoef &r, double *x, int flg, cudaStream_t st,
+                           const OddChain *oc) {
   SweepSet<double, RefCoef> s;
   s.n = 1;
   s.id[0] = comp;
   s.x[0] = x;
-  RefCoef r;
-  r.mu = mu;
-  r.rhs = rhs;
-  r.ax2 = h.ax2;
-  r.ay2 = h.ay2;
-  r.az2 = h.az2;
   s.coef[0] = r;
-  return odd_set(g, h, s, nullptr, flg, 0, 0, st, oc);
+  return odd_set(g, Helm{}, s, nullptr, flg, 0, 0, st, oc);
 }
 
 MuCoef mu_coef(const Phys &ph, const float *mu, const float *b, const float4 *bco) {

@@ -2349,9 +2349,8 @@ static int conv_diff_entry(tpls_ctx *c, int want_conv, double *o_u, double *o_v,
   TCK(cudaMemsetAsync(OU - XOFF, 0, bytes, c->st));
   TCK(cudaMemsetAsync(OV - XOFF, 0, bytes, c->st));
   TCK(cudaMemsetAsync(OW - XOFF, 0, bytes, c->st));
-  LCK(c, launch_conv_diff(0, want_conv, c->g, ph, U, V, W, c->scr_mu, OU, c->st));
-  LCK(c, launch_conv_diff(1, want_conv, c->g, ph, U, V, W, c->scr_mu, OV, c->st));
-  LCK(c, launch_conv_diff(2, want_conv, c->g, ph, U, V, W, c->scr_mu, OW, c->st));
+  double *const out[3] = {OU, OV, OW};
+  LCK(c, launch_conv_diff(want_conv, c->g, ph, U, V, W, c->scr_mu, out, c->st));
   TCK(d2h(c, o_u, OU, nz));
   TCK(d2h(c, o_v, OV, nz));
   TCK(d2h(c, o_w, OW, nz + 1));
@@ -2392,7 +2391,7 @@ static int jacobi_entry(tpls_ctx *c, int comp, double *x3, const double *x3_old,
   TCK(h2d(c, XO, x3_old, nzp));
   TCK(h2d(c, R, rhs, nzp));
   TCK(h2d_mu(c, c->scr_mu, va));
-  LCK(c, launch_jacobi(comp, c->g, ph, XO, R, c->scr_mu, nullptr, X, 0, 0, c->st));
+  LCK(c, launch_ref_jacobi(comp, c->g, ref_coef(comp, ph, R, c->scr_mu), XO, X, c->st));
   TCK(d2h(c, x3, X, nzp));
   TCK(cudaStreamSynchronize(c->st));
   return TPLS_OK;
@@ -2424,10 +2423,9 @@ static int sor_entry(tpls_ctx *c, int comp, double *x3, const double *rhs, const
   TCK(h2d(c, X, x3, nzp));
   TCK(h2d(c, R, rhs, nzp));
   TCK(h2d_mu(c, c->scr_mu, va));
-  if (*iteration_time % 2 == 0)
-    LCK(c, launch_sor(comp, c->g, ph, X, R, c->scr_mu, nullptr, *flg, *iteration_time, 0, 0, c->st));
-  else  // the column recurrence in chunks (as the step's sweeps), not one thread per column
-    LCK(c, launch_sor_ref_odd(comp, c->g, ph, X, R, c->scr_mu, *flg, c->st, odd_chain(c)));
+  const RefCoef rc = ref_coef(comp, ph, R, c->scr_mu);
+  if (*iteration_time % 2 == 0) LCK(c, launch_ref_even(comp, c->g, rc, X, *flg, c->st));
+  else LCK(c, launch_ref_odd(comp, c->g, rc, X, *flg, c->st, odd_chain(c)));
   TCK(d2h(c, x3, X, nzp));
   TCK(cudaStreamSynchronize(c->st));
   return TPLS_OK;

@@ -129,25 +129,10 @@ cudaError_t launch_mom_rhs64r32(int comp, const Geo &g, const Phys &ph,
                                 const double *c0, const double *s1,
                                 const double *s0, double *conv2,
                                 double *csf2, float *bdef, cudaStream_t st);
-// Standalone get_conv_all / get_diffusion_all (per-routine entries).
-cudaError_t launch_conv_diff(int comp, int want_conv, const Geo &g,
-                             const Phys &ph, const double *u2,
-                             const double *v2, const double *w2,
-                             const double *mu, double *out, cudaStream_t st);
-// jacobi_iteration_allflux.f90 / sor_iteration_allflux.f90 with the
-// boundary conditions of main_ns_hybrid.F90:756-887 fused in.
-//   bc: 0 = plain reference routine (only the routine's own BCs),
-//       1 = also the driver's post-sweep BCs (u: inlet copy, pressure outlet,
-//           fictitious point; v: inlet/outlet copies; w: walls, inlet,
-//           outlet).
-cudaError_t launch_jacobi(int comp, const Geo &g, const Phys &ph,
-                          const double *xo, const double *rhs,
-                          const double *mu, const double *pres, double *x,
-                          int bc, int fuse_ghosts, cudaStream_t st);
-cudaError_t launch_sor(int comp, const Geo &g, const Phys &ph, double *x,
-                       const double *rhs, const double *mu,
-                       const double *pres, int flg, int iteration_time,
-                       int bc, int fuse_ghosts, cudaStream_t st);
+// Standalone get_conv_all / get_diffusion_all (per-routine entries): out[q] =
+// conv or diff of component q on its domain (other entries are left untouched).
+cudaError_t launch_conv_diff(int want_conv, const Geo &g, const Phys &ph, const double *u2, const double *v2,
+                             const double *w2, const double *mu, double *const out[3], cudaStream_t st);
 // Tile-shape choice of the sweep kernels (autotuned per grid): jac / even =
 // block shape index (0: 32x4, 1: 32x8, 2: 64x4, 3: 16x8); odd is always 0
 // (the odd half-sweep has one shape).
@@ -171,17 +156,24 @@ struct OddChain {
 int odd_chain_segments(const Geo &g);
 
 // Coefficient source of the per-routine sweep entries: the FP64
-// viscosity_aug (device mu layout) and right-hand side of host arrays.
+// viscosity_aug (device mu layout) and right-hand side of host arrays, and
+// dt/(2 d^2) per axis (a quarter of it on the component's two other axes,
+// whose face viscosities are four-cell averages).
 struct RefCoef {
   const double *mu;
   const double *rhs;
-  double ax2, ay2, az2;
+  double cx, cy, cz;
 };
-// Odd-iteration half-sweep (iteration_time odd) of the per-routine entries
-// in the chunk-parallel column form, no boundary rows, no ghost fusing (the
-// reference's do_sor_u/v/w leave those to the driver).
-cudaError_t launch_sor_ref_odd(int comp, const Geo &g, const Phys &ph, double *x, const double *rhs,
-                               const double *mu, int flg, cudaStream_t st, const OddChain *oc);
+RefCoef ref_coef(int comp, const Phys &ph, const double *rhs, const double *mu);
+// The per-routine sweep entries (jacobi_iteration_allflux.f90,
+// sor_iteration_allflux.f90): only the routine's own boundary rows (those of
+// do_jacobi_v/w), no ghost rows.  The odd half-sweep (iteration_time odd) is
+// in the chunk-parallel column form.
+cudaError_t launch_ref_jacobi(int comp, const Geo &g, const RefCoef &s, const double *xo, double *x,
+                              cudaStream_t st);
+cudaError_t launch_ref_even(int comp, const Geo &g, const RefCoef &s, double *x, int flg, cudaStream_t st);
+cudaError_t launch_ref_odd(int comp, const Geo &g, const RefCoef &s, double *x, int flg, cudaStream_t st,
+                           const OddChain *oc);
 
 // FP32 sweeps in defect form: x holds d = x - X for the FP64 base X (the
 // component's state).  Their coefficients are recomputed per point from the

@@ -59,6 +59,54 @@ __device__ __forceinline__ FcT<T> faces(int comp, const Geo &g, const T *__restr
   return f;
 }
 
+// One point of the per-routine sweeps (jacobi_iteration_allflux.f90:84-90, the
+// same form in every Jacobi / SOR routine), whose coefficients come from the
+// FP64 viscosity.  Bound by the FP64 pipe: face viscosities as unscaled sums of
+// the pair of cells of the point's own face (`near`) and the neighbouring
+// pairs, the averages' quarter in the axis factor; the level's upper z face and
+// the next level's own pair are handed on, so that a thread marching up a
+// column forms each once; 1/diag from rcp_seed and one Newton step.
+// m: viscosity cell of the point (u, v: level k+1 of the p-grid; w: k); near =
+// m[0] + m[om] and lo (the lower z face) in; hi (the upper z face), near1 (near
+// of the level above) and h = 1/diag out.  Returns the right-hand side with
+// the x and y terms, to which the caller adds cz (hi zp + lo zm).
+template <int CC>
+__device__ __forceinline__ int ref_om(const Geo &g) {  // the far cell of a point's own face
+  return CC == 0 ? 1 : (CC == 1 ? -g.sy : g.szm);
+}
+template <int CC>
+__device__ __forceinline__ const double *ref_cell(const Geo &g, const RefCoef &s, int i, int j, int k) {
+  return s.mu + TPLS_IDXM(g, i, j + 1, CC == 2 ? k : k + 1);
+}
+template <int CC>
+__device__ __forceinline__ void ref_begin(const Geo &g, const double *m, double &near, double &lo) {
+  const int om = ref_om<CC>(g);
+  near = m[0] + m[om];
+  lo = (CC == 2) ? m[0] : near + (m[-g.szm] + m[-g.szm + om]);
+}
+template <int CC>
+__device__ __forceinline__ double ref_point(const Geo &g, const RefCoef &s, const double *m, double near, double lo,
+                                            double rhs, double xp, double xm, double yp, double ym, double &hi,
+                                            double &near1, double &h) {
+  const int om = ref_om<CC>(g), my = g.sy, mz = g.szm;
+  auto pair = [&](int o) { return m[o] + m[o + om]; };
+  const double fxp = (CC == 0) ? m[1] : near + pair(1), fxm = (CC == 0) ? m[0] : near + pair(-1);
+  const double fyp = (CC == 1) ? m[0] : near + pair(my), fym = (CC == 1) ? m[om] : near + pair(-my);
+  near1 = pair(mz);
+  hi = (CC == 2) ? m[mz] : near + near1;
+  double d = fma(s.cx, CC == 0 ? near : fxp + fxm, 1.0);
+  d = fma(s.cy, CC == 1 ? near : fyp + fym, d);
+  d = fma(s.cz, CC == 2 ? near : hi + lo, d);
+  if (rcp_range(d)) {
+    h = rcp_seed(d);
+    h = fma(h, fma(-d, h, 1.0), h);
+  } else {
+    h = div_slow(1.0, d);
+  }
+  const double t = fma(s.cx, fma(fxp, xp, fxm * xm), rhs);
+  return fma(s.cy, fma(fyp, yp, fym * ym), t);
+}
+
 // Slot of point (i, j, k) (linear index c, 1 <= i <= nx) in the coefficient
 // record arrays.  Each (j, k) row keeps the records of odd i in its first
 // half and of even i in its second half (the row pitch sy is a multiple of
