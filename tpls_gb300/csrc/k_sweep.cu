@@ -622,8 +622,11 @@ __global__ void __launch_bounds__(SOC_W * 32, sizeof(T) == 4 ? 8 : 5)  // 32 / 4
   }
 }
 
+// (FP64: with a bound of 1 block per SM the compiler takes the registers of 2
+// blocks and a half-sweep at 128x64x96 51 us instead of 40.5; bounds of 4 and
+// 5 blocks measured 40.8 and 42.)
 template <typename T, typename CS>
-__global__ void __launch_bounds__(SOC_W * 32, sizeof(T) == 4 ? 8 : 1)
+__global__ void __launch_bounds__(SOC_W * 32, sizeof(T) == 4 ? 8 : 3)
     k_sor_odd_c4(Geo g, Helm h, const __grid_constant__ SweepSet<T, CS> S, const double *__restrict__ P, int gx,
                  int flg, int bc, int fuse) {
   __shared__ OddShared<T> sh;
