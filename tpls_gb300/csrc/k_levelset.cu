@@ -3,12 +3,19 @@
 // levelset.f90:17-414, momentum_allflux.f90:474-521,
 // main_ns_hybrid.F90:646-724).
 //
-// Every kernel is a gather over the full halo'd index space: a thread
-// computes its own output element, including ghost planes, by evaluating
-// the reference's boundary rule (copy, linear extrapolation, inlet value)
-// on the interior values it needs.  That replaces the reference's sequence
-// of interior pass + boundary passes + exchange2d with one launch, with
-// identical values.
+// Every kernel writes the full halo'd index space in one launch, with the
+// values of the reference's sequence of interior pass, boundary passes and
+// exchange2d: a thread owns an interior column position (i, j) of its plane
+// and writes, beside its own element, the ghosts that copy it (periodic rows,
+// the outlet column) or that are its neighbours (the inlet column, the
+// extrapolated outlet column); the ghost z planes are blocks of their own that
+// evaluate the extrapolation.  With a thread per ghost element instead, a row
+// of nx + 2 points took a warp more than its nx / 32 for two of them, and a
+// warp's FP64 instructions hold the pipe as long for two lanes as for 32: 1.2
+// times the work at 256x128x192, 1.8 times at 64x32x48.  Measured, redistancing
+// and level-set update: 1584 -> 1374 us at 256x128x192, 609 -> 522 at
+// 192x96x112; the CSF force, whose end columns take their neighbour's value
+// from the next lane, 98 -> 48 us at 192x96x112.
 #include <cstring>
 #include <type_traits>
 
@@ -19,8 +26,27 @@ namespace tpls {
 
 constexpr int LS_BX = 32, LS_BY = 8;
 
-static inline dim3 full_grid(const Geo &g, int nzp) {
-  return dim3((g.nx + 2 + LS_BX - 1) / LS_BX, (g.ny + 2 + LS_BY - 1) / LS_BY, nzp);
+static inline dim3 owned_grid(const Geo &g, int nzp) {
+  return dim3((g.nx + LS_BX - 1) / LS_BX, (g.ny + LS_BY - 1) / LS_BY, nzp);
+}
+
+// w(q) for the element q = c of row j and for its periodic ghost row
+template <typename F>
+__device__ __forceinline__ void rows_of(const Geo &g, int j, int c, F w) {
+  w(c);
+  if (j == 1) w(c + g.sy * g.ny);
+  if (j == g.ny) w(c - g.sy * g.ny);
+}
+
+// levelset.f90 inlet value (k - 1/2) h - height at i = 0 (the ghost planes
+// extrapolated).  A call, not inline code: if-converted it would put its FP64
+// instructions on every lane's FP64 pipe, and only one column of the grid
+// takes it.
+__device__ __forceinline__ double ls_inlet(double h, double height, int k) { return (k * h - 0.5 * h) - height; }
+__device__ __noinline__ double inlet_plane(double h, double height, int k, int nz) {
+  if (k == 0) return 2.0 * ls_inlet(h, height, 1) - ls_inlet(h, height, 2);
+  if (k == nz + 1) return 2.0 * ls_inlet(h, height, nz) - ls_inlet(h, height, nz - 1);
+  return ls_inlet(h, height, k);
 }
 
 // ---------------------------------------------------------------------------
@@ -30,34 +56,39 @@ static inline dim3 full_grid(const Geo &g, int nzp) {
 __device__ __forceinline__ double ab3_val(const Geo &g, const Phys &ph, const double *phi2,
                                           const double *c0, const double *c1,
                                           const double *c2, int i, int j, int k) {
-  if (i == 0) return (k * ph.dz - 0.5 * ph.dz) - ph.height;
-  const int ii = (i == g.nx + 1) ? g.nx : i;
-  const int c = TPLS_IDX(g, ii, j, k);
+  const int c = TPLS_IDX(g, i, j, k);
   return phi2[c] - ph.dt * ((23.0 / 12.0) * c2[c] - (4.0 / 3.0) * c1[c] + (5.0 / 12.0) * c0[c]);
 }
 
 __global__ void k_ls_ab3(Geo g, Phys ph, const double *__restrict__ phi2,
                          const double *__restrict__ c0, const double *__restrict__ c1,
                          const double *__restrict__ c2, double *__restrict__ phi3) {
-  const int i = blockIdx.x * LS_BX + threadIdx.x, j = blockIdx.y * LS_BY + threadIdx.y;
+  const int i = blockIdx.x * LS_BX + threadIdx.x + 1, j = blockIdx.y * LS_BY + threadIdx.y + 1;
   const int k = blockIdx.z;
-  if (i > g.nx + 1 || j > g.ny + 1) return;
-  const int jj = wrapy(j, g.ny);
+  if (i > g.nx || j > g.ny) return;
   double v;
   if (k == 0)
-    v = 2.0 * ab3_val(g, ph, phi2, c0, c1, c2, i, jj, 1) - ab3_val(g, ph, phi2, c0, c1, c2, i, jj, 2);
+    v = 2.0 * ab3_val(g, ph, phi2, c0, c1, c2, i, j, 1) - ab3_val(g, ph, phi2, c0, c1, c2, i, j, 2);
   else if (k == g.nz + 1)
-    v = 2.0 * ab3_val(g, ph, phi2, c0, c1, c2, i, jj, g.nz) -
-        ab3_val(g, ph, phi2, c0, c1, c2, i, jj, g.nz - 1);
+    v = 2.0 * ab3_val(g, ph, phi2, c0, c1, c2, i, j, g.nz) -
+        ab3_val(g, ph, phi2, c0, c1, c2, i, j, g.nz - 1);
   else
-    v = ab3_val(g, ph, phi2, c0, c1, c2, i, jj, k);
-  phi3[TPLS_IDX(g, i, j, k)] = v;
+    v = ab3_val(g, ph, phi2, c0, c1, c2, i, j, k);
+  const int c = TPLS_IDX(g, i, j, k);
+  rows_of(g, j, c, [&](int q) {
+    phi3[q] = v;
+    if (i == g.nx) phi3[q + 1] = v;
+  });
+  if (i == 1) {
+    const double v0 = inlet_plane(ph.dz, ph.height, k, g.nz);
+    rows_of(g, j, c, [&](int q) { phi3[q - 1] = v0; });
+  }
 }
 
 cudaError_t launch_ls_ab3(const Geo &g, const Phys &ph, const double *phi2,
                           const double *c0, const double *c1, const double *c2,
                           double *phi3, cudaStream_t st) {
-  k_ls_ab3<<<full_grid(g, g.nz + 2), dim3(LS_BX, LS_BY), 0, st>>>(g, ph, phi2, c0, c1, c2, phi3);
+  k_ls_ab3<<<owned_grid(g, g.nz + 2), dim3(LS_BX, LS_BY), 0, st>>>(g, ph, phi2, c0, c1, c2, phi3);
   return cudaGetLastError();
 }
 
@@ -100,15 +131,21 @@ __device__ __noinline__ double status_distance(double h, double p, double pxp, d
 template <typename T>
 __global__ void k_ls_status(Geo g, double h, const double *__restrict__ phi, T *__restrict__ D,
                             signed char *__restrict__ flags) {
-  const int i = blockIdx.x * LS_BX + threadIdx.x, j = blockIdx.y * LS_BY + threadIdx.y;
+  const int i = blockIdx.x * LS_BX + threadIdx.x + 1, j = blockIdx.y * LS_BY + threadIdx.y + 1;
   const int k = blockIdx.z;
-  if (i > g.nx + 1 || j > g.ny + 1) return;
+  if (i > g.nx || j > g.ny) return;
   const int c = TPLS_IDX(g, i, j, k);
-  if (i < 1 || i > g.nx || j < 1 || j > g.ny || k < 1 || k > g.nz) {
-    D[c] = (T)0;
-    flags[c] = 0;
-    return;
-  }
+  const bool plane = k < 1 || k > g.nz;
+  rows_of(g, j, c, [&](int q) {  // the ghosts beside and beyond the thread's element
+    auto zero = [&](int o) {
+      D[o] = (T)0;
+      flags[o] = 0;
+    };
+    if (q != c || plane) zero(q);
+    if (i == 1) zero(q - 1);
+    if (i == g.nx) zero(q + 1);
+  });
+  if (plane) return;
   // FP64 in both forms: the status flags are discrete decisions, so the
   // FP32-mixed form takes them from the same arithmetic as the FP64 form
   // and only stores D in FP32.  Signs, the test min(p*q) <= 0 and the
@@ -129,12 +166,12 @@ __global__ void k_ls_status(Geo g, double h, const double *__restrict__ phi, T *
 
 cudaError_t launch_ls_status(const Geo &g, const Phys &ph, const double *phi3,
                              double *D, signed char *flags, cudaStream_t st) {
-  k_ls_status<double><<<full_grid(g, g.nz + 2), dim3(LS_BX, LS_BY), 0, st>>>(g, ph.dx, phi3, D, flags);
+  k_ls_status<double><<<owned_grid(g, g.nz + 2), dim3(LS_BX, LS_BY), 0, st>>>(g, ph.dx, phi3, D, flags);
   return cudaGetLastError();
 }
 cudaError_t launch_ls_status(const Geo &g, const Phys &ph, const double *phi3, float *D, signed char *flags,
                              cudaStream_t st) {
-  k_ls_status<float><<<full_grid(g, g.nz + 2), dim3(LS_BX, LS_BY), 0, st>>>(g, ph.dx, phi3, D, flags);
+  k_ls_status<float><<<owned_grid(g, g.nz + 2), dim3(LS_BX, LS_BY), 0, st>>>(g, ph.dx, phi3, D, flags);
   return cudaGetLastError();
 }
 
@@ -188,8 +225,7 @@ __device__ __forceinline__ TC rs_dc(const Geo &g, TC h, const LD &pr, TC p, cons
     const double az = dpos_bits(sp - dmin_bits(neg_if(pr[c - g.sz], m), neg_if(pr[c + g.sz], m)));
     const double a2 = (s == 2) ? ay : az, a3 = (s == 2) ? az : ay;
     // sqrt_rn: the same rounding with one FP64 operation instead of about
-    // eight; the point takes nine in all (16 before: 226 us per iteration at
-    // 256x128x192, 1086 at 512x256x256)
+    // eight; the point takes nine in all (16 before)
     return neg_if(sqrt_rn(ax * ax + a2 * a2 + a3 * a3) - h, m);
   } else {
     if (s == 2) {
@@ -226,20 +262,6 @@ __device__ __forceinline__ RT rs_update(const Geo &g, TC h, TC ktau, const TI *_
   else return (RT)pr0[c] - (RT)(ktau * dc);
 }
 
-// levelset.f90 inlet value (k - 1/2) h - height at i = 0.  A call, not
-// inline code: if-converted it would put its FP64 instructions on every
-// lane's FP64 pipe, and only one column of the grid takes it.
-__device__ __noinline__ double ls_inlet(double h, double height, int k) {
-  return (k * h - 0.5 * h) - height;
-}
-
-template <typename TC, typename TI, typename RT>
-__device__ __forceinline__ RT rs_val(const Geo &g, const Phys &ph, TC h, TC ktau, const TI *pr, const TC *D,
-                                     const signed char *flags, int i, int j, int k) {
-  if (i == 0) return (RT)ls_inlet((double)h, ph.height, k);
-  return rs_update<TC, TI, RT>(g, h, ktau, pr, D, flags, (i == g.nx + 1) ? g.nx : i, j, k);
-}
-
 // TI/TO: storage of the input/output iterate; TC: arithmetic (double for
 // the FP64 form; float for the FP32-mixed form, whose first iteration reads
 // the FP64 phi3 and whose last writes the FP64 state).
@@ -250,27 +272,29 @@ template <typename TC, typename TI, typename TO, bool ERR>
 __global__ void __launch_bounds__(LS_BX *LS_BY)
     k_ls_iter(Geo g, Phys ph, TC h, TC ktau, const TI *__restrict__ pr, const TC *__restrict__ D,
               const signed char *__restrict__ flags, TO *__restrict__ out, double *__restrict__ err_part) {
-  const int i = blockIdx.x * LS_BX + threadIdx.x, j = blockIdx.y * LS_BY + threadIdx.y;
+  const int i = blockIdx.x * LS_BX + threadIdx.x + 1, j = blockIdx.y * LS_BY + threadIdx.y + 1;
   const int k = blockIdx.z;
   double e = 0.0;
-  if (i <= g.nx + 1 && j <= g.ny + 1) {
-    const int jj = wrapy(j, g.ny);
+  if (i <= g.nx && j <= g.ny) {
     using RT = typename std::conditional<sizeof(TO) == sizeof(double), double, TC>::type;
+    auto val = [&](int kk) { return rs_update<TC, TI, RT>(g, h, ktau, pr, D, flags, i, j, kk); };
     RT v;
-    if (k == 0)
-      v = (RT)2 * rs_val<TC, TI, RT>(g, ph, h, ktau, pr, D, flags, i, jj, 1) -
-          rs_val<TC, TI, RT>(g, ph, h, ktau, pr, D, flags, i, jj, 2);
-    else if (k == g.nz + 1)
-      v = (RT)2 * rs_val<TC, TI, RT>(g, ph, h, ktau, pr, D, flags, i, jj, g.nz) -
-          rs_val<TC, TI, RT>(g, ph, h, ktau, pr, D, flags, i, jj, g.nz - 1);
-    else
-      v = rs_val<TC, TI, RT>(g, ph, h, ktau, pr, D, flags, i, jj, k);
+    if (k == 0) v = (RT)2 * val(1) - val(2);
+    else if (k == g.nz + 1) v = (RT)2 * val(g.nz) - val(g.nz - 1);
+    else v = val(k);
     const int c = TPLS_IDX(g, i, j, k);
-    if (ERR && i >= 1 && i <= g.nx && j >= 1 && j <= g.ny) {
+    if (ERR) {
       const double d = (double)pr[c] - (double)v;
       e = d * d;
     }
-    out[c] = (TO)v;
+    rows_of(g, j, c, [&](int q) {
+      out[q] = (TO)v;
+      if (i == g.nx) out[q + 1] = (TO)v;
+    });
+    if (i == 1) {
+      const RT v0 = (RT)inlet_plane((double)h, ph.height, k, g.nz);
+      rows_of(g, j, c, [&](int q) { out[q - 1] = (TO)v0; });
+    }
   }
   if constexpr (ERR) {
     __shared__ double s[LS_BX * LS_BY];
@@ -339,16 +363,18 @@ __device__ __forceinline__ float rs_dc_pair(const Geo &g, float h, const FFSrc<I
   return 0.0f;
 }
 
-// inlet row (levelset.f90:168-177), FP64, out of line (see below)
-__device__ __noinline__ FF ff_inlet(float h, double height, int k) {
-  return ff_split((k * (double)h - 0.5 * (double)h) - height);
+// inlet row (levelset.f90:168-177; the ghost planes extrapolated), FP64, out
+// of line (see below)
+__device__ __noinline__ FF ff_inlet(float h, double height, int k, int nz) {
+  auto in = [&](int q) { return ff_split(ls_inlet((double)h, height, q)); };
+  if (k == 0) return ff_split(2.0 * ff_dbl(in(1)) - ff_dbl(in(2)));
+  if (k == nz + 1) return ff_split(2.0 * ff_dbl(in(nz)) - ff_dbl(in(nz - 1)));
+  return in(k);
 }
 
 template <bool IN64>
-__device__ __forceinline__ FF ff_val(const Geo &g, const Phys &ph, float h, float ktau, const FFSrc<IN64> &src,
+__device__ __forceinline__ FF ff_val(const Geo &g, float h, float ktau, const FFSrc<IN64> &src,
                                      const float *D, const signed char *flags, int i, int j, int k) {
-  if (i == 0) return ff_inlet(h, ph.height, k);
-  if (i == g.nx + 1) i = g.nx;
   const int c = TPLS_IDX(g, i, j, k);
   const F2 p = src.pair(c);
   const float inc = ktau * rs_dc_pair<IN64>(g, h, src, p, D, flags[c], c);
@@ -360,11 +386,11 @@ __device__ __forceinline__ FF ff_val(const Geo &g, const Phys &ph, float h, floa
 // into the kernel body their FP64 instructions would be issued, predicated
 // off, for every point and fill GB300's slow FP64 pipe.
 template <bool IN64>
-__device__ __noinline__ FF ff_ghost_plane(const Geo &g, const Phys &ph, float h, float ktau, const FFSrc<IN64> &src,
+__device__ __noinline__ FF ff_ghost_plane(const Geo &g, float h, float ktau, const FFSrc<IN64> &src,
                                           const float *D, const signed char *flags, int i, int jj, int k) {
   const int k1 = (k == 0) ? 1 : g.nz, k2 = (k == 0) ? 2 : g.nz - 1;
-  return ff_split(2.0 * ff_dbl(ff_val<IN64>(g, ph, h, ktau, src, D, flags, i, jj, k1)) -
-                  ff_dbl(ff_val<IN64>(g, ph, h, ktau, src, D, flags, i, jj, k2)));
+  return ff_split(2.0 * ff_dbl(ff_val<IN64>(g, h, ktau, src, D, flags, i, jj, k1)) -
+                  ff_dbl(ff_val<IN64>(g, h, ktau, src, D, flags, i, jj, k2)));
 }
 
 template <bool IN64, bool OUT64>
@@ -372,26 +398,35 @@ __global__ void __launch_bounds__(LS_BX *LS_BY)
     k_ls_iter_ff(Geo g, Phys ph, float h, float ktau, FFSrc<IN64> src, const float *__restrict__ D,
                  const signed char *__restrict__ flags, double *__restrict__ out64, float *__restrict__ ohi,
                  float *__restrict__ olo, double *__restrict__ err_part) {
-  const int i = blockIdx.x * LS_BX + threadIdx.x, j = blockIdx.y * LS_BY + threadIdx.y;
+  const int i = blockIdx.x * LS_BX + threadIdx.x + 1, j = blockIdx.y * LS_BY + threadIdx.y + 1;
   const int k = blockIdx.z;
   float e = 0.0f;
-  if (i <= g.nx + 1 && j <= g.ny + 1) {
-    const int jj = wrapy(j, g.ny);
+  if (i <= g.nx && j <= g.ny) {
     const int c = TPLS_IDX(g, i, j, k);
     FF v;
     if (k == 0 || k == g.nz + 1)  // linear extrapolation, in FP64
-      v = ff_ghost_plane<IN64>(g, ph, h, ktau, src, D, flags, i, jj, k);
+      v = ff_ghost_plane<IN64>(g, h, ktau, src, D, flags, i, j, k);
     else
-      v = ff_val<IN64>(g, ph, h, ktau, src, D, flags, i, jj, k);
-    if (err_part && i >= 1 && i <= g.nx && j >= 1 && j <= g.ny) {  // the iteration's change, from pairs
+      v = ff_val<IN64>(g, h, ktau, src, D, flags, i, j, k);
+    if (err_part) {  // the iteration's change, from pairs
       const float d = dif(src.pair(c), F2{v.hi, v.lo});
       e = d * d;
     }
-    if (OUT64) {  // exact widening by integer operations, one FP64 add
-      out64[c] = widen_bits(v.hi) + widen_bits(v.lo);
-    } else {
-      ohi[c] = v.hi;
-      olo[c] = v.lo;
+    auto write = [&](int q, const FF &x) {
+      if (OUT64) {  // exact widening by integer operations, one FP64 add
+        out64[q] = widen_bits(x.hi) + widen_bits(x.lo);
+      } else {
+        ohi[q] = x.hi;
+        olo[q] = x.lo;
+      }
+    };
+    rows_of(g, j, c, [&](int q) {
+      write(q, v);
+      if (i == g.nx) write(q + 1, v);
+    });
+    if (i == 1) {
+      const FF v0 = ff_inlet(h, ph.height, k, g.nz);
+      rows_of(g, j, c, [&](int q) { write(q - 1, v0); });
     }
   }
   if (err_part) {
@@ -409,7 +444,7 @@ __global__ void __launch_bounds__(LS_BX *LS_BY)
 }
 
 int ls_iter_blocks(const Geo &g) {
-  dim3 gr = full_grid(g, g.nz + 2);
+  const dim3 gr = owned_grid(g, g.nz + 2);
   return (int)(gr.x * gr.y * gr.z);
 }
 
@@ -418,10 +453,10 @@ static cudaError_t ls_iter(const Geo &g, const Phys &ph, const TI *pr, const TC 
                            TO *pr_new, double *err_part, cudaStream_t st) {
   const double h = ph.dx, dtau = 0.3 * h;
   if (err_part)
-    k_ls_iter<TC, TI, TO, true><<<full_grid(g, g.nz + 2), dim3(LS_BX, LS_BY), 0, st>>>(
+    k_ls_iter<TC, TI, TO, true><<<owned_grid(g, g.nz + 2), dim3(LS_BX, LS_BY), 0, st>>>(
         g, ph, (TC)h, (TC)(dtau / h), pr, D, flags, pr_new, err_part);
   else
-    k_ls_iter<TC, TI, TO, false><<<full_grid(g, g.nz + 2), dim3(LS_BX, LS_BY), 0, st>>>(
+    k_ls_iter<TC, TI, TO, false><<<owned_grid(g, g.nz + 2), dim3(LS_BX, LS_BY), 0, st>>>(
         g, ph, (TC)h, (TC)(dtau / h), pr, D, flags, pr_new, err_part);
   return cudaGetLastError();
 }
@@ -433,7 +468,7 @@ cudaError_t launch_ls_iter_ff(const Geo &g, const Phys &ph, const double *in64, 
                               const float *lo, const float *D, const signed char *flags, double *out64,
                               float *ohi, float *olo, double *err_part, cudaStream_t st) {
   const float h = (float)ph.dx, ktau = (float)(0.3 * ph.dx / ph.dx);
-  const dim3 grd = full_grid(g, g.nz + 2), blk(LS_BX, LS_BY);
+  const dim3 grd = owned_grid(g, g.nz + 2), blk(LS_BX, LS_BY);
   if (in64) {
     const FFSrc<true> src{in64, nullptr, nullptr};
     if (out64)
@@ -526,32 +561,52 @@ __device__ __forceinline__ F3 csf_colval(const Geo &g, const Phys &ph, double mk
   return csf_point<T>(g, ph, mk, fi, i, j, k);
 }
 
+__device__ __forceinline__ F3 lane_of(const F3 &a, int l) {
+  F3 r = {__shfl_sync(0xffffffffu, a.x, l), __shfl_sync(0xffffffffu, a.y, l), __shfl_sync(0xffffffffu, a.z, l)};
+  return r;
+}
+
 // T: arithmetic of the curvature (double, or float in the FP32-mixed form);
 // TO: storage of the force components.
 template <typename T, typename TO>
 __global__ void k_csf(Geo g, Phys ph, double mk, const double *__restrict__ fi,
                       TO *__restrict__ fx, TO *__restrict__ fy, TO *__restrict__ fz) {
-  const int i = blockIdx.x * LS_BX + threadIdx.x, j = blockIdx.y * LS_BY + threadIdx.y;
+  const int i = blockIdx.x * LS_BX + threadIdx.x + 1, j = blockIdx.y * LS_BY + threadIdx.y + 1;
   const int k = blockIdx.z;
-  if (i > g.nx + 1 || j > g.ny + 1) return;
-  const int jj = wrapy(j, g.ny);
-  F3 v;
-  if (i == 0)
-    v = lin2(csf_colval<T>(g, ph, mk, fi, 1, jj, k), csf_colval<T>(g, ph, mk, fi, 2, jj, k));
-  else if (i == g.nx + 1)
-    v = lin2(csf_colval<T>(g, ph, mk, fi, g.nx, jj, k), csf_colval<T>(g, ph, mk, fi, g.nx - 1, jj, k));
-  else
-    v = csf_colval<T>(g, ph, mk, fi, i, jj, k);
+  if (j > g.ny) return;  // uniform per warp (one row)
+  F3 v = {0.0, 0.0, 0.0};
+  if (i <= g.nx) v = csf_colval<T>(g, ph, mk, fi, i, j, k);
+  // the inlet and outlet columns extrapolate from the last two columns: the
+  // inner one from the next lane, or by itself where that is in another warp
+  F3 in = {0.0, 0.0, 0.0};
+  if (blockIdx.x == 0) in = lane_of(v, 1);
+  if (blockIdx.x == gridDim.x - 1) {
+    const int last = (g.nx - 1) & 31;
+    if (last > 0) {
+      const F3 p = lane_of(v, last - 1);
+      if (i == g.nx) in = p;
+    } else if (i == g.nx) {
+      in = csf_colval<T>(g, ph, mk, fi, i - 1, j, k);
+    }
+  }
+  if (i > g.nx) return;
   const int c = TPLS_IDX(g, i, j, k);
-  fx[c] = (TO)v.x;
-  fy[c] = (TO)v.y;
-  fz[c] = (TO)v.z;
+  auto write = [&](int q, const F3 &x) {
+    fx[q] = (TO)x.x;
+    fy[q] = (TO)x.y;
+    fz[q] = (TO)x.z;
+  };
+  rows_of(g, j, c, [&](int q) { write(q, v); });
+  if (i == 1 || i == g.nx) {
+    const F3 e = lin2(v, in);
+    rows_of(g, j, c, [&](int q) { write(i == 1 ? q - 1 : q + 1, e); });
+  }
 }
 
 cudaError_t launch_csf(const Geo &g, const Phys &ph, const double *phi3,
                        double *fx, double *fy, double *fz, cudaStream_t st) {
   const double mk = 1.0 / fmin(fmin(ph.dx, ph.dy), ph.dz);
-  k_csf<double, double><<<full_grid(g, g.nz + 2), dim3(LS_BX, LS_BY), 0, st>>>(g, ph, mk, phi3, fx, fy, fz);
+  k_csf<double, double><<<owned_grid(g, g.nz + 2), dim3(LS_BX, LS_BY), 0, st>>>(g, ph, mk, phi3, fx, fy, fz);
   return cudaGetLastError();
 }
 cudaError_t launch_csf(const Geo &g, const Phys &ph, const double *phi3, float *fx, float *fy, float *fz,
@@ -560,7 +615,7 @@ cudaError_t launch_csf(const Geo &g, const Phys &ph, const double *phi3, float *
   // curvature stays FP64: its second differences of phi (~dx^2 |phi''|)
   // would lose ~1e-3 of their value to FP32 cancellation, a coherent error
   // in the surface-tension force at the interface; the force is stored FP32
-  k_csf<double, float><<<full_grid(g, g.nz + 2), dim3(LS_BX, LS_BY), 0, st>>>(g, ph, mk, phi3, fx, fy, fz);
+  k_csf<double, float><<<owned_grid(g, g.nz + 2), dim3(LS_BX, LS_BY), 0, st>>>(g, ph, mk, phi3, fx, fy, fz);
   return cudaGetLastError();
 }
 
