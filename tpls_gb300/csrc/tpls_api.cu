@@ -1156,13 +1156,13 @@ static int dim_stage(tpls_ctx *c, const double *conv2_phi) {
   cudaStream_t st = c->st;
   const DimK q = dim_constants(c->ph, c->prm.epn, c->prm.pe);
   LCK(c, launch_dim_prep(g, q, c->phi2, 0.5, c->dimE, c->D, st));
-  LCK(c, launch_dim_source(g, q, c->phi2, 0.5, c->dimE, c->D, conv2_phi, c->convprev, c->dimS, st));
+  LCK(c, launch_dim_source(g, q, c->phi2, 0.5, c->phi2, 0.5, c->dimE, c->D, conv2_phi, c->convprev, c->dimS, st));
   const double *pin = c->phi3d;
   double *pp[2] = {c->phiA, c->phiB};
   for (int it = 1; it <= c->prm.max_iteration_dim; it++) {
     double *out = pp[(it - 1) % 2];
     LCK(c, launch_dim_lap(g, q, pin, c->D, st));
-    LCK(c, launch_dim_update(g, q, c->phi2, 0.5, c->phi2, 0.5, c->dimS, pin, c->D, out, st));
+    LCK(c, launch_dim_update(g, q, c->dimS, pin, c->D, out, st));
     pin = out;
   }
   LCK(c, launch_dim_finish(g, pin, c->phi2, c->phi3d, st));
@@ -2275,13 +2275,13 @@ int tpls_dim(tpls_ctx *c, const int *maxl, const int *maxn, const double *dx, co
   TCK(h2d(c, CP, conv_prev_phi, nz + 2));
   TCK(h2d(c, N0, phi_new, nz + 2));
   LCK(c, launch_dim_prep(c->g, q, P, 0.0, N1, L, c->st));
-  LCK(c, launch_dim_source(c->g, q, P, 0.0, N1, L, C2, CP, S, c->st));
+  LCK(c, launch_dim_source(c->g, q, P, 0.0, O, 0.0, N1, L, C2, CP, S, c->st));
   const double *pin = N0;
   double *pp[2] = {N1, N0};
   for (int it = 1; it <= *max_iteration_dim; it++) {
     double *out = pp[(it - 1) % 2];
     LCK(c, launch_dim_lap(c->g, q, pin, L, c->st));
-    LCK(c, launch_dim_update(c->g, q, P, 0.0, O, 0.0, S, pin, L, out, c->st));
+    LCK(c, launch_dim_update(c->g, q, S, pin, L, out, c->st));
     pin = out;
   }
   TCK(d2h(c, phi_new, pin, nz + 2));

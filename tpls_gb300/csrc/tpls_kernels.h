@@ -54,18 +54,20 @@ struct DimK {
   double rdx2, rdy2, rdz2;  // 1/dx/dx, 1/dy/dy, 1/dz/dz
   double epn2, repn, rpe;   // epn^2, 1/epn, 1/Pe
   double c_nt2, c_en2;      // nmda*tao/2, epn^2*nmda/2
-  double dt, kc, tao, alfa1, rdiag;  // kc = dt*nmda/2/Pe, rdiag = 1/diagonal
+  double dt, ar;            // ar = alfa1/diagonal, the relaxation's weight
+  // the update: c_p phi + base + c_l d2phi + second differences of d2phi
+  double c_p, c_l, c_bx, c_by, c_bz;
   double dz, height, zden;  // inlet profile: 0.5+0.5 tanh((z-height)/zden)
 };
 DimK dim_constants(const Phys &ph, double epn, double pe);
 cudaError_t launch_dim_prep(const Geo &g, const DimK &q, const double *phi, double add, double *e0, double *l0,
                             cudaStream_t st);
-cudaError_t launch_dim_source(const Geo &g, const DimK &q, const double *phi, double add, const double *e0,
-                              const double *l0, const double *conv2, double *cprev, double *src, cudaStream_t st);
+cudaError_t launch_dim_source(const Geo &g, const DimK &q, const double *phi, double add, const double *phio,
+                              double addo, const double *e0, const double *l0, const double *conv2, double *cprev,
+                              double *base, cudaStream_t st);
 cudaError_t launch_dim_lap(const Geo &g, const DimK &q, const double *pin, double *l, cudaStream_t st);
-cudaError_t launch_dim_update(const Geo &g, const DimK &q, const double *phi, double add, const double *phio,
-                              double addo, const double *src, const double *pin, const double *l, double *pout,
-                              cudaStream_t st);
+cudaError_t launch_dim_update(const Geo &g, const DimK &q, const double *base, const double *pin, const double *l,
+                              double *pout, cudaStream_t st);
 cudaError_t launch_dim_finish(const Geo &g, const double *pfin, double *phi2, double *phi3, cudaStream_t st);
 
 // two_phase_levelset.f90 / levelset.f90
