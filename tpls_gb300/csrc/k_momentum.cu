@@ -235,7 +235,7 @@ enum { MOM_RHS, MOM_CONV, MOM_DIFF };
 
 template <int CC, int WHAT>
 __device__ __forceinline__ void mom_column(const Geo &g, const MomArgs &A, int i, int j, int ka, int kb) {
-  const int sy = g.sy, sz = g.sz, my = g.sy, mz = g.szm, nz = g.nz;
+  const int sy = g.sy, sz = g.sz, my = g.sym, mz = g.szm, nz = g.nz;
   const MomK &q = A.q[CC];
   const double *__restrict__ U = A.U, *__restrict__ V = A.V, *__restrict__ W = A.W;
   const double *__restrict__ S = (CC == 0) ? U : (CC == 1 ? V : W);

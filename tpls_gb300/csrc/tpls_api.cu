@@ -6,6 +6,7 @@
 #include <string.h>
 
 #include <array>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <vector>
@@ -330,12 +331,7 @@ static cudaError_t d2h(tpls_ctx *c, double *host, const double *dev0, int nzp) {
   if (e != cudaSuccess) return e;
   return cudaMemcpyAsync(host, c->stage, sizeof(double) * n, cudaMemcpyDeviceToHost, c->st);
 }
-// viscosity_aug (-1:nx+2,-1:ny+2,0:nz+1) <-> device mu (x 0..nx+1, y -1..ny+2)
-static cudaError_t h2d_mu(tpls_ctx *c, double *mu0, const double *host) {
-  const size_t w = sizeof(double) * (size_t)(c->nx + 2), n = (size_t)(c->nx + 4) * (c->ny + 4) * (c->nz + 2);
-  return cudaMemcpy2DAsync(mu0 - c->px, sizeof(double) * c->px, hmap(c, host, n) + 1, sizeof(double) * (c->nx + 4),
-                           w, (size_t)(c->ny + 4) * (c->nz + 2), cudaMemcpyDefault, c->st);
-}
+// device mu (x 0..nx+1, y -1..ny+2) -> viscosity_aug (-1:nx+2,-1:ny+2,0:nz+1)
 static cudaError_t d2h_mu(tpls_ctx *c, double *host, const double *mu0) {
   const size_t w = sizeof(double) * (size_t)(c->nx + 2), n = (size_t)(c->nx + 4) * (c->ny + 4) * (c->nz + 2);
   return cudaMemcpy2DAsync(hmap(c, host, n) + 1, sizeof(double) * (c->nx + 4), mu0 - c->px, sizeof(double) * c->px,
@@ -469,6 +465,7 @@ static int create_impl(int nx, int ny, int nz, const tpls_params *prm, const dou
   c->g.nz = nz;
   c->g.sy = c->px;
   c->g.sz = c->px * (ny + 2);
+  c->g.sym = c->px;
   c->g.szm = c->px * (ny + 4);
   TCK(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking));
   TCK(cudaEventCreateWithFlags(&c->front_ev, cudaEventDisableTiming));
@@ -661,6 +658,7 @@ long long tpls_footprint_bytes(int nx, int ny, int nz, int precision) {
   g.nz = nz;
   g.sy = (int)px;
   g.sz = (int)(px * (ny + 2));
+  g.sym = (int)px;
   g.szm = (int)(px * (ny + 4));
   size_t part = (size_t)ls_iter_blocks(g);
   const size_t d2 = (size_t)diff2_blocks(g, nz + 1);
@@ -2146,6 +2144,82 @@ static Phys phys_with(const tpls_ctx *c, const double *dx, const double *dy, con
   return ph;
 }
 
+// The per-routine entries that only run stencil kernels take their arrays in
+// the host layout (no row padding): a registered array's device mirror as it
+// is, any other by one copy into a scratch array.  Repacking every array to and
+// from the context's padded layout (and copying back whole velocities of which
+// the periodic rows alone had changed) cost 2.0 of 7.2 ms in the momentum calls
+// on registered arrays at 192x96x144, 0.33 of 1.64 ms in the interface calls on
+// plain ones at 128x64x96; the kernels, bound by the FP64 pipe, run at the same
+// speed on unpadded rows.
+static Geo host_geo(const tpls_ctx *c) {
+  Geo g = c->g;
+  g.sy = c->nx + 2;
+  g.sz = g.sy * (c->ny + 2);
+  g.sym = c->nx + 4;
+  g.szm = g.sym * (c->ny + 4);
+  return g;
+}
+static size_t host_len(const tpls_ctx *c, int nzp) { return (size_t)(c->nx + 2) * (c->ny + 2) * nzp; }
+static size_t host_len_mu(const tpls_ctx *c) { return (size_t)(c->nx + 4) * (c->ny + 4) * (c->nz + 2); }
+
+// An argument's host range; `out`: the routine writes it.
+struct HostArg {
+  const double *p;
+  size_t n;
+  bool out;
+};
+// Whether the kernels may work on the mirrors themselves: no written range
+// overlaps another argument (else every argument is copied, as the routine's
+// own copies in and out would have it).
+static bool args_disjoint(std::initializer_list<HostArg> v) {
+  for (const HostArg *x = v.begin(); x != v.end(); x++)
+    for (const HostArg *y = v.begin(); y != x; y++)
+      if ((x->out || y->out) && x->p < y->p + y->n && y->p < x->p + x->n) return false;
+  return true;
+}
+// The device copy of an argument that is read: *dev its mirror, or scr filled.
+static cudaError_t arg_in(tpls_ctx *c, bool direct, const double *host, size_t n, double *scr, double **dev) {
+  const double *m = hmap(c, host, n);
+  if (direct && m != host) {
+    *dev = const_cast<double *>(m);
+    return cudaSuccess;
+  }
+  *dev = scr;
+  return cudaMemcpyAsync(scr, m, sizeof(double) * n, m != host ? cudaMemcpyDefault : cudaMemcpyHostToDevice, c->st);
+}
+// Where an argument that is only written is computed.
+static double *arg_out(tpls_ctx *c, bool direct, double *host, size_t n, double *scr) {
+  double *m = hmap(c, host, n);
+  return (direct && m != host) ? m : scr;
+}
+static cudaError_t arg_done(tpls_ctx *c, double *host, size_t n, const double *dev) {
+  double *m = hmap(c, host, n);
+  if (m == dev) return cudaSuccess;
+  return cudaMemcpyAsync(m, dev, sizeof(double) * n, m != host ? cudaMemcpyDefault : cudaMemcpyDeviceToHost, c->st);
+}
+// The same for an array of which only the periodic rows changed.  In memory
+// row ny+1 of a plane and row 0 of the next are neighbours.
+static cudaError_t rows_done(tpls_ctx *c, double *host, int nzp, const double *dev) {
+  double *m = hmap(c, host, host_len(c, nzp));
+  if (m == dev) return cudaSuccess;
+  const cudaMemcpyKind kind = (m != host) ? cudaMemcpyDefault : cudaMemcpyDeviceToHost;
+  const size_t row = (size_t)c->nx + 2, plane = row * (c->ny + 2), D = sizeof(double);
+  const size_t last = plane * nzp - row, first = plane - row;
+  cudaError_t e = cudaMemcpyAsync(m, dev, D * row, kind, c->st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(m + last, dev + last, D * row, kind, c->st);
+  if (e == cudaSuccess && nzp > 1)
+    e = cudaMemcpy2DAsync(m + first, D * plane, dev + first, D * plane, D * 2 * row, nzp - 1, kind, c->st);
+  return e;
+}
+// viscosity_aug in the host layout, as the kernels index it (x, y from -1)
+static cudaError_t mu_in(tpls_ctx *c, bool direct, const double *va, const double **mu) {
+  double *dev = nullptr;
+  const cudaError_t e = arg_in(c, direct, va, host_len_mu(c), c->scr_mu - c->px, &dev);
+  *mu = dev + 1 + (c->nx + 4);
+  return e;
+}
+
 int tpls_exchange2d(tpls_ctx *c, double *uu, const int *ex, const int *ey, const int *ez, const int *sx,
                     const int *sy, const int *sz) {
   CHECKB(c, sx, ex, sy, ey);
@@ -2153,9 +2227,10 @@ int tpls_exchange2d(tpls_ctx *c, double *uu, const int *ex, const int *ey, const
   int s;
   if ((s = scratch(c))) return s;
   const int nzp = *ez + 1;
-  TCK(h2d(c, c->scr[0], uu, nzp));
-  LCK(c, launch_exchange(c->g, c->scr[0], nzp, c->st));
-  TCK(d2h(c, uu, c->scr[0], nzp));
+  double *U;
+  TCK(arg_in(c, true, uu, host_len(c, nzp), c->scr[0], &U));
+  LCK(c, launch_exchange(host_geo(c), U, nzp, c->st));
+  TCK(rows_done(c, uu, nzp, U));
   TCK(cudaStreamSynchronize(c->st));
   return TPLS_OK;
 }
@@ -2184,20 +2259,25 @@ int tpls_do_advect_phi(tpls_ctx *c, const double *phi2, double *u2, double *v2, 
   int s;
   if ((s = scratch(c))) return s;
   const Phys ph = phys_with(c, dx, dy, dz, nullptr);
-  double *P = c->scr[0], *U = c->scr[1], *V = c->scr[2], *W = c->scr[3], *C = c->scr[4];
-  TCK(h2d(c, P, phi2, nz + 2));
-  TCK(h2d(c, U, u2, nz));
-  TCK(h2d(c, V, v2, nz));
-  TCK(h2d(c, W, w2, nz + 1));
-  TCK(cudaMemsetAsync(C - XOFF, 0, sizeof(double) * ((size_t)c->px * (c->ny + 2) * (nz + 2)), c->st));
-  LCK(c, launch_advect(c->g, ph, P, U, V, W, C, c->st));
-  LCK(c, launch_exchange(c->g, U, nz, c->st));
-  LCK(c, launch_exchange(c->g, V, nz, c->st));
-  LCK(c, launch_exchange(c->g, W, nz + 1, c->st));
-  TCK(d2h(c, conv2_phi, C, nz + 2));
-  TCK(d2h(c, u2, U, nz));
-  TCK(d2h(c, v2, V, nz));
-  TCK(d2h(c, w2, W, nz + 1));
+  const Geo g = host_geo(c);
+  const size_t np = host_len(c, nz + 2), nu = host_len(c, nz), nw = host_len(c, nz + 1);
+  const bool dir = args_disjoint({{phi2, np, false}, {u2, nu, true}, {v2, nu, true}, {w2, nw, true},
+                                  {conv2_phi, np, true}});
+  double *P, *vel[3], *C = arg_out(c, dir, conv2_phi, np, c->scr[4]);
+  const int nzp[3] = {nz, nz, nz + 1};
+  TCK(arg_in(c, dir, phi2, np, c->scr[0], &P));
+  TCK(arg_in(c, dir, u2, nu, c->scr[1], &vel[0]));
+  TCK(arg_in(c, dir, v2, nu, c->scr[2], &vel[1]));
+  TCK(arg_in(c, dir, w2, nw, c->scr[3], &vel[2]));
+  TCK(cudaMemsetAsync(C, 0, sizeof(double) * np, c->st));
+  LCK(c, launch_advect(g, ph, P, vel[0], vel[1], vel[2], C, c->st));
+  LCK(c, launch_exchange_set<double>(g, 3, vel, nzp, c->st));
+  TCK(arg_done(c, conv2_phi, np, C));
+  double *const host[3] = {u2, v2, w2};
+  for (int q = 0; q < 3; q++) {
+    if (dir) TCK(rows_done(c, host[q], nzp[q], vel[q]));
+    else TCK(arg_done(c, host[q], host_len(c, nzp[q]), vel[q]));
+  }
   TCK(cudaStreamSynchronize(c->st));
   return TPLS_OK;
 }
@@ -2219,14 +2299,18 @@ int tpls_do_tpls(tpls_ctx *c, double *phi2, double *phi3, double *conv0_phi, dou
   if ((s = scratch(c))) return s;
   Phys ph = phys_with(c, dx, nullptr, dz, dt);
   ph.height = *height;
-  double *P2 = c->scr[0], *C0 = c->scr[1], *C1 = c->scr[2], *C2 = c->scr[3], *A = c->scr[4], *B = c->scr[5],
-         *OUT = c->scr[6], *Dd = c->scr[7];
-  TCK(h2d(c, P2, phi2, nz + 2));
-  TCK(h2d(c, C0, conv0_phi, nz + 2));
-  TCK(h2d(c, C1, conv1_phi, nz + 2));
-  TCK(h2d(c, C2, conv2_phi, nz + 2));
-  LCK(c, launch_ls_ab3(c->g, ph, P2, C0, C1, C2, A, c->st));
-  LCK(c, launch_ls_status(c->g, ph, A, Dd, c->scr_flags, c->st));
+  const Geo g = host_geo(c);
+  const size_t np = host_len(c, nz + 2);
+  const bool dir = args_disjoint({{phi2, np, false}, {conv0_phi, np, false}, {conv1_phi, np, false},
+                                  {conv2_phi, np, false}, {phi3, np, true}});
+  double *P2, *C0, *C1, *C2, *A = c->scr[4], *B = c->scr[5], *Dd = c->scr[7];
+  double *OUT = arg_out(c, dir, phi3, np, c->scr[6]);
+  TCK(arg_in(c, dir, phi2, np, c->scr[0], &P2));
+  TCK(arg_in(c, dir, conv0_phi, np, c->scr[1], &C0));
+  TCK(arg_in(c, dir, conv1_phi, np, c->scr[2], &C1));
+  TCK(arg_in(c, dir, conv2_phi, np, c->scr[3], &C2));
+  LCK(c, launch_ls_ab3(g, ph, P2, C0, C1, C2, A, c->st));
+  LCK(c, launch_ls_status(g, ph, A, Dd, c->scr_flags, c->st));
   const int L = *max_iteration_levelset;
   const double *src = A;
   if (L <= 0) {
@@ -2235,11 +2319,11 @@ int tpls_do_tpls(tpls_ctx *c, double *phi2, double *phi3, double *conv0_phi, dou
   for (int it = 1; it <= L; it++) {
     double *dst = (it == L) ? OUT : ((it % 2 == 1) ? B : A);
     if (it == 1 && L > 1) dst = B;
-    LCK(c, launch_ls_iter(c->g, ph, src, Dd, c->scr_flags, dst, (it == L) ? c->part : nullptr, c->st));
+    LCK(c, launch_ls_iter(g, ph, src, Dd, c->scr_flags, dst, (it == L) ? c->part : nullptr, c->st));
     src = dst;
   }
-  if (L > 0) FSUM(c, c->part, ls_iter_blocks(c->g), c->scal + SC_ERR_PHI, c->st);
-  TCK(d2h(c, phi3, src, nz + 2));
+  if (L > 0) FSUM(c, c->part, ls_iter_blocks(g), c->scal + SC_ERR_PHI, c->st);
+  TCK(arg_done(c, phi3, np, src));
   TCK(cudaMemcpyAsync(c->scal_host, c->scal, sizeof(double) * SC_N, cudaMemcpyDeviceToHost, c->st));
   TCK(cudaStreamSynchronize(c->st));
   *err2 = c->scal_host[SC_ERR_PHI];
@@ -2267,25 +2351,28 @@ int tpls_dim(tpls_ctx *c, const int *maxl, const int *maxn, const double *dx, co
   const DimK q = dim_constants(ph, *epn, *pe);
   // scr[5] holds bulkE0 until the source term is formed, then the iterate's
   // second buffer
-  double *P = c->scr[0], *O = c->scr[1], *C2 = c->scr[2], *CP = c->scr[3], *N0 = c->scr[4], *N1 = c->scr[5],
-         *L = c->scr[6], *S = c->scr[7];
-  TCK(h2d(c, P, phi, nz + 2));
-  TCK(h2d(c, O, phi_old, nz + 2));
-  TCK(h2d(c, C2, conv2_phi, nz + 2));
-  TCK(h2d(c, CP, conv_prev_phi, nz + 2));
-  TCK(h2d(c, N0, phi_new, nz + 2));
-  LCK(c, launch_dim_prep(c->g, q, P, 0.0, N1, L, c->st));
-  LCK(c, launch_dim_source(c->g, q, P, 0.0, O, 0.0, N1, L, C2, CP, S, c->st));
+  const Geo g = host_geo(c);
+  const size_t np = host_len(c, nz + 2);
+  const bool dir = args_disjoint({{phi, np, false}, {phi_old, np, false}, {conv2_phi, np, false},
+                                  {conv_prev_phi, np, true}, {phi_new, np, true}});
+  double *P, *O, *C2, *CP, *N0, *N1 = c->scr[5], *L = c->scr[6], *S = c->scr[7];
+  TCK(arg_in(c, dir, phi, np, c->scr[0], &P));
+  TCK(arg_in(c, dir, phi_old, np, c->scr[1], &O));
+  TCK(arg_in(c, dir, conv2_phi, np, c->scr[2], &C2));
+  TCK(arg_in(c, dir, conv_prev_phi, np, c->scr[3], &CP));
+  TCK(arg_in(c, dir, phi_new, np, c->scr[4], &N0));
+  LCK(c, launch_dim_prep(g, q, P, 0.0, N1, L, c->st));
+  LCK(c, launch_dim_source(g, q, P, 0.0, O, 0.0, N1, L, C2, CP, S, c->st));
   const double *pin = N0;
   double *pp[2] = {N1, N0};
   for (int it = 1; it <= *max_iteration_dim; it++) {
     double *out = pp[(it - 1) % 2];
-    LCK(c, launch_dim_lap(c->g, q, pin, L, c->st));
-    LCK(c, launch_dim_update(c->g, q, S, pin, L, out, c->st));
+    LCK(c, launch_dim_lap(g, q, pin, L, c->st));
+    LCK(c, launch_dim_update(g, q, S, pin, L, out, c->st));
     pin = out;
   }
-  TCK(d2h(c, phi_new, pin, nz + 2));
-  TCK(d2h(c, conv_prev_phi, CP, nz + 2));
+  TCK(arg_done(c, phi_new, np, pin));
+  TCK(arg_done(c, conv_prev_phi, np, CP));
   TCK(cudaStreamSynchronize(c->st));
   return TPLS_OK;
 }
@@ -2302,12 +2389,15 @@ int tpls_get_csf(tpls_ctx *c, double *fx_csf, double *fy_csf, double *fz_csf, co
   Phys ph = phys_with(c, dx, dy, dz, nullptr);
   ph.scap = *scap;
   ph.sw = *smooth_width;
-  const int nz = c->nz;
-  TCK(h2d(c, c->scr[0], fi, nz + 2));
-  LCK(c, launch_csf(c->g, ph, c->scr[0], c->scr[1], c->scr[2], c->scr[3], c->st));
-  TCK(d2h(c, fx_csf, c->scr[1], nz + 2));
-  TCK(d2h(c, fy_csf, c->scr[2], nz + 2));
-  TCK(d2h(c, fz_csf, c->scr[3], nz + 2));
+  const size_t np = host_len(c, c->nz + 2);
+  const bool dir = args_disjoint({{fi, np, false}, {fx_csf, np, true}, {fy_csf, np, true}, {fz_csf, np, true}});
+  double *F, *X = arg_out(c, dir, fx_csf, np, c->scr[1]), *Y = arg_out(c, dir, fy_csf, np, c->scr[2]),
+             *Z = arg_out(c, dir, fz_csf, np, c->scr[3]);
+  TCK(arg_in(c, dir, fi, np, c->scr[0], &F));
+  LCK(c, launch_csf(host_geo(c), ph, F, X, Y, Z, c->st));
+  TCK(arg_done(c, fx_csf, np, X));
+  TCK(arg_done(c, fy_csf, np, Y));
+  TCK(arg_done(c, fz_csf, np, Z));
   TCK(cudaStreamSynchronize(c->st));
   return TPLS_OK;
 }
@@ -2325,9 +2415,19 @@ int tpls_get_viscosity(tpls_ctx *c, double *viscosity_aug, const double *phi, co
   ph.re = *re;
   ph.mu_minus = *mu_minus;
   ph.mu_plus = *mu_plus;
-  TCK(h2d(c, c->scr[0], phi, c->nz + 2));
-  LCK(c, launch_visc(c->g, ph, c->scr[0], c->scr_mu, c->st));
-  TCK(d2h_mu(c, viscosity_aug, c->scr_mu));
+  const size_t np = host_len(c, c->nz + 2), nm = host_len_mu(c);
+  const bool dir = args_disjoint({{phi, np, false}, {viscosity_aug, nm, true}});
+  double *F, *M = hmap(c, viscosity_aug, nm);
+  TCK(arg_in(c, dir, phi, np, c->scr[0], &F));
+  Geo g = host_geo(c);  // the columns x = -1 and nx+2 keep their values
+  if (dir && M != viscosity_aug) {
+    LCK(c, launch_visc(g, ph, F, M + 1 + (c->nx + 4), c->st));
+  } else {
+    g.sym = c->g.sym;
+    g.szm = c->g.szm;
+    LCK(c, launch_visc(g, ph, F, c->scr_mu, c->st));
+    TCK(d2h_mu(c, viscosity_aug, c->scr_mu));
+  }
   TCK(cudaStreamSynchronize(c->st));
   return TPLS_OK;
 }
@@ -2340,20 +2440,21 @@ static int conv_diff_entry(tpls_ctx *c, int want_conv, double *o_u, double *o_v,
   if ((s = scratch(c))) return s;
   const Phys ph = phys_with(c, dx, dy, dz, nullptr);
   const int nz = c->nz;
-  double *U = c->scr[0], *V = c->scr[1], *W = c->scr[2], *OU = c->scr[3], *OV = c->scr[4], *OW = c->scr[5];
-  TCK(h2d(c, U, u2, nz));
-  TCK(h2d(c, V, v2, nz));
-  TCK(h2d(c, W, w2, nz + 1));
-  TCK(h2d_mu(c, c->scr_mu, va));
-  const size_t bytes = sizeof(double) * ((size_t)c->px * (c->ny + 2) * (nz + 2));
-  TCK(cudaMemsetAsync(OU - XOFF, 0, bytes, c->st));
-  TCK(cudaMemsetAsync(OV - XOFF, 0, bytes, c->st));
-  TCK(cudaMemsetAsync(OW - XOFF, 0, bytes, c->st));
-  double *const out[3] = {OU, OV, OW};
-  LCK(c, launch_conv_diff(want_conv, c->g, ph, U, V, W, c->scr_mu, out, c->st));
-  TCK(d2h(c, o_u, OU, nz));
-  TCK(d2h(c, o_v, OV, nz));
-  TCK(d2h(c, o_w, OW, nz + 1));
+  const size_t nu = host_len(c, nz), nw = host_len(c, nz + 1), n3[3] = {nu, nu, nw};
+  const bool dir = args_disjoint({{va, host_len_mu(c), false}, {u2, nu, false}, {v2, nu, false}, {w2, nw, false},
+                                  {o_u, nu, true}, {o_v, nu, true}, {o_w, nw, true}});
+  double *U, *V, *W, *const o[3] = {o_u, o_v, o_w}, *out[3];
+  const double *mu;
+  TCK(arg_in(c, dir, u2, nu, c->scr[0], &U));
+  TCK(arg_in(c, dir, v2, nu, c->scr[1], &V));
+  TCK(arg_in(c, dir, w2, nw, c->scr[2], &W));
+  TCK(mu_in(c, dir, va, &mu));
+  for (int q = 0; q < 3; q++) {
+    out[q] = arg_out(c, dir, o[q], n3[q], c->scr[3 + q]);
+    TCK(cudaMemsetAsync(out[q], 0, sizeof(double) * n3[q], c->st));
+  }
+  LCK(c, launch_conv_diff(want_conv, host_geo(c), ph, U, V, W, mu, out, c->st));
+  for (int q = 0; q < 3; q++) TCK(arg_done(c, o[q], n3[q], out[q]));
   TCK(cudaStreamSynchronize(c->st));
   return TPLS_OK;
 }
@@ -2386,13 +2487,16 @@ static int jacobi_entry(tpls_ctx *c, int comp, double *x3, const double *x3_old,
   if ((s = scratch(c))) return s;
   const Phys ph = phys_with(c, dx, dy, dz, dt);
   const int nzp = nz_planes(comp == 2 ? 2 : 1, c->nz);
-  double *X = c->scr[0], *XO = c->scr[1], *R = c->scr[2];
-  TCK(h2d(c, X, x3, nzp));
-  TCK(h2d(c, XO, x3_old, nzp));
-  TCK(h2d(c, R, rhs, nzp));
-  TCK(h2d_mu(c, c->scr_mu, va));
-  LCK(c, launch_ref_jacobi(comp, c->g, ref_coef(comp, ph, R, c->scr_mu), XO, X, c->st));
-  TCK(d2h(c, x3, X, nzp));
+  const size_t n = host_len(c, nzp);
+  const bool dir = args_disjoint({{x3, n, true}, {x3_old, n, false}, {rhs, n, false}, {va, host_len_mu(c), false}});
+  double *X, *XO, *R;
+  const double *mu;
+  TCK(arg_in(c, dir, x3, n, c->scr[0], &X));
+  TCK(arg_in(c, dir, x3_old, n, c->scr[1], &XO));
+  TCK(arg_in(c, dir, rhs, n, c->scr[2], &R));
+  TCK(mu_in(c, dir, va, &mu));
+  LCK(c, launch_ref_jacobi(comp, host_geo(c), ref_coef(comp, ph, R, mu), XO, X, c->st));
+  TCK(arg_done(c, x3, n, X));
   TCK(cudaStreamSynchronize(c->st));
   return TPLS_OK;
 }
@@ -2419,14 +2523,18 @@ static int sor_entry(tpls_ctx *c, int comp, double *x3, const double *rhs, const
   if ((s = scratch(c))) return s;
   const Phys ph = phys_with(c, dx, dy, dz, dt);
   const int nzp = nz_planes(comp == 2 ? 2 : 1, c->nz);
-  double *X = c->scr[0], *R = c->scr[1];
-  TCK(h2d(c, X, x3, nzp));
-  TCK(h2d(c, R, rhs, nzp));
-  TCK(h2d_mu(c, c->scr_mu, va));
-  const RefCoef rc = ref_coef(comp, ph, R, c->scr_mu);
-  if (*iteration_time % 2 == 0) LCK(c, launch_ref_even(comp, c->g, rc, X, *flg, c->st));
-  else LCK(c, launch_ref_odd(comp, c->g, rc, X, *flg, c->st, odd_chain(c)));
-  TCK(d2h(c, x3, X, nzp));
+  const Geo g = host_geo(c);
+  const size_t n = host_len(c, nzp);
+  const bool dir = args_disjoint({{x3, n, true}, {rhs, n, false}, {va, host_len_mu(c), false}});
+  double *X, *R;
+  const double *mu;
+  TCK(arg_in(c, dir, x3, n, c->scr[0], &X));
+  TCK(arg_in(c, dir, rhs, n, c->scr[1], &R));
+  TCK(mu_in(c, dir, va, &mu));
+  const RefCoef rc = ref_coef(comp, ph, R, mu);
+  if (*iteration_time % 2 == 0) LCK(c, launch_ref_even(comp, g, rc, X, *flg, c->st));
+  else LCK(c, launch_ref_odd(comp, g, rc, X, *flg, c->st, odd_chain(c)));
+  TCK(arg_done(c, x3, n, X));
   TCK(cudaStreamSynchronize(c->st));
   return TPLS_OK;
 }
@@ -2462,9 +2570,10 @@ int tpls_get_difference(tpls_ctx *c, const double *ua, const double *ub, const i
   int s;
   if ((s = scratch(c))) return s;
   const int nzp = *ez + 1;
-  TCK(h2d(c, c->scr[0], ua, nzp));
-  TCK(h2d(c, c->scr[1], ub, nzp));
-  LCK(c, launch_diff2(c->g, c->scr[0], c->scr[1], nzp, c->part, c->st));
+  double *UA, *UB;
+  TCK(arg_in(c, true, ua, host_len(c, nzp), c->scr[0], &UA));
+  TCK(arg_in(c, true, ub, host_len(c, nzp), c->scr[1], &UB));
+  LCK(c, launch_diff2(host_geo(c), UA, UB, nzp, c->part, c->st));
   FSUM(c, c->part, diff2_blocks(c->g, nzp), c->scal + SC_ERR_U, c->st);
   TCK(cudaMemcpyAsync(c->scal_host, c->scal, sizeof(double) * SC_N, cudaMemcpyDeviceToHost, c->st));
   TCK(cudaStreamSynchronize(c->st));
@@ -2482,11 +2591,14 @@ int tpls_get_source_pres(tpls_ctx *c, double *rhs, const double *u3, const doubl
   if ((s = scratch(c))) return s;
   const Phys ph = phys_with(c, dx, dy, dz, dt);
   const int nz = c->nz;
-  TCK(h2d(c, c->scr[0], u3, nz));
-  TCK(h2d(c, c->scr[1], v3, nz));
-  TCK(h2d(c, c->scr[2], w3, nz + 1));
-  LCK(c, launch_source(c->g, ph, c->scr[0], c->scr[1], c->scr[2], c->scr[3], c->st));
-  TCK(d2h(c, rhs, c->scr[3], nz + 2));
+  const size_t np = host_len(c, nz + 2), nu = host_len(c, nz), nw = host_len(c, nz + 1);
+  const bool dir = args_disjoint({{rhs, np, true}, {u3, nu, false}, {v3, nu, false}, {w3, nw, false}});
+  double *U, *V, *W, *R = arg_out(c, dir, rhs, np, c->scr[3]);
+  TCK(arg_in(c, dir, u3, nu, c->scr[0], &U));
+  TCK(arg_in(c, dir, v3, nu, c->scr[1], &V));
+  TCK(arg_in(c, dir, w3, nw, c->scr[2], &W));
+  LCK(c, launch_source(host_geo(c), ph, (const double *)U, (const double *)V, (const double *)W, R, c->st));
+  TCK(arg_done(c, rhs, np, R));
   TCK(cudaStreamSynchronize(c->st));
   return TPLS_OK;
 }

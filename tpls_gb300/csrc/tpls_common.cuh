@@ -24,7 +24,8 @@ struct Geo {
   int nx, ny, nz;
   int sy;   // y stride (elements) = PX
   int sz;   // z stride of p/u/v/w fields = PX*(ny+2)
-  int szm;  // z stride of the viscosity field = PX*(ny+4)
+  int sym;  // y stride of the viscosity field: PX, or the host array's nx + 4
+  int szm;  // z stride of the viscosity field = sym*(ny+4)
 };
 
 // Single-precision literals of the reference, widened exactly as Fortran does.
@@ -61,4 +62,4 @@ __device__ __forceinline__ double block_sum(double e, int t, double *sh) {
 }  // namespace tpls
 
 #define TPLS_IDX(g, i, j, k) ((i) + (g).sy * (j) + (g).sz * (k))
-#define TPLS_IDXM(g, i, j, k) ((i) + (g).sy * (j) + (g).szm * (k))
+#define TPLS_IDXM(g, i, j, k) ((i) + (g).sym * (j) + (g).szm * (k))

@@ -26,7 +26,7 @@ using Fc = FcT<double>;
 template <typename T>
 __device__ __forceinline__ FcT<T> faces(int comp, const Geo &g, const T *__restrict__ mu, int i, int j,
                                         int k) {
-  const int sy = g.sy, sz = g.szm;
+  const int sy = g.sym, sz = g.szm;
   FcT<T> f;
   if (comp == 0) {
     const T *m = mu + TPLS_IDXM(g, i, j + 1, k + 1);
@@ -72,7 +72,7 @@ __device__ __forceinline__ FcT<T> faces(int comp, const Geo &g, const T *__restr
 // the x and y terms, to which the caller adds cz (hi zp + lo zm).
 template <int CC>
 __device__ __forceinline__ int ref_om(const Geo &g) {  // the far cell of a point's own face
-  return CC == 0 ? 1 : (CC == 1 ? -g.sy : g.szm);
+  return CC == 0 ? 1 : (CC == 1 ? -g.sym : g.szm);
 }
 template <int CC>
 __device__ __forceinline__ const double *ref_cell(const Geo &g, const RefCoef &s, int i, int j, int k) {
@@ -88,7 +88,7 @@ template <int CC>
 __device__ __forceinline__ double ref_point(const Geo &g, const RefCoef &s, const double *m, double near, double lo,
                                             double rhs, double xp, double xm, double yp, double ym, double &hi,
                                             double &near1, double &h) {
-  const int om = ref_om<CC>(g), my = g.sy, mz = g.szm;
+  const int om = ref_om<CC>(g), my = g.sym, mz = g.szm;
   auto pair = [&](int o) { return m[o] + m[o + om]; };
   const double fxp = (CC == 0) ? m[1] : near + pair(1), fxm = (CC == 0) ? m[0] : near + pair(-1);
   const double fyp = (CC == 1) ? m[0] : near + pair(my), fym = (CC == 1) ? m[om] : near + pair(-my);
