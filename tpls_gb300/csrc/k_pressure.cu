@@ -61,6 +61,7 @@ struct PoissonSolver {
   double *cinv = nullptr;  // coarsest pseudo-inverse (nc x nc), or null
   int coarse_sweeps = 0;
   double *modes = nullptr;  // coarsest level by modes: Qz, Qy, lambda_z, lambda_y
+  double *dense = nullptr;  // and the matrices of its lines (dense_values), rows of up to DENSE_NX points
   double *x = nullptr, *r = nullptr, *p = nullptr, *q = nullptr, *bvec = nullptr;
   void *z = nullptr;           // preconditioned residual, in the level type
   float *r32 = nullptr;        // FP32 levels: r rounded once, for the V-cycle
@@ -913,6 +914,10 @@ static cudaError_t lj2_attr() {
 
 static size_t mg_dot_blocks(const PLevel &L);
 
+static ModeSweeps mode_sweeps(const PoissonSolver *S, const PLevel &L) {
+  return {L.nx, L.ny, L.nz, S->coarse_sweeps, L.cx, L.cy, L.cz, S->omega};
+}
+
 cudaError_t poisson_create(const Geo &g, double cx, double cy, double cz, int fp32,
                            PoissonSolver **out) {
   PoissonSolver *S = new PoissonSolver();
@@ -1008,6 +1013,16 @@ cudaError_t poisson_create(const Geo &g, double cx, double cy, double cz, int fp
       Qz.insert(Qz.end(), ly.begin(), ly.end());
       PCK(cudaMalloc(&S->modes, Qz.size() * sizeof(double)));
       PCK(cudaMemcpy(S->modes, Qz.data(), Qz.size() * sizeof(double), cudaMemcpyHostToDevice));
+      if (C.nx <= DENSE_NX) {
+        const ModeSweeps M = mode_sweeps(S, C);
+        const double *lzd = S->modes + (size_t)C.nz * C.nz + (size_t)C.ny * C.ny;
+        PCK(cudaMalloc(&S->dense, sizeof(double) * dense_values(C.nx, C.ny, C.nz)));
+        const int half = (C.nx + 1) / 2, warps = half <= 16 ? half : 2 * half;  // both parities per warp, or one
+        k_dense_build<<<dim3((warps + MODE_W - 1) / MODE_W, C.nz, mode_classes(C.ny)), 32 * MODE_W>>>(
+            M, lzd + C.nz, lzd, S->dense);
+        PCK(cudaGetLastError());
+        PCK(cudaStreamSynchronize(cudaStreamLegacy));  // before any stream of the context reads them
+      }
     }
   }
   const size_t nb = sizeof(double) * (size_t)S->N;
@@ -1049,6 +1064,7 @@ void poisson_destroy(PoissonSolver *S) {
   }
   cudaFree(S->cinv);
   cudaFree(S->modes);
+  cudaFree(S->dense);
   cudaFree(S->x);
   cudaFree(S->r);
   cudaFree(S->z);
@@ -1081,7 +1097,10 @@ size_t poisson_footprint(const Geo &g, int fp32, size_t (*rnd)(size_t)) {
     }
     const int cx = (nx % 2 == 0 && nx >= 4), cy = (ny % 2 == 0 && ny >= 4), cz = (nz % 2 == 0 && nz >= 4);
     if (!cx && !cy && !cz) {
-      if (!fp32 && modes_pay(nx, ny, nz)) tot += rnd(sizeof(double) * ((size_t)nz * nz + (size_t)ny * ny + nz + ny));
+      if (!fp32 && modes_pay(nx, ny, nz)) {
+        tot += rnd(sizeof(double) * ((size_t)nz * nz + (size_t)ny * ny + nz + ny));
+        if (nx <= DENSE_NX) tot += rnd(sizeof(double) * dense_values(nx, ny, nz));
+      }
       break;
     }
     nx = cx ? nx / 2 : nx;
@@ -1142,7 +1161,7 @@ static void mode_lines(const ModeSweeps &M, const double *Qy, const double *ly, 
 }
 static cudaError_t coarse_modes(const PoissonSolver *S, const PLevel &L, const double *b, double *t, double *u,
                                 double *e, cudaStream_t st, long *nl) {
-  const ModeSweeps M = {L.nx, L.ny, L.nz, S->coarse_sweeps, L.cx, L.cy, L.cz, S->omega};
+  const ModeSweeps M = mode_sweeps(S, L);
   const double *Qz = S->modes, *Qy = Qz + (size_t)L.nz * L.nz, *lz = Qy + (size_t)L.ny * L.ny, *ly = lz + L.nz;
   const int ncol = L.nx * L.ny, gc = (ncol + 31) / 32;
   constexpr int T = 32 * MODE_W;
@@ -1150,10 +1169,10 @@ static cudaError_t coarse_modes(const PoissonSolver *S, const PLevel &L, const d
   const int m4 = 2 * ((L.nz + 7) / 8), m1 = 2 * ((L.nz + 1) / 2);  // groups of four modes of one parity, of one
   if (gc * m4 >= MODE_WARPS) k_modes_z<4><<<dim3(gc, blocks(m4)), T, 0, st>>>(L.nz, ncol, Qz, b, t);
   else k_modes_z<1><<<dim3(gc, blocks(m1)), T, 0, st>>>(L.nz, ncol, Qz, b, t);
-  const int ppl = (L.nx + 31) / 32;
-  if (ppl == 1) mode_lines<1>(M, Qy, ly, lz, t, u, st);
-  else if (ppl == 2) mode_lines<2>(M, Qy, ly, lz, t, u, st);
-  else if (ppl <= 4) mode_lines<4>(M, Qy, ly, lz, t, u, st);
+  const dim3 lines((L.ny + MODE_W - 1) / MODE_W, L.nz);
+  if (S->dense && L.nx <= 32) k_mode_dense<false><<<lines, T, 0, st>>>(L.nx, L.ny, L.nz, Qy, S->dense, t, u);
+  else if (S->dense) k_mode_dense<true><<<lines, T, 0, st>>>(L.nx, L.ny, L.nz, Qy, S->dense, t, u);
+  else if (L.nx <= 128) mode_lines<4>(M, Qy, ly, lz, t, u, st);
   else mode_lines<MODE_PPL>(M, Qy, ly, lz, t, u, st);
   const int gi = (L.nx + 31) / 32, r4 = (L.ny + 3) / 4;
   if (gi * r4 * L.nz >= MODE_WARPS) k_points_y<4><<<dim3(gi, blocks(r4), L.nz), T, 0, st>>>(L.nx, L.ny, Qy, u, t);
