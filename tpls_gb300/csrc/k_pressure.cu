@@ -51,6 +51,7 @@ struct PLevel {
   void *b = nullptr, *e = nullptr, *e2 = nullptr, *r = nullptr, *t = nullptr;
   void *thomas = nullptr;  // [3 classes][nz][2] = (cprime, inv_den)
   int halved = 0;  // red-black level whose three axes are coarsened below it: the k_mg_* kernels
+  int planar = 0;  // FP64 red-black level of which x and y are coarsened, z (odd) is not: the same passes by planes
   int point = 0;  // near-isotropic level: red-black Gauss-Seidel instead of z-lines
   double invd[3][3];  // point smoother: 1/diagonal by x class (first, interior, last) and z class
 };
@@ -971,12 +972,13 @@ cudaError_t poisson_create(const Geo &g, double cx, double cy, double cz, int fp
       if (l + 1 < S->lv.size()) {
         const PLevel &c = S->lv[l + 1];
         L.halved = L.point && c.cxs && c.cys && c.czs;
+        L.planar = L.point && c.cxs && c.cys && !c.czs && !S->fp32;
       }
     }
     const size_t bytes = esz * (size_t)L.n;
     if (l > 0) PCK(cudaMalloc(&L.b, bytes));
     if (l > 0) PCK(cudaMalloc(&L.e, bytes));
-    if (!L.halved) {
+    if (!L.halved && !L.planar) {
       PCK(cudaMalloc(&L.e2, bytes));
       PCK(cudaMalloc(&L.r, bytes));
       PCK(cudaMalloc(&L.t, bytes));
@@ -1034,10 +1036,16 @@ cudaError_t poisson_create(const Geo &g, double cx, double cy, double cz, int fp
   PCK(cudaMalloc(&S->q, nb));
   PCK(cudaMalloc(&S->bvec, nb));
   PCK(cudaMalloc(&S->bin, sizeof(double) * (size_t)g.ny * g.nz));
-  S->rblk = nblocks(S->N) < 1216 ? nblocks(S->N) : 1216;  // 8 blocks per SM on 152 SMs
+  // Blocks of the reductions: 8 per SM on 152 SMs, which hide the loads of a
+  // large grid (7 iterations at 256x128x192: 5110 us, 5210 with 4 per SM); FP64,
+  // below 2M points, 4, half the blocks' own sums (15 iterations at 100x50x75:
+  // 3665 us with 8, 3510 with 4; 6 at 128x64x96: 1490, 1450).  (The FP32 form
+  // keeps one order of its sums for every size.)
+  const int rb = (!S->fp32 && S->N < 2000000) ? 608 : 1216;
+  S->rblk = nblocks(S->N) < rb ? nblocks(S->N) : rb;
   {
     size_t np = (size_t)S->rblk * 3;  // reductions of up to three sums, or one partial per block of k_mg_half_dot
-    if (S->lv[0].halved) {
+    if (S->lv[0].halved || S->lv[0].planar) {
       const size_t nb = S->fp32 ? 0 : mg_dot_blocks(S->lv[0]);
       if (nb > np) np = nb;
     }
@@ -1296,7 +1304,7 @@ static int mg_tiles(const PLevel &L, int cx, int cy, int cz) {
 }
 // blocks of the launch that forms r.z on the finest level (FP64)
 static size_t mg_dot_blocks(const PLevel &L) {
-  return mg_split<double>(L) ? mg_blocks(L, mg_kz(L)) : mg_tiles(L, 8, 2, 2);
+  return (L.planar || mg_split<double>(L)) ? mg_blocks(L, mg_kz(L)) : mg_tiles(L, 8, 2, 2);
 }
 
 // pre-smoothing from a zero start into e2: z-line Jacobi, or red then black
@@ -1351,7 +1359,7 @@ static cudaError_t mg_down_level(const MgLev<R> &M, const PLevel &L, int ncz, co
     mg_restrict_grid(L, ncz, &czb, &nb);
     if constexpr (sizeof(R) == sizeof(double)) k_mg_black<<<mg_blocks(L, kz), 256, 0, st>>>(M, b, e, kz);
     else k_mg_pre<<<mg_blocks(L, kz), 256, 0, st>>>(M, b, e, kz);
-    k_mg_restrict<R><<<nb, 256, 0, st>>>(M, b, e, bc, czb);
+    k_mg_restrict<R, true><<<nb, 256, 0, st>>>(M, b, e, bc, czb);
     *nl += 2;
   } else {
     k_mg_down<R, 8, 2, 2><<<mg_tiles(L, 8, 2, 2), 256, 0, st>>>(M, b, bc);
@@ -1360,12 +1368,44 @@ static cudaError_t mg_down_level(const MgLev<R> &M, const PLevel &L, int ncz, co
   return cudaGetLastError();
 }
 
+// The five passes of a level whose z axis is not coarsened (FP64), in place of
+// ten launches of the general ones: 34 us instead of 70 at 100x50x75.
+static cudaError_t mg_down_planar(const PLevel &L, const double *b, double *e, double *bc, cudaStream_t st, long *nl) {
+  const MgLev<double> M = mglev<double>(L);
+  const int kz = mg_kz(L);
+  int czb, nb;
+  mg_restrict_grid(L, L.nz, &czb, &nb);
+  k_mg_black<<<mg_blocks(L, kz), 256, 0, st>>>(M, b, e, kz);
+  k_mg_restrict<double, false><<<nb, 256, 0, st>>>(M, b, e, bc, czb);
+  *nl += 2;
+  return cudaGetLastError();
+}
+static cudaError_t mg_up_planar(PoissonSolver *S, const PLevel &L, bool finest, const double *b, const double *ec,
+                                double *e, cudaStream_t st, long *nl) {
+  const MgLev<double> M = mglev<double>(L);
+  const int kz = mg_kz(L), nb = mg_blocks(L, kz);
+  k_mg_prolong<false><<<nb, 256, 0, st>>>(M, b, ec, e, kz);
+  k_mg_half<<<nb, 256, 0, st>>>(M, 1, b, e, kz);
+  if (finest) k_mg_half_dot<<<nb, PB, 0, st>>>(M, b, e, kz, S->part, S->counter, S->s);
+  else k_mg_half<<<nb, 256, 0, st>>>(M, 0, b, e, kz);
+  *nl += 3;
+  return cudaGetLastError();
+}
+// (FP32 levels of that kind keep the general passes.)
+static cudaError_t mg_down_planar(const PLevel &, const float *, float *, float *, cudaStream_t, long *) {
+  return cudaErrorInvalidValue;
+}
+static cudaError_t mg_up_planar(PoissonSolver *, const PLevel &, bool, const float *, const float *, float *,
+                                cudaStream_t, long *) {
+  return cudaErrorInvalidValue;
+}
+
 // b and the coarse correction ec -> e; FP64: on the finest level r.z too.
 static cudaError_t mg_up_level(PoissonSolver *S, const MgLev<double> &M, const PLevel &L, bool finest,
                                const double *b, const double *ec, double *e, cudaStream_t st, long *nl) {
   if (mg_split<double>(L)) {
     const int kz = mg_kz(L), nb = mg_blocks(L, kz);
-    k_mg_prolong<<<nb, 256, 0, st>>>(M, b, ec, e, kz);
+    k_mg_prolong<true><<<nb, 256, 0, st>>>(M, b, ec, e, kz);
     k_mg_half<<<nb, 256, 0, st>>>(M, 1, b, e, kz);
     if (finest) k_mg_half_dot<<<nb, PB, 0, st>>>(M, b, e, kz, S->part, S->counter, S->s);
     else k_mg_half<<<nb, 256, 0, st>>>(M, 0, b, e, kz);
@@ -1395,7 +1435,7 @@ static cudaError_t mg_up_level(PoissonSolver *, const MgLev<float> &M, const PLe
 
 // r.z and beta of the preconditioned residual out.
 static cudaError_t mg_dot(PoissonSolver *S, const double *out, cudaStream_t st, long *nl) {
-  if (S->lv.size() > 1 && S->lv[0].halved) return cudaSuccess;  // formed by mg_up_level
+  if (S->lv.size() > 1 && (S->lv[0].halved || S->lv[0].planar)) return cudaSuccess;  // formed on the way up
   k_rdot<<<S->rblk, PB, 0, st>>>(S->N, S->r, out, S->part, S->counter, S->s);
   (*nl)++;
   return cudaGetLastError();
@@ -1407,8 +1447,8 @@ static cudaError_t mg_dot(PoissonSolver *S, const float *out, cudaStream_t st, l
 }
 
 // one symmetric V-cycle: out = M b0, and r.z into the CG scalars.  A level
-// whose axes are all coarsened runs the k_mg_* kernels in place in its
-// result array (L.halved); the others pre-smooth into their scratch e2 (one
+// whose axes are all coarsened, or all but z, runs the k_mg_* kernels in place
+// in its result array (L.halved, L.planar); the others pre-smooth into their scratch e2 (one
 // damped line-Jacobi sweep from zero, or red-black), restrict the residual,
 // add the prolonged coarse correction into e2 and post-smooth into the
 // result (out on the finest level, e elsewhere).  R: level type.
@@ -1449,6 +1489,10 @@ static cudaError_t vcycle(PoissonSolver *S, const R *b0, R *out, cudaStream_t st
       PCK(mg_down_level(M, L, C.nz, b, res, lvp(C.b), st, nl));
       continue;
     }
+    if (L.planar) {
+      PCK(mg_down_planar(L, b, res, lvp(C.b), st, nl));
+      continue;
+    }
     const LevArgs<R> A = largs<R>(L);
     pre_smooth<R>(L, w, w1, b, lvp(L.e2), st, nl);
     k_residual<R><<<mg_grid(L.nx, L.ny, L.nz), dim3(MG_BX, MG_BY), 0, st>>>(A, b, lvp(L.e2), lvp(L.r));
@@ -1464,6 +1508,8 @@ static cudaError_t vcycle(PoissonSolver *S, const R *b0, R *out, cudaStream_t st
     if (L.halved) {
       const MgLev<R> M = mglev<R>(L);
       PCK(mg_up_level(S, M, L, l == 0, b, lvp(C.e), res, st, nl));
+    } else if (L.planar) {
+      PCK(mg_up_planar(S, L, l == 0, b, lvp(C.e), res, st, nl));
     } else {
       PCK(prolong_chain<R>(L, C, lvp(C.e), lvp(L.t), lvp(L.e2), st, nl));
       post_smooth<R>(L, w, w1, b, lvp(L.e2), res, st, nl);

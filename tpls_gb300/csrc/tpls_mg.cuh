@@ -1,5 +1,6 @@
 // tpls_mg.cuh -- kernels of the symmetric red-black V-cycle on the levels
-// whose three axes are all coarsened (csrc/k_pressure.cu chooses the path).
+// whose three axes are all coarsened, or (FP64) x and y (csrc/k_pressure.cu
+// chooses the path).
 //
 // Red points have (i + j + k) even.  The pre-smoothing starts from zero, red
 // then black, so
@@ -105,12 +106,14 @@ __global__ void __launch_bounds__(256) k_mg_black(const __grid_constant__ MgLev<
 // e at the red points = b / d + P e_c.  P is trilinear with weights 3/4 and
 // 1/4 per axis (an index beyond a wall falls back on the wall's cell, y
 // wraps): 64 P = sum of products of 3 and 1, marched up z with the y- and
-// x-combined coarse values of three coarse levels in registers.
+// x-combined coarse values of three coarse levels in registers.  Z false: z is
+// not coarsened, 16 P in the point's own level.
+template <bool Z>
 __global__ void __launch_bounds__(256) k_mg_prolong(const __grid_constant__ MgLev<double> L, const double *__restrict__ b,
                                                     const double *__restrict__ ec, double *__restrict__ e, int kz) {
   const MgBlk B = mg_block(L, kz);  // kz even
   if (!B.in) return;
-  const int nx = L.nx, plane = nx * L.ny, ncx = nx / 2, ncy = L.ny / 2, ncz = L.nz / 2;
+  const int nx = L.nx, plane = nx * L.ny, ncx = nx / 2, ncy = L.ny / 2, ncz = Z ? L.nz / 2 : L.nz;
   const int y0 = B.j >> 1;
   int y1 = (B.j & 1) ? y0 + 1 : y0 - 1;
   y1 = y1 < 0 ? ncy - 1 : (y1 >= ncy ? 0 : y1);
@@ -124,6 +127,17 @@ __global__ void __launch_bounds__(256) k_mg_prolong(const __grid_constant__ MgLe
     ev = fma(3.0, h, fma(3.0, r0[o + xl], r1[o + xl]));
     od = fma(3.0, h, fma(3.0, r0[o + xr], r1[o + xr]));
   };
+  if constexpr (!Z) {
+    int c = 2 * B.i2 + nx * B.j + plane * B.k0;
+    for (int k = B.k0; k < B.k1; k++, c += plane) {
+      const int odd = (B.j + k) & 1;  // the pair's red point
+      double ev, od;
+      combine(k, ev, od);
+      const int x = odd ? ((2 * B.i2 + 1 == nx - 1) ? 2 : 1) : (B.i2 == 0 ? 0 : 1);
+      e[c + odd] = fma(b[c + odd], L.inv[x][mg_zc(k, L.nz)], (odd ? od : ev) * (1.0 / 16.0));
+    }
+    return;
+  }
   const int ja = B.j & 1;  // even level: the red point is the pair's odd one when j is odd
   double em, om, e0, o0, e1, o1;
   combine(B.k0 / 2 - 1, em, om);
@@ -287,6 +301,7 @@ __global__ void __launch_bounds__(256) k_mg_prolong32(const __grid_constant__ Mg
 // FP32 (arithmetic is 64 times cheaper): the residual of every point and all
 // taps, by the operations of k_residual and k_restrict_axis in their order,
 // equal to theirs bit for bit; bound by its loads.
+// Z false (FP64): z is not coarsened, R = P^T / 4 level by level.
 constexpr int MGR_FX = 60, MGR_FY = 14;
 
 // Four taps of a coarse point in the general restriction's order; w0, w1: 1
@@ -299,13 +314,13 @@ __device__ __forceinline__ R mg_taps(R w0, R w1, R am, R a0, R a1, R ap) {
   return fma((R)0.25, ap, v);
 }
 
-template <typename R>
+template <typename R, bool Z>
 __global__ void __launch_bounds__(256) k_mg_restrict(const __grid_constant__ MgLev<R> L, const R *__restrict__ b,
                                                      const R *__restrict__ e, R *__restrict__ bc, int czb) {
   using V2 = typename Pair2<R>::T;
   __shared__ R sx[2][MGR_FY + 2][32];
   const int nx = L.nx, ny = L.ny, nz = L.nz, plane = nx * ny;
-  const int ncx = nx / 2, ncy = ny / 2, ncz = nz / 2;
+  const int ncx = nx / 2, ncy = ny / 2, ncz = Z ? nz / 2 : nz;
   const int gx = (nx + MGR_FX - 1) / MGR_FX, gy = (ny + MGR_FY - 1) / MGR_FY;
   const int bx = blockIdx.x % gx, by = (blockIdx.x / gx) % gy, bz = blockIdx.x / (gx * gy);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -313,7 +328,7 @@ __global__ void __launch_bounds__(256) k_mg_restrict(const __grid_constant__ MgL
   const bool col = ic >= 0 && ic < ncx;
   const int y0 = by * MGR_FY;
   const int kc0 = bz * czb, kc1 = min(kc0 + czb, ncz);
-  const int ka = max(2 * kc0 - 1, 0), kb = min(2 * kc1, nz - 1);
+  const int ka = Z ? max(2 * kc0 - 1, 0) : kc0, kb = Z ? min(2 * kc1, nz - 1) : kc1 - 1;
   const V2 zero = {(R)0, (R)0};
   // this warp's two rows, 2 w and 2 w + 1 of the tile's 16 (fine y0 - 1 + row; past the grid's end they repeat rows)
   int o[2], om[2], op[2], jl[2];
@@ -387,6 +402,10 @@ __global__ void __launch_bounds__(256) k_mg_restrict(const __grid_constant__ MgL
       const R s2 = sx[buf][2 * w + 2][lane], s3 = sx[buf][2 * w + 3][lane];
       if constexpr (sizeof(R) == sizeof(double)) {
         const R v = fma((R)3, s1 + s2, s0 + s3);
+        if constexpr (!Z) {
+          out[cplane * k] = v * (R)(1.0 / 64.0);
+          continue;
+        }
         const R wz = (k == 0 || k == nz - 1) ? (R)4 : (R)3;
         if (k & 1) {  // k = 2 kc + 1: third tap of kc, first of kc + 1
           acc = fma(wz, v, acc);
@@ -408,7 +427,7 @@ __global__ void __launch_bounds__(256) k_mg_restrict(const __grid_constant__ MgL
       }
     }
   }
-  if (own && kc1 == ncz) {
+  if (Z && own && kc1 == ncz) {
     if constexpr (sizeof(R) == sizeof(double)) out[cplane * (ncz - 1)] = acc * (R)(1.0 / 512.0);
     else out[cplane * (ncz - 1)] = fma((R)0.25, first, acc) * (R)0.125;
   }
