@@ -203,7 +203,27 @@ __global__ void __launch_bounds__(SW_X *SW_Y)
 //      level's x is carried into the next super-chunk.
 // The rounding differs from the level-by-level order (the oracle's) by a
 // few ulp.
+// FP64 columns of one or two super-chunks: the chunks are of equal length and
+// so are the warps' runs in one (75 levels: 2 x 38 in runs of 5 instead of 64
+// and 11 in runs of 8), since a chunk takes as long as its busiest warp's
+// chain: 16 half-sweeps 453 -> 411 us at 100x50x75, 195 -> 172 at 37x19x23, 640 ->
+// 627 at 128x64x96.  Longer columns, which run by segments, keep 64 and 8, known
+// at compile time (3433 us at 256x128x192, 3482 with lengths at run time), and so
+// does FP32: another split would round differently, which the FP32-mixed
+// form's later steps amplify to its own accuracy.
 constexpr int SOC_W = 8, SOC_SC = 64;
+template <typename T>
+__device__ __forceinline__ bool odd_even_split(int nz) {
+  return sizeof(T) == 8 && nz <= 2 * SOC_SC;
+}
+template <typename T>
+__device__ __forceinline__ int odd_chunk(int nz) {  // levels of a super-chunk
+  return odd_even_split<T>(nz) ? (nz <= SOC_SC ? nz : (nz + 1) / 2) : SOC_SC;
+}
+template <typename T>
+__device__ __forceinline__ int odd_run(int nz, int n) {  // levels of a warp in a super-chunk of n
+  return odd_even_split<T>(nz) ? (n + SOC_W - 1) / SOC_W : SOC_SC / SOC_W;
+}
 
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
   unsigned v;
@@ -277,7 +297,7 @@ __device__ __forceinline__ void odd_produce_scan_levels(int comp, const Geo &g, 
     }
   }
   __syncthreads();
-  const int lb = w * PER, le = min(n, lb + PER);
+  const int per = odd_run<T>(g.nz, n), lb = w * per, le = min(n, lb + per);
   T yv = 0, pv = 1;
   for (int lk = lb; lk < le; lk++) {
     const T B = sB[lk][lane];
@@ -456,10 +476,11 @@ __device__ __forceinline__ void sor_odd_c4_tile(int comp_, const Geo &g, const H
   const bool act = (i2 < npair) && (i <= iend);
   constexpr int PER = SOC_SC / SOC_W;
   T carry = 0;  // x of the level below the super-chunk (k0 has B = 0)
-  for (int kc = k0; kc <= k1; kc += SOC_SC) {
-    const int n = min(SOC_SC, k1 - kc + 1);
+  const int sc = odd_chunk<T>(g.nz);
+  for (int kc = k0; kc <= k1; kc += sc) {
+    const int n = min(sc, k1 - kc + 1);
     odd_produce_scan_levels<T, CS, CC>(comp, g, coef, x, i, j, act, k0, kc, n, sA, sB, ey, ep);  // 1. produce, 2. scan
-    const int lb = w * PER, le = min(n, lb + PER);
+    const int per = odd_run<T>(g.nz, n), lb = w * per, le = min(n, lb + per);
     // 3. fold and write
     T xin = carry;
     for (int v = 0; v < w; v++) xin = fma(ep[v][lane], xin, ey[v][lane]);
