@@ -244,12 +244,12 @@ __device__ __forceinline__ void st_release_u32(unsigned *p, unsigned v) {
 // in place (y and P), its ends into ey/ep.  Synchronises the block.  A warp
 // per level, all (level, column) pairs independent.
 // The FP32 sweeps are bound by the latency of the loads, and more warps hide
-// it better than more loads per warp: one level at a time in 32 registers (8
-// blocks, all 64 warps of an SM) measured 404 us per half-sweep of three
-// components at 512x256x256, four levels in flight at 40 registers (6
+// it better than more loads per warp: two levels at a time in 32 registers (8
+// blocks, all 64 warps of an SM) measured 416 us per half-sweep of three
+// components at 512x256x256, one at a time 421, four in flight at 40 registers (6
 // blocks) 470.  Lanes past the row's end take the row's first point of this
-// colour (and store nothing), which frees the loads of their predicates: 404
-// against 422.
+// colour (and store nothing), which frees the loads of their predicates: 421
+// against 444.
 template <typename T, typename CS, int CC>
 __device__ __forceinline__ void odd_produce_scan_levels(int comp, const Geo &g, const CS &coef,
                                                         const T *__restrict__ x, int i, int j, bool act, int k0,
@@ -259,7 +259,7 @@ __device__ __forceinline__ void odd_produce_scan_levels(int comp, const Geo &g, 
   const int sy_ = g.sy, sz = g.sz, nz = g.nz;
   constexpr int PER = SOC_SC / SOC_W;
   const int ic = (sizeof(T) == 4 && !act) ? 1 + ((i & 1) ^ 1) : i;
-#pragma unroll(sizeof(T) == 4 ? 1 : 4)
+#pragma unroll(sizeof(T) == 4 ? 2 : 4)
   for (int r = 0; r < PER; r++) {
     const int lk = w + r * SOC_W, k = kc + lk;
     if (lk < n) {
@@ -401,6 +401,28 @@ __device__ __forceinline__ T odd_last_value(T xin, int n, bool col_in, T (*sA)[3
   return col_in ? fma(sB[n - 1][lane], xin, sA[n - 1][lane]) : (T)0;
 }
 
+// Boundary rows of a warp's levels lb .. le-1 (at most eight) of tile bx, after
+// its writes: a lane per level, lanes 0-15 for the first pair and 16-31 for the
+// last, so that the loads of all levels are in flight at once (by the pairs'
+// own lanes, level after level, they took 4.6 of 14.4 us at 64x32x48, 16 of 50 at
+// 192x96x112 in FP32; 16 half-sweeps now 222 instead of 237, and 608 instead of
+// 730).  The point a boundary copies was relaxed here (in sA) or
+// is of the other colour and final.  Nothing else in this sweep reads the
+// boundary values of these levels.  first: the relaxed point of the first pair.
+template <typename T>
+__device__ __forceinline__ void odd_bc(int comp, const Geo &g, const Helm &h, T *__restrict__ x,
+                                       const double *__restrict__ X, const double *__restrict__ P, int fuse, int bx,
+                                       int first, int j, int iend, int kc, int lb, int le, T (*sA)[32]) {
+  const int last = (iend - 1) / 2;
+  if (bx != 0 && bx != last / 32) return;
+  __syncwarp();
+  const int lane = threadIdx.x & 31, right = lane >> 4, lk = lb + (lane & 15), i2 = right ? last : 0;
+  if (lk >= le || bx != i2 / 32) return;
+  const int ib = right ? iend : 1;
+  const T src = (2 * i2 + first != ib) ? x[TPLS_IDX(g, ib, j, kc + lk)] : sA[lk][i2 & 31];
+  sor_bc(comp, g, h, x, X, P, i2, ib, iend, src, j, kc + lk, fuse);
+}
+
 // Phase 3: each warp writes x = y + P x_in from the value entering its own
 // chunk (given in xin for FP64; for FP32 xin enters the super-chunk and the
 // warp folds the chunk ends below its own into it first), then the
@@ -427,22 +449,8 @@ __device__ __forceinline__ T odd_write(int comp, const Geo &g, const Helm &h, T 
       sA[lk][lane] = v;  // kept for the boundary rows below
       if (lk == n - 1) last = v;
     }
-    // boundary rows of these levels, by the owners of the first and last
-    // pairs, after the writes: the point each boundary copies (relaxed
-    // here, or of the other colour and final) is loaded for all levels at
-    // once instead of level by level.  Nothing in this sweep reads the
-    // boundary values of these levels.
-    if (bc && (i2 == 0 || i2 == (iend - 1) / 2)) {
-      const int ib = (i2 == 0) ? 1 : iend;
-      T src[PER];
-#pragma unroll
-      for (int l = 0; l < PER; l++)
-        src[l] = (lb + l < le) ? ((i != ib) ? x[TPLS_IDX(g, ib, j, kc + lb + l)] : sA[lb + l][lane]) : (T)0;
-#pragma unroll
-      for (int l = 0; l < PER; l++)
-        if (lb + l < le) sor_bc(comp, g, h, x, X, P, i2, ib, iend, src[l], j, kc + lb + l, fuse);
-    }
   }
+  if (bc) odd_bc<T>(comp, g, h, x, X, P, fuse, (i2 - lane) / 32, 1 + ((i & 1) ^ 1), j, iend, kc, lb, le, sA);
   return last;
 }
 
@@ -474,7 +482,6 @@ __device__ __forceinline__ void sor_odd_c4_tile(int comp_, const Geo &g, const H
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int i2 = bx * 32 + lane, i = 2 * i2 + 1 + par;
   const bool act = (i2 < npair) && (i <= iend);
-  constexpr int PER = SOC_SC / SOC_W;
   T carry = 0;  // x of the level below the super-chunk (k0 has B = 0)
   const int sc = odd_chunk<T>(g.nz);
   for (int kc = k0; kc <= k1; kc += sc) {
@@ -494,22 +501,8 @@ __device__ __forceinline__ void sor_odd_c4_tile(int comp_, const Geo &g, const H
         sA[lk][lane] = v;  // kept for the boundary rows below
         if (lk == n - 1) scarry[lane] = v;
       }
-      // boundary rows of these levels, by the owners of the first and last
-      // pairs, after the writes: the point each boundary copies (relaxed
-      // here, or of the other colour and final) is loaded for all levels at
-      // once instead of level by level.  Nothing in this sweep reads the
-      // boundary values of these levels.
-      if (bc && (i2 == 0 || i2 == (iend - 1) / 2)) {
-        const int ib = (i2 == 0) ? 1 : iend;
-        T src[PER];
-#pragma unroll
-        for (int l = 0; l < PER; l++)
-          src[l] = (lb + l < le) ? ((i != ib) ? x[TPLS_IDX(g, ib, j, kc + lb + l)] : sA[lb + l][lane]) : (T)0;
-#pragma unroll
-        for (int l = 0; l < PER; l++)
-          if (lb + l < le) sor_bc(comp, g, h, x, X, P, i2, ib, iend, src[l], j, kc + lb + l, fuse);
-      }
     }
+    if (bc) odd_bc<T>(comp, g, h, x, X, P, fuse, bx, 1 + par, j, iend, kc, lb, le, sA);
     __syncthreads();
     carry = scarry[lane];
   }
@@ -611,10 +604,12 @@ __device__ __forceinline__ void sor_odd_segment(int comp_, const Geo &g, const H
     }                                             \
   } while (0)
 
-template <typename T, typename CS>
+// BC: with the boundary rows (the second half-sweep); the launches without
+// them then carry none of their registers.
+template <typename T, typename CS, bool BC>
 __global__ void __launch_bounds__(SOC_W * 32, sizeof(T) == 4 ? 8 : 5)  // 32 / 48 registers: 8 / 5 blocks per SM
     k_sor_odd_seg(Geo g, Helm h, const __grid_constant__ SweepSet<T, CS> S, const double *__restrict__ P, int flg,
-                  int bc, int fuse, OddChain oc, int gx, int limit) {
+                  int fuse, OddChain oc, int gx, int limit) {
   __shared__ OddShared<T> sh;
   __shared__ unsigned s_t, s_ep;
   if (threadIdx.x == 0) {
@@ -628,7 +623,7 @@ __global__ void __launch_bounds__(SOC_W * 32, sizeof(T) == 4 ? 8 : 5)  // 32 / 4
   const int q3 = ct / (gx * g.ny), tile = ct - q3 * gx * g.ny;
   const int comp = S.id[q3];
 #define TPLS_SEG(CC)                                                                                              \
-  sor_odd_segment<T, CS, CC>(comp, g, h, S.x[q3], S.coef[q3], P, S.X[q3], flg, bc, fuse, oc, limit, t, epoch, nct, \
+  sor_odd_segment<T, CS, CC>(comp, g, h, S.x[q3], S.coef[q3], P, S.X[q3], flg, BC, fuse, oc, limit, t, epoch, nct, \
                              seg, tile % gx, tile / gx + 1, sh)
   TPLS_BY_COMP(TPLS_SEG);
 #undef TPLS_SEG
@@ -646,14 +641,14 @@ __global__ void __launch_bounds__(SOC_W * 32, sizeof(T) == 4 ? 8 : 5)  // 32 / 4
 // (FP64: with a bound of 1 block per SM the compiler takes the registers of 2
 // blocks and a half-sweep at 128x64x96 51 us instead of 40.5; bounds of 4 and
 // 5 blocks measured 40.8 and 42.)
-template <typename T, typename CS>
+template <typename T, typename CS, bool BC>
 __global__ void __launch_bounds__(SOC_W * 32, sizeof(T) == 4 ? 8 : 3)
     k_sor_odd_c4(Geo g, Helm h, const __grid_constant__ SweepSet<T, CS> S, const double *__restrict__ P, int gx,
-                 int flg, int bc, int fuse) {
+                 int flg, int fuse) {
   __shared__ OddShared<T> sh;
   const int q3 = blockIdx.x / gx, bx = blockIdx.x - q3 * gx, comp = S.id[q3];
 #define TPLS_COL(CC) \
-  sor_odd_c4_tile<T, CS, CC>(comp, g, h, S.x[q3], S.coef[q3], P, S.X[q3], flg, bc, fuse, bx, blockIdx.y, sh)
+  sor_odd_c4_tile<T, CS, CC>(comp, g, h, S.x[q3], S.coef[q3], P, S.X[q3], flg, BC, fuse, bx, blockIdx.y, sh)
   TPLS_BY_COMP(TPLS_COL);
 #undef TPLS_COL
 }
@@ -775,9 +770,12 @@ static cudaError_t odd_set(const Geo &g, const Helm &h, const SweepSet<T, CS> &s
   // us, whole columns 764), the FP64 ones, bound by the FP64 pipe, do not
   // (128x64x96: 720, whole columns 646).
   if (oc && nseg >= (sizeof(T) == 4 ? 2 : 3) && oc->cap >= blocks) {
-    k_sor_odd_seg<T, CS><<<blocks, SOC_W * 32, 0, st>>>(g, h, s, pres, flg, bc, fuse, *oc, gx, 1 << 20);
+    if (bc) k_sor_odd_seg<T, CS, true><<<blocks, SOC_W * 32, 0, st>>>(g, h, s, pres, flg, fuse, *oc, gx, 1 << 20);
+    else k_sor_odd_seg<T, CS, false><<<blocks, SOC_W * 32, 0, st>>>(g, h, s, pres, flg, fuse, *oc, gx, 1 << 20);
   } else {  // one block per 32 columns of a row, the column in super-chunks
-    k_sor_odd_c4<T, CS><<<dim3(gx * s.n, g.ny), SOC_W * 32, 0, st>>>(g, h, s, pres, gx, flg, bc, fuse);
+    const dim3 grd(gx * s.n, g.ny);
+    if (bc) k_sor_odd_c4<T, CS, true><<<grd, SOC_W * 32, 0, st>>>(g, h, s, pres, gx, flg, fuse);
+    else k_sor_odd_c4<T, CS, false><<<grd, SOC_W * 32, 0, st>>>(g, h, s, pres, gx, flg, fuse);
   }
   return cudaGetLastError();
 }
