@@ -667,22 +667,33 @@ __device__ __forceinline__ CDT<float> conv_diff_pair(int comp, const Geo &g, con
 // rounding is not relative to the step's increment.  Stored: b = R / diag,
 // one float per point in record-slot order (the sweeps recompute the
 // coefficients from mu).  conv is stored into its FP64 history exactly.
-__global__ void __launch_bounds__(MB_X *MB_Y)
-    k_mom_rhs_pair(int comp, Geo g, MomF m, const double *__restrict__ U, const double *__restrict__ V,
-                   const double *__restrict__ W, const float *__restrict__ mu, const double *__restrict__ fc,
-                   const double *__restrict__ c1, const double *__restrict__ c0, const double *__restrict__ s1,
-                   const double *__restrict__ s0, double *__restrict__ conv2, double *__restrict__ csf2,
-                   float *__restrict__ bdef) {
-  const int i = blockIdx.x * MB_X + threadIdx.x + 1, j = blockIdx.y * MB_Y + threadIdx.y + 1;
-  const int k = blockIdx.z;
-  if (i > g.nx || j > g.ny) return;
+// The three components in one launch (gx blocks along x each).  Neither the
+// FP64 pipe (11 operations per point) nor the issue slots (700 instructions)
+// are full: it waits for loads and FP64 results, so many blocks per SM pay more
+// than registers do (BOUNDS_FIGURES; a launch per component, 9 blocks: 4050).
+// (The component stays a run-time value: as a template argument it changes
+// which products the compiler contracts, by last bits that the FP32 sweeps
+// amplify to their own accuracy.)
+struct MomPairArgs {
+  const double *U, *V, *W;
+  const float *mu;
+  const double *f[3], *c1[3], *c0[3], *s1[3], *s0[3];
+  double *conv2[3], *csf2[3];
+  float *b[3];
+};
+__global__ void __launch_bounds__(MB_X *MB_Y, 14)
+    k_mom_rhs_pair(Geo g, MomF m, const __grid_constant__ MomPairArgs A, int gx) {
+  const int comp = blockIdx.x / gx, i = (blockIdx.x - comp * gx) * MB_X + threadIdx.x + 1;
+  const int j = blockIdx.y * MB_Y + threadIdx.y + 1, k = blockIdx.z;
+  if (i > g.nx || j > g.ny || (comp != 2 && k == g.nz)) return;
+  const double *fc = A.f[comp];
   const int c = TPLS_IDX(g, i, j, k);
   CDT<float> cd = {0.0f, 0.0f};
   const bool valid = cd_valid(comp, g, i, k);
   FcT<float> f;
   if (valid) {
-    f = faces<float>(comp, g, mu, i, j, k);
-    cd = conv_diff_pair(comp, g, m, U, V, W, f, i, j, k);
+    f = faces<float>(comp, g, A.mu, i, j, k);
+    cd = conv_diff_pair(comp, g, m, A.U, A.V, A.W, f, i, j, k);
   }
   // main_ns_hybrid.F90:629-641 face averages of the CSF force
   double s2;
@@ -690,20 +701,18 @@ __global__ void __launch_bounds__(MB_X *MB_Y)
   else if (comp == 1) s2 = (fc[TPLS_IDX(g, i, j + 1, k + 1)] + fc[TPLS_IDX(g, i, j, k + 1)]) * 0.5;
   else s2 = (fc[TPLS_IDX(g, i, j + 1, k + 1)] + fc[TPLS_IDX(g, i, j + 1, k)]) * 0.5;
   const double conv = widen_bits(cd.conv);
-  conv2[c] = conv;
-  csf2[c] = s2;
+  A.conv2[comp][c] = conv;
+  A.csf2[comp][c] = s2;
   if (!valid) return;
-  const double abc = (23.0 / 12.0) * conv - (4.0 / 3.0) * c1[c] + (5.0 / 12.0) * c0[c];
-  const double abs_ = (23.0 / 12.0) * s2 - (4.0 / 3.0) * s1[c] + (5.0 / 12.0) * s0[c];
+  const double abc = (23.0 / 12.0) * conv - (4.0 / 3.0) * A.c1[comp][c] + (5.0 / 12.0) * A.c0[comp][c];
+  const double abs_ = (23.0 / 12.0) * s2 - (4.0 / 3.0) * A.s1[comp][c] + (5.0 / 12.0) * A.s0[comp][c];
   const double R = m.dt64 * (widen_bits(cd.diff) - abc + abs_);
   const float diag = 1.0f + m.ax2 * (f.px + f.mx) + m.ay2 * (f.py + f.my) + m.az2 * (f.pz + f.mz);
-  bdef[rec_slot(g, c, i)] = round_bits(R) / diag;
+  A.b[comp][rec_slot(g, c, i)] = round_bits(R) / diag;
 }
 
-cudaError_t launch_mom_rhs_pair(int comp, const Geo &g, const Phys &ph, const double *u2, const double *v2,
-                                const double *w2, const float *mu, const double *fcsf, const double *c1,
-                                const double *c0, const double *s1, const double *s0, double *conv2,
-                                double *csf2, float *bdef, cudaStream_t st) {
+cudaError_t launch_mom_rhs_pair(const Geo &g, const Phys &ph, const double *u2, const double *v2, const double *w2,
+                                const float *mu, const MomFields &q, float *const b[3], cudaStream_t st) {
   const Helm hm = helm_of(ph);
   MomF m;
   m.rdx = (float)(1.0 / ph.dx);
@@ -714,10 +723,19 @@ cudaError_t launch_mom_rhs_pair(int comp, const Geo &g, const Phys &ph, const do
   m.ax2 = (float)hm.ax2;
   m.ay2 = (float)hm.ay2;
   m.az2 = (float)hm.az2;
-  const int nk = (comp == 2) ? g.nz + 1 : g.nz;
-  dim3 grd((g.nx + MB_X - 1) / MB_X, (g.ny + MB_Y - 1) / MB_Y, nk);
-  k_mom_rhs_pair<<<grd, dim3(MB_X, MB_Y), 0, st>>>(comp, g, m, u2, v2, w2, mu, fcsf, c1, c0, s1, s0, conv2, csf2,
-                                                   bdef);
+  MomPairArgs A = {u2, v2, w2, mu};
+  for (int c = 0; c < 3; c++) {
+    A.f[c] = q.fcsf[c];
+    A.c1[c] = q.c1[c];
+    A.c0[c] = q.c0[c];
+    A.s1[c] = q.s1[c];
+    A.s0[c] = q.s0[c];
+    A.conv2[c] = q.conv2[c];
+    A.csf2[c] = q.csf2[c];
+    A.b[c] = b[c];
+  }
+  const int gx = (g.nx + MB_X - 1) / MB_X;
+  k_mom_rhs_pair<<<dim3(3 * gx, (g.ny + MB_Y - 1) / MB_Y, g.nz + 1), dim3(MB_X, MB_Y), 0, st>>>(g, m, A, gx);
   return cudaGetLastError();
 }
 

@@ -1391,12 +1391,7 @@ static int mixed_front(tpls_ctx *c) {
     }
     {
       PhaseScope ps(c, TPLS_T_MOM_RHS);
-      LCK(c, launch_mom_rhs_pair(0, g, ph, c->u2, c->v2, c->w2, c->mu32, c->fx, c->conv_u[s1], c->conv_u[s0],
-                                 c->csf_u[s1], c->csf_u[s0], c->conv_u[s2], c->csf_u[s2], c->bdef[0], st));
-      LCK(c, launch_mom_rhs_pair(1, g, ph, c->u2, c->v2, c->w2, c->mu32, c->fy, c->conv_v[s1], c->conv_v[s0],
-                                 c->csf_v[s1], c->csf_v[s0], c->conv_v[s2], c->csf_v[s2], c->bdef[1], st));
-      LCK(c, launch_mom_rhs_pair(2, g, ph, c->u2, c->v2, c->w2, c->mu32, c->fz, c->conv_w[s1], c->conv_w[s0],
-                                 c->csf_w[s1], c->csf_w[s0], c->conv_w[s2], c->csf_w[s2], c->bdef[2], st));
+      LCK(c, launch_mom_rhs_pair(g, ph, c->u2, c->v2, c->w2, c->mu32, mom_fields(c), c->bdef, st));
     }
   }
   return TPLS_OK;

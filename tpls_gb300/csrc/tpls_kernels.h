@@ -115,13 +115,8 @@ cudaError_t launch_mom_rhs(const Geo &g, const Phys &ph, const double *u2, const
 // FP32 pairs by integer operations and FP32 viscosity, FP64 CSF force and
 // AB3 combination; writes the defect-form b of the FP32 sweeps (one float
 // per point, rec_slot order) and the AB3 histories.
-cudaError_t launch_mom_rhs_pair(int comp, const Geo &g, const Phys &ph,
-                                const double *u2, const double *v2,
-                                const double *w2, const float *mu,
-                                const double *fcsf, const double *c1,
-                                const double *c0, const double *s1,
-                                const double *s0, double *conv2, double *csf2,
-                                float *coef, cudaStream_t st);
+cudaError_t launch_mom_rhs_pair(const Geo &g, const Phys &ph, const double *u2, const double *v2, const double *w2,
+                                const float *mu, const MomFields &q, float *const b[3], cudaStream_t st);
 // FP64 stencils writing the defect-form b of the FP32 sweeps (FP32-mixed
 // form with TPLS_PART_MOM_STENCIL; one float per point, rec_slot order).
 cudaError_t launch_mom_rhs64r32(int comp, const Geo &g, const Phys &ph,
