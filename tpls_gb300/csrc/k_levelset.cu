@@ -496,10 +496,16 @@ cudaError_t launch_ls_iter_ff(const Geo &g, const Phys &ph, const double *in64, 
 struct F3 {
   double x, y, z;
 };
+// Quotients of the parameters, formed once on the host (the same IEEE values):
+// four FP64 divisions of about nine operations each out of a band point's
+// 150.
+struct CsfK {
+  double rdx, rdy, rdz, a, sw, scap, max_kappa;  // a = 1/(2 sw)
+};
 
 template <typename T>
-__device__ __forceinline__ F3 csf_point(const Geo &g, const Phys &ph, double max_kappa,
-                                        const double *__restrict__ fi0, int i, int j, int k) {
+__device__ __forceinline__ F3 csf_point(const Geo &g, const CsfK &ph, const double *__restrict__ fi0, int i, int j,
+                                        int k) {
   const int c = TPLS_IDX(g, i, j, k);
   struct Ld {
     const double *p;
@@ -513,7 +519,7 @@ __device__ __forceinline__ F3 csf_point(const Geo &g, const Phys &ph, double max
   if (kp < dkey(-ph.sw) || kp > dkey(ph.sw)) return r;
   const T p = (T)p64;
   const int sy = g.sy, sz = g.sz;
-  const T rdx = (T)(1.0 / ph.dx), rdy = (T)(1.0 / ph.dy), rdz = (T)(1.0 / ph.dz);
+  const T rdx = (T)ph.rdx, rdy = (T)ph.rdy, rdz = (T)ph.rdz;
   const T r2dx = (T)0.5 * rdx, r2dy = (T)0.5 * rdy, r2dz = (T)0.5 * rdz, two = (T)2;
   const T d2x = (fi[c + 1] - two * p + fi[c - 1]) * (rdx * rdx);
   const T d2y = (fi[c + sy] - two * p + fi[c - sy]) * (rdy * rdy);
@@ -536,8 +542,8 @@ __device__ __forceinline__ F3 csf_point(const Geo &g, const Phys &ph, double max
     const T term3 = two * (gx * gy * d2xy + gx * gz * d2xz + gy * gz * d2yz) * inv15;
     kap = -(term1 - term2 - term3);
   }
-  if (kap > (T)max_kappa) kap = (T)max_kappa;
-  const T a = (T)(1.0 / (2.0 * ph.sw));
+  if (kap > (T)ph.max_kappa) kap = (T)ph.max_kappa;
+  const T a = (T)ph.a;
   const T dirac = a + a * cos((T)TPLS_PI_SP * p / (T)ph.sw);
   const T m = dirac * (T)ph.scap * kap;
   r.x = (double)(m * gx);
@@ -553,12 +559,11 @@ __device__ __forceinline__ F3 lin2(F3 a, F3 b) {  // 2a - b
 
 // value on the i = 1..nx columns including the extrapolated z ghost planes
 template <typename T>
-__device__ __forceinline__ F3 csf_colval(const Geo &g, const Phys &ph, double mk,
-                                         const double *fi, int i, int j, int k) {
-  if (k == 0) return lin2(csf_point<T>(g, ph, mk, fi, i, j, 1), csf_point<T>(g, ph, mk, fi, i, j, 2));
+__device__ __forceinline__ F3 csf_colval(const Geo &g, const CsfK &ph, const double *fi, int i, int j, int k) {
+  if (k == 0) return lin2(csf_point<T>(g, ph, fi, i, j, 1), csf_point<T>(g, ph, fi, i, j, 2));
   if (k == g.nz + 1)
-    return lin2(csf_point<T>(g, ph, mk, fi, i, j, g.nz), csf_point<T>(g, ph, mk, fi, i, j, g.nz - 1));
-  return csf_point<T>(g, ph, mk, fi, i, j, k);
+    return lin2(csf_point<T>(g, ph, fi, i, j, g.nz), csf_point<T>(g, ph, fi, i, j, g.nz - 1));
+  return csf_point<T>(g, ph, fi, i, j, k);
 }
 
 __device__ __forceinline__ F3 lane_of(const F3 &a, int l) {
@@ -568,14 +573,20 @@ __device__ __forceinline__ F3 lane_of(const F3 &a, int l) {
 
 // T: arithmetic of the curvature (double, or float in the FP32-mixed form);
 // TO: storage of the force components.
-template <typename T, typename TO>
-__global__ void k_csf(Geo g, Phys ph, double mk, const double *__restrict__ fi,
+// Blocks per SM (B): on large grids most warps only write zeros and six blocks
+// hide the few that evaluate the band (256x128x192: 86 us, 108 with the 3 that
+// its registers allow; 512x256x256: 385, 504); on small ones the band's own
+// chain is what a launch waits for, and the registers matter more (192x96x112: 45
+// us, 59 with six).
+template <typename T, typename TO, int B>
+__global__ void __launch_bounds__(LS_BX *LS_BY, B)
+    k_csf(Geo g, CsfK ph, const double *__restrict__ fi,
                       TO *__restrict__ fx, TO *__restrict__ fy, TO *__restrict__ fz) {
   const int i = blockIdx.x * LS_BX + threadIdx.x + 1, j = blockIdx.y * LS_BY + threadIdx.y + 1;
   const int k = blockIdx.z;
   if (j > g.ny) return;  // uniform per warp (one row)
   F3 v = {0.0, 0.0, 0.0};
-  if (i <= g.nx) v = csf_colval<T>(g, ph, mk, fi, i, j, k);
+  if (i <= g.nx) v = csf_colval<T>(g, ph, fi, i, j, k);
   // the inlet and outlet columns extrapolate from the last two columns: the
   // inner one from the next lane, or by itself where that is in another warp
   F3 in = {0.0, 0.0, 0.0};
@@ -586,7 +597,7 @@ __global__ void k_csf(Geo g, Phys ph, double mk, const double *__restrict__ fi,
       const F3 p = lane_of(v, last - 1);
       if (i == g.nx) in = p;
     } else if (i == g.nx) {
-      in = csf_colval<T>(g, ph, mk, fi, i - 1, j, k);
+      in = csf_colval<T>(g, ph, fi, i - 1, j, k);
     }
   }
   if (i > g.nx) return;
@@ -603,20 +614,28 @@ __global__ void k_csf(Geo g, Phys ph, double mk, const double *__restrict__ fi,
   }
 }
 
+static CsfK csf_constants(const Phys &ph) {
+  return {1.0 / ph.dx, 1.0 / ph.dy, 1.0 / ph.dz, 1.0 / (2.0 * ph.sw), ph.sw, ph.scap,
+          1.0 / fmin(fmin(ph.dx, ph.dy), ph.dz)};
+}
+template <typename T, typename TO>
+static cudaError_t csf(const Geo &g, const Phys &ph, const double *phi3, TO *fx, TO *fy, TO *fz, cudaStream_t st) {
+  const dim3 grd = owned_grid(g, g.nz + 2), blk(LS_BX, LS_BY);
+  const CsfK q = csf_constants(ph);
+  if ((size_t)g.nx * g.ny * g.nz > 4000000) k_csf<T, TO, 6><<<grd, blk, 0, st>>>(g, q, phi3, fx, fy, fz);
+  else k_csf<T, TO, 1><<<grd, blk, 0, st>>>(g, q, phi3, fx, fy, fz);
+  return cudaGetLastError();
+}
 cudaError_t launch_csf(const Geo &g, const Phys &ph, const double *phi3,
                        double *fx, double *fy, double *fz, cudaStream_t st) {
-  const double mk = 1.0 / fmin(fmin(ph.dx, ph.dy), ph.dz);
-  k_csf<double, double><<<owned_grid(g, g.nz + 2), dim3(LS_BX, LS_BY), 0, st>>>(g, ph, mk, phi3, fx, fy, fz);
-  return cudaGetLastError();
+  return csf<double>(g, ph, phi3, fx, fy, fz, st);
 }
 cudaError_t launch_csf(const Geo &g, const Phys &ph, const double *phi3, float *fx, float *fy, float *fz,
                        cudaStream_t st) {
-  const double mk = 1.0 / fmin(fmin(ph.dx, ph.dy), ph.dz);
   // curvature stays FP64: its second differences of phi (~dx^2 |phi''|)
   // would lose ~1e-3 of their value to FP32 cancellation, a coherent error
   // in the surface-tension force at the interface; the force is stored FP32
-  k_csf<double, float><<<owned_grid(g, g.nz + 2), dim3(LS_BX, LS_BY), 0, st>>>(g, ph, mk, phi3, fx, fy, fz);
-  return cudaGetLastError();
+  return csf<double>(g, ph, phi3, fx, fy, fz, st);
 }
 
 // ---------------------------------------------------------------------------
