@@ -139,10 +139,13 @@ __device__ __forceinline__ T yface(const Geo &g, const T *__restrict__ phi,
 }
 
 constexpr int ADV_BX = 32, ADV_BY = 8;
-// z levels per thread (column chunk): 16, halved to no less than 2 while the
-// grid has fewer than three blocks per SM.  A chunk forms one z-face more than
-// its levels; at 64x32x48, 24 blocks of 16 levels left 128 of 152 SMs idle
-// (285 us, against about 30 for its FP64 operations spread over all).
+// z levels per thread (column chunk), at most ADV_KC.  A chunk forms one z face
+// more than its levels, 3 kc + 1 faces per column, and the launch takes as long
+// as the SM with the most blocks: the choice with the least (blocks of that SM)
+// x (faces), a single block per SM counting 1.2 times (its barriers leave the FP64
+// pipe idle).  Against 16 halved until the grid has three blocks per SM: 53 ->
+// 45 us at 64x32x48, 33 -> 20 at 37x19x23, 182 -> 165 at 100x50x75, 252 -> 240 at
+// 128x64x96, 1786 -> 1700 at 256x128x192.
 constexpr int ADV_KC = 16;
 
 // One block covers 32 x 8 columns and a chunk of ADV_KC levels.  At each
@@ -403,8 +406,16 @@ cudaError_t launch_advect_tma(const Geo &g, const Phys &ph, const void *map128, 
 
 static int adv_levels(const Geo &g) {
   const int gxy = ((g.nx + ADV_BX - 1) / ADV_BX) * ((g.ny + ADV_BY - 1) / ADV_BY);
-  int kc = ADV_KC;
-  while (kc > 2 && gxy * ((g.nz + kc - 1) / kc) < 3 * 152) kc /= 2;
+  int kc = 1;
+  double best = 1e300;
+  for (int q = 1; q <= ADV_KC; q++) {
+    const int w = (gxy * ((g.nz + q - 1) / q) + 151) / 152;
+    const double t = (double)w * (3 * q + 1) * (w == 1 ? 1.2 : 1.0);
+    if (t < best) {
+      best = t;
+      kc = q;
+    }
+  }
   return kc;
 }
 
