@@ -847,58 +847,92 @@ RefCoef ref_coef(int comp, const Phys &ph, const double *rhs, const double *mu) 
           h.az2 * (comp == 2 ? 1.0 : 0.25)};
 }
 
-// get_difference: per-block partials of sum (a-b)^2 over i 1..nx, j 1..ny,
-// planes 0..nzp-1.
-// Sum of squared differences of two iterates (the sweeps' convergence
-// diagnostic), one partial per block.  FP64 iterates are differenced and
-// summed in FP64; FP32 iterates in FP32 up to the warp sums (exactly
-// widened), so the FP32 form issues no FP64 instruction per point.
+// get_difference of up to three pairs of iterates (the sweeps' convergence
+// diagnostic): out[q], q < nout, = sum (a-b)^2 over i 1..nx, j 1..ny, planes
+// 0..nzp-1, 0 without a pair.  One launch: rows to warps in a fixed order, a partial per
+// block, summed by the last block in a fixed order.  (A launch and one or two
+// more for the sum per component took 75 us of a step at 128x64x96, 30 at
+// 64x32x48; this 23 and 13.)  FP64 iterates are differenced and
+// summed in FP64; FP32 iterates in FP32 up to the sums of a warp's 32 points
+// (exactly widened), so the FP32 form issues one FP64 instruction per 32 points.
+constexpr int DF_B = 256, DF_W = DF_B / 32;
 template <typename T>
-__global__ void k_diff2(Geo g, const T *__restrict__ a, const T *__restrict__ b, double *__restrict__ part) {
-  const int i = blockIdx.x * MB_X + threadIdx.x + 1, j = blockIdx.y * MB_Y + threadIdx.y + 1;
-  const int k = blockIdx.z;
-  T e = (T)0;
-  if (i <= g.nx && j <= g.ny) {
-    const int c = TPLS_IDX(g, i, j, k);
-    const T d = a[c] - b[c];
-    e = d * d;
-  }
-  const int t = threadIdx.y * MB_X + threadIdx.x, blk = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-  if constexpr (sizeof(T) == sizeof(float)) {
-    __shared__ double s[MB_X * MB_Y / 32];
-    for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
-    if ((t & 31) == 0) s[t >> 5] = widen_bits(e);
-    __syncthreads();
-    if (t == 0) {
-      double acc = 0.0;
-      for (int q = 0; q < MB_X * MB_Y / 32; q++) acc += s[q];
-      part[blk] = acc;
+__global__ void __launch_bounds__(DF_B)
+    k_diff_set(Geo g, const __grid_constant__ DiffSet<T> s, int planes, double *__restrict__ part, unsigned *ctr,
+               double *__restrict__ out, int nout) {
+  __shared__ double sh[3][DF_B];
+  __shared__ bool last;
+  const int t = threadIdx.x, lane = t & 31, nb = gridDim.x;
+  double acc[3] = {0.0, 0.0, 0.0};
+  for (int row = blockIdx.x * DF_W + (t >> 5); row < g.ny * planes; row += nb * DF_W) {
+    const int k = row / g.ny, c0 = TPLS_IDX(g, 1, row - g.ny * k + 1, k);
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      if (!s.a[q] || k >= s.nzp[q]) continue;
+      const T *a = s.a[q] + c0, *b = s.b[q] + c0;
+#pragma unroll 4
+      for (int i = lane; i < ((g.nx + 31) & ~31); i += 32) {
+        T d = (T)0;
+        if (i < g.nx) d = a[i] - b[i];
+        if constexpr (sizeof(T) == sizeof(float)) {
+          float e = d * d;
+          for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+          acc[q] += widen_bits(e);
+        } else {
+          acc[q] = fma(d, d, acc[q]);
+        }
+      }
     }
-  } else {
-    __shared__ double s[MB_X * MB_Y];
-    const double acc = block_sum<MB_X * MB_Y / 32>(e, t, s);
-    if (t == 0) part[blk] = acc;
+  }
+  // the block's sums: FP64 lane by lane over the warps, then one warp's tree;
+  // FP32 (every lane holds the warp's sum) over the warps
+  auto block = [&](double (&v)[3], bool lanes) {  // in lane 0 of warp 0
+    __syncthreads();
+    for (int q = 0; q < 3; q++) sh[q][t] = v[q];
+    __syncthreads();
+    if (t < 32)
+      for (int q = 0; q < 3; q++) {
+        double x = sh[q][t];
+        for (int w = 1; w < DF_W; w++) x += sh[q][t + 32 * w];
+        if (lanes)
+          for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        v[q] = x;
+      }
+  };
+  block(acc, sizeof(T) == sizeof(double));
+  if (t == 0) {
+    for (int q = 0; q < 3; q++) part[q * nb + blockIdx.x] = acc[q];
+    __threadfence();
+    last = atomicAdd(ctr, 1u) == (unsigned)nb - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int q = 0; q < 3; q++) {
+    acc[q] = 0.0;
+    for (int b = t; b < nb; b += DF_B) acc[q] += __ldcg(part + q * nb + b);
+  }
+  block(acc, true);
+  if (t == 0) {
+    for (int q = 0; q < nout; q++) out[q] = acc[q];
+    *ctr = 0u;
   }
 }
 
-int diff2_blocks(const Geo &g, int nzp) {
-  return ((g.nx + MB_X - 1) / MB_X) * ((g.ny + MB_Y - 1) / MB_Y) * nzp;
-}
-
 template <typename T>
-static cudaError_t diff2(const Geo &g, const T *a, const T *b, int nzp, double *part, cudaStream_t st) {
-  dim3 grd((g.nx + MB_X - 1) / MB_X, (g.ny + MB_Y - 1) / MB_Y, nzp);
-  k_diff2<T><<<grd, dim3(MB_X, MB_Y), 0, st>>>(g, a, b, part);
+cudaError_t launch_diff_set(const Geo &g, const DiffSet<T> &s, double *part, unsigned *ctr, double *out, int nout,
+                            cudaStream_t st) {
+  int planes = 0;
+  for (int q = 0; q < 3; q++)
+    if (s.a[q] && s.nzp[q] > planes) planes = s.nzp[q];
+  const int need = (g.ny * planes + DF_W - 1) / DF_W, nb = need < 1 ? 1 : (need < DIFF_BLOCKS ? need : DIFF_BLOCKS);
+  k_diff_set<T><<<nb, DF_B, 0, st>>>(g, s, planes, part, ctr, out, nout);
   return cudaGetLastError();
 }
-cudaError_t launch_diff2(const Geo &g, const double *a, const double *b, int nzp, double *part,
-                         cudaStream_t st) {
-  return diff2(g, a, b, nzp, part, st);
-}
-cudaError_t launch_diff2(const Geo &g, const float *a, const float *b, int nzp, double *part,
-                         cudaStream_t st) {
-  return diff2(g, a, b, nzp, part, st);
-}
+template cudaError_t launch_diff_set<double>(const Geo &, const DiffSet<double> &, double *, unsigned *, double *, int,
+                                             cudaStream_t);
+template cudaError_t launch_diff_set<float>(const Geo &, const DiffSet<float> &, double *, unsigned *, double *, int,
+                                            cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // pressure.f90:16-56 get_source_pres on the full p-grid (zero outside the

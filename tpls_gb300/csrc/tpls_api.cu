@@ -338,6 +338,14 @@ static cudaError_t d2h_mu(tpls_ctx *c, double *host, const double *mu0) {
                            w, (size_t)(c->ny + 4) * (c->nz + 2), cudaMemcpyDefault, c->st);
 }
 
+// Partials of the reductions: one per block of the redistancing, of k_volume,
+// or three sums of launch_diff_set.
+static size_t part_values(const Geo &g) {
+  const size_t ls = ls_iter_blocks(g), vol = (size_t)((g.nx + 31) / 32) * ((g.ny + 3) / 4) * (g.nz + 1);
+  const size_t m = ls > vol ? ls : vol;
+  return m > 3 * DIFF_BLOCKS ? m : 3 * DIFF_BLOCKS;
+}
+
 static Phys phys_from(const tpls_params &p) {
   Phys ph;
   ph.dx = p.dx;
@@ -582,9 +590,7 @@ static int create_impl(int nx, int ny, int nz, const tpls_params *prm, const dou
     c->allocs.push_back(b);
     c->stage = (double *)b;
   }
-  c->part_len = (size_t)ls_iter_blocks(c->g);
-  size_t d2 = (size_t)diff2_blocks(c->g, nz + 1);
-  if (d2 > c->part_len) c->part_len = d2;
+  c->part_len = part_values(c->g);
   {
     void *b = nullptr;
     TCK(cudaMalloc(&b, sizeof(double) * (c->part_len + FS_TAIL)));
@@ -660,9 +666,7 @@ long long tpls_footprint_bytes(int nx, int ny, int nz, int precision) {
   g.sz = (int)(px * (ny + 2));
   g.sym = (int)px;
   g.szm = (int)(px * (ny + 4));
-  size_t part = (size_t)ls_iter_blocks(g);
-  const size_t d2 = (size_t)diff2_blocks(g, nz + 1);
-  if (d2 > part) part = d2;
+  const size_t part = part_values(g);
   t += round_alloc(D * (part + FS_TAIL)) + round_alloc(D * SC_N);
   const size_t oseg = (size_t)odd_chain_segments(g);  // odd half-sweep chain state
   t += round_alloc(sizeof(unsigned) * (4 + oseg)) + round_alloc(D * 32 * oseg);
@@ -1017,21 +1021,29 @@ static int mom32_begin(tpls_ctx *c, int comp) {
 }
 static int mom32_end(tpls_ctx *c, int comp, int N) {
   float **X = c->x3f[comp];
-  const int nzp = nz_planes(comp == 2 ? 2 : 1, c->nz);
   LCK(c, launch_defect_apply(mom32_base(c, comp) - XOFF, X[N % 2] - XOFF, c->x3[comp][0] - XOFF,
                              mom32_len(c, comp), c->st));
-  if (N >= 1) {
-    LCK(c, launch_diff2(c->g, X[N % 2], X[(N - 1) % 2], nzp, c->part, c->st));
-    FSUM(c, c->part, diff2_blocks(c->g, nzp), c->scal + SC_ERR_U + comp, c->st);
-  } else {
-    TCK(cudaMemsetAsync(c->scal + SC_ERR_U + comp, 0, sizeof(double), c->st));
-  }
   c->x3_final[comp] = 0;
   return TPLS_OK;
 }
 
 static int mom_iters(const tpls_ctx *c, int comp) {
   return (comp == 0 ? c->prm.mom_u : (comp == 1 ? c->prm.mom_v : c->prm.mom_w)) / 2;
+}
+// The logged get_difference of every component's last two iterates (0 for a
+// component without sweeps).
+template <typename T>
+static int mom_diff(tpls_ctx *c, T *const (&X)[3][2]) {
+  DiffSet<T> s;
+  for (int q = 0; q < 3; q++) {
+    const int N = mom_iters(c, q);
+    s.nzp[q] = nz_planes(q == 2 ? 2 : 1, c->nz);
+    if (N < 1) continue;
+    s.a[q] = X[q][N % 2];
+    s.b[q] = X[q][(N - 1) % 2];
+  }
+  LCK(c, launch_diff_set<T>(c->g, s, c->part, c->odd.ctr + 3, c->scal + SC_ERR_U, 3, c->st));
+  return TPLS_OK;
 }
 // The sweeps of the three components' Crank-Nicolson solves (main_ns_hybrid.
 // F90:756-887), which are independent of one another, in common launches:
@@ -1080,17 +1092,10 @@ static int momentum64(tpls_ctx *c) {
     const int N = mom_iters(c, q), nzp = nz_planes(q == 2 ? 2 : 1, c->nz);
     double **X = c->x3[q];
     c->x3_final[q] = N % 2;
-    if (N >= 1) {
-      // one sweep: the iterate before it is the start, which no launch wrote
-      if (N == 1) TCK(cudaMemsetAsync(X[0] - XOFF, 0, sizeof(double) * ((size_t)c->px * (c->ny + 2) * nzp + 8), c->st));
-      LCK(c, launch_diff2(c->g, X[N % 2], X[(N - 1) % 2], nzp, c->part, c->st));
-      FSUM(c, c->part, diff2_blocks(c->g, nzp), c->scal + SC_ERR_U + q, c->st);
-    } else {
-      TCK(cudaMemsetAsync(X[0] - XOFF, 0, sizeof(double) * ((size_t)c->px * (c->ny + 2) * nzp + 8), c->st));
-      TCK(cudaMemsetAsync(c->scal + SC_ERR_U + q, 0, sizeof(double), c->st));
-    }
+    // one sweep: the iterate before it is the start, which no launch wrote; none: the start is the result
+    if (N <= 1) TCK(cudaMemsetAsync(X[0] - XOFF, 0, sizeof(double) * ((size_t)c->px * (c->ny + 2) * nzp + 8), c->st));
   }
-  return TPLS_OK;
+  return mom_diff(c, c->x3);
 }
 }  // extern "C++"
 
@@ -1293,7 +1298,7 @@ static int sweeps32(tpls_ctx *c) {
   if ((s = momentum_sweeps<float, MuCoef>(c, coef, c->x3f))) return s;
   for (int q = 0; q < 3; q++)
     if ((s = mom32_end(c, q, mom_iters(c, q)))) return s;
-  return TPLS_OK;
+  return mom_diff(c, c->x3f);
 }
 
 // The FP32-mixed step in three stages: the front (viscosity, advection,
@@ -1809,6 +1814,7 @@ static int batch_capture(tpls_batch *b, int ph) {
       if (e != cudaSuccess) break;
       c->capturing = true;
       for (int comp = 0; comp < 3 && s == TPLS_OK; comp++) s = mom32_end(c, comp, mom_iters(c, comp));
+      if (s == TPLS_OK) s = mom_diff(c, c->x3f);
       if (s == TPLS_OK) s = mixed_back(c);
       c->capturing = false;
       if (s == TPLS_OK) e = cudaEventRecord(b->join[q], c->st);
@@ -2568,8 +2574,11 @@ int tpls_get_difference(tpls_ctx *c, const double *ua, const double *ub, const i
   double *UA, *UB;
   TCK(arg_in(c, true, ua, host_len(c, nzp), c->scr[0], &UA));
   TCK(arg_in(c, true, ub, host_len(c, nzp), c->scr[1], &UB));
-  LCK(c, launch_diff2(host_geo(c), UA, UB, nzp, c->part, c->st));
-  FSUM(c, c->part, diff2_blocks(c->g, nzp), c->scal + SC_ERR_U, c->st);
+  DiffSet<double> d;
+  d.a[0] = UA;
+  d.b[0] = UB;
+  d.nzp[0] = nzp;
+  LCK(c, launch_diff_set<double>(host_geo(c), d, c->part, c->odd.ctr + 3, c->scal + SC_ERR_U, 1, c->st));
   TCK(cudaMemcpyAsync(c->scal_host, c->scal, sizeof(double) * SC_N, cudaMemcpyDeviceToHost, c->st));
   TCK(cudaStreamSynchronize(c->st));
   *diff = c->scal_host[SC_ERR_U];

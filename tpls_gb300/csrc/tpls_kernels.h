@@ -143,7 +143,7 @@ struct SweepTiles {
 // of one row) a ready flag (epoch + 1) and the 32 values entering the
 // segment above it.  Zeroed at allocation.
 struct OddChain {
-  unsigned *ctr = nullptr;   // [0] tickets, [1] blocks done, [2] epoch
+  unsigned *ctr = nullptr;   // [0] tickets, [1] blocks done, [2] epoch; [3] launch_diff_set's counter
   unsigned *flag = nullptr;  // per segment
   double *incl = nullptr;    // per segment, 32 values
   double *kto = nullptr;     // waits that ran out (a context scalar)
@@ -235,11 +235,17 @@ cudaError_t launch_defect_apply(const double *X, const float *d, double *x, size
                                 cudaStream_t st);
 // One-time kernel attributes of the sweeps (dynamic shared memory).
 cudaError_t sweep_init();
-cudaError_t launch_diff2(const Geo &g, const double *a, const double *b,
-                         int nzp, double *part, cudaStream_t st);
-cudaError_t launch_diff2(const Geo &g, const float *a, const float *b,
-                         int nzp, double *part, cudaStream_t st);
-int diff2_blocks(const Geo &g, int nzp);
+// get_difference of up to three pairs (k_momentum.cu); part: 3 * DIFF_BLOCKS
+// doubles, ctr: a zeroed counter (left zero), out: the first nout sums.
+constexpr int DIFF_BLOCKS = 608;
+template <typename T>
+struct DiffSet {
+  const T *a[3] = {nullptr, nullptr, nullptr}, *b[3] = {nullptr, nullptr, nullptr};
+  int nzp[3] = {0, 0, 0};
+};
+template <typename T>
+cudaError_t launch_diff_set(const Geo &g, const DiffSet<T> &s, double *part, unsigned *ctr, double *out, int nout,
+                            cudaStream_t st);
 
 // pressure.f90
 cudaError_t launch_source(const Geo &g, const Phys &ph, const double *u3,
