@@ -129,14 +129,14 @@ def _algorithmic_bytes(nx, ny, nz, mom, esz=8):
     relaxed colour, that colour written).  FP32 sweeps (esz 4; x, mu and the
     defect b in FP32): Jacobi 16 B, half-sweep 12 B.  Returns (Jacobi bytes,
     odd half-sweep bytes, Jacobi launches, odd half-sweep launches) of one
-    step."""
+    step; a launch sweeps the three components."""
     pts = [(nx - 1) * ny * nz, nx * ny * nz, nx * ny * (nz - 1)]
     outer = mom // 2
     n_odd = (outer + 1) // 2  # outer iterations 1, 3, 5, ... use the odd sweep
     jac_pt, half_pt = (32.0, 28.0) if esz == 8 else (16.0, 12.0)
     jac = sum(jac_pt * p for p in pts) * outer
     sor_odd = sum(half_pt * p for p in pts) * 2 * n_odd
-    return jac, sor_odd, 3 * outer, 6 * n_odd
+    return jac, sor_odd, outer, 2 * n_odd
 
 
 def _profile_figure(tag: str, kernel: str, workload: str | None) -> dict | None:
@@ -270,8 +270,8 @@ def run_gpu(args, ws, rank, local) -> dict | None:
     # (k_sor_odd_c4), its launches timed with CUDA events on the library's
     # stream in the phase pass
     sor_ms, sor_l = phases["sor_odd"]
-    # (one block per 64-level segment for columns of 3 or more segments)
-    dominant = "k_sor_odd_seg" if (not args.odd_columns and (nz - 1) // 64 + 1 >= 3) else "k_sor_odd_c4"
+    # (one block per 64-level segment for columns of 3 or more segments, of 2 in FP32)
+    dominant = "k_sor_odd_seg" if (not args.odd_columns and (nz - 1) // 64 + 1 >= (3 if esz == 8 else 2)) else "k_sor_odd_c4"
     per_launch_b = sor_b / sor_n
     avg_ms = sor_ms / max(sor_l, 1)
     achieved = per_launch_b / (avg_ms / 1e3) / 1e9

@@ -1,7 +1,7 @@
 // k_advect.cu -- level-set advection: WENO5 face values and the
 // conservative flux divergence (advect_phi.f90:19-119, weno.f90:18-215).
 //
-// One thread per (i,j) column of p-cells, marching a chunk of 16 z levels
+// One thread per (i,j) column of p-cells, marching a chunk of z levels
 // (one z-face below the chunk is computed at its start).  Each face value
 // is computed once: the x-face left of a thread is its left neighbour's
 // right face and the y-face below is the lower row's upper face, both
@@ -148,7 +148,7 @@ constexpr int ADV_BX = 32, ADV_BY = 8;
 // 128x64x96, 1786 -> 1700 at 256x128x192.
 constexpr int ADV_KC = 16;
 
-// One block covers 32 x 8 columns and a chunk of ADV_KC levels.  At each
+// One block covers 32 x 8 columns and a chunk of kc levels.  At each
 // level every thread computes the x-face right of its cell and the y-face
 // above it; the faces left of the block's first column (8, one per row) are
 // computed by eight lanes of warp 1 and those below its first row (32) by

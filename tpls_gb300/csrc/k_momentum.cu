@@ -13,8 +13,8 @@
 // checkerboard mod(k+j+flg,2), every point of a colour is independent and
 // one thread updates one point.  For an odd iteration_time the colouring is
 // mod(j+flg,2) in every plane, so the reference's sequential loop lets a
-// point see the already-relaxed point below it: one thread marches each
-// (i,j) column upward, carrying the relaxed value in a register.
+// point see the already-relaxed point below it: a recurrence up each column,
+// run in chunks (k_sweep.cu).
 // Periodic ghost rows are written by the thread that writes the row they
 // copy (legal for even ny: no point of the colour being relaxed reads a
 // ghost row written in the same half-sweep); for odd ny the caller runs a

@@ -18,12 +18,16 @@
 // Solver: CG preconditioned by one symmetric multigrid V-cycle.
 //   levels: cell-centred coarsening of every dimension that is even and
 //           >= 4 (y >= 4), down to <= 512 cells or no coarsenable dimension;
-//   smoother: damped z-line Jacobi (one tridiagonal solve per (x,y) column
-//           with precomputed Thomas factors -- the operator's z couplings
-//           are (dx/dz)^2 times stronger than x/y on the channel grids);
+//   smoother: red-black Gauss-Seidel (red, black before the coarse correction,
+//           black, red after it) on near-isotropic levels of even y extent,
+//           damped z-line Jacobi (precomputed Thomas factors) on the others;
+//           levels that halve in all axes, or (FP64) in x and y, run the
+//           kernels of tpls_mg.cuh;
 //   transfer: trilinear prolongation P, restriction R = P^T / 2^d;
 //   coarse operator: rediscretisation; coarsest grid: dense FP64
-//           pseudo-inverse built from the separable eigen-decomposition.
+//           pseudo-inverse built from the separable eigen-decomposition up to
+//           512 cells, else forty smoothing sweeps (FP64: by modes,
+//           tpls_modes.cuh).
 // All reductions are deterministic (per-block partials summed in a fixed
 // order), so a solve's iterates do not depend on timing.
 #include <math.h>

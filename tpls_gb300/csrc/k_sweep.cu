@@ -6,7 +6,7 @@
 // k_mom_rhs writes, once per timestep, one record per point of a velocity
 // component: the six neighbour coefficients and rhs/diag, already divided
 // by the Helmholtz diagonal, and the odd half-sweep's factor 1.2 czm (see
-// write_coef in k_momentum.cu).  A sweep
+// mom_column in k_momentum.cu).  A sweep
 // point is then x_new = sum(c_n x_n) + b: seven FMAs instead of the face
 // averages, diagonal and division of the reference's form, evaluated once
 // per step instead of once per sweep: on GB300's FP64 pipe the 64-byte
@@ -14,8 +14,8 @@
 // FP32-mixed form take the other side: FP32 arithmetic is 64x faster, so
 // they recompute the coefficients per point from the FP32 viscosity and read
 // only b (4 bytes), cutting a Jacobi point from ~40 to ~16 bytes of traffic.
-// Templated on the arithmetic type and the coefficient source (records, or
-// MuCoef).
+// Templated on the arithmetic type and the coefficient source (records,
+// MuCoef, or for the per-routine odd half-sweep RefCoef).
 #include <type_traits>
 #include "tpls_sweep.cuh"
 
