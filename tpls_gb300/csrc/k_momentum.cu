@@ -853,8 +853,10 @@ RefCoef ref_coef(int comp, const Phys &ph, const double *rhs, const double *mu) 
 // block, summed by the last block in a fixed order.  (A launch and one or two
 // more for the sum per component took 75 us of a step at 128x64x96, 30 at
 // 64x32x48; this 23 and 13.)  FP64 iterates are differenced and
-// summed in FP64; FP32 iterates in FP32 up to the sums of a warp's 32 points
-// (exactly widened), so the FP32 form issues one FP64 instruction per 32 points.
+// summed in FP64; FP32 iterates are differenced in FP32 and each thread sums
+// its squares as an FP32 pair (error-free sums), widened at the end: no FP64
+// instruction per point (with a warp's FP32 sum widened per 32 points 450 us at
+// 512x256x256, 200 with pairs).
 constexpr int DF_B = 256, DF_W = DF_B / 32;
 template <typename T>
 __global__ void __launch_bounds__(DF_B)
@@ -864,6 +866,7 @@ __global__ void __launch_bounds__(DF_B)
   __shared__ bool last;
   const int t = threadIdx.x, lane = t & 31, nb = gridDim.x;
   double acc[3] = {0.0, 0.0, 0.0};
+  float hi[3] = {0.0f, 0.0f, 0.0f}, lo[3] = {0.0f, 0.0f, 0.0f};
   for (int row = blockIdx.x * DF_W + (t >> 5); row < g.ny * planes; row += nb * DF_W) {
     const int k = row / g.ny, c0 = TPLS_IDX(g, 1, row - g.ny * k + 1, k);
 #pragma unroll
@@ -871,22 +874,23 @@ __global__ void __launch_bounds__(DF_B)
       if (!s.a[q] || k >= s.nzp[q]) continue;
       const T *a = s.a[q] + c0, *b = s.b[q] + c0;
 #pragma unroll 4
-      for (int i = lane; i < ((g.nx + 31) & ~31); i += 32) {
-        T d = (T)0;
-        if (i < g.nx) d = a[i] - b[i];
+      for (int i = lane; i < g.nx; i += 32) {
+        const T d = a[i] - b[i];
         if constexpr (sizeof(T) == sizeof(float)) {
-          float e = d * d;
-          for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-          acc[q] += widen_bits(e);
+          const float e = __fmul_rn(d, d), s1 = hi[q] + e, z = s1 - hi[q];  // hi + e = s1 + its rounding
+          lo[q] += (hi[q] - (s1 - z)) + (e - z);
+          hi[q] = s1;
         } else {
           acc[q] = fma(d, d, acc[q]);
         }
       }
     }
   }
-  // the block's sums: FP64 lane by lane over the warps, then one warp's tree;
-  // FP32 (every lane holds the warp's sum) over the warps
-  auto block = [&](double (&v)[3], bool lanes) {  // in lane 0 of warp 0
+  if constexpr (sizeof(T) == sizeof(float))
+    for (int q = 0; q < 3; q++) acc[q] = widen_bits(hi[q]) + widen_bits(lo[q]);
+  // the block's sums, in lane 0 of warp 0: lane by lane over the warps, then one
+  // warp's tree
+  auto block = [&](double (&v)[3]) {
     __syncthreads();
     for (int q = 0; q < 3; q++) sh[q][t] = v[q];
     __syncthreads();
@@ -894,12 +898,11 @@ __global__ void __launch_bounds__(DF_B)
       for (int q = 0; q < 3; q++) {
         double x = sh[q][t];
         for (int w = 1; w < DF_W; w++) x += sh[q][t + 32 * w];
-        if (lanes)
-          for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
         v[q] = x;
       }
   };
-  block(acc, sizeof(T) == sizeof(double));
+  block(acc);
   if (t == 0) {
     for (int q = 0; q < 3; q++) part[q * nb + blockIdx.x] = acc[q];
     __threadfence();
@@ -912,7 +915,7 @@ __global__ void __launch_bounds__(DF_B)
     acc[q] = 0.0;
     for (int b = t; b < nb; b += DF_B) acc[q] += __ldcg(part + q * nb + b);
   }
-  block(acc, true);
+  block(acc);
   if (t == 0) {
     for (int q = 0; q < nout; q++) out[q] = acc[q];
     *ctr = 0u;
