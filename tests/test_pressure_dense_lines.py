@@ -4,8 +4,8 @@
 CPU: the folded matrices (even and odd part about the line's middle, one
 matrix for the sine and cosine modes of a wavenumber), indexed as the kernels
 do, give what the sweeps along the line give.  GPU: solves on grids of one
-level with lines of up to 64 points, and just above, against the oracle's exact
-solve."""
+level with lines of up to 64 points, and just above or with more matrices than
+the limit, against the oracle's exact solve."""
 import numpy as np
 import pytest
 
@@ -70,7 +70,8 @@ def test_folded_matrices_equal_the_sweeps(nx):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("size", [(5, 9, 23), (33, 7, 11), (63, 5, 9), (65, 5, 9), (25, 25, 75)])
+@pytest.mark.parametrize("size", [(5, 9, 23), (33, 7, 11), (63, 5, 9), (65, 5, 9), (25, 25, 75), (63, 35, 75),
+                                  (31, 69, 121)])
 def test_solves_match_the_oracle(size):
     """Converged to 1e-13 on both sides; the tolerance is the per-routine
     parity tests' 1e-11 of the maximum."""

@@ -504,7 +504,10 @@ __global__ void __launch_bounds__(LJB)
 // assemble the line right-hand sides into shared memory, one warp runs the
 // Thomas forward/backward substitution in shared memory, all threads write
 // the damped result.  Dynamic shared memory: nz * 32 values of float.
-constexpr int LJ2_T = 256;
+// 1024 threads: a level has few blocks (20 at 25x25x75), and with 256 each
+// thread assembled and wrote its ten levels one load after another (875 launches
+// of a solve's V-cycles at 100x50x75 8.4 -> 7.1 ms, at 145x70x99 21.7 -> 18.3).
+constexpr int LJ2_T = 1024;
 
 __global__ void __launch_bounds__(LJ2_T)
     k_line_jacobi2(LevArgs<float> L, float omega, float one_m_omega, int zero_init, const float *__restrict__ thomas,

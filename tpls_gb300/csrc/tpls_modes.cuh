@@ -138,13 +138,16 @@ __device__ __forceinline__ void line_sweeps(const ModeSweeps &M, const ModePoint
 // two matrices of half the order.  D[class][mz][j][i] = (even, odd), i
 // consecutive, half = (nx+1)/2 of each; the sine and cosine modes of y share
 // theirs (class = (my+1)/2).  Up to 64 points because half a line then fits a
-// warp; the matrices of the largest such level (lines of 63, 69 rows, 141
-// planes) take 78 MB and 3.5 ms to build, those of 25x25x75 3.4 MB and 0.15 ms.
+// warp, and up to 16 MB of matrices: those of 25x25x75 take 2.6 MB and 0.15 ms to
+// build, those of 63x69x141 would take 83 MB and 3.5 ms for 0.1 ms less per cycle.
 constexpr int DENSE_NX = 64;
 __host__ __device__ inline int mode_classes(int ny) { return ny / 2 + 1; }
 inline size_t dense_values(int nx, int ny, int nz) {
   const size_t half = (nx + 1) / 2;
   return 2 * half * half * (size_t)mode_classes(ny) * nz;
+}
+inline bool dense_pays(int nx, int ny, int nz) {
+  return nx <= DENSE_NX && dense_values(nx, ny, nz) * sizeof(double) <= (size_t)16 << 20;
 }
 
 // A column j of the matrices: the sweeps of the unit pair at j and nx-1-j, on
@@ -257,7 +260,7 @@ __global__ void __launch_bounds__(32 * MODE_W)
 }
 
 // y modes of the z-transformed right-hand side and all sweeps of their x
-// lines, of more than DENSE_NX points: a warp per line, PPL consecutive x
+// lines, where dense_pays says no: a warp per line, PPL consecutive x
 // points per lane.
 template <int PPL>
 __global__ void __launch_bounds__(32 * MODE_W)
