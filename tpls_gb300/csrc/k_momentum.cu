@@ -188,7 +188,7 @@ cudaError_t launch_mom_rhs64r32(int comp, const Geo &g, const Phys &ph, const do
 
 // ---------------------------------------------------------------------------
 // FP64 right-hand sides and sweep records (the FP64 form).  Bound by the FP64
-// pipe, so written for few operations (73 per point against 105 in the point
+// pipe, so written for few operations (74 per point against 105 in the point
 // form above):
 //   * a thread marches kc levels of a column: the z faces' viscosity sums,
 //     shear and difference products of a level's upper face are the next
@@ -196,8 +196,12 @@ cudaError_t launch_mom_rhs64r32(int comp, const Geo &g, const Phys &ph, const do
 //   * conv and diff share the normal stress p dE - m dW of the component's own
 //     axis; every axis' scales (1/2 of the centred difference, 1/4 of a
 //     four-cell average, the grid spacings) are one factor;
-//   * the AB3 and Crank-Nicolson combination is seven FMAs on factors that
-//     carry dt; 1/diag comes from rcp_seed and one Newton step.
+//   * the AB3 and Crank-Nicolson combination is a product and six FMAs on
+//     factors that carry dt, then the sum with the state: begun from the state,
+//     it is rounded seven times at the state's size (3012 us at 256x128x192, 3044
+//     so); 1/diag comes from rcp_seed and one Newton step.
+// No output is further from a long-double evaluation than with the point form
+// (conv 0.70-0.95 of its RMS error, diff 0.99-1.00, the step's u3, v3, w3 0.73-0.99).
 // All three components in one launch (gx blocks along x each).
 //
 // The record of one point (8 doubles): the neighbour coefficients divided by
@@ -280,7 +284,8 @@ __device__ __forceinline__ void mom_column(const Geo &g, const MomArgs &A, int i
       const double near = mn + mf;  // the two cells of this point's own face
       double mn1 = 0.0, mf1 = 0.0;
       MomFace hi;
-      double xt = 0.0, dT, dB2, ws1 = 0.0;  // dB2: the centred difference's lower half
+      // dT: the component's difference over the upper face, dsh: the shear's; dB2: the centred difference's lower half
+      double xt = 0.0, dT, dB2, dsh = 0.0, ws1 = 0.0;
       if (CC == 2) {
         hi.m = mf;  // mu of level k+1
         xt = S[c + sz];
@@ -303,7 +308,8 @@ __device__ __forceinline__ void mom_column(const Geo &g, const MomArgs &A, int i
         hi.m = near + (mn1 + mf1);
         const double w0 = W[c + sz], w1 = W[c + sz + oq];
         ws1 = w0 + w1;
-        hi.sh = hi.m * (CC == 0 ? w1 - w0 : w0 - w1);
+        dsh = CC == 0 ? w1 - w0 : w0 - w1;
+        hi.sh = hi.m * dsh;
         pz = hi.m;
         mzv = lo.m;
         if (CC == 0) {
@@ -329,11 +335,12 @@ __device__ __forceinline__ void mom_column(const Geo &g, const MomArgs &A, int i
         xt = S[c + sz];
         dT = xt - x;
         hi.own = hi.m * dT;
-        lo.own = lo.m * fma(-1.0 / 3.0, xt, 3.0 * x);
+        lo.own = lo.m * (x - fma(1.0 / 3.0, xt, -2.0 * x));
         dz = x + xt;
       } else if (k == nz - 1) {
         const double xb = S[c - sz];
-        hi.own = hi.m * fma(1.0 / 3.0, xb, -3.0 * x);
+        dT = fma(1.0 / 3.0, xb, -2.0 * x) - x;
+        hi.own = hi.m * dT;
         dz = -(x + xb);
       } else {
         xt = S[c + sz];
@@ -366,24 +373,15 @@ __device__ __forceinline__ void mom_column(const Geo &g, const MomArgs &A, int i
         shx = fma(px, b1 - b0, -mx * (a1 - a0));
         shy = fma(py, e1 - e0, -myv * (d1 - d0));
       }
-      const double nx_ = fma(px, dE, -mx * dW), ny_ = fma(py, dN, -myv * dS), nz_ = hi.own - lo.own;
-      conv = q.vx * ((xe - xw) * vx);
-      conv = fma(q.vy, (xn - xs) * vy, conv);
+      const double nx_ = fma(px, dE, -mx * dW), ny_ = fma(py, dN, -myv * dS), nz_ = fma(hi.m, dT, -lo.own);
+      // shear of conv (the component's own axis shares diff's normal stress), then its convective terms, the streamwise
+      // one last: the sum is rounded at its full size once
+      conv = -q.tx * (CC == 0 ? nx_ : shx);
+      conv = fma(-q.ty, CC == 1 ? ny_ : shy, conv);
+      conv = fma(-q.tz, CC == 2 ? nz_ : fma(hi.m, dsh, -lo.sh), conv);
       conv = fma(q.vz, dz * vz, conv);
-      // shear of conv: the component's own axis shares diff's normal stress
-      if (CC == 0) {
-        conv = fma(-q.tx, nx_, conv);
-        conv = fma(-q.ty, shy, conv);
-        conv = fma(-q.tz, hi.sh - lo.sh, conv);
-      } else if (CC == 1) {
-        conv = fma(-q.tx, shx, conv);
-        conv = fma(-q.ty, ny_, conv);
-        conv = fma(-q.tz, hi.sh - lo.sh, conv);
-      } else {
-        conv = fma(-q.tx, shx, conv);
-        conv = fma(-q.ty, shy, conv);
-        conv = fma(-q.tz, nz_, conv);
-      }
+      conv = fma(q.vy, (xn - xs) * vy, conv);
+      conv = fma(q.vx, (xe - xw) * vx, conv);
       diff = q.lx * nx_;
       diff = fma(q.ly, ny_, diff);
       diff = fma(q.lz, nz_, diff);
@@ -412,13 +410,13 @@ __device__ __forceinline__ void mom_column(const Geo &g, const MomArgs &A, int i
     csf2[c] = s2;
     if (valid) {
       // main_ns_hybrid.F90:743-751 (AB3 convection and CSF, CN diffusion)
-      double r = fma(q.k2, conv, xc);
+      double r = q.k2 * conv;
       r = fma(q.k1, c1[c], r);
       r = fma(q.k0, c0[c], r);
       r = fma(q.hd, diff, r);
       r = fma(q.l2, s2, r);
       r = fma(q.l1, s1[c], r);
-      r = fma(q.l0, s0[c], r);
+      r = fma(q.l0, s0[c], r) + xc;
       // the own axis' two faces are the two cells `near` sums (u: px + mx, v: py + my, w: pz + mz)
       double d = fma(q.ax, CC == 0 ? sx : px + mx, 1.0);
       d = fma(q.ay, CC == 1 ? sx : py + myv, d);
@@ -741,8 +739,10 @@ cudaError_t launch_mom_rhs_pair(const Geo &g, const Phys &ph, const double *u2, 
 
 // jacobi_iteration_allflux.f90:21-282 with the routine's own boundary rows
 // (v, w): the per-routine entry.  A thread marches kc levels of a column.
-// 146 us per component at 192x96x144 (28 FP64 operations per point; the point
-// form with averages and a division 197).
+// 149 us per component at 192x96x144 (29 FP64 operations per point; the point
+// form with averages and a division 197).  The right-hand side is added last
+// and the quotient rounded once, as in that form, whose error this has: as a
+// product with 1/diag, begun from the right-hand side, 146 us and 1.1 times it.
 template <int CC>
 __global__ void __launch_bounds__(MB_X *MB_Y)
     k_ref_jacobi(Geo g, RefCoef s, const double *__restrict__ xo, double *__restrict__ x, int kc) {
@@ -757,8 +757,8 @@ __global__ void __launch_bounds__(MB_X *MB_Y)
   ref_begin<CC>(g, m, near, lo);
   double xc = xo[c], zm = (CC == 2 || ka > 0) ? xo[c - sz] : 0.0;
   for (int k = ka; k < kb; k++) {
-    double hi, near1, h;
-    double t = ref_point<CC>(g, s, m, near, lo, s.rhs[c], xo[c + 1], xo[c - 1], xo[c + sy], xo[c - sy], hi, near1, h);
+    double hi, near1, d;
+    double t = ref_point<CC, false>(g, s, m, near, lo, 0.0, xo[c + 1], xo[c - 1], xo[c + sy], xo[c - sy], hi, near1, d);
     double zp = 0.0;
     if (CC == 2 || k < nz - 1) zp = xo[c + sz];
     // the no-slip ghost values below k = 0 and above k = nz-1 (jacobi_iteration_allflux.f90:63-73)
@@ -766,7 +766,7 @@ __global__ void __launch_bounds__(MB_X *MB_Y)
     if (CC != 2 && k == 0) zb = fma(zp, 1.0 / 3.0, -2.0 * xc);
     if (CC != 2 && k == nz - 1) zt = fma(zm, 1.0 / 3.0, -2.0 * xc);
     t = fma(s.cz, fma(hi, zt, lo * zb), t);
-    const double v = t * h;
+    const double v = div_inf(t + s.rhs[c], d);
     x[c] = v;
     if (CC == 1) {  // jacobi_iteration_allflux.f90:178-189
       if (i == 1) x[c - 1] = v;
@@ -805,8 +805,8 @@ cudaError_t launch_ref_jacobi(int comp, const Geo &g, const RefCoef &s, const do
 }
 
 // sor_iteration_allflux.f90:54-99 (and v, w): 3-D checkerboard half-sweep of
-// the per-routine entry.  79 us per component at 192x96x144 (with averages and
-// a division 105).
+// the per-routine entry, its quotient as the Jacobi point's.  84 us per
+// component at 192x96x144 (with averages and a division 105).
 template <int CC>
 __global__ void __launch_bounds__(MB_X *MB_Y)
     k_ref_even(Geo g, RefCoef s, double *__restrict__ x, int flg) {
@@ -816,9 +816,9 @@ __global__ void __launch_bounds__(MB_X *MB_Y)
   if (i > iend || j > g.ny) return;
   const int sy = g.sy, sz = g.sz, c = TPLS_IDX(g, i, j, k);
   const double *m = ref_cell<CC>(g, s, i, j, k);
-  double near, lo, hi, near1, h;
+  double near, lo, hi, near1, d;
   ref_begin<CC>(g, m, near, lo);
-  double t = ref_point<CC>(g, s, m, near, lo, s.rhs[c], x[c + 1], x[c - 1], x[c + sy], x[c - sy], hi, near1, h);
+  double t = ref_point<CC, false>(g, s, m, near, lo, 0.0, x[c + 1], x[c - 1], x[c + sy], x[c - sy], hi, near1, d);
   const double xc = x[c];
   double zp, zm;
   if (CC == 2) {
@@ -828,8 +828,8 @@ __global__ void __launch_bounds__(MB_X *MB_Y)
     zp = (k < nz - 1) ? x[c + sz] : fma(x[c - sz], 1.0 / 3.0, -2.0 * xc);
     zm = (k > 0) ? x[c - sz] : fma(zp, 1.0 / 3.0, -2.0 * xc);
   }
-  t = fma(s.cz, fma(hi, zp, lo * zm), t);
-  x[c] = fma(1.2, fma(t, h, -xc), xc);
+  t = fma(s.cz, fma(hi, zp, lo * zm), t) + s.rhs[c];
+  x[c] = fma(1.2, div_inf(t, d) - xc, xc);
 }
 
 cudaError_t launch_ref_even(int comp, const Geo &g, const RefCoef &s, double *x, int flg, cudaStream_t st) {

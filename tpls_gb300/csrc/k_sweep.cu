@@ -89,7 +89,8 @@ __device__ __forceinline__ void ref_odd(const Geo &g, const RefCoef &s, const do
                                         const double *m, int c, int k, int k0, double xc, double zp, double near,
                                         double lo, double &near1, double &hi, double &A, double &B) {
   double h;
-  double t = ref_point<CC>(g, s, m, near, lo, s.rhs[c], x[c + 1], x[c - 1], x[c + g.sy], x[c - g.sy], hi, near1, h);
+  double t =
+      ref_point<CC, true>(g, s, m, near, lo, s.rhs[c], x[c + 1], x[c - 1], x[c + g.sy], x[c - g.sy], hi, near1, h);
   double below = lo;  // weight of the point below
   double zt = zp;
   if (CC != 2 && k == g.nz - 1) {  // ghost -2 x + x(k-1)/3 above

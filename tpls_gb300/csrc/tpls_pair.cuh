@@ -95,6 +95,14 @@ __device__ __forceinline__ double div_fast(double n, double d) {
   return fma(fma(-d, q, n), r, q);
 }
 
+// The same for any numerator: an infinite quotient is not corrected (its
+// remainder would be NaN).
+__device__ __forceinline__ double div_inf(double n, double d) {
+  if (!rcp_range(d)) return div_slow(n, d);
+  const double r = rcp_seed(d), q = n * r, v = fma(fma(-d, q, n), r, q);
+  return (__double2hiint(q) & 0x7ff00000) == 0x7ff00000 ? q : v;
+}
+
 // sqrt(a), correctly rounded, with one FP64 operation: an FP32 pair (sh, sl)
 // of the root to about 2^-43, joined to a double s0 by integer addition; the
 // exact residual a - s0^2 by one FMA; the correction c = residual / (2 s0) in

@@ -65,11 +65,12 @@ __device__ __forceinline__ FcT<T> faces(int comp, const Geo &g, const T *__restr
 // the pair of cells of the point's own face (`near`) and the neighbouring
 // pairs, the averages' quarter in the axis factor; the level's upper z face and
 // the next level's own pair are handed on, so that a thread marching up a
-// column forms each once; 1/diag from rcp_seed and one Newton step.
+// column forms each once.
 // m: viscosity cell of the point (u, v: level k+1 of the p-grid; w: k); near =
 // m[0] + m[om] and lo (the lower z face) in; hi (the upper z face), near1 (near
-// of the level above) and h = 1/diag out.  Returns the right-hand side with
-// the x and y terms, to which the caller adds cz (hi zp + lo zm).
+// of the level above) and q out, the diagonal (RCP: its reciprocal, from rcp_seed
+// and one Newton step).  Returns rhs with the x and y terms, to which the caller
+// adds cz (hi zp + lo zm).
 template <int CC>
 __device__ __forceinline__ int ref_om(const Geo &g) {  // the far cell of a point's own face
   return CC == 0 ? 1 : (CC == 1 ? -g.sym : g.szm);
@@ -84,10 +85,10 @@ __device__ __forceinline__ void ref_begin(const Geo &g, const double *m, double 
   near = m[0] + m[om];
   lo = (CC == 2) ? m[0] : near + (m[-g.szm] + m[-g.szm + om]);
 }
-template <int CC>
+template <int CC, bool RCP>
 __device__ __forceinline__ double ref_point(const Geo &g, const RefCoef &s, const double *m, double near, double lo,
                                             double rhs, double xp, double xm, double yp, double ym, double &hi,
-                                            double &near1, double &h) {
+                                            double &near1, double &q) {
   const int om = ref_om<CC>(g), my = g.sym, mz = g.szm;
   auto pair = [&](int o) { return m[o] + m[o + om]; };
   const double fxp = (CC == 0) ? m[1] : near + pair(1), fxm = (CC == 0) ? m[0] : near + pair(-1);
@@ -97,11 +98,14 @@ __device__ __forceinline__ double ref_point(const Geo &g, const RefCoef &s, cons
   double d = fma(s.cx, CC == 0 ? near : fxp + fxm, 1.0);
   d = fma(s.cy, CC == 1 ? near : fyp + fym, d);
   d = fma(s.cz, CC == 2 ? near : hi + lo, d);
-  if (rcp_range(d)) {
-    h = rcp_seed(d);
-    h = fma(h, fma(-d, h, 1.0), h);
-  } else {
-    h = div_slow(1.0, d);
+  q = d;
+  if constexpr (RCP) {
+    if (rcp_range(d)) {
+      q = rcp_seed(d);
+      q = fma(q, fma(-d, q, 1.0), q);
+    } else {
+      q = div_slow(1.0, d);
+    }
   }
   const double t = fma(s.cx, fma(fxp, xp, fxm * xm), rhs);
   return fma(s.cy, fma(fyp, yp, fym * ym), t);
