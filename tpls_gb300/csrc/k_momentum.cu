@@ -858,6 +858,21 @@ RefCoef ref_coef(int comp, const Phys &ph, const double *rhs, const double *mu) 
 // instruction per point (with a warp's FP32 sum widened per 32 points 450 us at
 // 512x256x256, 200 with pairs).
 constexpr int DF_B = 256, DF_W = DF_B / 32;
+// A thread's squares of one pair summed in FP64, where their FP32 sum is not
+// finite (it overflowed, or a square is infinite or NaN: the pair's rounding is
+// NaN then).  Out of the loop, in which a test per square doubled the time.
+static __device__ __noinline__ double wide_squares(const Geo &g, const float *__restrict__ x,
+                                                   const float *__restrict__ y, int nzp) {
+  double s = 0.0;
+  for (int row = blockIdx.x * DF_W + (threadIdx.x >> 5); row < g.ny * nzp; row += gridDim.x * DF_W) {
+    const int k = row / g.ny, c0 = TPLS_IDX(g, 1, row - g.ny * k + 1, k);
+    for (int i = threadIdx.x & 31; i < g.nx; i += 32) {
+      const float d = x[c0 + i] - y[c0 + i];
+      s += widen_bits(__fmul_rn(d, d));
+    }
+  }
+  return s;
+}
 template <typename T>
 __global__ void __launch_bounds__(DF_B)
     k_diff_set(Geo g, const __grid_constant__ DiffSet<T> s, int planes, double *__restrict__ part, unsigned *ctr,
@@ -887,7 +902,9 @@ __global__ void __launch_bounds__(DF_B)
     }
   }
   if constexpr (sizeof(T) == sizeof(float))
-    for (int q = 0; q < 3; q++) acc[q] = widen_bits(hi[q]) + widen_bits(lo[q]);
+    for (int q = 0; q < 3; q++)
+      acc[q] = hi[q] <= 0x1.fffffep127f ? widen_bits(hi[q]) + widen_bits(lo[q])
+                                        : wide_squares(g, s.a[q], s.b[q], s.nzp[q]);
   // the block's sums, in lane 0 of warp 0: lane by lane over the warps, then one
   // warp's tree
   auto block = [&](double (&v)[3]) {
