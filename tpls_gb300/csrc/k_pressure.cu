@@ -66,7 +66,7 @@ struct PoissonSolver {
   double *cinv = nullptr;  // coarsest pseudo-inverse (nc x nc), or null
   int coarse_sweeps = 0;
   double *modes = nullptr;  // coarsest level by modes: Qz, Qy, lambda_z, lambda_y
-  double *dense = nullptr;  // and the matrices of its lines (dense_values), rows of up to DENSE_NX points
+  double *dense = nullptr;  // and the matrices of its lines (dense_values), where dense_pays
   double *x = nullptr, *r = nullptr, *p = nullptr, *q = nullptr, *bvec = nullptr;
   void *z = nullptr;           // preconditioned residual, in the level type
   float *r32 = nullptr;        // FP32 levels: r rounded once, for the V-cycle
@@ -1034,7 +1034,7 @@ cudaError_t poisson_create(const Geo &g, double cx, double cy, double cz, int fp
       Qz.insert(Qz.end(), ly.begin(), ly.end());
       PCK(cudaMalloc(&S->modes, Qz.size() * sizeof(double)));
       PCK(cudaMemcpy(S->modes, Qz.data(), Qz.size() * sizeof(double), cudaMemcpyHostToDevice));
-      if (C.nx <= DENSE_NX) {
+      if (dense_pays(C.nx)) {
         const ModeSweeps M = mode_sweeps(S, C);
         const double *lzd = S->modes + (size_t)C.nz * C.nz + (size_t)C.ny * C.ny;
         PCK(cudaMalloc(&S->dense, sizeof(double) * dense_values(C.nx, C.ny, C.nz)));
@@ -1126,7 +1126,7 @@ size_t poisson_footprint(const Geo &g, int fp32, size_t (*rnd)(size_t)) {
     if (!cx && !cy && !cz) {
       if (!fp32 && modes_pay(nx, ny, nz)) {
         tot += rnd(sizeof(double) * ((size_t)nz * nz + (size_t)ny * ny + nz + ny));
-        if (nx <= DENSE_NX) tot += rnd(sizeof(double) * dense_values(nx, ny, nz));
+        if (dense_pays(nx)) tot += rnd(sizeof(double) * dense_values(nx, ny, nz));
       }
       break;
     }

@@ -138,17 +138,19 @@ __device__ __forceinline__ void line_sweeps(const ModeSweeps &M, const ModePoint
 // two matrices of half the order.  D[class][mz][j][i] = (even, odd), i
 // consecutive, half = (nx+1)/2 of each; the sine and cosine modes of y share
 // theirs (class = (my+1)/2).  Up to 64 points because half a line then fits a
-// warp, and up to 16 MB of matrices: those of 25x25x75 take 2.6 MB and 0.15 ms to
-// build, those of 63x69x141 would take 83 MB and 3.5 ms for 0.1 ms less per cycle.
+// warp.  No limit on their size beyond modes_pay's on the level (81 MB at
+// 63x69x141, a seventh of the context): building them is repaid within two steps
+// at every size.  Without / with them, creation and one step: 63x35x75 (22 MB)
+// 2.4 / 3.4 and 3.33 / 2.79 ms; 47x45x121 (26 MB) 2.6 / 4.1 and 7.60 / 5.99 ms;
+// 31x69x121 (17 MB) 2.6 / 3.5 and 6.79 / 5.74 ms; 63x69x141 2.7 / 6.1 and 18.2 /
+// 15.3 ms.
 constexpr int DENSE_NX = 64;
 __host__ __device__ inline int mode_classes(int ny) { return ny / 2 + 1; }
 inline size_t dense_values(int nx, int ny, int nz) {
   const size_t half = (nx + 1) / 2;
   return 2 * half * half * (size_t)mode_classes(ny) * nz;
 }
-inline bool dense_pays(int nx, int ny, int nz) {
-  return nx <= DENSE_NX && dense_values(nx, ny, nz) * sizeof(double) <= (size_t)16 << 20;
-}
+inline bool dense_pays(int nx) { return nx <= DENSE_NX; }
 
 // A column j of the matrices: the sweeps of the unit pair at j and nx-1-j, on
 // half the line (its other half is plus or minus the mirror image), a point
@@ -260,7 +262,7 @@ __global__ void __launch_bounds__(32 * MODE_W)
 }
 
 // y modes of the z-transformed right-hand side and all sweeps of their x
-// lines, where dense_pays says no: a warp per line, PPL consecutive x
+// lines, of more than DENSE_NX points: a warp per line, PPL consecutive x
 // points per lane.
 template <int PPL>
 __global__ void __launch_bounds__(32 * MODE_W)
