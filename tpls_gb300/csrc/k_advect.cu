@@ -74,7 +74,7 @@ __device__ __forceinline__ T weno_up(bool pos, T m2, T m1, T c0, T p1, T p2, T p
 // 40 operations with the quotient of div_fast against 57 with the form above,
 // and smaller roundings (the correction is a small part of v3).
 struct Weno {
-  double d1, d2, d3, d4, s1, s2, s3;
+  double d2, d3, s1, s2, s3;
 };
 __device__ __forceinline__ double weno_ratio(const Weno &w, double e1, double e2, double e3) {
   // e_m = s_m^2 + 12/13 eps
@@ -92,13 +92,11 @@ __device__ __forceinline__ double weno_up64(bool pos, double m2, double m1, doub
                                             double p3) {
   const double v1 = pos ? m2 : p3, v2 = pos ? m1 : p2, v3 = pos ? c0 : p1, v4 = pos ? p1 : c0, v5 = pos ? p2 : m1;
   Weno w;
-  w.d1 = v2 - v1;
   w.d2 = v3 - v2;
   w.d3 = v4 - v3;
-  w.d4 = v5 - v4;
-  w.s1 = w.d2 - w.d1;
+  w.s1 = w.d2 - (v2 - v1);
   w.s2 = w.d3 - w.d2;
-  w.s3 = w.d4 - w.d3;
+  w.s3 = (v5 - v4) - w.d3;
   return fma(weno_ratio(w, fma(w.s1, w.s1, WENO_E), fma(w.s2, w.s2, WENO_E), fma(w.s3, w.s3, WENO_E)), 1.0 / 6.0,
              v3);
 }

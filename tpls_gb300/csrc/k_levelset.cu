@@ -503,52 +503,45 @@ struct CsfK {
   double rdx, rdy, rdz, a, sw, scap, max_kappa;  // a = 1/(2 sw)
 };
 
-template <typename T>
-__device__ __forceinline__ F3 csf_point(const Geo &g, const CsfK &ph, const double *__restrict__ fi0, int i, int j,
+__device__ __forceinline__ F3 csf_point(const Geo &g, const CsfK &ph, const double *__restrict__ fi, int i, int j,
                                         int k) {
   const int c = TPLS_IDX(g, i, j, k);
-  struct Ld {
-    const double *p;
-    __device__ T operator[](int q) const { return (T)p[q]; }
-  } fi{fi0};
-  const double p64 = fi0[c];
+  const double p = fi[c];
   F3 r = {0.0, 0.0, 0.0};
-  // band decision on the FP64 value in both forms, by order keys of the bit
-  // patterns (exact; no FP64 compare)
-  const long long kp = dkey(p64);
+  // band decision by order keys of the bit patterns (exact; no FP64 compare)
+  const long long kp = dkey(p);
   if (kp < dkey(-ph.sw) || kp > dkey(ph.sw)) return r;
-  const T p = (T)p64;
   const int sy = g.sy, sz = g.sz;
-  const T rdx = (T)ph.rdx, rdy = (T)ph.rdy, rdz = (T)ph.rdz;
-  const T r2dx = (T)0.5 * rdx, r2dy = (T)0.5 * rdy, r2dz = (T)0.5 * rdz, two = (T)2;
-  const T d2x = (fi[c + 1] - two * p + fi[c - 1]) * (rdx * rdx);
-  const T d2y = (fi[c + sy] - two * p + fi[c - sy]) * (rdy * rdy);
-  const T d2z = (fi[c + sz] - two * p + fi[c - sz]) * (rdz * rdz);
-  const T gx = (fi[c + 1] - fi[c - 1]) * r2dx;
-  const T gy = (fi[c + sy] - fi[c - sy]) * r2dy;
-  const T gz = (fi[c + sz] - fi[c - sz]) * r2dz;
-  const T d2xz = ((fi[c + 1 + sz] - fi[c - 1 + sz]) - (fi[c + 1 - sz] - fi[c - 1 - sz])) * (r2dx * r2dz);
-  const T d2yz = ((fi[c + sy + sz] - fi[c - sy + sz]) - (fi[c + sy - sz] - fi[c - sy - sz])) * (r2dy * r2dz);
-  const T d2xy = ((fi[c + 1 + sy] - fi[c - 1 + sy]) - (fi[c + 1 - sy] - fi[c - 1 - sy])) * (r2dx * r2dy);
-  const T nrm = gx * gx + gy * gy + gz * gz;
-  T kap;
-  if (nrm < (T)1e-10) {
-    kap = (T)0;
+  const double rdx = ph.rdx, rdy = ph.rdy, rdz = ph.rdz;
+  const double r2dx = 0.5 * rdx, r2dy = 0.5 * rdy, r2dz = 0.5 * rdz, two = 2.0;
+  const double d2x = (fi[c + 1] - two * p + fi[c - 1]) * (rdx * rdx);
+  const double d2y = (fi[c + sy] - two * p + fi[c - sy]) * (rdy * rdy);
+  const double d2z = (fi[c + sz] - two * p + fi[c - sz]) * (rdz * rdz);
+  const double gx = (fi[c + 1] - fi[c - 1]) * r2dx;
+  const double gy = (fi[c + sy] - fi[c - sy]) * r2dy;
+  const double gz = (fi[c + sz] - fi[c - sz]) * r2dz;
+  const double d2xz = ((fi[c + 1 + sz] - fi[c - 1 + sz]) - (fi[c + 1 - sz] - fi[c - 1 - sz])) * (r2dx * r2dz);
+  const double d2yz = ((fi[c + sy + sz] - fi[c - sy + sz]) - (fi[c + sy - sz] - fi[c - sy - sz])) * (r2dy * r2dz);
+  const double d2xy = ((fi[c + 1 + sy] - fi[c - 1 + sy]) - (fi[c + 1 - sy] - fi[c - 1 - sy])) * (r2dx * r2dy);
+  const double nrm = gx * gx + gy * gy + gz * gz;
+  double kap;
+  if (nrm < 1e-10) {
+    kap = 0.0;
   } else {
-    const T s = sqrt(nrm);             // nrm**0.5
-    const T inv15 = (T)1 / (nrm * s);  // nrm**(-1.5)
-    const T term1 = (d2x + d2y + d2z) / s;
-    const T term2 = (gx * gx * d2x + gy * gy * d2y + gz * gz * d2z) * inv15;
-    const T term3 = two * (gx * gy * d2xy + gx * gz * d2xz + gy * gz * d2yz) * inv15;
+    const double s = sqrt(nrm);            // nrm**0.5
+    const double inv15 = 1.0 / (nrm * s);  // nrm**(-1.5)
+    const double term1 = (d2x + d2y + d2z) / s;
+    const double term2 = (gx * gx * d2x + gy * gy * d2y + gz * gz * d2z) * inv15;
+    const double term3 = two * (gx * gy * d2xy + gx * gz * d2xz + gy * gz * d2yz) * inv15;
     kap = -(term1 - term2 - term3);
   }
-  if (kap > (T)ph.max_kappa) kap = (T)ph.max_kappa;
-  const T a = (T)ph.a;
-  const T dirac = a + a * cos((T)TPLS_PI_SP * p / (T)ph.sw);
-  const T m = dirac * (T)ph.scap * kap;
-  r.x = (double)(m * gx);
-  r.y = (double)(m * gy);
-  r.z = (double)(m * gz);
+  if (kap > ph.max_kappa) kap = ph.max_kappa;
+  const double a = ph.a;
+  const double dirac = a + a * cos(TPLS_PI_SP * p / ph.sw);
+  const double m = dirac * ph.scap * kap;
+  r.x = m * gx;
+  r.y = m * gy;
+  r.z = m * gz;
   return r;
 }
 
@@ -558,12 +551,11 @@ __device__ __forceinline__ F3 lin2(F3 a, F3 b) {  // 2a - b
 }
 
 // value on the i = 1..nx columns including the extrapolated z ghost planes
-template <typename T>
 __device__ __forceinline__ F3 csf_colval(const Geo &g, const CsfK &ph, const double *fi, int i, int j, int k) {
-  if (k == 0) return lin2(csf_point<T>(g, ph, fi, i, j, 1), csf_point<T>(g, ph, fi, i, j, 2));
+  if (k == 0) return lin2(csf_point(g, ph, fi, i, j, 1), csf_point(g, ph, fi, i, j, 2));
   if (k == g.nz + 1)
-    return lin2(csf_point<T>(g, ph, fi, i, j, g.nz), csf_point<T>(g, ph, fi, i, j, g.nz - 1));
-  return csf_point<T>(g, ph, fi, i, j, k);
+    return lin2(csf_point(g, ph, fi, i, j, g.nz), csf_point(g, ph, fi, i, j, g.nz - 1));
+  return csf_point(g, ph, fi, i, j, k);
 }
 
 __device__ __forceinline__ F3 lane_of(const F3 &a, int l) {
@@ -571,22 +563,23 @@ __device__ __forceinline__ F3 lane_of(const F3 &a, int l) {
   return r;
 }
 
-// T: arithmetic of the curvature (double, or float in the FP32-mixed form);
-// TO: storage of the force components.
+// FP64 in both forms: the curvature's second differences of phi (~dx^2 |phi''|)
+// would lose ~1e-3 of their value to FP32 cancellation, a coherent error in the
+// surface-tension force at the interface.
 // Blocks per SM (B): on large grids most warps only write zeros and six blocks
 // hide the few that evaluate the band (256x128x192: 86 us, 108 with the 3 that
 // its registers allow; 512x256x256: 385, 504); on small ones the band's own
 // chain is what a launch waits for, and the registers matter more (192x96x112: 45
 // us, 59 with six).
-template <typename T, typename TO, int B>
+template <int B>
 __global__ void __launch_bounds__(LS_BX *LS_BY, B)
-    k_csf(Geo g, CsfK ph, const double *__restrict__ fi,
-                      TO *__restrict__ fx, TO *__restrict__ fy, TO *__restrict__ fz) {
+    k_csf(Geo g, CsfK ph, const double *__restrict__ fi, double *__restrict__ fx, double *__restrict__ fy,
+          double *__restrict__ fz) {
   const int i = blockIdx.x * LS_BX + threadIdx.x + 1, j = blockIdx.y * LS_BY + threadIdx.y + 1;
   const int k = blockIdx.z;
   if (j > g.ny) return;  // uniform per warp (one row)
   F3 v = {0.0, 0.0, 0.0};
-  if (i <= g.nx) v = csf_colval<T>(g, ph, fi, i, j, k);
+  if (i <= g.nx) v = csf_colval(g, ph, fi, i, j, k);
   // the inlet and outlet columns extrapolate from the last two columns: the
   // inner one from the next lane, or by itself where that is in another warp
   F3 in = {0.0, 0.0, 0.0};
@@ -597,15 +590,15 @@ __global__ void __launch_bounds__(LS_BX *LS_BY, B)
       const F3 p = lane_of(v, last - 1);
       if (i == g.nx) in = p;
     } else if (i == g.nx) {
-      in = csf_colval<T>(g, ph, fi, i - 1, j, k);
+      in = csf_colval(g, ph, fi, i - 1, j, k);
     }
   }
   if (i > g.nx) return;
   const int c = TPLS_IDX(g, i, j, k);
   auto write = [&](int q, const F3 &x) {
-    fx[q] = (TO)x.x;
-    fy[q] = (TO)x.y;
-    fz[q] = (TO)x.z;
+    fx[q] = x.x;
+    fy[q] = x.y;
+    fz[q] = x.z;
   };
   rows_of(g, j, c, [&](int q) { write(q, v); });
   if (i == 1 || i == g.nx) {
@@ -618,24 +611,13 @@ static CsfK csf_constants(const Phys &ph) {
   return {1.0 / ph.dx, 1.0 / ph.dy, 1.0 / ph.dz, 1.0 / (2.0 * ph.sw), ph.sw, ph.scap,
           1.0 / fmin(fmin(ph.dx, ph.dy), ph.dz)};
 }
-template <typename T, typename TO>
-static cudaError_t csf(const Geo &g, const Phys &ph, const double *phi3, TO *fx, TO *fy, TO *fz, cudaStream_t st) {
-  const dim3 grd = owned_grid(g, g.nz + 2), blk(LS_BX, LS_BY);
-  const CsfK q = csf_constants(ph);
-  if ((size_t)g.nx * g.ny * g.nz > 4000000) k_csf<T, TO, 6><<<grd, blk, 0, st>>>(g, q, phi3, fx, fy, fz);
-  else k_csf<T, TO, 1><<<grd, blk, 0, st>>>(g, q, phi3, fx, fy, fz);
-  return cudaGetLastError();
-}
 cudaError_t launch_csf(const Geo &g, const Phys &ph, const double *phi3,
                        double *fx, double *fy, double *fz, cudaStream_t st) {
-  return csf<double>(g, ph, phi3, fx, fy, fz, st);
-}
-cudaError_t launch_csf(const Geo &g, const Phys &ph, const double *phi3, float *fx, float *fy, float *fz,
-                       cudaStream_t st) {
-  // curvature stays FP64: its second differences of phi (~dx^2 |phi''|)
-  // would lose ~1e-3 of their value to FP32 cancellation, a coherent error
-  // in the surface-tension force at the interface; the force is stored FP32
-  return csf<double>(g, ph, phi3, fx, fy, fz, st);
+  const dim3 grd = owned_grid(g, g.nz + 2), blk(LS_BX, LS_BY);
+  const CsfK q = csf_constants(ph);
+  if ((size_t)g.nx * g.ny * g.nz > 4000000) k_csf<6><<<grd, blk, 0, st>>>(g, q, phi3, fx, fy, fz);
+  else k_csf<1><<<grd, blk, 0, st>>>(g, q, phi3, fx, fy, fz);
+  return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------

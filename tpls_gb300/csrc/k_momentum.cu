@@ -558,7 +558,7 @@ __device__ __forceinline__ F2 ld2(const double *__restrict__ p) { return split_b
 
 // float constants of one step (computed on the host in FP64, then rounded)
 struct MomF {
-  float rdx, rdy, rdz, dt, ax2, ay2, az2;
+  float rdx, rdy, rdz, ax2, ay2, az2;
   double dt64;
 };
 
@@ -716,7 +716,6 @@ cudaError_t launch_mom_rhs_pair(const Geo &g, const Phys &ph, const double *u2, 
   m.rdx = (float)(1.0 / ph.dx);
   m.rdy = (float)(1.0 / ph.dy);
   m.rdz = (float)(1.0 / ph.dz);
-  m.dt = (float)ph.dt;
   m.dt64 = ph.dt;
   m.ax2 = (float)hm.ax2;
   m.ay2 = (float)hm.ay2;

@@ -703,8 +703,6 @@ cudaError_t launch_odd_multi(int comp, const SweepMember *mem, const int *prefix
   return cudaGetLastError();
 }
 
-cudaError_t sweep_init() { return cudaSuccess; }
-
 // tile: the block shape (threads over i, or i pairs, by threads over j) the
 // autotuner chooses among for the Jacobi and even-SOR kernels: 0 = 32x4 (the
 // default), 1 = 32x8, 2 = 64x4, 3 = 16x8.
@@ -765,17 +763,19 @@ static cudaError_t odd_set(const Geo &g, const Helm &h, const SweepSet<T, CS> &s
                            int fuse, cudaStream_t st, const OddChain *oc) {
   const int gx = ((g.nx + 1) / 2 + 31) / 32, nseg = (g.nz - 1) / SOC_SC + 1;
   const int blocks = nseg * s.n * gx * g.ny;
+  constexpr bool rows = !std::is_same<CS, RefCoef>::value;  // the per-routine entries write no boundary rows
   // One block per segment, chained, for columns of 2 (FP32) or 3 (FP64) and
   // more segments.  With 2, half the blocks wait on the other half: the FP32
   // sweeps gain more from twice the blocks (16 half-sweeps at 192x96x112: 722
   // us, whole columns 764), the FP64 ones, bound by the FP64 pipe, do not
   // (128x64x96: 720, whole columns 646).
   if (oc && nseg >= (sizeof(T) == 4 ? 2 : 3) && oc->cap >= blocks) {
-    if (bc) k_sor_odd_seg<T, CS, true><<<blocks, SOC_W * 32, 0, st>>>(g, h, s, pres, flg, fuse, *oc, gx, 1 << 20);
+    if (rows && bc)
+      k_sor_odd_seg<T, CS, rows><<<blocks, SOC_W * 32, 0, st>>>(g, h, s, pres, flg, fuse, *oc, gx, 1 << 20);
     else k_sor_odd_seg<T, CS, false><<<blocks, SOC_W * 32, 0, st>>>(g, h, s, pres, flg, fuse, *oc, gx, 1 << 20);
   } else {  // one block per 32 columns of a row, the column in super-chunks
     const dim3 grd(gx * s.n, g.ny);
-    if (bc) k_sor_odd_c4<T, CS, true><<<grd, SOC_W * 32, 0, st>>>(g, h, s, pres, gx, flg, fuse);
+    if (rows && bc) k_sor_odd_c4<T, CS, rows><<<grd, SOC_W * 32, 0, st>>>(g, h, s, pres, gx, flg, fuse);
     else k_sor_odd_c4<T, CS, false><<<grd, SOC_W * 32, 0, st>>>(g, h, s, pres, gx, flg, fuse);
   }
   return cudaGetLastError();

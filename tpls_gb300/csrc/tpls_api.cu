@@ -184,7 +184,7 @@ struct PhaseScope {
   ~PhaseScope();
 };
 
-// The odd half-sweep state for launch_sor_c: null walks each column in one
+// The odd half-sweep state for launch_sor_set: null walks each column in one
 // block (TPLS_FLAG_ODD_COLUMNS; the same results).
 static const OddChain *odd_chain(const tpls_ctx *c) {
   return (c->odd.cap > 0 && !(c->prm.flags & TPLS_FLAG_ODD_COLUMNS)) ? &c->odd : nullptr;
@@ -477,7 +477,6 @@ static int create_impl(int nx, int ny, int nz, const tpls_params *prm, const dou
   c->g.szm = c->px * (ny + 4);
   TCK(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking));
   TCK(cudaEventCreateWithFlags(&c->front_ev, cudaEventDisableTiming));
-  TCK(sweep_init());
   c->mixed = (prm->precision == TPLS_PREC_FP32_MIXED);
   c->n_p = (size_t)c->px * (ny + 2) * (nz + 2) + 8;
   c->n_uv = (size_t)c->px * (ny + 2) * nz + 8;

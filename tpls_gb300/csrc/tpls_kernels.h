@@ -97,8 +97,6 @@ cudaError_t launch_ls_iter_ff(const Geo &g, const Phys &ph, const double *in64,
                               const signed char *flags, double *out64,
                               float *ohi, float *olo, double *err_part,
                               cudaStream_t st);
-cudaError_t launch_csf(const Geo &g, const Phys &ph, const double *phi3,
-                       float *fx, float *fy, float *fz, cudaStream_t st);
 cudaError_t launch_visc(const Geo &g, const Phys &ph, const double *phi2,
                         float *mu, cudaStream_t st);
 
@@ -233,8 +231,6 @@ cudaError_t launch_sor_set(const Geo &g, const Phys &ph, const SweepSet32 &s, co
 cudaError_t launch_defect_init(const double *X, float *d, size_t n, cudaStream_t st);
 cudaError_t launch_defect_apply(const double *X, const float *d, double *x, size_t n,
                                 cudaStream_t st);
-// One-time kernel attributes of the sweeps (dynamic shared memory).
-cudaError_t sweep_init();
 // get_difference of up to three pairs (k_momentum.cu); part: 3 * DIFF_BLOCKS
 // doubles, ctr: a zeroed counter (left zero), out: the first nout sums.
 constexpr int DIFF_BLOCKS = 608;
