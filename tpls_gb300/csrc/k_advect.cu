@@ -142,8 +142,8 @@ constexpr int ADV_BX = 32, ADV_BY = 8;
 // as the SM with the most blocks: the choice with the least (blocks of that SM)
 // x (faces), a single block per SM counting 1.2 times (its barriers leave the FP64
 // pipe idle).  Against 16 halved until the grid has three blocks per SM: 53 ->
-// 45 us at 64x32x48, 33 -> 20 at 37x19x23, 182 -> 165 at 100x50x75, 252 -> 240 at
-// 128x64x96, 1786 -> 1700 at 256x128x192.
+// 45 us at 64x32x48, 33 -> 20 at 37x19x23, 182 -> 170 at 100x50x75, 252 -> 233 at
+// 128x64x96, 1786 -> 1686 at 256x128x192.
 constexpr int ADV_KC = 16;
 
 // One block covers 32 x 8 columns and a chunk of kc levels.  At each

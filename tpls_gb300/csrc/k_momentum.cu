@@ -668,7 +668,9 @@ __device__ __forceinline__ CDT<float> conv_diff_pair(int comp, const Geo &g, con
 // The three components in one launch (gx blocks along x each).  Neither the
 // FP64 pipe (11 operations per point) nor the issue slots (700 instructions)
 // are full: it waits for loads and FP64 results, so many blocks per SM pay more
-// than registers do (BOUNDS_FIGURES; a launch per component, 9 blocks: 4050).
+// than registers do.  Blocks (registers, spilled bytes) and us at 512x256x256 and
+// 192x96x112: 8 (60, 0) 3997, 256; 10 (48, 20) 3434, 221; 12 (40, 164) 3175, 205; 14 and 16
+// (32, 248) 2767, 182.  (A launch per component, 9 blocks: 4050 at 512x256x256.)
 // (The component stays a run-time value: as a template argument it changes
 // which products the compiler contracts, by last bits that the FP32 sweeps
 // amplify to their own accuracy.)

@@ -81,9 +81,10 @@ __device__ __forceinline__ Rec<float> get_rec(int comp, const Geo &g, const MuCo
 // The per-routine entries (sor_iteration_allflux.f90 on host arrays): A and B
 // of point (i, j, k) of the odd half-sweep from the FP64 viscosity (ref_point),
 // x the field, zp its value above (unused at the wall levels of u and v).
-// near and lo in, near1 and hi out, as ref_point.  (111 us per half-sweep of a
-// component at 192x96x144; with the coefficients normalised one by one by a
-// division 163.)
+// near and lo in, near1 and hi out, as ref_point.  (112 us per half-sweep of a
+// component at 192x96x144, where the segment kernel's bound of 5 blocks, chosen
+// for the record form, spills 424 bytes of a thread's 48 registers; with the
+// coefficients normalised one by one by a division 163.)
 template <int CC>
 __device__ __forceinline__ void ref_odd(const Geo &g, const RefCoef &s, const double *__restrict__ x,
                                         const double *m, int c, int k, int k0, double xc, double zp, double near,
